@@ -227,8 +227,8 @@ int omdg_tile_counts(omdg_ctx* ctx, int* tiles, int* staged);
  * height; its kernels run one thread per centre), "tb_block" (kept for
  * callers that set it; the three-body kernels run 128-thread blocks),
  * "nbr_hshift" (log2 of the neighbour slice height),
- * "build_lanes" (list build: 0 cell CTAs, else threads per atom), "io_blocks"
- * (blocks of omdg_step_io's downloads beside the step's kernels), "nbr_capacity"
+ * "build_lanes" (list build: 1 or 8 threads per atom; 0 and 4: by the number
+ * of atoms), "io_blocks" (blocks of omdg_step_io's downloads beside the step's kernels), "nbr_capacity"
  * (row capacity of the next first list build; 0 sizes it from the density;
  * rows grow by themselves when a build needs more), "tb_persistent" (the
  * Tersoff register pass as one resident grid), "fuse_kick" (the step's second

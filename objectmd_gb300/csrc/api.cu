@@ -182,9 +182,9 @@ static void free_atoms(Context* c) {
     void* ptrs[] = {c->x,    c->y,     c->z,      c->vx,     c->vy,          c->vz,          c->fx,
                     c->fy,   c->fz,    c->pe,     c->vir,    c->pack,        c->xref,        c->loc,         c->type,
                     c->id,   c->inv,   c->fp,     c->femb,   c->cell,        c->perm,        c->stage_d,
-                    c->stage_i, c->cell_sorted, c->f64, c->extra, c->stage_extra, c->nnb, c->d_red, c->aflag,
+                    c->stage_i, c->f64, c->extra, c->stage_extra, c->nnb, c->d_red, c->aflag,
                     c->snap_d, c->snap_i,
-                    c->ters_wide, c->nbmask};
+                    c->ters_wide, c->nbmask, c->cell_sorted};
     for (void* p : ptrs) cudaFree(p);
     c->x = c->y = c->z = c->vx = c->vy = c->vz = nullptr;
     c->fx = c->fy = c->fz = c->pe = c->vir = nullptr;
@@ -192,13 +192,12 @@ static void free_atoms(Context* c) {
     c->xref = nullptr;
     c->loc = nullptr;
     c->nbmask = nullptr;
-    c->nbmask_valid = false;
+    c->cell_sorted = nullptr;
     c->type = c->id = c->inv = c->ters_wide = nullptr;
     c->fp = c->femb = nullptr;
     c->cell = c->perm = nullptr;
     c->stage_d = nullptr;
     c->stage_i = nullptr;
-    c->cell_sorted = nullptr;
     c->f64 = nullptr;
     c->snap_d = nullptr;
     c->snap_i = nullptr;
@@ -215,10 +214,10 @@ static int alloc_atoms(Context* c, int n) {
     bool ok = dalloc(c->x, cap) && dalloc(c->y, cap) && dalloc(c->z, cap) && dalloc(c->vx, cap) &&
               dalloc(c->vy, cap) && dalloc(c->vz, cap) && dalloc(c->fx, cap) && dalloc(c->fy, cap) &&
               dalloc(c->fz, cap) && dalloc(c->pe, cap) && dalloc(c->vir, cap) && dalloc(c->pack, cap) &&
-              dalloc(c->xref, cap) && dalloc(c->loc, cap) && dalloc(c->nbmask, cap) && dalloc(c->type, cap) && dalloc(c->id, cap) && dalloc(c->inv, cap) &&
+              dalloc(c->xref, cap) && dalloc(c->loc, (size_t)cap + LOC_PAD) && dalloc(c->nbmask, cap) && dalloc(c->cell_sorted, cap) && dalloc(c->type, cap) && dalloc(c->id, cap) && dalloc(c->inv, cap) &&
               dalloc(c->fp, cap) && dalloc(c->femb, cap) && dalloc(c->cell, cap) && dalloc(c->perm, cap) &&
               dalloc(c->stage_d, (size_t)6 * cap) && dalloc(c->stage_i, (size_t)3 * cap) && dalloc(c->aflag, cap) &&
-              dalloc(c->cell_sorted, cap) && dalloc(c->nnb, cap) && dalloc(c->ters_wide, (size_t)cap + 1);
+              dalloc(c->nnb, cap) && dalloc(c->ters_wide, (size_t)cap + 1);
     // block partials: the kick's blocks, or a force kernel's with the kick in its epilogue (>= 8 atoms a block)
     int nb = grid_for(cap, 8) + 1;
     ok = ok && dalloc(c->d_red, (size_t)4 * nb);
@@ -1909,27 +1908,6 @@ static int time_forces(Context* c, int reps, double& best) {
     if (!rc) rc = check_status(c);
     return rc;
 }
-// Best of `reps` list builds (binning, permutation, list) in milliseconds.
-static int time_build(Context* c, int reps, double& best) {
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    best = 1e30;
-    int rc = nlist_build(c);  // warm
-    for (int r = 0; r < reps && !rc; r++) {
-        cudaEventRecord(a, c->stream);
-        rc = nlist_build(c);
-        cudaEventRecord(b, c->stream);
-        cudaEventSynchronize(b);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, a, b);
-        if (ms < best) best = ms;
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    if (!rc) rc = check_status(c);
-    return rc;
-}
 }  // namespace omdg
 
 extern "C" {
@@ -2011,25 +1989,8 @@ int omdg_autotune(omdg_ctx* c, int reps, double* best_ms) {
             for (int stage : {0, 1}) cands.push_back(Cand{lanes, 128, stage, tile_on});
     }
     int rc = OMDG_OK;
-    // list build: cell-CTA, 8 or 4 lanes per atom, or one thread per atom
-    // (cells holding few atoms leave most of a cell CTA idle)
     if (!c->list_valid && (rc = build_list(c))) return rc;
-    {
-        int best_bl = c->build_lanes;
-        double tbest = 1e30;
-        for (int bl : {0, 8, 4, 1}) {
-            c->build_lanes = bl;
-            double t;
-            if ((rc = time_build(c, reps, t))) return rc;
-            if (t < tbest) {
-                tbest = t;
-                best_bl = bl;
-            }
-        }
-        c->build_lanes = best_bl;
-        if ((rc = build_list(c))) return rc;
-        if ((rc = threebody_prepare(c))) return rc;
-    }
+    if ((rc = threebody_prepare(c))) return rc;
     if (cands.empty()) {
         invalidate_graph(c);
         if (best_ms) return time_forces(c, reps, *best_ms);

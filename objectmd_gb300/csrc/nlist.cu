@@ -373,18 +373,13 @@ __global__ void k_rep_build_done(int nrep, int full, int* __restrict__ rflag, in
 }
 
 
-// Cell of each sorted atom (cell[] is indexed by the previous order).
-
 // Replica mode: every replica has its own periodic lengths and cell grid,
 // and its cells occupy the global cell range [cell_base, cell_base + cells).
-// base and hf are the replica's cell reference points in the pack frame
-// (LocFrame below).
 struct RepGeom {
     double lo[3], L[3], cell_org[3], cell_h[3], inv_h[3];
     int nc[3], periodic[3];
     int cell_base;
     ShiftF S;
-    float base[3], hf[3];
 };
 
 // The pack coordinate is X = x + Q with Q = P - org, formed as FP32 hi + lo
@@ -393,65 +388,42 @@ struct PackFrame {
     float Qh[3], Ql[3];
 };
 
-// The list screen works in a cell-local frame: each cell has an FP32
-// reference point R(c) = fma(c, h, base) per axis (base = the pack-frame
-// corner of cell 0), and an atom's local coordinate u = (X_hi - R) + X_lo is
-// exact up to its final FP32 rounding (X_hi - R is Sterbenz-exact).  The
-// build recomputes R(c) with the same expression.
-struct LocFrame {
-    int nc[3];
-    float base[3], h[3];
-};
-
-__device__ __forceinline__ float cell_ref(int c, float h, float base) { return fmaf((float)c, h, base); }
-
+// loc: the position rounded to FP32, which the list build screens (w: the type)
 __global__ void k_pack(int n, const double* __restrict__ x, const double* __restrict__ y,
                        const double* __restrict__ z, const int* __restrict__ type, PackFrame f,
-                       PosPack* __restrict__ pack, float4* __restrict__ xref, const int* __restrict__ cell,
-                       LocFrame lf, const int* __restrict__ rep_of, const RepGeom* __restrict__ rg,
+                       PosPack* __restrict__ pack, float4* __restrict__ xref, const int* __restrict__ rep_of,
                        const unsigned* __restrict__ aflag, float4* __restrict__ loc, unsigned* umax,
                        const int* __restrict__ rflag) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float m = 0.f;
     if (i < n && (!rflag || rflag[rep_of[i]])) {
         PosPack p;
-        pack_coord(x[i], f.Qh[0], f.Ql[0], p.hi.x, p.lo.x);
-        pack_coord(y[i], f.Qh[1], f.Ql[1], p.hi.y, p.lo.y);
-        pack_coord(z[i], f.Qh[2], f.Ql[2], p.hi.z, p.lo.z);
+        const double X = x[i], Y = y[i], Z = z[i];
+        pack_coord(X, f.Qh[0], f.Ql[0], p.hi.x, p.lo.x);
+        pack_coord(Y, f.Qh[1], f.Ql[1], p.hi.y, p.lo.y);
+        pack_coord(Z, f.Qh[2], f.Ql[2], p.hi.z, p.lo.z);
         p.hi.w = __int_as_float(type[i]);
         p.lo.w = 0.f;
         pack[i] = p;
         if (xref) xref[i] = make_float4(p.hi.x, p.hi.y, p.hi.z, 0.f);
         if (loc) {
-            int c = cell[i];
-            if (rep_of) {  // the replica's own grid and reference points
-                const RepGeom& g = rg[rep_of[i]];
-                c -= g.cell_base;
-                for (int d = 0; d < 3; d++) {
-                    lf.nc[d] = g.nc[d];
-                    lf.h[d] = g.hf[d];
-                    lf.base[d] = g.base[d];
-                }
-            }
-            const int cx = c % lf.nc[0], cy = (c / lf.nc[0]) % lf.nc[1], cz = c / (lf.nc[0] * lf.nc[1]);
-            const float ux = __fadd_rn(__fsub_rn(p.hi.x, cell_ref(cx, lf.h[0], lf.base[0])), p.lo.x);
-            const float uy = __fadd_rn(__fsub_rn(p.hi.y, cell_ref(cy, lf.h[1], lf.base[1])), p.lo.y);
-            const float uz = __fadd_rn(__fsub_rn(p.hi.z, cell_ref(cz, lf.h[2], lf.base[2])), p.lo.z);
             if (aflag && !(aflag[i] & 1u)) {
                 // inactive (SetActive false): far from every centre, so no
-                // list takes it, and outside the band's max |u|
+                // list takes it, and outside the band's max |x|
                 loc[i] = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f);
             } else {
-                loc[i] = make_float4(ux, uy, uz, __int_as_float(type[i]));  // w: the type, for the row's type mask
+                const float ux = f2_from(X).hi, uy = f2_from(Y).hi, uz = f2_from(Z).hi;
+                loc[i] = make_float4(ux, uy, uz, p.hi.w);
                 m = fmaxf(fabsf(ux), fmaxf(fabsf(uy), fabsf(uz)));
                 if (!(m <= 3.0e38f)) m = 3.0e38f;  // non-finite: flagged by the cell assignment
             }
         }
     }
     if (loc) {
-        // the largest |u| sets the width of the screening band
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(umax, __float_as_uint(m));
+        // the largest |x| sets the width of the screening band
+        m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+        if ((threadIdx.x & 31) == 0 && m > 0.f && __float_as_uint(m) > *(volatile unsigned*)umax)
+            atomicMax(umax, __float_as_uint(m));
     }
 }
 
@@ -472,15 +444,14 @@ struct TileOut {
 struct BuildParams {
     TileOut to;
     int n, maxnb, hshift;
+    int cap;              // LANES = 1: row entries a thread keeps in shared memory
     int nc[3];
     int periodic[3];
     ShiftF L;
     double L64[3];
     double rsq;           // Rv*Rv in FP64 (VerletList.cpp:161)
-    float rsq_lo, rsq_hi; // FP32 screening band around rsq
     float rv;             // Rv rounded to FP32
-    float base[3], h[3];  // cell reference points (LocFrame)
-    float hmax;           // largest cell size over all grids (screening band)
+    float lmax;           // largest periodic length (screening band)
 };
 
 // Per axis, how many (cell, image) candidates a cell has and the idx-th one,
@@ -514,11 +485,35 @@ __device__ __forceinline__ bool axis_cell(int c, int nc, int periodic, int idx, 
     return k >= 0 && k < nc;
 }
 
-// The reference's FP64 test (dx = x_i - (x_j + s), r2 = (dx*dx + dy*dy) +
-// dz*dz <= Rv^2) for the rare pairs inside the FP32 screening band.
+// The candidates along x of the cells a..b as runs of consecutive cells under
+// one image (the atoms of consecutive cells lie back to back): the cells
+// a-1..b+1, cut where a periodic axis wraps; a periodic axis of fewer than 3
+// cells gives one run per (cell, image).
+__device__ __forceinline__ int axis_runs(int a, int b, int nc, int periodic) {
+    if (!periodic) return 1;
+    if (nc < 3) return 3 * nc;
+    return 1 + (a == 0) + (b == nc - 1);
+}
+
+__device__ __forceinline__ void axis_run(int a, int b, int nc, int periodic, int idx, int& c0, int& c1, int& shift) {
+    if (periodic && nc < 3) {
+        c0 = c1 = idx / 3;
+        shift = idx % 3 - 1;
+        return;
+    }
+    if (periodic && a == 0) idx--;  // run -1: the last cell's image below
+    shift = idx < 0 ? -1 : idx;
+    c0 = idx < 0 ? nc - 1 : (idx == 0 ? max(a - 1, 0) : 0);
+    c1 = idx < 0 ? nc - 1 : (idx == 0 ? min(b + 1, nc - 1) : 0);
+}
+
+// A pair inside the FP32 screening band, or closer than it can tell from an
+// overlap: the reference's FP64 test (dx = x_i - (x_j + s), r2 = (dx*dx +
+// dy*dy) + dz*dz <= Rv^2) and its overlap check (gadget.cpp:149).  Rare, out
+// of line.
 __device__ __noinline__ bool exact_within(double Lx, double Ly, double Lz, double rsq, const double* __restrict__ x,
                                           const double* __restrict__ y, const double* __restrict__ z, int i, int k,
-                                          unsigned code) {
+                                          unsigned code, unsigned* status) {
     const int sx = nbr_sx(code), sy = nbr_sy(code), sz = nbr_sz(code);
     double gx = sx == 0 ? 0.0 : (sx > 0 ? Lx : -Lx);
     double gy = sy == 0 ? 0.0 : (sy > 0 ? Ly : -Ly);
@@ -527,132 +522,228 @@ __device__ __noinline__ bool exact_within(double Lx, double Ly, double Lz, doubl
     double dy = __dsub_rn(y[i], __dadd_rn(y[k], gy));
     double dz = __dsub_rn(z[i], __dadd_rn(z[k], gz));
     double rr = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-    return rr <= rsq && !(k == i && code == nbr_encode(0, 0, 0, 0));
+    if (!(rr <= rsq)) return false;
+    if (rr < OMD_PROXIMITY) report_overlap(status, i, k);
+    return true;
 }
 
-// One thread per centre atom, screening in the cell-local frame: a
-// candidate costs one 16-byte load of its local coordinate, the difference
-// against the centre shifted by the (cell, image) offset R(c_i) - R(c_k) - sL
-// (computed once per cell), and the squared length.  Every FP32 step is
-// bounded by a few ulps of max(|u|, h); pairs within that band of Rv take
-// the reference's FP64 test, so the list is the reference's exactly.  Rows
-// come out in the traversal order of the other build variants.
+// The list build.  The candidates of the 27 cells are 9 runs of back-to-back
+// atoms (axis_run); a candidate costs one 16-byte load of its FP32 position,
+// four of them in flight, and the squared length of the difference.  Every
+// FP32 step errs by at most an ulp of max|x| + L, so pairs within a band of
+// Rv (a few 1e-4 A for boxes of a few hundred A: one atom in thirty has such
+// a pair), and pairs close enough to be an overlap, take the reference's FP64
+// test, out of line: the list is the reference's exactly, in the traversal
+// order of the cells.
 //
-// Grid accessors: the single box reads the kernel parameters, a replica its
-// RepGeom entry (both inline to plain loads).
-struct BoxGrid {
-    const BuildParams& p;
-    __device__ int nc(int d) const { return p.nc[d]; }
-    __device__ int periodic(int d) const { return p.periodic[d]; }
-    __device__ float base(int d) const { return p.base[d]; }
-    __device__ float h(int d) const { return p.h[d]; }
-    __device__ double L64(int d) const { return p.L64[d]; }
-    __device__ const ShiftF& L() const { return p.L; }
-    __device__ int cell_base() const { return 0; }
-};
+// Accepted entries wait in a shared-memory column per thread: some lane of
+// the warp accepts nearly every candidate, so the append has to be a
+// predicated store and an add, not a branch around address arithmetic.
+//
+// LANES = 1: one thread per centre walks every run; its column holds the
+// whole row (longer ones go out in pieces) and goes out as whole 32-byte
+// sectors of the sliced layout.  Bound by instruction issue and the latency
+// of the loads (370 warp instructions per EAM atom at 53 % issue; six loads
+// in flight: with four 165 us, with eight 170).  256,000 EAM atoms, 13 a
+// cell: 154 us, against 498 us for one CTA per cell on hi/lo packs and 200
+// for one thread per centre with a loop per cell; 512,000 Tersoff atoms, 1.6
+// a cell: 90 us against 113.  One warp per cell, its lanes over the
+// candidates and eight centres in registers, took 239 us on EAM: appending
+// by ballot or by bit mask costs more instructions than the loads it saves.
+//
+// LANES = 8, for boxes too small to fill the chip with a thread per centre:
+// eight lanes take a run each, and after each round of eight runs the lanes'
+// counts are scanned to place their entries.
+constexpr int BUILD_THREADS = 128;
+constexpr int BUILD_AHEAD = LOC_PAD;  // candidate loads in flight per thread
+constexpr int BUILD_RUN = 32;      // LANES = 8: a lane's entries of one run in shared memory
 
-struct RepGrid {
-    const RepGeom* r;
-    __device__ int nc(int d) const { return r->nc[d]; }
-    __device__ int periodic(int d) const { return r->periodic[d]; }
-    __device__ float base(int d) const { return r->base[d]; }
-    __device__ float h(int d) const { return r->hf[d]; }
-    __device__ double L64(int d) const { return r->L[d]; }
-    __device__ const ShiftF& L() const { return r->S; }
-    __device__ int cell_base() const { return r->cell_base; }
-};
-
-
-template <bool TILES, class G>
-__device__ __forceinline__ void build_row(const BuildParams& p, const G& g, int i, const float4* __restrict__ loc,
+// One run of candidates for the centre at (px, py, pz): the accepted entries
+// go to the column at w (stride BUILD_THREADS), which out() empties when it
+// is full.
+template <bool ONE, class Out, class Slot>
+__device__ __forceinline__ void build_run(const float4* __restrict__ u, int left, unsigned ent, unsigned self_ent,
+                                          float px, float py, float pz, float rsq_lo, float rsq_hi, float rsq_ov,
                                           const double* __restrict__ x, const double* __restrict__ y,
-                                          const double* __restrict__ z, const int* __restrict__ cell,
-                                          const int* __restrict__ start, const unsigned* __restrict__ umax,
-                                          unsigned* __restrict__ nbr, int* __restrict__ nnb, unsigned* status,
-                                          int* need, unsigned* __restrict__ nbmask) {
-    // band: per component |error| <= 3 ulp(2 max(|u|, h)) (two operand
-    // roundings, the offset, the difference); 2x margin, then sqrt(3) for
-    // the length and 1e-6 relative for the squares
-    const float U = fmaxf(__uint_as_float(*umax), p.hmax);
-    const float dlt = 1.7320509f * (12.f * U * 2.3841858e-7f) + 1e-6f * p.rv;
-    const float rl = fmaxf(p.rv - dlt, 0.f), rh = p.rv + dlt;
-    const float rsq_lo = rl * rl * (1.f - 1e-6f), rsq_hi = rh * rh * (1.f + 1e-6f);
+                                          const double* __restrict__ z, int i, double rsq, double Lx, double Ly,
+                                          double Lz, unsigned* status, unsigned*& w, const unsigned* w_full,
+                                          unsigned& tmask, Out&& out, Slot&& slot) {
+    const unsigned band = __float_as_uint(rsq_hi) - __float_as_uint(rsq_lo);
+#pragma unroll 1
+    for (; left > 0; left -= BUILD_AHEAD, u += BUILD_AHEAD, ent += BUILD_AHEAD) {
+        if (w > w_full) out();
+        float4 uk[BUILD_AHEAD];
+#pragma unroll
+        for (int t = 0; t < BUILD_AHEAD; t++) uk[t] = __ldg(u + t);  // the array is padded
+        float r2[BUILD_AHEAD];
+        bool in[BUILD_AHEAD];
+        bool rare = false;
+#pragma unroll
+        for (int t = 0; t < BUILD_AHEAD; t++) {
+            const float dx = px - uk[t].x, dy = py - uk[t].y, dz = pz - uk[t].z;
+            r2[t] = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+            in[t] = r2[t] <= rsq_hi && t < left;
+            rare |= (__float_as_uint(r2[t]) - __float_as_uint(rsq_lo)) <= band || r2[t] < rsq_ov;
+        }
+        if (rare) {  // one in the band, the centre itself or an overlap
+#pragma unroll
+            for (int t = 0; t < BUILD_AHEAD; t++) {
+                if (ent + t == self_ent) in[t] = false;
+                if (in[t] && (r2[t] >= rsq_lo || r2[t] < rsq_ov))
+                    in[t] = exact_within(Lx, Ly, Lz, rsq, x, y, z, i, (int)(ent & (unsigned)INDEX_MASK) + t, ent,
+                                         status);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < BUILD_AHEAD; t++) {
+            if (!ONE && in[t]) tmask |= 1u << (__float_as_int(uk[t].w) & 31);
+            if (in[t]) {
+                slot((int)(ent & (unsigned)INDEX_MASK) + t);
+                *w = ent + t;
+                w += BUILD_THREADS;
+            }
+        }
+    }
+}
+
+// REP: the centre's replica supplies the grid and lengths.  TILES (LANES = 1):
+// the rows also go out as EAM tile slots.  ONE: a single atom type (no type
+// mask).
+template <int LANES, bool REP, bool TILES, bool ONE>
+__global__ void __launch_bounds__(BUILD_THREADS, 7) k_build(
+    BuildParams p, const RepGeom* __restrict__ rg, const int* __restrict__ rep_of, const float4* __restrict__ loc,
+    const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+    const int* __restrict__ cell, const int* __restrict__ start, const unsigned* __restrict__ umax,
+    unsigned* __restrict__ nbr, int* __restrict__ nnb, unsigned* status, int* need, const int* __restrict__ rflag,
+    unsigned* __restrict__ nbmask) {
+    extern __shared__ unsigned s_row[];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t / LANES, lane = t % LANES;
+    if (i >= p.n) return;  // LANES = 8: whole groups leave together
+    const RepGeom* g = REP ? rg + rep_of[i] : nullptr;
+    if (REP && rflag && !rflag[rep_of[i]]) return;  // the replica keeps its list
     const float4 ui = loc[i];
     if (ui.x == 3.0e38f) {  // inactive centre (k_pack): an empty row
-        nnb[i] = 0;
-        nbmask[i] = 0u;
+        if (lane == 0) {
+            nnb[i] = 0;
+            nbmask[i] = 0u;
+        }
         return;
     }
-    unsigned tmask = 0u;  // types the row holds
-    const int nx = g.nc(0), ny = g.nc(1), nz = g.nc(2);
-    const int ci = cell[i] - g.cell_base();
+    // band: per component the two positions, the image length and two
+    // differences each round by half an ulp of at most U; 2x margin, sqrt(3)
+    // for the length and 1e-6 relative for the squares
+    const float U = __uint_as_float(*umax) + p.lmax;
+    const float dlt = 1.7320509f * (6.f * U * 1.1920929e-7f) + 1e-6f * p.rv;
+    const float rl = fmaxf(p.rv - dlt, 0.f), rh = p.rv + dlt, ro = 1.0e-3f + dlt;
+    const float rsq_lo = rl * rl * (1.f - 1e-6f), rsq_hi = rh * rh * (1.f + 1e-6f), rsq_ov = ro * ro;
+    const int nx = REP ? g->nc[0] : p.nc[0], ny = REP ? g->nc[1] : p.nc[1], nz = REP ? g->nc[2] : p.nc[2];
+    const int perx = REP ? g->periodic[0] : p.periodic[0], pery = REP ? g->periodic[1] : p.periodic[1],
+              perz = REP ? g->periodic[2] : p.periodic[2];
+    const int cbase = REP ? g->cell_base : 0;
+    const ShiftF& L = REP ? g->S : p.L;
+    const double* L64 = REP ? g->L : p.L64;
+    const int ci = cell[i] - cbase;
     const int cx = ci % nx, cy = (ci / nx) % ny, cz = ci / (nx * ny);
+    const int mx = axis_runs(cx, cx, nx, perx), my = axis_count(ny, pery), mz = axis_count(nz, perz);
+    const unsigned self_ent = nbr_encode(i, 0, 0, 0);
+    unsigned tmask = 0u;  // types the row holds
+    unsigned* const out = nbr + nbr_at(i, 0, p.hshift, p.maxnb);
+    unsigned* const col = s_row + threadIdx.x;
+    unsigned* w = col;
+    const unsigned* const w_full = col + ((LANES == 1 ? p.cap : BUILD_RUN) - BUILD_AHEAD) * BUILD_THREADS;
+    int cnt = 0;  // entries of the row already out
     // tile slots (single box only): the centre's tile, where it is staged
     const unsigned short* tsb = nullptr;
     unsigned short* trow = nullptr;
     int tox = 0, toy = 0, toz = 0;
     if (TILES) {
         const int tx = cx / p.to.T[0], ty = cy / p.to.T[1], tz = cz / p.to.T[2];
-        const int t = (tz * p.to.nt[1] + ty) * p.to.nt[0] + tx;
-        if (p.to.nst[t] <= p.to.cap) {
-            tsb = p.to.sb + (size_t)t * p.to.HC;
+        const int tt = (tz * p.to.nt[1] + ty) * p.to.nt[0] + tx;
+        if (p.to.nst[tt] <= p.to.cap) {
+            tsb = p.to.sb + (size_t)tt * p.to.HC;
             trow = p.to.slot + (size_t)i * p.to.stride;
             tox = cx - tx * p.to.T[0];
             toy = cy - ty * p.to.T[1];
             toz = cz - tz * p.to.T[2];
         }
     }
-    const float rx = cell_ref(cx, g.h(0), g.base(0)), ry = cell_ref(cy, g.h(1), g.base(1)),
-                rz = cell_ref(cz, g.h(2), g.base(2));
-    const int mx = axis_count(nx, g.periodic(0));
-    const int my = axis_count(ny, g.periodic(1));
-    const int mz = axis_count(nz, g.periodic(2));
-    const unsigned self_code = nbr_encode(0, 0, 0, 0);
-    int cnt = 0;
-#pragma unroll 1
-    for (int a = 0; a < mz; a++) {
-        int kz, sz;
-        if (!axis_cell(cz, nz, g.periodic(2), a, kz, sz)) continue;
-        const float pz = ui.z + (((rz - cell_ref(kz, g.h(2), g.base(2))) - sel_shift(sz, g.L().hz)) -
-                                 sel_shift(sz, g.L().lz));
-#pragma unroll 1
-        for (int b = 0; b < my; b++) {
-            int ky, sy;
-            if (!axis_cell(cy, ny, g.periodic(1), b, ky, sy)) continue;
-            const float py = ui.y + (((ry - cell_ref(ky, g.h(1), g.base(1))) - sel_shift(sy, g.L().hy)) -
-                                     sel_shift(sy, g.L().ly));
-#pragma unroll 1
-            for (int q = 0; q < mx; q++) {
-                int kx, sx;
-                if (!axis_cell(cx, nx, g.periodic(0), q, kx, sx)) continue;
-                const float px = ui.x + (((rx - cell_ref(kx, g.h(0), g.base(0))) - sel_shift(sx, g.L().hx)) -
-                                         sel_shift(sx, g.L().lx));
-                const int c = g.cell_base() + (kz * ny + ky) * nx + kx;
-                const unsigned code = nbr_encode(0, sx, sy, sz);
-                const int e = start[c + 1];
-                // slot of candidate k in the tile's staged halo: tb + k
-                const int tb =
-                    TILES && trow ? (int)tsb[((toz + a) * p.to.hy + (toy + b)) * p.to.hx + (tox + q)] - start[c] : 0;
-                for (int k = start[c]; k < e; k++) {
-                    const float4 uk = loc[k];
-                    const float dx = px - uk.x, dy = py - uk.y, dz = pz - uk.z;
-                    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                    if (r2 > rsq_hi) continue;
-                    if (k == i && code == self_code) continue;
-                    // borderline pairs: the reference's FP64 arithmetic, out of line
-                    if (!(r2 < rsq_lo) &&
-                        !exact_within(g.L64(0), g.L64(1), g.L64(2), p.rsq, x, y, z, i, k, code))
-                        continue;
-                    if (r2 < 1e-6f) report_overlap(status, i, k);
-                    tmask |= 1u << (__float_as_int(uk.w) & 31);
-                    if (cnt < p.maxnb) {
-                        nbr[nbr_at(i, cnt, p.hshift, p.maxnb)] = code | (unsigned)k;
-                        if (TILES && trow) trow[cnt] = (unsigned short)(tb + k);
-                    }
-                    cnt++;
-                }
-            }
+    const auto flush = [&]() {
+        const int m = (int)(w - col) / BUILD_THREADS;
+        const int put = min(m, p.maxnb - cnt);
+        for (int s = 0; s < put; s++) out[(size_t)(cnt + s) << p.hshift] = col[s * BUILD_THREADS];
+        cnt += m;
+        w = col;
+    };
+    // run (a, b, q): its cells, image and candidates
+    const auto run = [&](int a, int b, int q, auto&& emit) {
+        int kz, sz, ky, sy, c0, c1, sx;
+        if (!axis_cell(cz, nz, perz, a, kz, sz) || !axis_cell(cy, ny, pery, b, ky, sy)) return;
+        axis_run(cx, cx, nx, perx, q, c0, c1, sx);
+        const int row0 = cbase + (kz * ny + ky) * nx;
+        const int k0 = start[row0 + c0], e = start[row0 + c1 + 1];
+        // slot of candidate k in the tile's staged halo: tb + k (halo cells
+        // along x are staged back to back, as the run is)
+        int tb = 0;
+        if (TILES && trow) {
+            const int hx = sx < 0 ? 0 : (sx > 0 ? 2 : c0 - cx + 1);  // the run's first halo cell
+            tb = (int)tsb[((toz + a) * p.to.hy + (toy + b)) * p.to.hx + (tox + hx)] - k0;
         }
+        build_run<ONE>(loc + k0, e - k0, nbr_encode(k0, sx, sy, sz), self_ent, ui.x - sel_shift(sx, L.hx),
+                       ui.y - sel_shift(sy, L.hy), ui.z - sel_shift(sz, L.hz), rsq_lo, rsq_hi, rsq_ov, x, y, z, i,
+                       p.rsq, L64[0], L64[1], L64[2], status, w, w_full, tmask, emit, [&](int k) {
+                           if (TILES && trow) {
+                               const int at = cnt + (int)(w - col) / BUILD_THREADS;
+                               if (at < p.maxnb) trow[at] = (unsigned short)(tb + k);
+                           }
+                       });
+    };
+    if (LANES == 1) {
+#pragma unroll 1
+        for (int a = 0; a < mz; a++)
+#pragma unroll 1
+            for (int b = 0; b < my; b++)
+#pragma unroll 1
+                for (int q = 0; q < mx; q++) run(a, b, q, flush);
+        flush();
+    } else {
+        const unsigned group = 0xffu << (threadIdx.x & 24);
+        const int runs = mx * my * mz;
+#pragma unroll 1
+        for (int r0 = 0; r0 < runs; r0 += LANES) {
+            // a run of more than BUILD_RUN accepted entries is placed by
+            // walking it twice: once to count, once from its place
+            const int r = r0 + lane;
+            const int q = r % mx, b = (r / mx) % my, a = r / (mx * my);
+            int spilled = 0;
+            w = col;
+            if (r < runs)
+                run(a, b, q, [&]() {
+                    spilled += (int)(w - col) / BUILD_THREADS;
+                    w = col;
+                });
+            const int m = (int)(w - col) / BUILD_THREADS;
+            int incl = spilled + m;
+            for (int o = 1; o < LANES; o <<= 1) {
+                const int v = __shfl_up_sync(group, incl, o, LANES);
+                if (lane >= o) incl += v;
+            }
+            const int total = __shfl_sync(group, incl, LANES - 1, LANES);
+            const int row_cnt = cnt;
+            cnt += incl - spilled - m;  // this lane's first place
+            if (spilled) {
+                w = col;
+                run(a, b, q, flush);
+                flush();
+            } else {
+                flush();
+            }
+            cnt = row_cnt + total;
+            w = col;
+        }
+        if (!ONE)
+            for (int o = 1; o < LANES; o <<= 1) tmask |= __shfl_xor_sync(group, tmask, o, LANES);
+        if (lane != 0) return;
     }
     if (cnt > p.maxnb) {
         atomicOr(status, ERR_NBR_OVERFLOW);
@@ -660,28 +751,7 @@ __device__ __forceinline__ void build_row(const BuildParams& p, const G& g, int 
         cnt = p.maxnb;
     }
     nnb[i] = cnt;
-    nbmask[i] = tmask;
-}
-
-// REP: the atom's replica supplies the grid, reference points and lengths.
-// TILES: the rows also go out as EAM tile slots.
-template <bool REP, bool TILES = false>
-__global__ void __launch_bounds__(128, REP ? 7 : 8) k_build(BuildParams p, const RepGeom* __restrict__ rg,
-                                               const int* __restrict__ rep_of, const float4* __restrict__ loc,
-                                               const double* __restrict__ x, const double* __restrict__ y,
-                                               const double* __restrict__ z, const int* __restrict__ cell,
-                                               const int* __restrict__ start, const unsigned* __restrict__ umax,
-                                               unsigned* __restrict__ nbr, int* __restrict__ nnb, unsigned* status,
-                                               int* need, const int* __restrict__ rflag,
-                                               unsigned* __restrict__ nbmask) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
-    if (REP && rflag && !rflag[rep_of[i]]) return;  // the replica keeps its list
-    if (REP)
-        build_row<false>(p, RepGrid{rg + rep_of[i]}, i, loc, x, y, z, cell, start, umax, nbr, nnb, status, need,
-                         nbmask);
-    else
-        build_row<TILES>(p, BoxGrid{p}, i, loc, x, y, z, cell, start, umax, nbr, nnb, status, need, nbmask);
+    nbmask[i] = ONE ? (cnt > 0 ? 1u : 0u) : tmask;
 }
 
 // ------------------------------------------------------------------ EAM cell tiles
@@ -784,212 +854,6 @@ __global__ void k_cell_assign_rep(int n, double* __restrict__ x, double* __restr
     atomicAdd(&count[c], 1);
 }
 
-// Same list as k_build with LANES threads per atom: the lanes test
-// consecutive atoms of a cell together and append the accepted ones in lane
-// order (ballot + prefix popcount), so each row keeps exactly the
-// cell-traversal order of the one-thread build.
-template <int LANES>
-__global__ void __launch_bounds__(256) k_build_lanes(BuildParams p, const PosPack* __restrict__ pack,
-                                                     const double* __restrict__ x, const double* __restrict__ y,
-                                                     const double* __restrict__ z, const int* __restrict__ cell,
-                                                     const int* __restrict__ start, unsigned* __restrict__ nbr,
-                                                     int* __restrict__ nnb, unsigned* status, int* need) {
-    const int lane = threadIdx.x & (LANES - 1);
-    const int gbase = (threadIdx.x & 31) & ~(LANES - 1);
-    const unsigned gmask = (LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u)) << gbase;
-    const int i = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
-    if (i >= p.n) return;  // whole groups leave together
-    const PosPack pi = pack[i];
-    const int ci = cell[i];
-    const int cx = ci % p.nc[0], cy = (ci / p.nc[0]) % p.nc[1], cz = ci / (p.nc[0] * p.nc[1]);
-    const int mx = axis_count(p.nc[0], p.periodic[0]);
-    const int my = axis_count(p.nc[1], p.periodic[1]);
-    const int mz = axis_count(p.nc[2], p.periodic[2]);
-    int cnt = 0;
-    for (int a = 0; a < mz; a++)
-        for (int b = 0; b < my; b++)
-            for (int q = 0; q < mx; q++) {
-                int kz, sz, ky, sy, kx, sx;
-                if (!axis_cell(cz, p.nc[2], p.periodic[2], a, kz, sz) ||
-                    !axis_cell(cy, p.nc[1], p.periodic[1], b, ky, sy) ||
-                    !axis_cell(cx, p.nc[0], p.periodic[0], q, kx, sx))
-                    continue;
-                const int c = (kz * p.nc[1] + ky) * p.nc[0] + kx;
-                const unsigned code = nbr_encode(0, sx, sy, sz);
-                const bool self_image = (sx == 0 && sy == 0 && sz == 0);
-                const int e = start[c + 1];
-                for (int k0 = start[c]; k0 < e; k0 += LANES) {
-                    const int k = k0 + lane;
-                    bool in = false;
-                    if (k < e && !(self_image && k == i)) {
-                        const PosPack pk = pack[k];
-                        const float3 d = pair_delta(pi.hi, pi.lo, pk.hi, pk.lo, code, p.L);
-                        const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
-                        if (r2 <= p.rsq_hi) {
-                            in = r2 < p.rsq_lo;
-                            if (!in) {
-                                // borderline: the reference's FP64 arithmetic decides
-                                double gx = sx == 0 ? 0.0 : (sx > 0 ? p.L64[0] : -p.L64[0]);
-                                double gy = sy == 0 ? 0.0 : (sy > 0 ? p.L64[1] : -p.L64[1]);
-                                double gz = sz == 0 ? 0.0 : (sz > 0 ? p.L64[2] : -p.L64[2]);
-                                double dx = __dsub_rn(x[i], __dadd_rn(x[k], gx));
-                                double dy = __dsub_rn(y[i], __dadd_rn(y[k], gy));
-                                double dz = __dsub_rn(z[i], __dadd_rn(z[k], gz));
-                                double rr = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                                      __dmul_rn(dz, dz));
-                                in = rr <= p.rsq;
-                            }
-                            if (in && r2 < 1e-6f) report_overlap(status, i, k);
-                        }
-                    }
-                    const unsigned bal = __ballot_sync(gmask, in) >> gbase;
-                    if (in) {
-                        const int pos = cnt + __popc(bal & ((1u << lane) - 1u));
-                        if (pos < p.maxnb) nbr[nbr_at(i, pos, p.hshift, p.maxnb)] = code | (unsigned)k;
-                    }
-                    cnt += __popc(bal);
-                }
-            }
-    if (lane == 0) {
-        if (cnt > p.maxnb) {
-            atomicOr(status, ERR_NBR_OVERFLOW);
-            atomicMax(need, cnt);
-            cnt = p.maxnb;
-        }
-        nnb[i] = cnt;
-    }
-}
-
-// Cell-centric build: one CTA per cell.  The CTA copies the packs of every
-// (cell, image) of the cell's neighbourhood into shared memory in traversal
-// order (chunks of `cap` candidates when the neighbourhood is larger), and
-// groups of 8 lanes test one centre atom each against the staged candidates,
-// appending in lane order.  Rows come out identical to k_build's.
-constexpr int BUILD_CELL_THREADS = 128;
-constexpr int BUILD_GROUP = 8;
-
-__global__ void __launch_bounds__(BUILD_CELL_THREADS) k_build_cells(BuildParams p, const PosPack* __restrict__ pack,
-                                                                    const double* __restrict__ x,
-                                                                    const double* __restrict__ y,
-                                                                    const double* __restrict__ z,
-                                                                    const int* __restrict__ start, int cap,
-                                                                    unsigned* __restrict__ nbr, int* __restrict__ nnb,
-                                                                    unsigned* status, int* need) {
-    extern __shared__ float4 s_cand[];  // 2 float4 per candidate: hi (w = atom index), lo (w = image code)
-    __shared__ int s_cell[64], s_code[64], s_pref[65];
-    __shared__ float4 s_sh[64], s_sl[64];  // split image shift by the entry's 6 image bits
-    for (int k = threadIdx.x; k < 64; k += blockDim.x) {
-        const float fx = (float)((k & 3) - 1), fy = (float)(((k >> 2) & 3) - 1), fz = (float)(((k >> 4) & 3) - 1);
-        s_sh[k] = make_float4(fx * p.L.hx, fy * p.L.hy, fz * p.L.hz, 0.f);
-        s_sl[k] = make_float4(fx * p.L.lx, fy * p.L.ly, fz * p.L.lz, 0.f);
-    }
-    const int c = blockIdx.x;
-    const int cx = c % p.nc[0], cy = (c / p.nc[0]) % p.nc[1], cz = c / (p.nc[0] * p.nc[1]);
-    const int mx = axis_count(p.nc[0], p.periodic[0]);
-    const int my = axis_count(p.nc[1], p.periodic[1]);
-    const int mz = axis_count(p.nc[2], p.periodic[2]);
-    const int ncombo = mx * my * mz;  // <= 27 unless a periodic axis has fewer than 3 cells
-    // enumerate (cell, image) combos in traversal order (combo t = (a, b, q)
-    // with q fastest); the first two warps look up one combo each in parallel
-    if (threadIdx.x < 64) {
-        const int t = threadIdx.x;
-        int cnt = 0, cc = 0;
-        unsigned code = 0;
-        if (t < ncombo) {
-            const int q = t % mx, b = (t / mx) % my, a = t / (mx * my);
-            int kz, sz, ky, sy, kx, sx;
-            if (axis_cell(cz, p.nc[2], p.periodic[2], a, kz, sz) && axis_cell(cy, p.nc[1], p.periodic[1], b, ky, sy) &&
-                axis_cell(cx, p.nc[0], p.periodic[0], q, kx, sx)) {
-                cc = (kz * p.nc[1] + ky) * p.nc[0] + kx;
-                cnt = start[cc + 1] - start[cc];
-                code = nbr_encode(0, sx, sy, sz);
-            }
-        }
-        s_cell[t] = cc;
-        s_code[t] = (int)code;
-        s_pref[t + 1] = cnt;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_pref[0] = 0;
-        for (int t = 0; t < 64; t++) s_pref[t + 1] += s_pref[t];
-    }
-    __syncthreads();
-    const int nc_used = ncombo < 64 ? ncombo : 64;
-    const int total = s_pref[nc_used];
-    const int c_begin = start[c], c_end = start[c + 1];
-    const int group = threadIdx.x / BUILD_GROUP, lane = threadIdx.x & (BUILD_GROUP - 1);
-    const int gbase = (threadIdx.x & 31) & ~(BUILD_GROUP - 1);
-    const unsigned gmask = ((1u << BUILD_GROUP) - 1u) << gbase;
-    const unsigned self_code = nbr_encode(0, 0, 0, 0);
-    for (int batch = c_begin; batch < c_end; batch += BUILD_CELL_THREADS / BUILD_GROUP) {
-        const int i = batch + group;
-        const bool active = i < c_end;
-        PosPack pi;
-        if (active) pi = pack[i];
-        int cnt = 0;
-        for (int c0 = 0; c0 < total; c0 += cap) {
-            const int c1 = min(total, c0 + cap);
-            __syncthreads();
-            for (int t = c0 + threadIdx.x; t < c1; t += blockDim.x) {
-                int lo = 0, hi = nc_used;  // combo holding candidate t
-                while (hi - lo > 1) {
-                    int mid = (lo + hi) >> 1;
-                    if (s_pref[mid] <= t) lo = mid;
-                    else hi = mid;
-                }
-                const int k = start[s_cell[lo]] + (t - s_pref[lo]);
-                PosPack pk = pack[k];
-                pk.hi.w = __int_as_float(k);
-                pk.lo.w = __int_as_float(s_code[lo]);
-                s_cand[2 * (t - c0)] = pk.hi;
-                s_cand[2 * (t - c0) + 1] = pk.lo;
-            }
-            __syncthreads();
-            if (active) {
-                for (int k0 = c0; k0 < c1; k0 += BUILD_GROUP) {
-                    const int t = k0 + lane;
-                    bool in = false;
-                    unsigned entry = 0;
-                    if (t < c1) {
-                        const float4 hk = s_cand[2 * (t - c0)], lk = s_cand[2 * (t - c0) + 1];
-                        const unsigned code = __float_as_uint(lk.w);
-                        entry = code | __float_as_uint(hk.w);
-                        const float4 sh = s_sh[code >> 26], sl = s_sl[code >> 26];
-                        const float dx = __fadd_rn(__fsub_rn(__fsub_rn(pi.hi.x, hk.x), sh.x),
-                                                   __fsub_rn(__fsub_rn(pi.lo.x, lk.x), sl.x));
-                        const float dy = __fadd_rn(__fsub_rn(__fsub_rn(pi.hi.y, hk.y), sh.y),
-                                                   __fsub_rn(__fsub_rn(pi.lo.y, lk.y), sl.y));
-                        const float dz = __fadd_rn(__fsub_rn(__fsub_rn(pi.hi.z, hk.z), sh.z),
-                                                   __fsub_rn(__fsub_rn(pi.lo.z, lk.z), sl.z));
-                        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                        // the atom itself is the only candidate at exactly zero distance
-                        in = r2 < p.rsq_lo && r2 > 0.f;
-                        if (r2 >= p.rsq_lo && r2 <= p.rsq_hi)
-                            in = exact_within(p.L64[0], p.L64[1], p.L64[2], p.rsq, x, y, z, i,
-                                              (int)(entry & (unsigned)INDEX_MASK), code);
-                        if (in && r2 < 1e-6f) report_overlap(status, i, (int)(entry & (unsigned)INDEX_MASK));
-                    }
-                    const unsigned bal = __ballot_sync(gmask, in) >> gbase;
-                    if (in) {
-                        const int pos = cnt + __popc(bal & ((1u << lane) - 1u));
-                        if (pos < p.maxnb) nbr[nbr_at(i, pos, p.hshift, p.maxnb)] = entry;
-                    }
-                    cnt += __popc(bal);
-                }
-            }
-        }
-        if (active && lane == 0) {
-            if (cnt > p.maxnb) {
-                atomicOr(status, ERR_NBR_OVERFLOW);
-                atomicMax(need, cnt);
-                cnt = p.maxnb;
-            }
-            nnb[i] = cnt;
-        }
-    }
-}
-
 // rev at (i, s): the slot of (i, -image) in the row of j = nbr at (i, s).
 // For every list entry (i, s) -> j, the slot of i in row j: REV_LANES
 // threads per centre, each searching for every REV_LANES-th entry (the
@@ -1021,6 +885,12 @@ __global__ void k_reverse(int n, int hshift, int maxnb, const unsigned* __restri
 }
 
 // ---------------------------------------------------------------- host side
+
+// Centres per SM up to which the list build takes eight lanes each: the chip
+// holds 896 threads of it a SM, so a thread per centre fills a quarter of
+// that or less.  14,212 EAM atoms: 25 us against 54; 4,000 LJ atoms (79 a row): 36
+// against 90; 512 Tersoff atoms: 14 against 23.
+constexpr int BUILD_SMALL_PER_SM = 256;
 
 // Cells along an axis of extent ext: as many as fit with each at least
 // Rv (1 + 1e-12) wide (the margin absorbs cell_coord's rounding).
@@ -1057,7 +927,7 @@ int replica_prepare(Context* c) {
     std::vector<RepGeom> rg(c->nrep);
     std::vector<ShiftF> sh(c->nrep);
     int base = 0;
-    double hmax = 0.0;
+    double lmax = 0.0;
     for (int r = 0; r < c->nrep; r++) {
         RepGeom& g = rg[r];
         for (int d = 0; d < 3; d++) {
@@ -1076,9 +946,7 @@ int replica_prepare(Context* c) {
                 g.cell_h[d] = ext / g.nc[d];
             }
             g.inv_h[d] = 1.0 / g.cell_h[d];
-            g.base[d] = (float)(g.cell_org[d] - c->box.org[d] + c->box.P[d]);
-            g.hf[d] = (float)g.cell_h[d];
-            hmax = std::max(hmax, g.cell_h[d]);
+            if (g.periodic[d]) lmax = std::max(lmax, g.L[d]);
         }
         const float lh[3] = {(float)g.L[0], (float)g.L[1], (float)g.L[2]};
         g.S.hx = lh[0];
@@ -1092,7 +960,7 @@ int replica_prepare(Context* c) {
         base += g.nc[0] * g.nc[1] * g.nc[2];
     }
     c->rep_cells = base;
-    c->rep_hmax = hmax;
+    c->rep_lmax = lmax;
     // The step graph holds these pointers: allocate once (omdg_set_replicas
     // frees them) and reallocate only for a larger atom capacity, dropping
     // the graph then.  Contents are rewritten in place.
@@ -1109,7 +977,13 @@ int replica_prepare(Context* c) {
         e = cudaMalloc(&c->d_rep_builds, sizeof(int) * c->nrep);
         if (e == cudaSuccess) e = cudaMemsetAsync(c->d_rep_builds, 0, sizeof(int) * c->nrep, c->stream);
     }
-    if (e == cudaSuccess && !c->d_cell_rep) e = cudaMalloc(&c->d_cell_rep, sizeof(int) * std::max(1, base));
+    if (e == cudaSuccess && (!c->d_cell_rep || c->rep_cells_cap < base)) {
+        cudaFree(c->d_cell_rep);
+        c->d_cell_rep = nullptr;
+        e = cudaMalloc(&c->d_cell_rep, sizeof(int) * std::max(1, base));
+        c->rep_cells_cap = base;
+        invalidate_graph(c);
+    }
     if (e == cudaSuccess && (!c->d_rep_of || c->rep_of_cap < c->cap)) {
         cudaFree(c->d_rep_of);
         c->d_rep_of = nullptr;
@@ -1272,8 +1146,7 @@ int integrate_pack(Context* c) {
     if (c->n == 0) return OMDG_OK;
     // xref keeps the positions of the last build (the displacement reference)
     k_pack<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->x, c->y, c->z, c->type, pack_frame(c), c->pack,
-                                                       nullptr, nullptr, LocFrame{}, nullptr, nullptr,
-                                                       nullptr, nullptr, nullptr, nullptr);
+                                                       nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     c->launches++;
     return check_cuda(c, cudaGetLastError(), "pack");
 }
@@ -1348,18 +1221,12 @@ int nlist_build(Context* c) {
     c->launches += 2;
     prof_end(c);
     prof_begin(c, "pack");
-    LocFrame lf;
-    for (int d = 0; d < 3; d++) {
-        lf.nc[d] = g.nc[d];
-        lf.h[d] = (float)g.h[d];
-        lf.base[d] = (float)(g.org[d] - c->box.org[d] + c->box.P[d]);
-    }
+    const RepGeom* rg = reps ? static_cast<const RepGeom*>(c->d_rep_geom) : nullptr;
     unsigned* umax = reinterpret_cast<unsigned*>(c->d_flags + 3);
     k_zero_ints<<<1, 32, 0, s>>>(1, c->d_flags + 3, c->d_flags + 3);
-    const RepGeom* rg = reps ? static_cast<const RepGeom*>(c->d_rep_geom) : nullptr;
     k_pack<<<grid_for(n, 256), 256, 0, s>>>(n, c->x, c->y, c->z, c->type, pack_frame(c), c->pack, c->xref,
-                                            cell_sorted, lf, reps ? c->d_rep_of : nullptr, rg,
-                                            c->flags_used ? c->aflag : nullptr, c->loc, umax, rflag);
+                                            reps ? c->d_rep_of : nullptr, c->flags_used ? c->aflag : nullptr, c->loc,
+                                            umax, rflag);
     c->launches += 2;
     prof_end(c);
 
@@ -1410,54 +1277,34 @@ int nlist_build(Context* c) {
     bp.L = make_shift(c->box);
     double rv = c->rc_max + c->skin;
     bp.rsq = rv * rv;
-    bp.rsq_lo = (float)(bp.rsq * (1.0 - 2e-5));
-    bp.rsq_hi = (float)(bp.rsq * (1.0 + 2e-5));
     bp.rv = (float)rv;
-    bp.hmax = 0.f;
-    for (int d = 0; d < 3; d++) {
-        bp.base[d] = lf.base[d];
-        bp.h[d] = lf.h[d];
-        bp.hmax = fmaxf(bp.hmax, lf.h[d]);
-    }
-    if (reps) bp.hmax = (float)c->rep_hmax;
     prof_begin(c, "nlist_build");
-    int combos = 1;
-    for (int d = 0; d < 3; d++) combos *= (g.periodic[d] && g.nc[d] < 3) ? 3 * g.nc[d] : 3;
-    // the cell-local builds also write each row's type mask
-    c->nbmask_valid = reps || c->flags_used || tiles || !(c->build_lanes == 0 && combos <= 64 && !sparse) &&
-                                                   c->build_lanes != 8 && c->build_lanes != 4;
-    if (reps) {
-        k_build<true><<<grid_for(n, 128), 128, 0, s>>>(bp, rg, c->d_rep_of, c->loc, c->x, c->y, c->z, cell_sorted,
-                                                       c->cell_start, umax, reinterpret_cast<unsigned*>(c->nbr),
-                                                       c->nnb, c->d_status, c->d_flags + 1, rflag, c->nbmask);
-    } else if (tiles) {  // only the cell-local build writes tile slots
-        k_build<false, true><<<grid_for(n, 128), 128, 0, s>>>(bp, nullptr, nullptr, c->loc, c->x, c->y, c->z,
-                                                              cell_sorted, c->cell_start, umax,
-                                                              reinterpret_cast<unsigned*>(c->nbr), c->nnb,
-                                                              c->d_status, c->d_flags + 1, nullptr, c->nbmask);
-    } else if (c->flags_used) {  // only the cell-local build skips inactive atoms
-        k_build<false><<<grid_for(n, 128), 128, 0, s>>>(bp, nullptr, nullptr, c->loc, c->x, c->y, c->z,
-                                                        cell_sorted, c->cell_start, umax,
-                                                        reinterpret_cast<unsigned*>(c->nbr), c->nnb, c->d_status,
-                                                        c->d_flags + 1, nullptr, c->nbmask);
-    } else if (c->build_lanes == 0 && combos <= 64 && !sparse) {  // a cell CTA wants >= 8 atoms per cell
-        const int cap = 1024;  // staged candidates per chunk (32 bytes each)
-        k_build_cells<<<m, BUILD_CELL_THREADS, cap * 2 * sizeof(float4), s>>>(
-            bp, c->pack, c->x, c->y, c->z, c->cell_start, cap, reinterpret_cast<unsigned*>(c->nbr), c->nnb,
-            c->d_status, c->d_flags + 1);
-    } else if (c->build_lanes == 8) {
-        k_build_lanes<8><<<grid_for(n, 256 / 8), 256, 0, s>>>(bp, c->pack, c->x, c->y, c->z, cell_sorted,
-                                                               c->cell_start, reinterpret_cast<unsigned*>(c->nbr),
-                                                               c->nnb, c->d_status, c->d_flags + 1);
-    } else if (c->build_lanes == 4) {
-        k_build_lanes<4><<<grid_for(n, 256 / 4), 256, 0, s>>>(bp, c->pack, c->x, c->y, c->z, cell_sorted,
-                                                               c->cell_start, reinterpret_cast<unsigned*>(c->nbr),
-                                                               c->nnb, c->d_status, c->d_flags + 1);
+    bp.lmax = 0.f;
+    for (int d = 0; d < 3; d++)
+        if (g.periodic[d]) bp.lmax = fmaxf(bp.lmax, (float)g.L[d]);
+    if (reps) bp.lmax = (float)c->rep_lmax;
+    // shared-memory columns: maxnb is twice the mean row and 32 at first, so
+    // half of it and 8 holds nearly every row; 64 entries (32 KB a block)
+    // keep seven blocks on a SM.  Longer rows go out in pieces.
+    bp.cap = std::max(2 * BUILD_AHEAD, std::min(64, c->maxnb / 2 + 8));
+    const bool one = c->ntypes == 1;
+    // eight lanes a centre while a thread per centre would leave most of the
+    // chip's warp slots empty (BUILD_SMALL_PER_SM)
+    const bool small = c->build_lanes == 8 || (c->build_lanes != 1 && n <= BUILD_SMALL_PER_SM * c->num_sms);
+    const int lanes = small && !tiles ? 8 : 1;  // only the one-thread form writes tile slots
+    const size_t smem = sizeof(unsigned) * BUILD_THREADS * (lanes == 1 ? bp.cap : BUILD_RUN);
+    const auto launch = [&](auto kernel) {
+        kernel<<<grid_for(n, BUILD_THREADS / lanes), BUILD_THREADS, smem, s>>>(
+            bp, rg, c->d_rep_of, c->loc, c->x, c->y, c->z, cell_sorted, c->cell_start, umax,
+            reinterpret_cast<unsigned*>(c->nbr), c->nnb, c->d_status, c->d_flags + 1, rflag, c->nbmask);
+    };
+    if (lanes == 8) {
+        if (reps) one ? launch(k_build<8, true, false, true>) : launch(k_build<8, true, false, false>);
+        else one ? launch(k_build<8, false, false, true>) : launch(k_build<8, false, false, false>);
     } else {
-        k_build<false><<<grid_for(n, 128), 128, 0, s>>>(bp, nullptr, nullptr, c->loc, c->x, c->y, c->z,
-                                                        cell_sorted, c->cell_start, umax,
-                                                        reinterpret_cast<unsigned*>(c->nbr), c->nnb, c->d_status,
-                                                        c->d_flags + 1, nullptr, c->nbmask);
+        if (reps) one ? launch(k_build<1, true, false, true>) : launch(k_build<1, true, false, false>);
+        else if (tiles) launch(k_build<1, false, true, true>);  // the tiled passes take one type
+        else one ? launch(k_build<1, false, false, true>) : launch(k_build<1, false, false, false>);
     }
     c->launches++;
     if (c->build_in_step) {

@@ -165,9 +165,8 @@ struct Context {
     float *pe = nullptr, *vir = nullptr;
     PosPack* pack = nullptr;
     float4* xref = nullptr;   // pack-frame position at the last build (FP32)
-    float4* loc = nullptr;    // position relative to its cell's corner at the last build (FP32); w = the type
-    unsigned* nbmask = nullptr;  // per atom: bit t set when its row holds an atom of type t (cell-local build)
-    bool nbmask_valid = false;   // the last build wrote nbmask
+    float4* loc = nullptr;    // position at the last build rounded to FP32; w = the type
+    unsigned* nbmask = nullptr;  // per atom: bit t set when its row holds an atom of type t
     int* type = nullptr;
     int* id = nullptr;        // caller index of sorted atom
     int* inv = nullptr;       // sorted index of caller atom
@@ -184,7 +183,8 @@ struct Context {
     std::vector<double> rep_lo, rep_hi;  // nrep x 3
     int rep_periodic[3] = {1, 1, 0};
     int rep_cells = 0;                   // cells over all replicas
-    double rep_hmax = 0.0;               // largest replica cell size (list screening band)
+    double rep_lmax = 0.0;               // largest periodic replica length (list screening band)
+    int rep_cells_cap = 0;               // entries of d_cell_rep
     int* d_rep_of = nullptr;             // replica of each atom (index order)
     int rep_of_cap = 0;
     void* d_rep_geom = nullptr;          // RepGeom[nrep] (nlist.cu)
@@ -200,6 +200,7 @@ struct Context {
     bool kick_fused = false;             // the last force launch did the step's second half-kick
     int ncell_cap = 0;
     int* scan_partials = nullptr;
+    int* cell_sorted = nullptr;
     double* stage_d = nullptr;   // permutation staging: 6 FP64 arrays x cap
     int* stage_i = nullptr;      // permutation staging: 2 int arrays x cap
     unsigned* aflag = nullptr;   // per atom: bit 0 FLAG_ACTIVE (base.h:230), bits 8..15 group membership
@@ -207,7 +208,6 @@ struct Context {
     double* extra = nullptr;     // optional per-atom FP64 state carried through sorts
     double* stage_extra = nullptr;
     int extra_n = 0;
-    int* cell_sorted = nullptr;
     double* f64 = nullptr;       // FP64 forces (3n) + FP64 per-atom energy (n), FP64 kernels only
     bool use_f64 = false;
     double* d_mass = nullptr;    // mass per type (device)
@@ -250,8 +250,7 @@ struct Context {
     // launch shapes (defaults; the tuner may change them)
     int num_sms = 152;
     int io_blocks = 152;       // blocks of the download kernels beside a step (omdg_step_io)
-    int build_lanes = 0;       // list build: 1, 4, 8 threads per atom; 0 cell-centric (shared memory)
-                               // on grids of >= 8 atoms per cell, else one thread per atom
+    int build_lanes = 0;       // list build: 1 or 8 threads per centre; else by the box's size
     int nbr_hshift = 3;        // sliced-ELL slice height H = 2^hshift
     int eam_block = 256;
     int eam_lanes = 4;         // threads per atom
@@ -322,7 +321,7 @@ struct Context {
     // device status and reductions
     unsigned* d_status = nullptr;   // error bits
     int* d_flags = nullptr;         // [0] rebuild request, [1] row length needed, [2] ghost count,
-                                    // [3] largest cell-local coordinate of the last build (float bits),
+                                    // [3] largest coordinate of the last build (float bits),
                                     // [4] blocks done in the current kick (reset by the last block)
     double* d_red = nullptr;        // block partials
     int red_cap = 0;
@@ -426,6 +425,7 @@ int post_force_modifies(Context* c);  // ForceDamper / CoordClamp after the forc
 int io_set_flags(Context* c, const unsigned* flags, unsigned keep_mask);  // caller order; bits in keep_mask survive
 int io_get_flags(Context* c, unsigned* flags);
 
+constexpr int LOC_PAD = 6;    // entries past the last atom the list build may load
 constexpr int LEDGER_W = 12;  // doubles per ledger row
 constexpr int RED_BLOCK = 256;  // threads of the kick kernel's blocks (one 32-byte partial each)
 

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(512) k_pair32(PairParams p, const PosPack* __r
         bool any = valid && (p.all_types || ti == p.ta || ti == p.tb);
         // with the rows' type masks, a row without the partner type is skipped
         // whole (most rows of a mixed system: a Si atom with no Ar near)
-        if (any && !p.all_types && nbmask)
+        if (any && !p.all_types)
             any = (nbmask[ii] & ((ti == p.ta ? want_a : 0u) | (ti == p.tb ? want_b : 0u))) != 0u;
         int m = any ? nnb[ii] : 0;
         Kahan ax, ay, az, ae;
@@ -184,7 +184,7 @@ static void launch32(Context* c, const PairParams& p, int block) {
     int per_block = block / LANES;
     k_pair32<LANES><<<grid_for(c->n, per_block), block, 0, c->stream>>>(
         p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->fx, c->fy, c->fz, c->pe, c->vir,
-        c->d_status, c->nbmask_valid ? c->nbmask : nullptr);
+        c->d_status, c->nbmask);
 }
 
 int pair_launch(Context* c, Potential& pot, bool first) {

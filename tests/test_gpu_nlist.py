@@ -83,3 +83,29 @@ def test_build_variants_match_oracle_and_each_other(omdg_lib, oracle_lib, geomet
             forces.append(ctx.get_state()["f"])
     for mode, f in zip(MODES[1:], forces[1:]):
         assert np.array_equal(f, forces[0]), mode
+
+
+# Rows longer than a thread's shared-memory column (64 entries at one thread
+# per centre, 32 per run of cells at eight), at the widths where the candidate
+# loop's last group is ragged, for one and two atom types.
+@pytest.mark.parametrize("n,side,ntypes", [(1500, 3.05, 1), (3001, 3.3, 1), (2003, 2.2, 2), (700, 1.4, 1)])
+def test_rows_past_the_shared_columns(omdg_lib, oracle_lib, n, side, ntypes):
+    from objectmd_gb300 import inputs
+
+    oc = oracle_lib
+    rv = cutoff(oc)
+    rng = np.random.default_rng(n)
+    L = np.full(3, side * rv)
+    x = rng.uniform(0.0, 1.0, (n, 3)) * L
+    ref = nbr_set(*oc.neighbors(oc.make_box(np.zeros(3), L, (1, 1, 1)), x, rv, 2048))
+    assert len(ref) > 100 * n
+    for mode in (1, 8):
+        with omdg_lib.Context(0) as ctx:
+            ctx.set_box(np.zeros(3), L, (True, True, True))
+            ctx.set_atoms(x, types=rng.integers(0, ntypes, n), masses=[inputs.md_mass("aluminum")] * ntypes,
+                          znum=[13.0] * ntypes)
+            ctx.add_eam(EAM_TABLE)
+            ctx.set_neighbor(SKIN, 1)
+            ctx.set_launch("build_lanes", mode)
+            ctx.build_neighbors()
+            assert nbr_set(*ctx.neighbors()) == ref, mode
