@@ -114,54 +114,109 @@ __global__ void __launch_bounds__(512) k_pair32(PairParams p, const PosPack* __r
     }
 }
 
-// FP64 end to end: dx = x_i - (x_j + s), r = sqrt(r2), TableReader in FP64.
-// PAIR64_LANES lanes per atom take every PAIR64_LANES-th row entry, and the
-// lanes' FP64 sums meet in a fixed xor tree, so the FP64 work of a small box
-// spreads over the whole chip (one thread per atom left most SMs idle).
-constexpr int PAIR64_LANES = 32;
+// FP64 end to end.  The FP64 pipe (one warp instruction in about 18 cycles of
+// an SM) sets the time, so the pass counts FP64 instructions: about 30 a pair.
+//   - the centre minus the image's length is formed once per centre and picked
+//     by the entry's image bits (integer selects cost nothing here);
+//   - 1/r comes from the hardware's reciprocal-square-root estimate and one
+//     third-order step (y + y e (1/2 + 3/8 e), e = 1 - r^2 y^2: the estimate's
+//     error cubed, below an ulp), r = r^2 / r takes one Newton step to half
+//     an ulp, and the force factor a product where the reference divides;
+//   - the knot index comes from FP32; a value it puts in the segment next
+//     door is off by the spline's third-derivative jump times 1e-4 knots
+//     cubed, far below an ulp;
+//   - value and slope share their Horner steps.
+// Reads below the first knot, with the reference's edge rules, go through
+// tab_read64 out of line.  The IEEE sequences (root, two divisions, separate
+// adds and products) took about 110 FP64 instructions a pair: 4,000 LJ argon
+// atoms 66 us, now 33.  Against quad precision the forces are as far off as
+// theirs (1.3-1.4e-15 of the norm).
+__device__ __noinline__ void tab_read64_slow(const DevTable& t, double r, double* v, double* dv, unsigned* status) {
+    tab_read64(t, r, *v, *dv, status);
+}
 
-__global__ void __launch_bounds__(128) k_pair64(PairParams p, const double* __restrict__ x,
+// double to float by the bits (truncated; normal, positive, in float's range)
+__device__ __forceinline__ float d2f_bits(double d) {
+    const int hi = __double2hiint(d), lo = __double2loint(d);
+    return __int_as_float(__funnelshift_l(lo, hi - 0x38000000, 3));
+}
+
+constexpr int P64_BLOCK = 32;  // one warp a block: the pipe is shared evenly (4,000 atoms: 30.9 us, 33.7 at 128)
+
+// LANES lanes per atom take every LANES-th row entry, and the lanes' FP64
+// sums meet in a fixed xor tree.
+template <int LANES>
+__global__ void __launch_bounds__(P64_BLOCK) k_pair64(PairParams p, const double* __restrict__ x,
                                                 const double* __restrict__ y, const double* __restrict__ z,
                                                 const int* __restrict__ type, const unsigned* __restrict__ nbr,
                                                 const int* __restrict__ nnb, double* __restrict__ f64,
                                                 float* __restrict__ pe, float* __restrict__ vir, unsigned* status) {
-    const int lane = threadIdx.x & (PAIR64_LANES - 1);
-    const int i = blockIdx.x * (blockDim.x / PAIR64_LANES) + threadIdx.x / PAIR64_LANES;
-    if (i >= p.n) return;  // whole warps leave together
+    const int lane = threadIdx.x & (LANES - 1);
+    const int at = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
+    const bool valid = at < p.n;
+    const int i = valid ? at : p.n - 1;
     const int ti = type[i];
     const double xi = x[i], yi = y[i], zi = z[i];
+    const double xm = xi - p.L64[0], xp = xi + p.L64[0], ym = yi - p.L64[1], yp = yi + p.L64[1], zm = zi - p.L64[2],
+                 zp = zi + p.L64[2];
     double ax = 0, ay = 0, az = 0, ae = 0, av = 0;
-    const bool any = p.all_types || ti == p.ta || ti == p.tb;
+    const bool any = valid && (p.all_types || ti == p.ta || ti == p.tb);
     const int m = any ? nnb[i] : 0;
-    for (int s = lane; s < m; s += PAIR64_LANES) {
+    const long long rc_bits = __double_as_longlong(p.rc64);
+    for (int s = lane; s < m; s += LANES) {
         const unsigned e = __ldg(&nbr[nbr_at(i, s, p.hshift, p.maxnb)]);
         const int j = nbr_index(e);
         if (!p.all_types && !types_match(ti, type[j], p.ta, p.tb)) continue;
         const int sx = nbr_sx(e), sy = nbr_sy(e), sz = nbr_sz(e);
-        const double gx = __dadd_rn(x[j], sx == 0 ? 0.0 : (sx > 0 ? p.L64[0] : -p.L64[0]));
-        const double gy = __dadd_rn(y[j], sy == 0 ? 0.0 : (sy > 0 ? p.L64[1] : -p.L64[1]));
-        const double gz = __dadd_rn(z[j], sz == 0 ? 0.0 : (sz > 0 ? p.L64[2] : -p.L64[2]));
-        const double dx = __dsub_rn(xi, gx), dy = __dsub_rn(yi, gy), dz = __dsub_rn(zi, gz);
-        const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-        const double r = __dsqrt_rn(r2);
-        if (!(r < p.rc64)) continue;
+        const double dx = (sx == 0 ? xi : (sx > 0 ? xm : xp)) - x[j];
+        const double dy = (sy == 0 ? yi : (sy > 0 ? ym : yp)) - y[j];
+        const double dz = (sz == 0 ? zi : (sz > 0 ? zm : zp)) - z[j];
+        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+        double w;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(w) : "d"(r2));
+        const double err = fma(-(r2 * w), w, 1.0);
+        double rinv = fma(fma(0.375, err, 0.5), w * err, w);
+        double r = r2 * rinv;
+        r = fma(fma(-r, r, r2), 0.5 * rinv, r);  // the root to half an ulp, as the reference's
+        const bool tiny = __double_as_longlong(r2) < 0x3D70000000000000ll;  // r below 2^-20: the estimate may not hold
+        if (tiny) {
+            r = __dsqrt_rn(r2);
+            rinv = 1.0 / r;
+        }
+        if (!(__double_as_longlong(r) < rc_bits)) continue;  // r < rc, on the bits of non-negative doubles
+        const double rval = r - p.phi.off64;
         double ph, dph;
-        tab_read64(p.phi, r, ph, dph, status);
-        const double fr = __ddiv_rn(-dph, r);
-        ax = __dadd_rn(ax, __dmul_rn(dx, fr));
-        ay = __dadd_rn(ay, __dmul_rn(dy, fr));
-        az = __dadd_rn(az, __dmul_rn(dz, fr));
-        ae = __dadd_rn(ae, __dmul_rn(0.5, ph));
-        av = __dadd_rn(av, __dmul_rn(fr, r2));
+        // at or below the first knot, or a table so long that FP32 may miss its knot by one
+        if (tiny || __double_as_longlong(rval) < (1ll << 52) || p.phi.n > (1 << 16)) {
+            tab_read64_slow(p.phi, r, &ph, &dph, status);
+        } else {
+            const int k = min((int)(d2f_bits(rval) * p.phi.inv_dr), p.phi.n - 2);
+            const double d = fma(-f2d_exact((float)k), p.phi.dr64, rval);
+            const double4_32a cf = p.phi.coef64[k];
+            const double u = fma(d, cf.x, cf.y), h = fma(d, u, cf.z);
+            ph = fma(d, h, cf.w);
+            dph = fma(d, fma(d, cf.x, u), h);
+            if (p.phi.rmult) {
+                ph *= rinv;
+                dph = (dph - ph) * rinv;
+            }
+        }
+        const double fr = -dph * rinv;
+        ax = fma(dx, fr, ax);
+        ay = fma(dy, fr, ay);
+        az = fma(dz, fr, az);
+        ae = fma(0.5, ph, ae);
+        av = fma(fr, r2, av);
     }
-    for (int o = PAIR64_LANES / 2; o > 0; o >>= 1) {
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
         ax += __shfl_xor_sync(0xffffffffu, ax, o);
         ay += __shfl_xor_sync(0xffffffffu, ay, o);
         az += __shfl_xor_sync(0xffffffffu, az, o);
         ae += __shfl_xor_sync(0xffffffffu, ae, o);
         av += __shfl_xor_sync(0xffffffffu, av, o);
     }
-    if (lane != 0) return;
+    if (lane != 0 || !valid) return;
     if (p.first) {
         f64[3 * (size_t)i + 0] = ax;
         f64[3 * (size_t)i + 1] = ay;
@@ -177,6 +232,25 @@ __global__ void __launch_bounds__(128) k_pair64(PairParams p, const double* __re
         vir[i] += (float)av;
         f64[3 * (size_t)p.n + i] += ae;
     }
+}
+
+template <int LANES>
+static void launch64(Context* c, const PairParams& p) {
+    k_pair64<LANES><<<grid_for(c->n, P64_BLOCK / LANES), P64_BLOCK, 0, c->stream>>>(
+        p, c->x, c->y, c->z, c->type, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->f64, c->pe, c->vir,
+        c->d_status);
+}
+
+// Few lanes an atom waste the least on ragged rows and on the sums' exchange,
+// many shorten the dependent chain where the chip is not full (a warp alone
+// takes about 2 us per row entry).  LJ argon, 79 entries, us with 8 / 16 / 32
+// lanes before the root's Newton step: 500 atoms 25.7 / 17.1 / 14.0, 2,048
+// atoms 26.1 / 19.9 / 23.7, 4,000 atoms 30.9 / 31.8 / 40.0, 16,384 atoms 95 /
+// 104 / 132.
+static void launch64(Context* c, const PairParams& p) {
+    if (c->n >= 20 * c->num_sms) launch64<8>(c, p);
+    else if (c->n >= 8 * c->num_sms) launch64<16>(c, p);
+    else launch64<32>(c, p);
 }
 
 template <int LANES>
@@ -208,9 +282,7 @@ int pair_launch(Context* c, Potential& pot, bool first) {
     int block = c->pair_block;
     if (pot.fp64) {
         prof_begin(c, "pair64");
-        k_pair64<<<grid_for(c->n, 128 / PAIR64_LANES), 128, 0, c->stream>>>(p, c->x, c->y, c->z, c->type,
-                                                              reinterpret_cast<const unsigned*>(c->nbr), c->nnb,
-                                                              c->f64, c->pe, c->vir, c->d_status);
+        launch64(c, p);
     } else {
         prof_begin(c, "pair32");
         switch (c->pair_lanes) {

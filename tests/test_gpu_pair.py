@@ -115,3 +115,57 @@ def test_berendsen_thermostat_default_counts_owners(omdg_lib, oracle_lib):
         if step:
             v *= oc.berendsen_factor(dt, tau, tset, (2.0 / 3.0) / 8.61734279e-05 * k / n)
     np.testing.assert_allclose(kin, ref, rtol=1e-6)
+
+
+def _lj(omdg, x, types, ntypes, lo, hi, pairs):
+    from objectmd_gb300 import inputs
+
+    ctx = omdg.Context(0)
+    ctx.set_box(lo, hi)
+    ctx.set_atoms(x, types=types, masses=[inputs.md_mass("argon")] * ntypes, znum=[18.0] * ntypes)
+    for a, b in pairs:
+        ctx.add_pair_table(LJ, a, b, fp64=True)
+    ctx.set_neighbor(0.3, 1)
+    return ctx
+
+
+# The FP64 pass takes 32, 16 or 8 lanes an atom by the box's size (1,216 and
+# 3,040 atoms on 152 SMs); untyped and typed, against the oracle.
+@pytest.mark.parametrize("ncell,ntypes", [(4, 1), (6, 2), (7, 1), (8, 2), (9, 1), (10, 2)])
+def test_fp64_pair_lanes_match_oracle(omdg_lib, oracle_lib, ncell, ntypes):
+    from objectmd_gb300 import inputs
+
+    oc = oracle_lib
+    x, _, (lo, hi) = inputs.lj_argon(ncell=ncell)
+    x = inputs.perturb(x, 0.15, 7, lo, hi)
+    types = np.random.default_rng(8).integers(0, ntypes, len(x)).astype(np.int32)
+    phi = oc.Table.from_file(LJ, "")
+    nb = oc.neighbors(oc.make_box(lo, hi, (1, 1, 1)), x, phi.max_range() + 0.3)
+    off, j, _ = nb
+    f, e = oc.pair_table(oc.make_box(lo, hi, (1, 1, 1)), x, nb, phi)[:2]
+    with _lj(omdg_lib, x, types, ntypes, lo, hi, [(0, 0), (0, 1), (1, 1)][:1 if ntypes == 1 else 3]) as ctx:
+        ctx.compute_forces()
+        st = ctx.get_state()
+    assert np.abs(st["f"] - f).max() < 1e-10
+    assert np.abs(st["pot"] - e).max() < 1e-12 + 2.0 ** -23 * np.abs(e).max()
+
+
+# A pair closer than the first knot is refused (treader.cpp:199-218), and so is a
+# pair moved onto one point without a rebuild of the list in between.
+@pytest.mark.parametrize("gap,later", [(1.9, None), (0.5, None), (3.0, 1.95), (2.1, 1.95), (2.01, 0.0)])
+def test_fp64_pair_below_the_first_knot(omdg_lib, gap, later):
+    lo, hi = np.zeros(3), np.full(3, 40.0)
+    x = np.array([[10.0, 10.0, 10.0], [10.0 + gap, 10.0, 10.0]])
+    with _lj(omdg_lib, x, np.zeros(2, np.int32), 1, lo, hi, [(0, 0)]) as ctx:
+        if later is None:
+            with pytest.raises(omdg_lib.OMDGError) as err:
+                ctx.compute_forces()
+            assert err.value.code == omdg_lib.OMDG_ERANGE
+        else:
+            ctx.set_neighbor(20.0 if later == 0.0 else 3.0, 0)
+            ctx.compute_forces()
+            x[1, 0] = 10.0 + later
+            ctx.set_positions(x)
+            with pytest.raises(omdg_lib.OMDGError) as err:
+                ctx.compute_forces()
+            assert err.value.code in (omdg_lib.OMDG_ERANGE, omdg_lib.OMDG_EOVERLAP)
