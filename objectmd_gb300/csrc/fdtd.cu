@@ -16,12 +16,11 @@
 // reference built with -ffp-contract=off.  A face's conductance
 // K = con_a con_b / (con_a + con_b) is the same number seen from either cell
 // (both operations commute), so k_fd_faces computes it once per face when
-// the conductivity is uploaded and the step reads it: the step's FP64
-// divisions drop from seven per cell to the one by cap.  The step then moves
-// 8 B of the old vector, 24 B of its own three face conductances, 8 B cap,
-// 8 B S, 8 B E, 4 B map and 1 B mask read and 8 B written per cell (69 B; E
-// and S are cleared only where not zero); the neighbours' T and conductances
-// come from L1/L2.  A face whose conductance is zero adds nothing, as in the
+// the conductivity is uploaded and the step reads it, and the division by
+// cap takes the capacity's reciprocal (fd_quotient).  The step then moves
+// 8 B of the old vector, 24 B of its own three face conductances, 16 B cap
+// and its reciprocal, 8 B S, 8 B E, 4 B map and 1 B mask read and 8 B written
+// per cell (77 B); the neighbours' T and conductances come from L1/L2.  A face whose conductance is zero adds nothing, as in the
 // reference for finite cell values.
 //
 // Host side (the string path of FDTDSolver, fdtd.cpp:100-118, 506-597): the
@@ -30,6 +29,7 @@
 // pruning, applied to host images that are uploaded when they change.  A
 // '{...}' value is an expression for muParser (a third-party library the
 // reference does not vendor): it is refused with OMDG_EINVAL.
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cstring>
@@ -53,16 +53,16 @@ FDDev fd_dev(const FDGrid* g) {
     p.nz = g->nz;
     p.dim = g->dim;
     p.dt = g->timestep;
-    p.h2inv = g->h2inv;
+    p.h2inv2 = 2.0 * g->h2inv;
     p.map = g->dmap;
     p.mask = g->dmask[g->solves > 0 ? 1 : 0];
     p.K = g->dK;
     p.cap = g->dcap;
+    p.rcap = g->drcap;
     p.S = g->dS;
     p.E = g->dE;
     p.mask_first = p.mask_later = nullptr;
     p.solves = p.active = nullptr;
-    p.keep_S = 0;
     return p;
 }
 
@@ -89,6 +89,36 @@ __global__ void __launch_bounds__(FD_BLOCK) k_fd_faces(int nx, int ny, int nz, c
 __device__ __forceinline__ double fd_face(const double* __restrict__ T, double K, int nb, double ti, double acc) {
     if (K != 0.0) acc = __dadd_rn(acc, __dmul_rn(K, __dsub_rn(T[nb], ti)));
     return acc;
+}
+
+// The reciprocal of each capacity, correctly rounded, for fd_quotient; NaN
+// where the step must divide (not positive, out of the range in which no
+// intermediate leaves the normal numbers, or a mantissa of ones, which the
+// theorem excludes).
+__global__ void __launch_bounds__(FD_BLOCK) k_fd_rcp(int dim, const double* __restrict__ cap,
+                                                     double* __restrict__ rcap) {
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= dim) return;
+    const double c = cap[idx];
+    const long long b = __double_as_longlong(c), m = b & 0xFFFFFFFFFFFFFll;
+    const int e = (int)(b >> 52);  // negative for negative capacities
+    rcap[idx] = (e >= 723 && e <= 1323 && m != 0xFFFFFFFFFFFFFll) ? __ddiv_rn(1.0, c) : __longlong_as_double(-1ll);
+}
+
+// x / c, correctly rounded, with r the correctly rounded 1 / c: a quotient
+// refined once is within an ulp, and then one residual step rounds correctly
+// (P. Markstein, IBM J. Res. Dev. 34, 111 (1990)).  Five FP64 instructions
+// where the division takes about ten.
+__device__ __forceinline__ double fd_quotient(double x, double c, double r) {
+    const int e = (__double2hiint(x) >> 20) & 0x7FF;
+    const bool zero = (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) == 0;
+    if (r == r && ((e >= 723 && e <= 1323) || zero)) {
+        if (zero) return x;  // c is positive
+        double q = __dmul_rn(x, r);
+        q = __fma_rn(__fma_rn(-q, c, x), r, q);
+        return __fma_rn(__fma_rn(-q, c, x), r, q);
+    }
+    return __ddiv_rn(x, c);
 }
 
 __global__ void __launch_bounds__(FD_BLOCK) k_fd_solve(FDDev p, const double* __restrict__ T, double* __restrict__ A) {
@@ -125,12 +155,18 @@ __global__ void __launch_bounds__(FD_BLOCK) k_fd_solve(FDDev p, const double* __
         }
     }
     // A = T + (2 A h2inv + S + E) dt / cap (fdtd.cpp:664)
+    // (2 acc is exact, so its product with h2inv is acc's with 2 h2inv; adding
+    // a zero changes nothing but the sign of a zero sum, restored below)
     const double si = p.S[idx], ei = p.E[idx];
-    const double q = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(2.0, acc), p.h2inv), si), ei);
-    A[idx] = __dadd_rn(ti, __ddiv_rn(__dmul_rn(q, p.dt), p.cap[idx]));
-    // E[i] = S[i] = 0 (fdtd.cpp:665), written only where not zero already
+    double q = __dmul_rn(acc, p.h2inv2);
+    if (si != 0.0) q = __dadd_rn(q, si);
+    if (ei != 0.0) q = __dadd_rn(q, ei);
+    if (q == 0.0 && !(__double_as_longlong(si) < 0 && __double_as_longlong(ei) < 0)) q = 0.0;
+    const double x = __dmul_rn(q, p.dt);
+    A[idx] = __dadd_rn(ti, p.rcap ? fd_quotient(x, p.cap[idx], p.rcap[idx]) : __ddiv_rn(x, p.cap[idx]));
+    // E[i] = 0 (fdtd.cpp:665), written only where not zero already; the source
+    // pattern stays, the host decides whether the next solve sees it
     if (ei != 0.0) p.E[idx] = 0.0;
-    if (!p.keep_S && si != 0.0) p.S[idx] = 0.0;
 }
 
 int fd_solve(FDGrid* g, cudaStream_t s) {
@@ -251,8 +287,12 @@ static void check_expression(std::string& str, int& t0, int& t1, bool& isequ) {
 
 // AssignArray(ptr, str) (fdtd.cpp:528-592): tokens outside their time range
 // are dropped from str, ranged ones in range are kept (an unranged token is
-// kept for good).
-static int assign_array(FDGrid* g, std::vector<double>& a, std::string& str, bool& changed) {
+// kept for good).  until: the last step at which the tokens applied now are
+// the ones that apply (INT_MAX when they stay).  standing: a holds these
+// assignments already, only the string is pruned.
+static int assign_array(FDGrid* g, std::vector<double>& a, std::string& str, bool& changed, int& until,
+                        bool standing = false) {
+    until = INT_MAX;
     if (str.empty()) return OMDG_OK;
     std::istringstream ss(str);
     str.clear();
@@ -263,11 +303,13 @@ static int assign_array(FDGrid* g, std::vector<double>& a, std::string& str, boo
         bool isequ;
         check_expression(val, t0, t1, isequ);
         if (!(g->step >= t0 && g->step <= t1)) continue;
+        until = std::min(until, t1);
         if (t0 != t1) {
             if (isequ) str += tok + " {" + val + ":" + std::to_string(t0) + ":" + std::to_string(t1) + "} ";
             else str += tok + " " + val + ":" + std::to_string(t0) + ":" + std::to_string(t1) + " ";
         }
         if (isequ) return fd_fail(g, OMDG_EINVAL, "'{...}' expressions need muParser, which is not built: " + val);
+        if (standing) continue;
         if (tok[0] == '@') {
             // coordinates before '=', the value after it (without '=' the
             // whole token is both, as val.erase(0, npos + 1) erases nothing)
@@ -298,40 +340,62 @@ static int assign_array(FDGrid* g, std::vector<double>& a, std::string& str, boo
                 return rc;
             }
         } else {  // every cell whose symbol is in tok ('*' all, '.' cells outside the symbol map)
-            double dv;
+            // (one pass over the cells: the token's symbols take the same value)
+            double dv = 0.0;
             const bool ok = to_double(val, dv);
+            const int nsym = (int)g->bound.size();
+            std::vector<char> takes(nsym + 1, 0);  // last: cells outside the symbol map
             for (char c : tok)
-                for (int i = 0; i < g->nx; i++)
-                    for (int j = 0; j < g->ny; j++)
-                        for (int k = 0; k < g->nz; k++) {
-                            const int idx = index3(g, i, j, k);
-                            const int m = g->map[idx];
-                            const char sym = (m < 0 || m >= (int)g->bound.size()) ? '.' : g->bound[m].sym;
-                            if (c == '*' || sym == c) {
-                                if (!ok) return fd_fail(g, OMDG_EINVAL, "conversion error: " + val);
-                                if (!(a[idx] == dv) || std::signbit(a[idx]) != std::signbit(dv)) changed = true;
-                                a[idx] = dv;
-                            }
-                        }
+                for (int m = 0; m <= nsym; m++)
+                    if (c == '*' || (m < nsym ? g->bound[m].sym : '.') == c) takes[m] = 1;
+            for (int idx = 0; idx < g->dim; idx++) {
+                const int m = g->map[idx];
+                if (!takes[m < 0 || m >= nsym ? nsym : m]) continue;
+                if (!ok) return fd_fail(g, OMDG_EINVAL, "conversion error: " + val);
+                if (!(a[idx] == dv) || std::signbit(a[idx]) != std::signbit(dv)) changed = true;
+                a[idx] = dv;
+            }
         }
     }
     return OMDG_OK;
 }
 
-// assignments to S: the device S is zero after every solve, so any value
-// written since makes the host image the one to upload
-static int assign_source(FDGrid* g, std::string& str) {
+static int assign_source(FDGrid* g, std::string& str, int& until, bool standing = false) {
     bool changed = false;
-    const int rc = assign_array(g, g->hS, str, changed);
+    const int rc = assign_array(g, g->hS, str, changed, until, standing);
     if (changed) g->dirty_S = g->s_any = true;
     return rc;
 }
 
-int fd_sync_data(FDGrid* g) {
+// The kept strings of the current step.  Applying the same tokens again gives
+// the same values (each writes constants, in order), so conductivity and
+// capacity are left alone until a token drops out or the caller assigns; and
+// a source pattern that the same tokens make from the cleared S stays on the
+// device, where the solve reads it again (S is zero to the caller between
+// steps, fdtd.cpp:665).  A layered 96 x 80 x 72 sample with two materials and
+// a source spent 5.7 ms a step in applying them; ten steps and a read-back
+// went from 62 ms to 0.63.
+int fd_sync_data(FDGrid* g, bool again) {
+    using K = FDGrid::Kept;
     bool ccon = false, ccap = false;
-    int rc = assign_source(g, g->str_src);
-    if (!rc) rc = assign_array(g, g->hcon, g->str_con, ccon);
-    if (!rc) rc = assign_array(g, g->hcap, g->str_cap, ccap);
+    int rc = OMDG_OK;
+    const auto stands = [&](const K& k) { return !again && k.applied && g->step <= k.until; };
+    if (!(stands(g->k_src) && g->k_src.pruned && !g->s_any)) {
+        // S as the last assignment left it (not yet solved with), or cleared
+        const bool now = stands(g->k_src) && !g->k_src.pruned;
+        const bool clean = !g->s_any || (now && g->k_src.clean);
+        rc = assign_source(g, g->str_src, g->k_src.until, now);
+        if (g->s_live) g->dirty_S = true;  // replaces the pattern that stayed on the device
+        g->s_live = false;
+        g->k_src.applied = g->k_src.pruned = !rc && clean;
+    }
+    const auto sync = [&](K& k, std::vector<double>& a, std::string& str, bool& changed) {
+        if (rc || (stands(k) && k.pruned)) return;
+        rc = assign_array(g, a, str, changed, k.until, stands(k));
+        k.applied = k.pruned = !rc;
+    };
+    sync(g->k_con, g->hcon, g->str_con, ccon);
+    sync(g->k_cap, g->hcap, g->str_cap, ccap);
     g->dirty_con |= ccon;
     g->dirty_cap |= ccap;
     return rc;
@@ -350,7 +414,15 @@ int fd_upload(FDGrid* g, cudaStream_t s) {
             e = cudaGetLastError();
         }
     }
-    if (e == cudaSuccess && g->dirty_cap) e = cudaMemcpyAsync(g->dcap, g->hcap.data(), b, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess && g->dirty_cap) {
+        e = cudaMemcpyAsync(g->dcap, g->hcap.data(), b, cudaMemcpyHostToDevice, s);
+        g->rcap_ok = false;
+    }
+    if (e == cudaSuccess && !g->rcap_ok) {
+        k_fd_rcp<<<grid_for(g->dim, FD_BLOCK), FD_BLOCK, 0, s>>>(g->dim, g->dcap, g->drcap);
+        e = cudaGetLastError();
+        g->rcap_ok = e == cudaSuccess;
+    }
     if (e != cudaSuccess) return fd_fail(g, OMDG_ECUDA, std::string("fdtd upload: ") + cudaGetErrorString(e));
     g->dirty_S = g->dirty_con = g->dirty_cap = false;
     return OMDG_OK;
@@ -413,6 +485,7 @@ int omdg_fdtd_create(omdg_fdtd** out, int device, int nx, int ny, int nz, const 
     if (e == cudaSuccess) e = cudaMalloc(&g->dcon, b8);
     if (e == cudaSuccess) e = cudaMalloc(&g->dK, 3 * b8);
     if (e == cudaSuccess) e = cudaMalloc(&g->dcap, b8);
+    if (e == cudaSuccess) e = cudaMalloc(&g->drcap, b8);
     if (e == cudaSuccess) e = cudaMalloc(&g->dmap, sizeof(int) * g->dim);
     for (int k = 0; k < 2 && e == cudaSuccess; k++) e = cudaMalloc(&g->dmask[k], g->dim);
     if (e != cudaSuccess) return fd_fail(g, OMDG_ENOMEM, std::string("fdtd allocation: ") + cudaGetErrorString(e));
@@ -443,6 +516,7 @@ int omdg_fdtd_destroy(omdg_fdtd* g) {
     cudaFree(g->dcon);
     cudaFree(g->dK);
     cudaFree(g->dcap);
+    cudaFree(g->drcap);
     cudaFree(g->dmap);
     if (g->own_stream) cudaStreamDestroy(g->stream);
     delete g;
@@ -474,7 +548,8 @@ int omdg_fdtd_assign(omdg_fdtd* g, int which, const char* str) {
     if (which == 0) {
         if ((rc = fd_download_A(g))) return rc;
         bool changed = false;
-        if ((rc = assign_array(g, g->hA, s, changed))) return rc;
+        int until;
+        if ((rc = assign_array(g, g->hA, s, changed, until))) return rc;
         cudaError_t e = cudaMemcpyAsync(g->dA[g->cur], g->hA.data(), sizeof(double) * g->dim,
                                         cudaMemcpyHostToDevice, g->stream);
         if (e != cudaSuccess) return fd_fail(g, OMDG_ECUDA, std::string("fdtd: ") + cudaGetErrorString(e));
@@ -484,9 +559,17 @@ int omdg_fdtd_assign(omdg_fdtd* g, int which, const char* str) {
     // apply a copy of it now (fdtd.hpp:126-133)
     std::string& kept = which == 1 ? g->str_src : (which == 2 ? g->str_con : g->str_cap);
     kept = str;
-    if (which == 1) return assign_source(g, s);
+    FDGrid::Kept& k = which == 1 ? g->k_src : (which == 2 ? g->k_con : g->k_cap);
+    k.applied = k.pruned = false;
     bool changed = false;
-    rc = assign_array(g, which == 2 ? g->hcon : g->hcap, s, changed);
+    if (which == 1) {
+        k.clean = !g->s_any;
+        rc = assign_source(g, s, k.until);
+    } else {
+        rc = assign_array(g, which == 2 ? g->hcon : g->hcap, s, changed, k.until);
+    }
+    k.applied = !rc;
+    if (which == 1) return rc;
     if (which == 2) g->dirty_con |= changed;
     else g->dirty_cap |= changed;
     return rc;
@@ -502,9 +585,10 @@ int omdg_fdtd_step(omdg_fdtd* g, int n) {
         if (!rc) rc = fd_upload(g, g->stream);
         if (!rc) rc = fd_solve(g, g->stream);
         if (rc) return rc;
-        if (g->s_any) {  // Solve clears S (fdtd.cpp:665), on the device too
+        if (g->s_any) {  // Solve clears S (fdtd.cpp:665); the device keeps the pattern for fd_sync_data
             std::fill(g->hS.begin(), g->hS.end(), 0.0);
             g->s_any = false;
+            g->s_live = true;
         }
         g->step += 1;
     }

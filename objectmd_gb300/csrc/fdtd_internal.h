@@ -28,14 +28,14 @@ enum : uint8_t { FD_R = 1, FD_L = 2, FD_B = 4, FD_T = 8, FD_N = 16, FD_F = 32 };
 // character outside the symbol map) and mask the exchange directions.
 struct FDDev {
     int nx, ny, nz, dim;
-    double dt, h2inv;
+    double dt, h2inv2;  // time step; 2 / h^2
     const int* map;
     const uint8_t* mask;
     const double* K;  // face conductances: x faces [0, dim), y faces [dim, 2 dim), z faces [2 dim, 3 dim)
     const double* cap;
-    double* S;
+    const double* rcap;  // 1 / cap, or NaN where the step divides; null: it divides everywhere
+    double* S;  // not cleared by the solve (coupled: the kept strings' fixed pattern)
     double* E;
-    int keep_S;  // coupled: S is the kept strings' fixed pattern, not cleared by the solve
     // coupled to the atoms (a replayed step graph): the mask chosen on the
     // device from the solve count, and the step skipped while the model is
     // not active; null for host-driven steps
@@ -62,9 +62,20 @@ struct FDGrid {
     std::vector<double> hA, hS, hcon, hcap; // host images of the assigned arrays
     bool dirty_S = true, dirty_con = true, dirty_cap = true;  // the host image changed since the last upload
     bool s_any = false;                  // hS holds a non-zero value (cleared after each solve)
+    bool s_live = false;                 // dS holds the last solve's pattern while hS is cleared
+    // a kept string's last application stands until a token drops out (the
+    // step is past `until`) or the caller assigns
+    struct Kept {
+        bool applied = false;  // the array holds the string's assignments
+        bool pruned = false;   // the string was pruned by a step since
+        bool clean = false;    // source: S was clear before the assignment
+        int until = 0;
+    } k_src, k_con, k_cap;
     double* dA[2] = {nullptr, nullptr};
     int cur = 0;                         // dA[cur] holds the cell vector
     double *dS = nullptr, *dE = nullptr, *dcon = nullptr, *dcap = nullptr;
+    double* drcap = nullptr;             // 1 / cap
+    bool rcap_ok = false;                // drcap belongs to dcap
     double* dK = nullptr;                // face conductances from dcon (3 x dim), refreshed with it
     int* dmap = nullptr;
     uint8_t* dmask[2] = {nullptr, nullptr};  // first, later
@@ -80,8 +91,9 @@ int fd_solve(FDGrid* g, cudaStream_t s);
 // coupling left it), writes dA[0].
 cudaError_t fd_solve_coupled(const FDDev& p, const double* T, double* A, cudaStream_t s);
 // sync_data (fdtd.cpp:599-603): the kept source, conductivity and capacity
-// strings re-applied at the current step.
-int fd_sync_data(FDGrid* g);
+// strings at the current step (again: every string applied, whatever the
+// last step left).
+int fd_sync_data(FDGrid* g, bool again = false);
 FDDev fd_dev(const FDGrid* g);
 
 }  // namespace omdg

@@ -590,7 +590,7 @@ int ttm_pre(Context* c) {
         q.fd.mask_later = fg->dmask[1];
         q.fd.solves = t.dev_ctr;
         q.fd.active = t.dev_ctr + 1;
-        q.fd.keep_S = 1;  // the unranged source tokens would assign the same pattern every step
+        q.fd.rcap = nullptr;  // the model writes the capacities every step
         q.A = fg->dA[0];
         q.T = fg->dA[1];
         q.cap = fg->dcap;
@@ -762,7 +762,7 @@ int omdg_set_ttm_grid(omdg_ctx* c, omdg_fdtd* grid, const double* origin) {
     ttm_grid_detach(c, t);
     // the kept strings once more (they are unranged: every later step would
     // apply the same values), then their images on the device
-    int rc = fd_sync_data(grid);
+    int rc = fd_sync_data(grid, true);
     if (!rc) rc = fd_upload(grid, grid->stream);
     if (rc) return set_error(c, rc, grid->err);
     cudaError_t e = cudaSuccess;
@@ -791,6 +791,7 @@ int omdg_set_ttm_grid(omdg_ctx* c, omdg_fdtd* grid, const double* origin) {
     for (int d = 0; d < 3; d++) t.org[d] = origin[d];
     t.grid = grid;
     grid->coupled = true;
+    grid->rcap_ok = false;
     invalidate_graph(c);
     return OMDG_OK;
 }

@@ -122,3 +122,69 @@ def test_errors_are_reported(omdg_lib):
     with pytest.raises(omdg_lib.OMDGError) as ei:
         omdg_lib.FDTD(4, 4, 1, "a pppp", "a" * 15)
     assert "map string count" in str(ei.value)
+
+
+# The kept strings stand from step to step until a token drops out or the
+# caller assigns again, the source pattern stays on the device in between, and
+# the division by the capacity takes its reciprocal where that rounds
+# correctly.  Every step against the oracle, bit for bit: tokens that drop out
+# and uncover an earlier one, single-step tokens, assignments and reads
+# between steps, capacities the reciprocal does not take.
+@pytest.mark.parametrize("dims,cap", [((9, 7, 5), "* 3.0"), ((33, 5, 1), "a 0.7 b 1e-280:0:6"),
+                                      ((16, 16, 3), "* 1.9999999999999998 b 1e200"), ((5, 4, 4), "a -2.0 b 7:0:3")])
+def test_strings_that_stand_equal_the_oracle(omdg_lib, dims, cap):
+    nx, ny, nz = dims
+    dim = nx * ny * (1 if nz <= 2 else nz)
+    rng = np.random.default_rng(dim)
+    cmap = "".join("ab"[int(q)] for q in rng.integers(0, 2, dim))
+    flags = "pppppp" if nz > 2 else "pppp"
+    symbol = "a %s b %s" % (flags, flags)
+    ref = fo.Grid(nx, ny, nz, symbol, cmap)
+    con = "a 0.25 b 0.5:0:5 @ 1,1,0=2:0:3 @ 2,1,0=3:4"
+    src = "a 5:0:7 @ 1,2,0=9:2:4 b 1.5"
+    with omdg_lib.FDTD(nx, ny, nz, symbol, cmap) as g:
+        for o in (ref, g):
+            o.set_spacestep(1.0)
+            o.set_timestep(0.01)
+            o.set_cell("* 300 @ 0,0,0,2,2,0=900")
+            o.set_conductivity(con)
+            o.set_capacity(cap)
+            o.set_source(src)
+        for k in range(14):
+            if k == 9:  # a pattern that stood is replaced, and one is added to
+                for o in (ref, g):
+                    o.set_source("b 2")
+                    o.set_source("@ 0,0,0=4")
+            if k == 11:
+                for o in (ref, g):
+                    o.set_source("a 0")
+                    o.set_conductivity("* 1")
+            ext = np.zeros(dim)
+            if k in (3, 10):
+                ext[dim // 2] = -3.0
+            ref.E = ext.copy()
+            g.set_ext(ext)
+            ref.run_step()
+            g.step(1)
+            assert np.array_equal(g.vector(), ref.A, equal_nan=True), k
+            assert np.array_equal(g.get(g.SOURCE), ref.S), k
+            assert np.array_equal(g.get(g.CONDUCTIVITY), ref.con), k
+            assert np.array_equal(g.get(g.CAPACITY), ref.cap), k
+
+
+# Quotients by the reciprocal against the FP64 division, over mantissas and
+# exponents: one cell per pair, no exchange, A = T + E dt / cap with T = 0.
+def test_quotients_equal_the_division(omdg_lib):
+    rng = np.random.default_rng(3)
+    n = 64
+    e = rng.uniform(1.0, 2.0, n * n) * 2.0 ** rng.integers(-40, 40, n * n) * rng.choice([-1.0, 1.0], n * n)
+    cap = rng.uniform(1.0, 2.0, n)
+    cap[:4] = [1.0, 2.0 - 2.0 ** -52, 1.0 + 2.0 ** -52, 2.0 - 2.0 ** -51]
+    cap *= 2.0 ** rng.integers(-30, 30, n)
+    with omdg_lib.FDTD(n, n, 1, "a ----", "a" * (n * n)) as g:
+        g.set_timestep(1.0)
+        g.set_cell("* 0")
+        g.set_capacity(" ".join("@ 0,%d,0,%d,%d,0=%.17g" % (j, n - 1, j, cap[j]) for j in range(n)))
+        g.set_ext(e)
+        g.step(1)
+        assert np.array_equal(g.vector(), e / np.repeat(cap, n))
