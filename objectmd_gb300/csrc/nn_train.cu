@@ -9,11 +9,12 @@
 //   2. k_nn_conf_energy  per configuration: dE = (sum E_i - E_ref) / N
 //   3. k_nn_force      F_k = sum_s (J_ks^T u_k - J_(j,rev)^T u_j), force residual
 //   4. k_nn_vvec       v_i = dL/du_i = sum_s J_is (rho_i - rho_j)
-//   5. k_nn_atom_grad  per-atom vectors of the energy and force gradients
-//                      (the force term differentiates u_i . v_i through the
-//                      network: forward-mode tangent, then reverse mode)
-//   6. k_nn_wgrad_*    outer-product sums over atoms, fixed order (deterministic)
-//   7. k_nn_adam       Adam update of the FP32 parameters
+//   5. k_nn_grad       per chunk of atoms the energy and force gradients (the
+//                      force term differentiates u_i . v_i through the network:
+//                      forward-mode tangent, then reverse mode) and their
+//                      outer-product sums, fixed order (deterministic)
+//   6. k_nn_step       sums of the chunks and the loss, Adam update of the
+//                      FP32 parameters
 // Loss: L = wE mean_c (dE_c)^2 + wF mean_(k,a) (F_ka - F_ka^ref)^2.
 #include <algorithm>
 #include <cmath>
@@ -23,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "device_common.cuh"
 #include "nn_desc.cuh"
 #include "tc_common.cuh"
 
@@ -68,11 +70,13 @@ struct omdg_nn {
     float* d_ew = nullptr;       // per configuration dL/dE_i
     float* d_lossE = nullptr;    // per batch configuration
     float* d_lossF = nullptr;    // per batch atom
-    float* d_vecs = nullptr;     // per batch atom: 7 x 64 vectors + e
+    float* d_acts = nullptr;     // per batch chunk: the forward pass's activations (NT_ACTS x 32 atoms)
     float* d_partial = nullptr;  // per chunk x NN_PARAMS
-    double* d_loss = nullptr;
+    double* d_loss = nullptr;    // per batch of the queued epochs
+    long cap_loss = 0;
     int* d_list = nullptr;       // atom order of the epoch
-    int* d_clist = nullptr;      // configuration order of the epoch
+    int* d_clist = nullptr;      // configuration order of the queued epochs, then where each one's atoms begin
+    long cap_clist = 0;
     unsigned* d_status = nullptr;
     long cap_batch_atoms = 0;
     long adam_t = 0;
@@ -81,8 +85,7 @@ struct omdg_nn {
 
 namespace omdg {
 
-constexpr int NN_VEC_STRIDE = 7 * NN_H + 1;  // zeta1 d1 zeta2 d2 a1 da1 w3g | e
-constexpr int NN_CHUNK = 32;                  // atoms per gradient partial
+constexpr int NN_CHUNK = 32;  // atoms per block and gradient partial
 
 // ------------------------------------------------------------------ dataset kernels
 __device__ __forceinline__ double nn_min_image(double d, double L) { return d - L * rint(d / L); }
@@ -210,50 +213,210 @@ __global__ void k_nn_normalize(NNDescParams p, long n, const float* __restrict__
 }
 
 // ------------------------------------------------------------------ training kernels
-// Parameters staged in shared memory (FP32).
-__device__ __forceinline__ void load_params(const float* __restrict__ w, float* s) {
-    for (int k = threadIdx.x; k < NN_PARAMS; k += blockDim.x) s[k] = w[k];
-    __syncthreads();
+// A block takes NN_CHUNK = 32 atoms.  Weights and the atoms' vectors sit in
+// shared memory, a vector as one row of 32 atoms per feature (stride 36), and
+// the layers are register-tiled products: a thread holds four atoms by two
+// of 64 features.  Every output
+// sums its terms in the order of the feature index, in FP32.  Bound by the
+// shared loads' latency and wavefronts at two blocks a SM (LSU 50 %).  For a
+// batch of 16 x 512 atoms a step's kernels take 17 (forward), 7 (forces), 6
+// (dL/du), 25 (gradient) and 12 us (sums and Adam) under ncu, a step 82 us in
+// the loop; one thread per atom, as it was, ran 64 blocks of 128 threads with
+// 64-wide vectors in local memory and took 348 us a step.
+constexpr int NT_THREADS = 256;
+constexpr int NT_TO = NT_THREADS / 8;   // threads along the features; eight along the atoms (four each)
+constexpr int NT_R = NN_H / NT_TO;      // features of 64 a thread
+constexpr int NT_AS = NN_CHUNK + 4;     // stride of a feature row
+constexpr int NT_W1S = NN_DESC + 4;     // stride of a row of W1 (64 x 32)
+constexpr int NT_W2S = NN_H + 4;        // stride of a row of W2 (64 x 64)
+constexpr int NT_ACTS = 3 * NN_H;       // features kept from the forward pass: a1, a2, W2^T d2
+constexpr int NT_VEC = 4 * NN_H;        // b1, b2, w3, b3
+constexpr int NT_W_FLOATS = NN_H * NT_W1S + NN_H * NT_W2S + NT_VEC;
+constexpr int NT_FWD_FLOATS = NT_W_FLOATS + (NN_DESC + 3 * NN_H) * NT_AS;
+constexpr int NT_GRAD_FLOATS = NT_W_FLOATS + (2 * NN_DESC + 7 * NN_H) * NT_AS + NN_CHUNK;
+
+struct NTWeights {
+    float *W1, *W2, *b1, *b2, *w3, *b3;
+};
+
+__device__ __forceinline__ NTWeights nt_load_weights(const float* __restrict__ w, float* s) {
+    NTWeights q;
+    q.W1 = s;
+    q.W2 = q.W1 + NN_H * NT_W1S;
+    q.b1 = q.W2 + NN_H * NT_W2S;
+    q.b2 = q.b1 + NN_H;
+    q.w3 = q.b2 + NN_H;
+    q.b3 = q.w3 + NN_H;
+    const float4* w1 = reinterpret_cast<const float4*>(w + NN_OFF_W1);
+    const float4* w2 = reinterpret_cast<const float4*>(w + NN_OFF_W2);
+#pragma unroll
+    for (int c = 0; c < NN_H * NN_DESC / 4 / NT_THREADS; c++) {
+        const int k = c * NT_THREADS + threadIdx.x;
+        *reinterpret_cast<float4*>(q.W1 + (k / (NN_DESC / 4)) * NT_W1S + 4 * (k % (NN_DESC / 4))) = __ldg(w1 + k);
+    }
+#pragma unroll
+    for (int c = 0; c < NN_H * NN_H / 4 / NT_THREADS; c++) {
+        const int k = c * NT_THREADS + threadIdx.x;
+        *reinterpret_cast<float4*>(q.W2 + (k / (NN_H / 4)) * NT_W2S + 4 * (k % (NN_H / 4))) = __ldg(w2 + k);
+    }
+    for (int k = threadIdx.x; k < NN_H; k += NT_THREADS) {
+        q.b1[k] = __ldg(w + NN_OFF_B1 + k);
+        q.b2[k] = __ldg(w + NN_OFF_B2 + k);
+        q.w3[k] = __ldg(w + NN_OFF_W3 + k);
+    }
+    if (threadIdx.x == 0) q.b3[0] = __ldg(w + NN_OFF_B3);
+    return q;
 }
 
-// E_i and u_i (raw descriptor units) for the atoms list[a0 .. a0 + na).
-__global__ void __launch_bounds__(128) k_nn_fwd(const float* __restrict__ w, const float* __restrict__ Gt,
-                                                NNDescParams p, const int* __restrict__ list, int a0, int na,
-                                                float* __restrict__ E, float* __restrict__ U) {
-    extern __shared__ float sw[];
-    load_params(w, sw);
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= na) return;
-    const int atom = list[a0 + t];
-    const float* W1 = sw + NN_OFF_W1;
-    const float* W2 = sw + NN_OFF_W2;
-    float g[NN_DESC];
-    for (int d = 0; d < NN_DESC; d++) g[d] = Gt[(size_t)atom * NN_DESC + d];
-    float a1[NN_H];
-    for (int j = 0; j < NN_H; j++) {
-        float z = sw[NN_OFF_B1 + j];
-        for (int d = 0; d < NN_DESC; d++) z = fmaf(W1[j * NN_DESC + d], g[d], z);
-        a1[j] = tanhf(z);
+// acc[o][a] += sum_k W[row o][k] X[k][a], rows to + NT_TO o, atoms 4 ta + a
+template <int K, int WS>
+__device__ __forceinline__ void nt_rows(const float* W, const float* X, int to, int ta, float (&acc)[NT_R][4]) {
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+        float4 w[NT_R];
+#pragma unroll
+        for (int o = 0; o < NT_R; o++) w[o] = *reinterpret_cast<const float4*>(W + (to + NT_TO * o) * WS + k);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float4 x = *reinterpret_cast<const float4*>(X + (k + q) * NT_AS + 4 * ta);
+#pragma unroll
+            for (int o = 0; o < NT_R; o++) {
+                const float v = q == 0 ? w[o].x : (q == 1 ? w[o].y : (q == 2 ? w[o].z : w[o].w));
+                acc[o][0] = fmaf(v, x.x, acc[o][0]);
+                acc[o][1] = fmaf(v, x.y, acc[o][1]);
+                acc[o][2] = fmaf(v, x.z, acc[o][2]);
+                acc[o][3] = fmaf(v, x.w, acc[o][3]);
+            }
+        }
     }
-    float d2[NN_H];
-    float e = sw[NN_OFF_B3];
-    for (int o = 0; o < NN_H; o++) {
-        float z = sw[NN_OFF_B2 + o];
-        for (int j = 0; j < NN_H; j++) z = fmaf(W2[o * NN_H + j], a1[j], z);
-        const float a2 = tanhf(z);
-        e = fmaf(sw[NN_OFF_W3 + o], a2, e);
-        d2[o] = sw[NN_OFF_W3 + o] * (1.f - a2 * a2);
+}
+
+// acc[c][a] += sum_k X[k][a] W[k][NC to + c]
+template <int NC, int WS>
+__device__ __forceinline__ void nt_cols(const float* W, const float* X, int to, int ta, float (&acc)[NC][4]) {
+#pragma unroll 4
+    for (int k = 0; k < NN_H; k++) {
+        const float4 x = *reinterpret_cast<const float4*>(X + k * NT_AS + 4 * ta);
+        float v[NC];
+        if (NC == 2) {
+            const float2 w = *reinterpret_cast<const float2*>(W + k * WS + 2 * to);
+            v[0] = w.x, v[NC - 1] = w.y;
+        } else {
+            v[0] = W[k * WS + to];
+        }
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            acc[c][0] = fmaf(v[c], x.x, acc[c][0]);
+            acc[c][1] = fmaf(v[c], x.y, acc[c][1]);
+            acc[c][2] = fmaf(v[c], x.z, acc[c][2]);
+            acc[c][3] = fmaf(v[c], x.w, acc[c][3]);
+        }
     }
-    float u[NN_DESC];
-    for (int d = 0; d < NN_DESC; d++) u[d] = 0.f;
-    for (int j = 0; j < NN_H; j++) {
-        float s = 0.f;
-        for (int o = 0; o < NN_H; o++) s = fmaf(d2[o], W2[o * NN_H + j], s);
-        const float d1 = s * (1.f - a1[j] * a1[j]);
-        for (int d = 0; d < NN_DESC; d++) u[d] = fmaf(d1, W1[j * NN_DESC + d], u[d]);
+}
+
+template <int N>
+__device__ __forceinline__ void nt_zero(float (&acc)[N][4]) {
+#pragma unroll
+    for (int o = 0; o < N; o++) acc[o][0] = acc[o][1] = acc[o][2] = acc[o][3] = 0.f;
+}
+
+__device__ __forceinline__ float4& nt_at(float* X, int row, int ta) {
+    return *reinterpret_cast<float4*>(X + row * NT_AS + 4 * ta);
+}
+
+// 32-wide rows of the chunk's atoms into feature rows; absent atoms give zeros
+template <bool SCALE>
+__device__ __forceinline__ void nt_load_rows(const float* __restrict__ src, const float* scale,
+                                             const int* __restrict__ list, int cnt, float* X) {
+    const int d = threadIdx.x & 31;
+    for (int a = threadIdx.x >> 5; a < NN_CHUNK; a += NT_THREADS / 32) {
+        float v = a < cnt ? src[(size_t)__ldg(list + a) * NN_DESC + d] : 0.f;
+        if (SCALE) v *= scale[d];
+        X[d * NT_AS + a] = v;
     }
-    E[atom] = e;
-    for (int d = 0; d < NN_DESC; d++) U[(size_t)atom * NN_DESC + d] = u[d] * p.isig[d];
+}
+
+// E_i and u_i (raw descriptor units) for the atoms list[a0 .. a0 + na); with
+// acts, the activations the gradient needs; with eatom, the per-atom energy
+// residuals (dL/dE_i) and their loss terms.
+__global__ void __launch_bounds__(NT_THREADS) k_nn_fwd(const float* __restrict__ w, const float* __restrict__ Gt,
+                                                       NNDescParams p, const int* __restrict__ list, int a0, int na,
+                                                       float* __restrict__ E, float* __restrict__ U,
+                                                       float* __restrict__ acts, const float* __restrict__ eatom,
+                                                       float wE, float* __restrict__ ewa,
+                                                       float* __restrict__ lossE) {
+    extern __shared__ __align__(16) float sm[];
+    const NTWeights q = nt_load_weights(w, sm);
+    float* G = sm + NT_W_FLOATS;
+    float* A1 = G + NN_DESC * NT_AS;
+    float* D2 = A1 + NN_H * NT_AS;
+    float* A2 = D2 + NN_H * NT_AS;
+    const int t0 = blockIdx.x * NN_CHUNK, cnt = min(NN_CHUNK, na - t0);
+    list += a0 + t0;
+    nt_load_rows<false>(Gt, nullptr, list, cnt, G);
+    __syncthreads();
+    const int ta = threadIdx.x & 7, to = threadIdx.x >> 3;
+    float* act = acts ? acts + (size_t)blockIdx.x * NT_ACTS * NN_CHUNK + 4 * ta : nullptr;
+    float z[NT_R][4];
+#pragma unroll
+    for (int o = 0; o < NT_R; o++) z[o][0] = z[o][1] = z[o][2] = z[o][3] = q.b1[to + NT_TO * o];
+    nt_rows<NN_DESC, NT_W1S>(q.W1, G, to, ta, z);
+#pragma unroll
+    for (int o = 0; o < NT_R; o++) {
+        const float4 v = make_float4(tanhf(z[o][0]), tanhf(z[o][1]), tanhf(z[o][2]), tanhf(z[o][3]));
+        nt_at(A1, to + NT_TO * o, ta) = v;
+        if (act) *reinterpret_cast<float4*>(act + (to + NT_TO * o) * NN_CHUNK) = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int o = 0; o < NT_R; o++) z[o][0] = z[o][1] = z[o][2] = z[o][3] = q.b2[to + NT_TO * o];
+    nt_rows<NN_H, NT_W2S>(q.W2, A1, to, ta, z);
+#pragma unroll
+    for (int o = 0; o < NT_R; o++) {
+        const float4 v = make_float4(tanhf(z[o][0]), tanhf(z[o][1]), tanhf(z[o][2]), tanhf(z[o][3]));
+        const float w3 = q.w3[to + NT_TO * o];
+        nt_at(A2, to + NT_TO * o, ta) = v;
+        nt_at(D2, to + NT_TO * o, ta) = make_float4(w3 * (1.f - v.x * v.x), w3 * (1.f - v.y * v.y),
+                                                 w3 * (1.f - v.z * v.z), w3 * (1.f - v.w * v.w));
+        if (act) *reinterpret_cast<float4*>(act + (NN_H + to + NT_TO * o) * NN_CHUNK) = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < cnt) {
+        float e = q.b3[0];
+#pragma unroll 8
+        for (int o = 0; o < NN_H; o++) e = fmaf(q.w3[o], A2[o * NT_AS + threadIdx.x], e);
+        const int atom = list[threadIdx.x];
+        E[atom] = e;
+        if (eatom) {
+            const float r = e - eatom[atom];
+            ewa[atom] = 2.f * wE * r / na;
+            lossE[t0 + threadIdx.x] = wE * r * r / na;
+        }
+    }
+    nt_zero(z);
+    nt_cols<NT_R, NT_W2S>(q.W2, D2, to, ta, z);
+    __syncthreads();  // D2 is done: it takes d1
+#pragma unroll
+    for (int c = 0; c < NT_R; c++) {
+        const int j = NT_R * to + c;
+        const float4 a1 = nt_at(A1, j, ta);
+        if (act)
+            *reinterpret_cast<float4*>(act + (2 * NN_H + j) * NN_CHUNK) = make_float4(z[c][0], z[c][1], z[c][2], z[c][3]);
+        nt_at(D2, j, ta) = make_float4(z[c][0] * (1.f - a1.x * a1.x), z[c][1] * (1.f - a1.y * a1.y),
+                                       z[c][2] * (1.f - a1.z * a1.z), z[c][3] * (1.f - a1.w * a1.w));
+    }
+    __syncthreads();
+    float u[NT_R / 2][4];
+    nt_zero(u);
+    nt_cols<NT_R / 2, NT_W1S>(q.W1, D2, to, ta, u);
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+        if (4 * ta + a < cnt)
+#pragma unroll
+            for (int c = 0; c < NT_R / 2; c++) {
+                const int d = NT_R / 2 * to + c;
+                U[(size_t)list[4 * ta + a] * NN_DESC + d] = u[c][a] * p.isig[d];
+            }
 }
 
 // One block per batch configuration: energy residual and its loss term.
@@ -279,43 +442,36 @@ __global__ void k_nn_conf_energy(const int* __restrict__ clist, int c0, int nb, 
     }
 }
 
-// Per-atom energy residuals (per-atom energy loss): dL/dE_i and the loss terms.
-__global__ void k_nn_atom_energy(const int* __restrict__ list, int a0, int na, const float* __restrict__ E,
-                                 const float* __restrict__ eatom, float wE, float* __restrict__ ewa,
-                                 float* __restrict__ lossE) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= na) return;
-    const int i = list[a0 + t];
-    const float r = E[i] - eatom[i];
-    ewa[i] = 2.f * wE * r / na;
-    lossE[t] = wE * r * r / na;
-}
-
 // Forces from J and u; the force residual, rho = dL/dF and its loss term.
-__global__ void k_nn_force(const int* __restrict__ list, int a0, int na, const int* __restrict__ slot_start,
-                           const int* __restrict__ slot_j, const int* __restrict__ rev, const float* __restrict__ J,
-                           const float* __restrict__ U, const float* __restrict__ fref, float wF_over_ncomp,
-                           const float* __restrict__ fw, const int* __restrict__ atom_conf, float* __restrict__ F,
-                           float* __restrict__ rho, float* __restrict__ lossF) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per atom, a lane per descriptor: the Jacobian's rows (32 floats)
+// and u are read as whole lines, and the descriptors sum in an xor tree.
+__global__ void __launch_bounds__(256) k_nn_force(const int* __restrict__ list, int a0, int na,
+                                                  const int* __restrict__ slot_start, const int* __restrict__ slot_j,
+                                                  const int* __restrict__ rev, const float* __restrict__ J,
+                                                  const float* __restrict__ U, const float* __restrict__ fref,
+                                                  float wF_over_ncomp, const float* __restrict__ fw,
+                                                  const int* __restrict__ atom_conf, float* __restrict__ F,
+                                                  float* __restrict__ rho, float* __restrict__ lossF) {
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (t >= na) return;
     const int k = list[a0 + t];
-    if (fref) wF_over_ncomp *= fw[atom_conf[k]];
-    float uk[NN_DESC];
-    for (int d = 0; d < NN_DESC; d++) uk[d] = U[(size_t)k * NN_DESC + d];
+    const int s0 = slot_start[k], s1 = slot_start[k + 1];
+    const float uk = U[(size_t)k * NN_DESC + lane];
     float f[3] = {0.f, 0.f, 0.f};
-    for (int s = slot_start[k]; s < slot_start[k + 1]; s++) {
-        const int j = slot_j[s];
-        const float* Js = J + (size_t)s * 3 * NN_DESC;
-        const float* Jr = J + (size_t)rev[s] * 3 * NN_DESC;
-        const float* uj = U + (size_t)j * NN_DESC;
-        for (int c = 0; c < 3; c++) {
-            float acc = 0.f;
-            for (int d = 0; d < NN_DESC; d++) acc = fmaf(Js[c * NN_DESC + d], uk[d], acc);
-            for (int d = 0; d < NN_DESC; d++) acc = fmaf(-Jr[c * NN_DESC + d], uj[d], acc);
-            f[c] += acc;
-        }
+#pragma unroll 2
+    for (int s = s0; s < s1; s++) {
+        const float* Js = J + (size_t)s * 3 * NN_DESC + lane;
+        const float* Jr = J + (size_t)rev[s] * 3 * NN_DESC + lane;
+        const float uj = U[(size_t)slot_j[s] * NN_DESC + lane];
+#pragma unroll
+        for (int c = 0; c < 3; c++) f[c] = fmaf(-Jr[c * NN_DESC], uj, fmaf(Js[c * NN_DESC], uk, f[c]));
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; c++) f[c] += __shfl_xor_sync(0xffffffffu, f[c], o);
+    if (lane != 0) return;
+    if (fref) wF_over_ncomp *= fw[atom_conf[k]];
     float l = 0.f;
     for (int c = 0; c < 3; c++) {
         F[3 * (size_t)k + c] = f[c];
@@ -328,181 +484,257 @@ __global__ void k_nn_force(const int* __restrict__ list, int a0, int na, const i
     if (fref) lossF[t] = wF_over_ncomp * l;
 }
 
-// v_i = dL/du_i = sum_s J_is (rho_i - rho_j)
-__global__ void k_nn_vvec(const int* __restrict__ list, int a0, int na, const int* __restrict__ slot_start,
-                          const int* __restrict__ slot_j, const float* __restrict__ J, const float* __restrict__ rho,
-                          float* __restrict__ V) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// v_i = dL/du_i = sum_s J_is (rho_i - rho_j); a warp per atom, a lane per descriptor
+__global__ void __launch_bounds__(256) k_nn_vvec(const int* __restrict__ list, int a0, int na,
+                                                 const int* __restrict__ slot_start, const int* __restrict__ slot_j,
+                                                 const float* __restrict__ J, const float* __restrict__ rho,
+                                                 float* __restrict__ V) {
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (t >= na) return;
     const int i = list[a0 + t];
-    float v[NN_DESC];
-    for (int d = 0; d < NN_DESC; d++) v[d] = 0.f;
+    const int s0 = slot_start[i], s1 = slot_start[i + 1];
+    float v = 0.f;
     const float ri[3] = {rho[3 * (size_t)i], rho[3 * (size_t)i + 1], rho[3 * (size_t)i + 2]};
-    for (int s = slot_start[i]; s < slot_start[i + 1]; s++) {
+#pragma unroll 2
+    for (int s = s0; s < s1; s++) {
         const int j = slot_j[s];
-        const float* Js = J + (size_t)s * 3 * NN_DESC;
-        for (int c = 0; c < 3; c++) {
-            const float dr = ri[c] - rho[3 * (size_t)j + c];
-            for (int d = 0; d < NN_DESC; d++) v[d] = fmaf(Js[c * NN_DESC + d], dr, v[d]);
-        }
+        const float* Js = J + (size_t)s * 3 * NN_DESC + lane;
+#pragma unroll
+        for (int c = 0; c < 3; c++) v = fmaf(Js[c * NN_DESC], ri[c] - rho[3 * (size_t)j + c], v);
     }
-    for (int d = 0; d < NN_DESC; d++) V[(size_t)i * NN_DESC + d] = v[d];
+    V[(size_t)i * NN_DESC + lane] = v;
 }
 
-// Per-atom vectors of dL/dw: the energy term (weight e = dL/dE_i) and the
-// force term d(u . v)/dw (u = dE/dG, v = dL/du) by a forward tangent dz1 = W1 v~
-// followed by reverse mode through the tangent computation.
-__global__ void __launch_bounds__(128) k_nn_atom_grad(const float* __restrict__ w, const float* __restrict__ Gt,
-                                                      const float* __restrict__ V, NNDescParams p,
-                                                      const int* __restrict__ list, const int* __restrict__ atom_conf,
-                                                      const float* __restrict__ ew, const int* __restrict__ ew_index,
-                                                      int a0, int na,
-                                                      float* __restrict__ vecs) {
-    extern __shared__ float sw[];
-    load_params(w, sw);
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= na) return;
-    const int atom = list[a0 + t];
-    const float e = ew[ew_index ? ew_index[atom] : atom];
-    const float* W1 = sw + NN_OFF_W1;
-    const float* W2 = sw + NN_OFF_W2;
-    const float* w3 = sw + NN_OFF_W3;
-    float g[NN_DESC], vt[NN_DESC];
-    for (int d = 0; d < NN_DESC; d++) {
-        g[d] = Gt[(size_t)atom * NN_DESC + d];
-        vt[d] = V[(size_t)atom * NN_DESC + d] * p.isig[d];
-    }
-    float a1[NN_H], dz1[NN_H], da1[NN_H];
-    for (int j = 0; j < NN_H; j++) {
-        float z = sw[NN_OFF_B1 + j], dz = 0.f;
-        for (int d = 0; d < NN_DESC; d++) {
-            z = fmaf(W1[j * NN_DESC + d], g[d], z);
-            dz = fmaf(W1[j * NN_DESC + d], vt[d], dz);
-        }
-        a1[j] = tanhf(z);
-        dz1[j] = dz;
-        da1[j] = (1.f - a1[j] * a1[j]) * dz;
-    }
-    float* out = vecs + (size_t)t * NN_VEC_STRIDE;
-    float d2[NN_H], r2[NN_H];
-    for (int o = 0; o < NN_H; o++) {
-        float z = sw[NN_OFF_B2 + o], dz = 0.f;
-        for (int j = 0; j < NN_H; j++) {
-            z = fmaf(W2[o * NN_H + j], a1[j], z);
-            dz = fmaf(W2[o * NN_H + j], da1[j], dz);
-        }
-        const float a2 = tanhf(z), s2 = 1.f - a2 * a2;
-        d2[o] = w3[o] * s2;
-        r2[o] = w3[o] * dz * (-2.f * a2 * s2);
-        out[2 * NN_H + o] = e * d2[o] + r2[o];      // zeta2
-        out[3 * NN_H + o] = d2[o];                  // delta2
-        out[6 * NN_H + o] = e * a2 + s2 * dz;       // w3 gradient
-    }
-    for (int j = 0; j < NN_H; j++) {
-        float sd = 0.f, sr = 0.f;
-        for (int o = 0; o < NN_H; o++) {
-            sd = fmaf(d2[o], W2[o * NN_H + j], sd);
-            sr = fmaf(r2[o], W2[o * NN_H + j], sr);
-        }
-        const float s1 = 1.f - a1[j] * a1[j];
-        const float d1 = sd * s1;
-        const float r1 = sr * s1 + sd * dz1[j] * (-2.f * a1[j] * s1);
-        out[0 * NN_H + j] = e * d1 + r1;  // zeta1
-        out[1 * NN_H + j] = d1;           // delta1
-        out[4 * NN_H + j] = a1[j];
-        out[5 * NN_H + j] = da1[j];
-    }
-    out[7 * NN_H] = e;
+// sum of a feature over the chunk's atoms: four a thread, then over the eight lanes along the atoms
+__device__ __forceinline__ float nt_sum(float4 v) {
+    float s = ((v.x + v.y) + v.z) + v.w;
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
 }
 
-// Partial dL/dw over a chunk of NN_CHUNK batch atoms (fixed order).
-__global__ void __launch_bounds__(256) k_nn_wgrad_partial(const float* __restrict__ vecs, const float* __restrict__ Gt,
-                                                          const float* __restrict__ V, NNDescParams p,
-                                                          const int* __restrict__ list, int a0, int na,
-                                                          float* __restrict__ partial) {
-    extern __shared__ float sm[];
-    float* sv = sm;                              // NN_CHUNK x NN_VEC_STRIDE
-    float* sg = sv + NN_CHUNK * NN_VEC_STRIDE;   // NN_CHUNK x 32
-    float* sr = sg + NN_CHUNK * NN_DESC;         // NN_CHUNK x 32 (v~)
-    const int t0 = blockIdx.x * NN_CHUNK;
-    const int cnt = min(NN_CHUNK, na - t0);
-    for (int q = threadIdx.x; q < NN_CHUNK * NN_VEC_STRIDE; q += blockDim.x) {
-        const int a = q / NN_VEC_STRIDE;
-        sv[q] = a < cnt ? vecs[(size_t)(t0 + a) * NN_VEC_STRIDE + q % NN_VEC_STRIDE] : 0.f;
-    }
-    for (int q = threadIdx.x; q < NN_CHUNK * NN_DESC; q += blockDim.x) {
-        const int a = q / NN_DESC, d = q % NN_DESC;
-        const int atom = a < cnt ? list[a0 + t0 + a] : 0;
-        sg[q] = a < cnt ? Gt[(size_t)atom * NN_DESC + d] : 0.f;
-        sr[q] = a < cnt ? V[(size_t)atom * NN_DESC + d] * p.isig[d] : 0.f;
-    }
-    __syncthreads();
-    float* out = partial + (size_t)blockIdx.x * NN_PARAMS;
-    for (int k = threadIdx.x; k < NN_PARAMS; k += blockDim.x) {
-        float s = 0.f;
-        if (k < NN_OFF_B1) {
-            const int j = k / NN_DESC, d = k % NN_DESC;
-            for (int a = 0; a < NN_CHUNK; a++) {
-                const float* v = sv + a * NN_VEC_STRIDE;
-                s = fmaf(v[j], sg[a * NN_DESC + d], s);
-                s = fmaf(v[NN_H + j], sr[a * NN_DESC + d], s);
+// out[r][c] = sum over the chunk's atoms of P[r] X[c] + Q[r] Y[c], rows
+// to + NT_TO o, columns tc + 8 k, both products of an atom before the next atom's
+template <int NCOL, int COLS>
+__device__ __forceinline__ void nt_outer(const float* P, const float* X, const float* Q, const float* Y,
+                                         float* __restrict__ out) {
+    const int tc = threadIdx.x & 7, to = threadIdx.x >> 3;
+    float acc[NT_R][NCOL];
+#pragma unroll
+    for (int o = 0; o < NT_R; o++)
+#pragma unroll
+        for (int k = 0; k < NCOL; k++) acc[o][k] = 0.f;
+#pragma unroll 1
+    for (int a = 0; a < NN_CHUNK; a += 4) {
+        float4 pr[NT_R], qr[NT_R];
+#pragma unroll
+        for (int o = 0; o < NT_R; o++) {
+            pr[o] = *reinterpret_cast<const float4*>(P + (to + NT_TO * o) * NT_AS + a);
+            qr[o] = *reinterpret_cast<const float4*>(Q + (to + NT_TO * o) * NT_AS + a);
+        }
+#pragma unroll
+        for (int k = 0; k < NCOL; k++) {
+            const float4 x = *reinterpret_cast<const float4*>(X + (tc + 8 * k) * NT_AS + a);
+            const float4 y = *reinterpret_cast<const float4*>(Y + (tc + 8 * k) * NT_AS + a);
+#pragma unroll
+            for (int o = 0; o < NT_R; o++) {
+                float v = acc[o][k];
+                v = fmaf(qr[o].x, y.x, fmaf(pr[o].x, x.x, v));
+                v = fmaf(qr[o].y, y.y, fmaf(pr[o].y, x.y, v));
+                v = fmaf(qr[o].z, y.z, fmaf(pr[o].z, x.z, v));
+                acc[o][k] = fmaf(qr[o].w, y.w, fmaf(pr[o].w, x.w, v));
             }
-        } else if (k < NN_OFF_W2) {
-            const int j = k - NN_OFF_B1;
-            for (int a = 0; a < NN_CHUNK; a++) s += sv[a * NN_VEC_STRIDE + j];
-        } else if (k < NN_OFF_B2) {
-            const int o = (k - NN_OFF_W2) / NN_H, j = (k - NN_OFF_W2) % NN_H;
-            for (int a = 0; a < NN_CHUNK; a++) {
-                const float* v = sv + a * NN_VEC_STRIDE;
-                s = fmaf(v[2 * NN_H + o], v[4 * NN_H + j], s);
-                s = fmaf(v[3 * NN_H + o], v[5 * NN_H + j], s);
-            }
-        } else if (k < NN_OFF_W3) {
-            const int o = k - NN_OFF_B2;
-            for (int a = 0; a < NN_CHUNK; a++) s += sv[a * NN_VEC_STRIDE + 2 * NN_H + o];
-        } else if (k < NN_OFF_B3) {
-            const int o = k - NN_OFF_W3;
-            for (int a = 0; a < NN_CHUNK; a++) s += sv[a * NN_VEC_STRIDE + 6 * NN_H + o];
-        } else {
-            for (int a = 0; a < NN_CHUNK; a++) s += sv[a * NN_VEC_STRIDE + 7 * NN_H];
         }
-        out[k] = s;
     }
+#pragma unroll
+    for (int o = 0; o < NT_R; o++)
+#pragma unroll
+        for (int k = 0; k < NCOL; k++) out[(to + NT_TO * o) * COLS + tc + 8 * k] = acc[o][k];
 }
 
-__global__ void k_nn_wgrad_final(const float* __restrict__ partial, int nchunks, float* __restrict__ grad) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= NN_PARAMS) return;
-    double s = 0.0;
-    for (int c = 0; c < nchunks; c++) s += (double)partial[(size_t)c * NN_PARAMS + k];
-    grad[k] = (float)s;
-}
-
-__global__ void k_nn_loss(const float* __restrict__ lossE, int nb, const float* __restrict__ lossF, int na,
-                          double* __restrict__ loss) {
-    __shared__ double red[256];
-    double s = 0.0;
-    for (int q = threadIdx.x; q < nb; q += blockDim.x) s += (double)lossE[q];
-    for (int q = threadIdx.x; q < na; q += blockDim.x) s += (double)lossF[q];
-    red[threadIdx.x] = s;
+// The loss terms' sum in FP64, by one block.
+__device__ __forceinline__ void nt_loss(const float* __restrict__ lossE, int nE, const float* __restrict__ lossF,
+                                        int nF, double* red, double* __restrict__ loss) {
+    // four sums a thread: the latency of the FP64 adds, not their number, sets this block's time
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int k = threadIdx.x; k < nE; k += 4 * NT_THREADS)
+#pragma unroll
+        for (int q = 0; q < 4; q++) s[q] += k + q * NT_THREADS < nE ? (double)__ldg(lossE + k + q * NT_THREADS) : 0.0;
+    for (int k = threadIdx.x; k < nF; k += 4 * NT_THREADS)
+#pragma unroll
+        for (int q = 0; q < 4; q++) s[q] += k + q * NT_THREADS < nF ? (double)__ldg(lossF + k + q * NT_THREADS) : 0.0;
+    red[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
     __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
+    for (int off = NT_THREADS / 2; off > 0; off >>= 1) {
         if (threadIdx.x < off) red[threadIdx.x] += red[threadIdx.x + off];
         __syncthreads();
     }
     if (threadIdx.x == 0) loss[0] = red[0];
 }
 
-__global__ void k_nn_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                          float* __restrict__ v, float lr_t, float b1, float b2, float eps) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= NN_PARAMS) return;
-    const float gk = g[k];
-    const float mk = b1 * m[k] + (1.f - b1) * gk;
-    const float vk = b2 * v[k] + (1.f - b2) * gk * gk;
+// Partial dL/dw of a chunk of atoms: the energy term (weight e = dL/dE_i) and
+// the force term d(u . v)/dw (u = dE/dG, v = dL/du) by a forward tangent
+// dz1 = W1 v~ followed by reverse mode through the tangent computation, then
+// the outer products over the chunk, all from shared memory.  One block more
+// sums the loss meanwhile.
+__global__ void __launch_bounds__(NT_THREADS) k_nn_grad(const float* __restrict__ w, const float* __restrict__ Gt,
+                                                        const float* __restrict__ V, NNDescParams p,
+                                                        const float* __restrict__ acts, const int* __restrict__ list,
+                                                        const float* __restrict__ ew,
+                                                        const int* __restrict__ ew_index, int a0, int na,
+                                                        float* __restrict__ partial, const float* __restrict__ lossE,
+                                                        int nE, const float* __restrict__ lossF,
+                                                        double* __restrict__ loss) {
+    extern __shared__ __align__(16) float sm[];
+    if (blockIdx.x * NN_CHUNK >= na) {  // the block past the chunks
+        nt_loss(lossE, nE, lossF, na, reinterpret_cast<double*>(sm), loss);
+        return;
+    }
+    const NTWeights q = nt_load_weights(w, sm);
+    float* G = sm + NT_W_FLOATS;
+    float* VT = G + NN_DESC * NT_AS;
+    float* A1 = VT + NN_DESC * NT_AS;
+    float* DA1 = A1 + NN_H * NT_AS;
+    float* D1 = DA1 + NN_H * NT_AS;
+    float* Z1 = D1 + NN_H * NT_AS;   // first the part of r1 that needs dz1
+    float* Z2 = Z1 + NN_H * NT_AS;
+    float* D2 = Z2 + NN_H * NT_AS;
+    float* R2 = D2 + NN_H * NT_AS;
+    float* e = R2 + NN_H * NT_AS;    // NN_CHUNK
+    const int t0 = blockIdx.x * NN_CHUNK, cnt = min(NN_CHUNK, na - t0);
+    list += a0 + t0;
+    float* out = partial + (size_t)blockIdx.x * NN_PARAMS;
+    nt_load_rows<false>(Gt, nullptr, list, cnt, G);
+    nt_load_rows<true>(V, p.isig, list, cnt, VT);
+    if (threadIdx.x < NN_CHUNK) {
+        const int atom = threadIdx.x < cnt ? list[threadIdx.x] : 0;
+        float v = threadIdx.x < cnt ? ew[ew_index ? ew_index[atom] : atom] : 0.f;
+        e[threadIdx.x] = v;
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (threadIdx.x == 0) out[NN_OFF_B3] = v;
+    }
+    __syncthreads();
+    const int ta = threadIdx.x & 7, to = threadIdx.x >> 3;
+    const float* act = acts + (size_t)blockIdx.x * NT_ACTS * NN_CHUNK + 4 * ta;
+    const float4 e4 = *reinterpret_cast<const float4*>(e + 4 * ta);
+    // absent atoms of the last chunk: the forward pass gave them a1 = tanh(b1)
+    // and so on; their tangents and weights are zero here, and the terms that
+    // survive (d1, d2 against zero inputs or tangents) multiply zeros
+    float z[NT_R][4];
+    nt_zero(z);
+    nt_rows<NN_DESC, NT_W1S>(q.W1, VT, to, ta, z);
+#pragma unroll
+    for (int o = 0; o < NT_R; o++) {
+        const int j = to + NT_TO * o;
+        const float4 a1 = *reinterpret_cast<const float4*>(act + j * NN_CHUNK);
+        const float4 sd = *reinterpret_cast<const float4*>(act + (2 * NN_H + j) * NN_CHUNK);
+        float4 da, d1, r;
+        const auto one = [](float a, float s, float dz, float& da_, float& d1_, float& r_) {
+            const float s1 = 1.f - a * a;
+            da_ = s1 * dz;
+            d1_ = s * s1;
+            r_ = s * dz * (-2.f * a * s1);
+        };
+        one(a1.x, sd.x, z[o][0], da.x, d1.x, r.x);
+        one(a1.y, sd.y, z[o][1], da.y, d1.y, r.y);
+        one(a1.z, sd.z, z[o][2], da.z, d1.z, r.z);
+        one(a1.w, sd.w, z[o][3], da.w, d1.w, r.w);
+        nt_at(A1, j, ta) = a1;
+        nt_at(DA1, j, ta) = da;
+        nt_at(D1, j, ta) = d1;
+        nt_at(Z1, j, ta) = r;
+    }
+    __syncthreads();
+    nt_zero(z);
+    nt_rows<NN_H, NT_W2S>(q.W2, DA1, to, ta, z);
+#pragma unroll
+    for (int o = 0; o < NT_R; o++) {
+        const int j = to + NT_TO * o;
+        const float w3 = q.w3[j];
+        const float4 a2 = *reinterpret_cast<const float4*>(act + (NN_H + j) * NN_CHUNK);
+        float4 d2, r2, z2, g3;
+        const auto one = [&](float a, float dz, float ei, float& d2_, float& r2_, float& z2_, float& g3_) {
+            const float s2 = 1.f - a * a;
+            d2_ = w3 * s2;
+            r2_ = w3 * dz * (-2.f * a * s2);
+            z2_ = ei * d2_ + r2_;
+            g3_ = ei * a + s2 * dz;
+        };
+        one(a2.x, z[o][0], e4.x, d2.x, r2.x, z2.x, g3.x);
+        one(a2.y, z[o][1], e4.y, d2.y, r2.y, z2.y, g3.y);
+        one(a2.z, z[o][2], e4.z, d2.z, r2.z, z2.z, g3.z);
+        one(a2.w, z[o][3], e4.w, d2.w, r2.w, z2.w, g3.w);
+        nt_at(D2, j, ta) = d2;
+        nt_at(R2, j, ta) = r2;
+        nt_at(Z2, j, ta) = z2;
+        const float gw3 = nt_sum(g3), gb2 = nt_sum(z2);
+        if (ta == 0) {
+            out[NN_OFF_W3 + j] = gw3;
+            out[NN_OFF_B2 + j] = gb2;
+        }
+    }
+    __syncthreads();
+    nt_zero(z);
+    nt_cols<NT_R, NT_W2S>(q.W2, R2, to, ta, z);
+#pragma unroll
+    for (int c = 0; c < NT_R; c++) {
+        const int j = NT_R * to + c;
+        const float4 a1 = nt_at(A1, j, ta), d1 = nt_at(D1, j, ta), r = nt_at(Z1, j, ta);
+        const float4 z1 = make_float4(e4.x * d1.x + (z[c][0] * (1.f - a1.x * a1.x) + r.x),
+                                      e4.y * d1.y + (z[c][1] * (1.f - a1.y * a1.y) + r.y),
+                                      e4.z * d1.z + (z[c][2] * (1.f - a1.z * a1.z) + r.z),
+                                      e4.w * d1.w + (z[c][3] * (1.f - a1.w * a1.w) + r.w));
+        nt_at(Z1, j, ta) = z1;
+        const float gb1 = nt_sum(z1);
+        if (ta == 0) out[NN_OFF_B1 + j] = gb1;
+    }
+    __syncthreads();
+    nt_outer<8, NN_H>(Z2, A1, D2, DA1, out + NN_OFF_W2);
+    nt_outer<4, NN_DESC>(Z1, G, D1, VT, out + NN_OFF_W1);
+}
+
+// One Adam step's factors; on = 0: leave the weights alone.
+struct NTAdam {
+    int on;
+    float lr, b1, b2, eps;
+};
+
+// The chunks' partial gradients summed in FP64 (each of NT_SPLIT threads a
+// run of the chunks, the runs in order), the gradient stored and the weights
+// stepped.
+constexpr int NT_SPLIT = 8;
+constexpr int NT_FINAL_BLOCKS = (NN_PARAMS + 31) / 32;
+
+__global__ void __launch_bounds__(32 * NT_SPLIT) k_nn_step(const float* __restrict__ partial, int nchunks,
+                                                           float* __restrict__ grad, NTAdam ad, float* __restrict__ w,
+                                                           float* __restrict__ m, float* __restrict__ v) {
+    __shared__ double red[32 * NT_SPLIT];
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    double s = 0.0;
+    const int k = blockIdx.x * 32 + lane;
+    const int per = (nchunks + NT_SPLIT - 1) / NT_SPLIT, c0 = part * per, c1 = min(nchunks, c0 + per);
+    if (k < NN_PARAMS) {
+#pragma unroll 8
+        for (int c = c0; c < c1; c++) s += f2d_exact(__ldg(partial + (size_t)c * NN_PARAMS + k));  // no FP64 conversion
+    }
+    red[threadIdx.x] = s;
+    __syncthreads();
+    if (part != 0 || k >= NN_PARAMS) return;
+    for (int q = 1; q < NT_SPLIT; q++) s += red[q * 32 + lane];
+    const float gk = (float)s;
+    grad[k] = gk;
+    if (!ad.on) return;
+    const float mk = ad.b1 * m[k] + (1.f - ad.b1) * gk;
+    const float vk = ad.b2 * v[k] + (1.f - ad.b2) * gk * gk;
     m[k] = mk;
     v[k] = vk;
-    w[k] -= lr_t * mk / (sqrtf(vk) + eps);
+    w[k] -= ad.lr * mk / (sqrtf(vk) + ad.eps);
+}
+
+// The atoms of the configurations in the epoch's order, back to back.
+__global__ void k_nn_order(const int* __restrict__ clist, const int* __restrict__ at,
+                           const int* __restrict__ conf_start, int* __restrict__ list) {
+    const int c = clist[blockIdx.x], a = conf_start[c], n = conf_start[c + 1] - a;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) list[at[blockIdx.x] + k] = a + k;
 }
 
 }  // namespace omdg
@@ -541,16 +773,16 @@ static void nn_free_data(omdg_nn* t) {
     void* ptrs[] = {t->d_conf_start, t->d_atom_conf, t->d_x,     t->d_L,      t->d_eref,    t->d_fref,   t->d_slot_start,
                     t->d_slot_j,     t->d_slot_rev,  t->d_slot_d, t->d_G,     t->d_Gt,      t->d_J,      t->d_E,
                     t->d_u,          t->d_F,         t->d_rho,   t->d_vvec,   t->d_ew,      t->d_lossE,  t->d_lossF,
-                    t->d_vecs,       t->d_partial,   t->d_list,  t->d_clist};
+                    t->d_acts,       t->d_partial,   t->d_list,  t->d_clist};
     for (void* p : ptrs) cudaFree(p);
     t->d_conf_start = t->d_atom_conf = t->d_slot_start = t->d_slot_j = t->d_slot_rev = t->d_list = t->d_clist = nullptr;
     t->d_x = t->d_L = nullptr;
     t->d_eref = t->d_fref = t->d_G = t->d_Gt = t->d_J = t->d_E = t->d_u = t->d_F = t->d_rho = t->d_vvec = nullptr;
-    t->d_ew = t->d_lossE = t->d_lossF = t->d_vecs = t->d_partial = nullptr;
+    t->d_ew = t->d_lossE = t->d_lossF = t->d_acts = t->d_partial = nullptr;
     t->d_slot_d = nullptr;
     t->nconf = 0;
     t->natoms = t->nslots = 0;
-    t->cap_batch_atoms = 0;
+    t->cap_batch_atoms = t->cap_clist = 0;
 }
 
 template <typename T>
@@ -576,7 +808,6 @@ int omdg_nn_create(omdg_nn** out, int device) {
     if (e == cudaSuccess) e = dalloc(&t->d_adam_m, NN_PARAMS);
     if (e == cudaSuccess) e = dalloc(&t->d_adam_v, NN_PARAMS);
     if (e == cudaSuccess) e = dalloc(&t->d_grad, NN_PARAMS);
-    if (e == cudaSuccess) e = dalloc(&t->d_loss, 1);
     if (e != cudaSuccess) {
         delete t;
         return OMDG_ECUDA;
@@ -735,7 +966,6 @@ int omdg_nn_set_dataset(omdg_nn* t, int nconf, const int* natoms, const double* 
     if (e == cudaSuccess) e = dalloc(&t->d_vvec, n * NN_DESC);
     if (e == cudaSuccess) e = dalloc(&t->d_ew, nconf);
     if (e == cudaSuccess) e = dalloc(&t->d_list, n);
-    if (e == cudaSuccess) e = dalloc(&t->d_clist, nconf);
     if (e != cudaSuccess) return nn_cuda(t, e, "dataset allocation");
     cudaStream_t s = t->stream;
     cudaMemcpyAsync(t->d_conf_start, start.data(), sizeof(int) * (nconf + 1), cudaMemcpyHostToDevice, s);
@@ -863,73 +1093,99 @@ static int ensure_batch(omdg_nn* t, long atoms) {
     if (atoms <= t->cap_batch_atoms) return OMDG_OK;
     cudaFree(t->d_lossE);
     cudaFree(t->d_lossF);
-    cudaFree(t->d_vecs);
+    cudaFree(t->d_acts);
     cudaFree(t->d_partial);
     const long chunks = (atoms + NN_CHUNK - 1) / NN_CHUNK;
     cudaError_t e = dalloc(&t->d_lossE, std::max<long>(t->nconf, atoms));
     if (e == cudaSuccess) e = dalloc(&t->d_lossF, atoms);
-    if (e == cudaSuccess) e = dalloc(&t->d_vecs, (size_t)atoms * NN_VEC_STRIDE);
+    if (e == cudaSuccess) e = dalloc(&t->d_acts, (size_t)chunks * NT_ACTS * NN_CHUNK);
     if (e == cudaSuccess) e = dalloc(&t->d_partial, (size_t)chunks * NN_PARAMS);
     if (e != cudaSuccess) return nn_cuda(t, e, "batch allocation");
     t->cap_batch_atoms = atoms;
     return OMDG_OK;
 }
 
+static void nn_kernel_attributes() {
+    cudaFuncSetAttribute(k_nn_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(float) * NT_FWD_FLOATS);
+    cudaFuncSetAttribute(k_nn_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(float) * NT_GRAD_FLOATS);
+}
+
 // Loss and gradient over the configurations clist[c0 .. c0 + nb) whose atoms
-// are list[a0 .. a0 + na); leaves dL/dw in d_grad and L in d_loss.
-static int nn_loss_grad(omdg_nn* t, int c0, int nb, long a0, long na, double wE, double wF) {
+// are list[a0 .. a0 + na); leaves dL/dw in d_grad and L in loss, and steps the
+// weights when ad says so.
+static int nn_loss_grad(omdg_nn* t, const int* clist, int c0, int nb, long a0, long na, double wE, double wF,
+                        const NTAdam& ad, double* loss) {
     int rc = ensure_batch(t, na);
     if (rc) return rc;
     cudaStream_t s = t->stream;
     const NNDescParams& p = t->model.dp;
-    const size_t wsm = sizeof(float) * NN_PARAMS;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_nn_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
-        cudaFuncSetAttribute(k_nn_atom_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
-        cudaFuncSetAttribute(k_nn_wgrad_partial, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(float) * NN_CHUNK * (NN_VEC_STRIDE + 2 * NN_DESC)));
-        attr = true;
-    }
-    const unsigned gb = (unsigned)((na + 127) / 128);
-    k_nn_fwd<<<gb, 128, wsm, s>>>(t->d_params, t->d_Gt, p, t->d_list, (int)a0, (int)na, t->d_E, t->d_u);
-    if (t->d_eatom)
-        k_nn_atom_energy<<<gb, 128, 0, s>>>(t->d_list, (int)a0, (int)na, t->d_E, t->d_eatom, (float)wE, t->d_ewa,
+    nn_kernel_attributes();
+    const int chunks = (int)((na + NN_CHUNK - 1) / NN_CHUNK);
+    const unsigned wb = (unsigned)((na + 7) / 8);  // blocks of eight warps, an atom each
+    k_nn_fwd<<<chunks, NT_THREADS, sizeof(float) * NT_FWD_FLOATS, s>>>(
+        t->d_params, t->d_Gt, p, t->d_list, (int)a0, (int)na, t->d_E, t->d_u, t->d_acts, t->d_eatom, (float)wE,
+        t->d_ewa, t->d_lossE);
+    if (!t->d_eatom)
+        k_nn_conf_energy<<<nb, 256, 0, s>>>(clist, c0, nb, t->d_conf_start, t->d_E, t->d_eref, (float)wE, t->d_ew,
                                             t->d_lossE);
-    else
-        k_nn_conf_energy<<<nb, 256, 0, s>>>(t->d_clist, c0, nb, t->d_conf_start, t->d_E, t->d_eref, (float)wE,
-                                            t->d_ew, t->d_lossE);
-    k_nn_force<<<gb, 128, 0, s>>>(t->d_list, (int)a0, (int)na, t->d_slot_start, t->d_slot_j, t->d_slot_rev, t->d_J,
+    k_nn_force<<<wb, 256, 0, s>>>(t->d_list, (int)a0, (int)na, t->d_slot_start, t->d_slot_j, t->d_slot_rev, t->d_J,
                                   t->d_u, t->d_fref, (float)(wF / (3.0 * na)), t->d_fw, t->d_atom_conf, t->d_F,
                                   t->d_rho, t->d_lossF);
-    k_nn_vvec<<<gb, 128, 0, s>>>(t->d_list, (int)a0, (int)na, t->d_slot_start, t->d_slot_j, t->d_J, t->d_rho,
+    k_nn_vvec<<<wb, 256, 0, s>>>(t->d_list, (int)a0, (int)na, t->d_slot_start, t->d_slot_j, t->d_J, t->d_rho,
                                  t->d_vvec);
-    k_nn_atom_grad<<<gb, 128, wsm, s>>>(t->d_params, t->d_Gt, t->d_vvec, p, t->d_list, t->d_atom_conf,
-                                        t->d_eatom ? t->d_ewa : t->d_ew, t->d_eatom ? nullptr : t->d_atom_conf,
-                                        (int)a0, (int)na, t->d_vecs);
-    const int chunks = (int)((na + NN_CHUNK - 1) / NN_CHUNK);
-    k_nn_wgrad_partial<<<chunks, 256, sizeof(float) * NN_CHUNK * (NN_VEC_STRIDE + 2 * NN_DESC), s>>>(
-        t->d_vecs, t->d_Gt, t->d_vvec, p, t->d_list, (int)a0, (int)na, t->d_partial);
-    k_nn_wgrad_final<<<(NN_PARAMS + 255) / 256, 256, 0, s>>>(t->d_partial, chunks, t->d_grad);
-    k_nn_loss<<<1, 256, 0, s>>>(t->d_lossE, t->d_eatom ? (int)na : nb, t->d_lossF, (int)na, t->d_loss);
+    k_nn_grad<<<chunks + 1, NT_THREADS, sizeof(float) * NT_GRAD_FLOATS, s>>>(
+        t->d_params, t->d_Gt, t->d_vvec, p, t->d_acts, t->d_list, t->d_eatom ? t->d_ewa : t->d_ew,
+        t->d_eatom ? nullptr : t->d_atom_conf, (int)a0, (int)na, t->d_partial, t->d_lossE,
+        t->d_eatom ? (int)na : nb, t->d_lossF, loss);
+    k_nn_step<<<NT_FINAL_BLOCKS, 32 * NT_SPLIT, 0, s>>>(t->d_partial, chunks, t->d_grad, ad, t->d_params, t->d_adam_m,
+                                                        t->d_adam_v);
     return nn_cuda(t, cudaGetLastError(), "training step");
 }
 
-static int upload_order(omdg_nn* t, const std::vector<int>& confs, std::vector<long>& conf_atoms0) {
-    std::vector<int> list;
-    list.reserve(t->natoms);
-    conf_atoms0.assign(confs.size() + 1, 0);
-    for (size_t k = 0; k < confs.size(); k++) {
-        const int c = confs[k];
-        for (int a = t->conf_start[c]; a < t->conf_start[c + 1]; a++) list.push_back(a);
-        conf_atoms0[k + 1] = (long)list.size();
+// The configuration orders of `epochs` epochs (confs, back to back) to the
+// device; conf_atoms0 gives where each configuration's atoms begin in its
+// epoch's atom order, which nn_order writes.
+static int upload_orders(omdg_nn* t, const std::vector<int>& confs, int epochs, std::vector<int>& conf_atoms0) {
+    const size_t n = confs.size(), per = n / epochs;
+    std::vector<int> up(confs);
+    up.resize(2 * n);
+    conf_atoms0.assign((per + 1) * epochs, 0);
+    for (int ep = 0; ep < epochs; ep++) {
+        int* at = conf_atoms0.data() + (per + 1) * ep;
+        for (size_t k = 0; k < per; k++) {
+            const int c = confs[per * ep + k];
+            up[n + per * ep + k] = at[k];
+            at[k + 1] = at[k] + (t->conf_start[c + 1] - t->conf_start[c]);
+        }
     }
-    cudaError_t e = cudaMemcpyAsync(t->d_list, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice,
-                                    t->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(t->d_clist, confs.data(), sizeof(int) * confs.size(), cudaMemcpyHostToDevice, t->stream);
+    if ((long)up.size() > t->cap_clist) {
+        cudaFree(t->d_clist);
+        t->d_clist = nullptr;
+        t->cap_clist = 0;
+        cudaError_t e = dalloc(&t->d_clist, up.size());
+        if (e != cudaSuccess) return nn_cuda(t, e, "batch order");
+        t->cap_clist = (long)up.size();
+    }
+    cudaError_t e = cudaMemcpyAsync(t->d_clist, up.data(), sizeof(int) * up.size(), cudaMemcpyHostToDevice, t->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
     return nn_cuda(t, e, "batch order");
+}
+
+// The atom order of one uploaded epoch (n configurations in all epochs, per of them in each).
+static void nn_order(omdg_nn* t, size_t n, size_t per, int ep) {
+    k_nn_order<<<(unsigned)per, 256, 0, t->stream>>>(t->d_clist + per * ep, t->d_clist + n + per * ep, t->d_conf_start,
+                                                    t->d_list);
+}
+
+static int ensure_losses(omdg_nn* t, long n) {
+    if (n <= t->cap_loss) return OMDG_OK;
+    cudaFree(t->d_loss);
+    t->d_loss = nullptr;
+    t->cap_loss = 0;
+    cudaError_t e = dalloc(&t->d_loss, n);
+    if (e != cudaSuccess) return nn_cuda(t, e, "loss allocation");
+    t->cap_loss = n;
+    return OMDG_OK;
 }
 
 int omdg_nn_gradient(omdg_nn* t, int conf0, int nconf, double wE, double wF, double* loss, float* grad) {
@@ -937,10 +1193,12 @@ int omdg_nn_gradient(omdg_nn* t, int conf0, int nconf, double wE, double wF, dou
     cudaSetDevice(t->device);
     std::vector<int> confs(nconf);
     std::iota(confs.begin(), confs.end(), conf0);
-    std::vector<long> ca;
-    int rc = upload_order(t, confs, ca);
+    std::vector<int> ca;
+    int rc = upload_orders(t, confs, 1, ca);
+    if (!rc) rc = ensure_losses(t, 1);
     if (rc) return rc;
-    if ((rc = nn_loss_grad(t, 0, nconf, 0, ca[nconf], wE, wF))) return rc;
+    nn_order(t, confs.size(), confs.size(), 0);
+    if ((rc = nn_loss_grad(t, t->d_clist, 0, nconf, 0, ca[nconf], wE, wF, NTAdam{}, t->d_loss))) return rc;
     cudaError_t e = cudaSuccess;
     if (loss) e = cudaMemcpyAsync(loss, t->d_loss, sizeof(double), cudaMemcpyDeviceToHost, t->stream);
     if (grad && e == cudaSuccess)
@@ -956,40 +1214,54 @@ int omdg_nn_train(omdg_nn* t, int epochs, int batch_confs, double lr, double lr_
     cudaSetDevice(t->device);
     std::mt19937 rng(seed);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    std::vector<int> confs(t->nconf);
+    std::vector<int> confs(t->nconf), orders, ca;
     std::iota(confs.begin(), confs.end(), 0);
-    for (int ep = 0; ep < epochs; ep++) {
-        // cosine decay from lr (first epoch) to lr_final (last epoch)
-        const double lr_ep =
-            epochs > 1 ? lr_final + 0.5 * (lr - lr_final) * (1.0 + std::cos(M_PI * ep / (epochs - 1))) : lr;
-        std::shuffle(confs.begin(), confs.end(), rng);
-        std::vector<long> ca;
-        int rc = upload_order(t, confs, ca);
-        if (rc) return rc;
-        double sum = 0.0;
-        int nbatch = 0;
-        for (int c0 = 0; c0 < t->nconf; c0 += batch_confs) {
-            const int nb = std::min(batch_confs, t->nconf - c0);
-            if ((rc = nn_loss_grad(t, c0, nb, ca[c0], ca[c0 + nb] - ca[c0], wE, wF))) return rc;
-            t->adam_t++;
-            const double bc1 = 1.0 - std::pow((double)b1, (double)t->adam_t);
-            const double bc2 = 1.0 - std::pow((double)b2, (double)t->adam_t);
-            const float lr_t = (float)(lr_ep * std::sqrt(bc2) / bc1);
-            k_nn_adam<<<(NN_PARAMS + 255) / 256, 256, 0, t->stream>>>(t->d_params, t->d_grad, t->d_adam_m,
-                                                                      t->d_adam_v, lr_t, b1, b2, eps);
-            if (epoch_loss) {
-                double l = 0;
-                cudaMemcpyAsync(&l, t->d_loss, sizeof(double), cudaMemcpyDeviceToHost, t->stream);
-                cudaStreamSynchronize(t->stream);
-                sum += l;
-            }
-            nbatch++;
+    // epochs are queued in groups (orders of up to 2^20 configurations); the
+    // host waits, and reads the batches' losses, once per group
+    const int nbatch = (t->nconf + batch_confs - 1) / batch_confs;
+    const int group = std::max(1, std::min(epochs, (1 << 20) / t->nconf));
+    std::vector<double> losses((size_t)group * nbatch);
+    int rc = ensure_losses(t, (long)losses.size());
+    if (rc) return rc;
+    for (int e0 = 0; e0 < epochs; e0 += group) {
+        const int ne = std::min(group, epochs - e0);
+        orders.clear();
+        for (int k = 0; k < ne; k++) {
+            std::shuffle(confs.begin(), confs.end(), rng);
+            orders.insert(orders.end(), confs.begin(), confs.end());
         }
-        cudaError_t e = cudaStreamSynchronize(t->stream);
+        if ((rc = upload_orders(t, orders, ne, ca))) return rc;
+        for (int k = 0; k < ne; k++) {
+            const int ep = e0 + k;
+            // cosine decay from lr (first epoch) to lr_final (last epoch)
+            const double lr_ep =
+                epochs > 1 ? lr_final + 0.5 * (lr - lr_final) * (1.0 + std::cos(M_PI * ep / (epochs - 1))) : lr;
+            const int* at = ca.data() + (size_t)(t->nconf + 1) * k;
+            nn_order(t, orders.size(), t->nconf, k);
+            for (int c0 = 0, b = 0; c0 < t->nconf; c0 += batch_confs, b++) {
+                const int nb = std::min(batch_confs, t->nconf - c0);
+                t->adam_t++;
+                const double bc1 = 1.0 - std::pow((double)b1, (double)t->adam_t);
+                const double bc2 = 1.0 - std::pow((double)b2, (double)t->adam_t);
+                const float lr_t = (float)(lr_ep * std::sqrt(bc2) / bc1);
+                rc = nn_loss_grad(t, t->d_clist + (size_t)t->nconf * k, c0, nb, at[c0], at[c0 + nb] - at[c0], wE, wF,
+                                  NTAdam{1, lr_t, b1, b2, eps}, t->d_loss + (size_t)nbatch * k + b);
+                if (rc) return rc;
+            }
+        }
+        cudaError_t e = cudaSuccess;
+        if (epoch_loss)
+            e = cudaMemcpyAsync(losses.data(), t->d_loss, sizeof(double) * (size_t)ne * nbatch,
+                                cudaMemcpyDeviceToHost, t->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
         if (e != cudaSuccess) return nn_cuda(t, e, "training");
-        if (epoch_loss) epoch_loss[ep] = sum / std::max(1, nbatch);
+        for (int k = 0; epoch_loss && k < ne; k++) {
+            double sum = 0.0;
+            for (int b = 0; b < nbatch; b++) sum += losses[(size_t)nbatch * k + b];
+            epoch_loss[e0 + k] = sum / std::max(1, nbatch);
+        }
     }
-    int rc = nn_status(t);
+    rc = nn_status(t);
     if (rc) return rc;
     return omdg_nn_get_weights(t, t->model.w.data(), NN_PARAMS);
 }
@@ -1004,23 +1276,23 @@ int omdg_nn_predict(omdg_nn* t, int conf0, int nconf, int fp32, double* energy_p
     if ((rc = nn_net_upload(t->net, t->model, t->stream, t->err))) return rc;
     std::vector<int> confs(nconf);
     std::iota(confs.begin(), confs.end(), conf0);
-    std::vector<long> ca;
-    if ((rc = upload_order(t, confs, ca))) return rc;
+    std::vector<int> ca;
+    if ((rc = upload_orders(t, confs, 1, ca))) return rc;
+    nn_order(t, confs.size(), confs.size(), 0);
     const long a0 = t->conf_start[conf0], na = t->conf_start[conf0 + nconf] - a0;
-    const unsigned gb = (unsigned)((na + 127) / 128);
     cudaError_t e = cudaSuccess;
     if (fp32) {
-        const size_t wsm = sizeof(float) * NN_PARAMS;
-        cudaFuncSetAttribute(k_nn_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
-        k_nn_fwd<<<gb, 128, wsm, t->stream>>>(t->d_params, t->d_Gt, t->model.dp, t->d_list, 0, (int)na, t->d_E,
-                                              t->d_u);
+        nn_kernel_attributes();
+        k_nn_fwd<<<(unsigned)((na + NN_CHUNK - 1) / NN_CHUNK), NT_THREADS, sizeof(float) * NT_FWD_FLOATS, t->stream>>>(
+            t->d_params, t->d_Gt, t->model.dp, t->d_list, 0, (int)na, t->d_E, t->d_u, nullptr, nullptr, 0.f, nullptr,
+            nullptr);
         e = cudaGetLastError();
     } else {
         e = nn_mlp_launch(t->net, t->d_Gt + a0 * NN_DESC, (int)na, t->d_E + a0, t->d_u + a0 * NN_DESC, t->d_status,
                           t->num_sms, t->stream);
     }
     if (e != cudaSuccess) return nn_cuda(t, e, "network");
-    k_nn_force<<<gb, 128, 0, t->stream>>>(t->d_list, 0, (int)na, t->d_slot_start, t->d_slot_j, t->d_slot_rev, t->d_J,
+    k_nn_force<<<(unsigned)((na + 7) / 8), 256, 0, t->stream>>>(t->d_list, 0, (int)na, t->d_slot_start, t->d_slot_j, t->d_slot_rev, t->d_J,
                                           t->d_u, nullptr, 0.f, nullptr, nullptr, t->d_F, nullptr, nullptr);
     std::vector<float> E(na), F(3 * na);
     e = cudaGetLastError();

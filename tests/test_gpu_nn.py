@@ -114,6 +114,53 @@ def test_training_gradient_matches_oracle(omdg_lib, dataset, per_atom):
     assert np.linalg.norm(g - ref) / np.linalg.norm(ref) < 1e-3
 
 
+# Batches that leave the last chunk of 32 atoms ragged (cells with vacancies),
+# against the oracle, and the queued epochs against Adam steps taken here from
+# the gradient entry point (one batch: the order of its configurations only
+# reorders FP64 sums of chunks).
+@pytest.mark.parametrize("sizes,per_atom", [((63,), True), ((33, 62), False), ((31, 64, 50), True), ((17,), False)])
+def test_ragged_batches_and_queued_epochs(omdg_lib, oracle_lib, sizes, per_atom):
+    from objectmd_gb300 import inputs
+    from oracle import nn_oracle as nn
+
+    oc = oracle_lib
+    p = nn.descriptor_params()
+    confs = []
+    for k, n in enumerate(sizes):
+        x, v, (lo, hi) = inputs.diamond_silicon(ncell=2, a=5.431, sigma=0.1, temp=300.0, seed_pos=40 + k, seed_vel=50)
+        x = x[np.sort(np.random.default_rng(k).permutation(64)[:n])]
+        box = oc.make_box(lo, hi, (1, 1, 1))
+        f, e, _ = oc.tersoff(box, x, oc.neighbors(box, x, 3.15), oc.TersoffParam(**TP))
+        G, jac = nn.descriptors(x, lo, hi, p)
+        confs.append(dict(x=x, lo=lo, hi=hi, E=e.sum(), Ea=e, F=f, G=G, jac=jac))
+    net, w, norm = make_network(omdg_lib, confs)
+    if per_atom:
+        net.set_atom_energies(np.concatenate([c["Ea"] for c in confs]))
+    loss, g = net.gradient(0, len(sizes), 1.0, 2.0)
+    L, grad = nn.loss_and_grad(w, norm, [(c["G"], c["jac"], c["Ea"] if per_atom else c["E"], c["F"]) for c in confs],
+                               1.0, 2.0, per_atom)
+    ref = nn.flatten(grad).astype(np.float64)
+    assert abs(loss - L) < 1e-4 * abs(L)
+    assert np.linalg.norm(g - ref) / np.linalg.norm(ref) < 1e-3
+    W = net.weights()
+    m, v = np.zeros_like(W), np.zeros_like(W)
+    ws, losses = W.copy(), []
+    for k in range(3):
+        net.set_weights(ws)
+        l, g = net.gradient(0, len(sizes), 1.0, 2.0)
+        losses.append(l)
+        m, v = np.float32(0.9) * m + np.float32(0.1) * g, np.float32(0.999) * v + np.float32(0.001) * g * g
+        lr = 1e-3 * np.sqrt(1.0 - 0.999 ** (k + 1)) / (1.0 - 0.9 ** (k + 1))
+        ws = ws - np.float32(lr) * m / (np.sqrt(v) + np.float32(1e-8))
+    net.set_weights(W)
+    hist = net.train(3, len(sizes), 1e-3, 1.0, 2.0)
+    net2 = net.weights()
+    net.close()
+    np.testing.assert_allclose(hist, losses, rtol=1e-4)
+    # weights move by about lr a step; where a gradient is at its rounding noise the two may step apart
+    assert np.linalg.norm(net2 - ws) < 1e-2 * np.linalg.norm(ws - W)
+
+
 def surrogate_context(omdg, c, model, fallback):
     from objectmd_gb300 import inputs
 
