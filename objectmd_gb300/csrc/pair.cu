@@ -40,6 +40,72 @@ __device__ __forceinline__ void lanes_twosum(float& s, float& c) {
     }
 }
 
+// One lane's share of the row of atom ii (entries lane, lane + LANES, ...).
+template <int LANES>
+__device__ __forceinline__ void pair32_sum(const PairParams& p, const PosPack* __restrict__ pack,
+                                           const unsigned* __restrict__ nbr, int ii, const PosPack& pi, int ti, int m,
+                                           int lane, Kahan& ax, Kahan& ay, Kahan& az, Kahan& ae, float& av,
+                                           unsigned* status) {
+    const ShiftF L = p.rep_L ? p.rep_L[p.rep_of[ii]] : p.L;
+    for (int s = lane; s < m; s += LANES) {
+        unsigned e = __ldg(&nbr[nbr_at(ii, s, p.hshift, p.maxnb)]);
+        int j = nbr_index(e);
+        const float4* pj = reinterpret_cast<const float4*>(pack + j);
+        const float4 hj = __ldg(pj);  // the type word first: most rows of a mixed system skip here
+        if (!p.all_types && !types_match(ti, pack_type(hj), p.ta, p.tb)) continue;
+        const float4 lj = __ldg(pj + 1);
+        float3 d = pair_delta(pi.hi, pi.lo, hj, lj, e, L);
+        float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
+        if (r2 >= p.rc2) continue;
+        float rinv = rsqrtf(r2);
+        float r = r2 * rinv;
+        if (!(r < p.rc)) continue;
+        float ph, dph;
+        tab_read(p.phi, p.phi.coef, r, rinv, ph, dph, status);
+        float fr = -dph * rinv;
+        ax.add(d.x * fr);
+        ay.add(d.y * fr);
+        az.add(d.z * fr);
+        ae.add(0.5f * ph);
+        av = fmaf(fr, r2, av);
+    }
+    lanes_twosum<LANES>(ax.s, ax.c);
+    lanes_twosum<LANES>(ay.s, ay.c);
+    lanes_twosum<LANES>(az.s, az.c);
+    lanes_twosum<LANES>(ae.s, ae.c);
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) av += __shfl_xor_sync(0xffffffffu, av, off);
+}
+
+__device__ __forceinline__ void pair32_store(const PairParams& p, int i, int m, const Kahan& ax, const Kahan& ay,
+                                             const Kahan& az, const Kahan& ae, float av, float* __restrict__ fx,
+                                             float* __restrict__ fy, float* __restrict__ fz, float* __restrict__ pe,
+                                             float* __restrict__ vir) {
+    const float vfx = __fsub_rn(ax.s, ax.c), vfy = __fsub_rn(ay.s, ay.c), vfz = __fsub_rn(az.s, az.c);
+    const float ve = __fsub_rn(ae.s, ae.c);
+    if (p.first) {
+        fx[i] = vfx;
+        fy[i] = vfy;
+        fz[i] = vfz;
+        pe[i] = ve;
+        vir[i] = av;
+    } else if (m) {
+        fx[i] += vfx;
+        fy[i] += vfy;
+        fz[i] += vfz;
+        pe[i] += ve;
+        vir[i] += av;
+    }
+}
+
+// A typed pair: the row of an atom of type ta or tb that holds an atom of the
+// other type (the rows' type masks; most rows of a mixed system, a Si atom
+// with no Ar near, have none).
+__device__ __forceinline__ bool pair32_wanted(const PairParams& p, int ti, unsigned mask) {
+    const unsigned want_a = 1u << (p.tb & 31), want_b = 1u << (p.ta & 31);
+    return (mask & ((ti == p.ta ? want_a : 0u) | (ti == p.tb ? want_b : 0u))) != 0u;
+}
+
 template <int LANES>
 __global__ void __launch_bounds__(512) k_pair32(PairParams p, const PosPack* __restrict__ pack,
                                                 const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
@@ -49,68 +115,52 @@ __global__ void __launch_bounds__(512) k_pair32(PairParams p, const PosPack* __r
                                                 const unsigned* __restrict__ nbmask) {
     const int lane = threadIdx.x & (LANES - 1);
     const int per_block = blockDim.x / LANES;
-    // a typed pair: the partner type(s) a centre of each type looks for
-    const unsigned want_a = 1u << (p.tb & 31), want_b = 1u << (p.ta & 31);
     for (int base = blockIdx.x * per_block; base < p.n; base += gridDim.x * per_block) {
         int i = base + threadIdx.x / LANES;
         bool valid = i < p.n;
         int ii = valid ? i : p.n - 1;
         PosPack pi = pack[ii];
         int ti = pack_type(pi.hi);
-        const ShiftF L = p.rep_L ? p.rep_L[p.rep_of[ii]] : p.L;
-        bool any = valid && (p.all_types || ti == p.ta || ti == p.tb);
-        // with the rows' type masks, a row without the partner type is skipped
-        // whole (most rows of a mixed system: a Si atom with no Ar near)
-        if (any && !p.all_types)
-            any = (nbmask[ii] & ((ti == p.ta ? want_a : 0u) | (ti == p.tb ? want_b : 0u))) != 0u;
-        int m = any ? nnb[ii] : 0;
+        const bool any = valid && (p.all_types || pair32_wanted(p, ti, nbmask[ii]));
+        const int m = any ? nnb[ii] : 0;
         Kahan ax, ay, az, ae;
         float av = 0.f;
-        for (int s = lane; s < m; s += LANES) {
-            unsigned e = __ldg(&nbr[nbr_at(ii, s, p.hshift, p.maxnb)]);
-            int j = nbr_index(e);
-            const float4* pj = reinterpret_cast<const float4*>(pack + j);
-            const float4 hj = __ldg(pj);  // the type word first: most rows of a mixed system skip here
-            if (!p.all_types && !types_match(ti, pack_type(hj), p.ta, p.tb)) continue;
-            const float4 lj = __ldg(pj + 1);
-            float3 d = pair_delta(pi.hi, pi.lo, hj, lj, e, L);
-            float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
-            if (r2 >= p.rc2) continue;
-            float rinv = rsqrtf(r2);
-            float r = r2 * rinv;
-            if (!(r < p.rc)) continue;
-            float ph, dph;
-            tab_read(p.phi, p.phi.coef, r, rinv, ph, dph, status);
-            float fr = -dph * rinv;
-            ax.add(d.x * fr);
-            ay.add(d.y * fr);
-            az.add(d.z * fr);
-            ae.add(0.5f * ph);
-            av = fmaf(fr, r2, av);
-        }
-        lanes_twosum<LANES>(ax.s, ax.c);
-        lanes_twosum<LANES>(ay.s, ay.c);
-        lanes_twosum<LANES>(az.s, az.c);
-        lanes_twosum<LANES>(ae.s, ae.c);
-#pragma unroll
-        for (int off = LANES / 2; off > 0; off >>= 1) av += __shfl_xor_sync(0xffffffffu, av, off);
-        if (lane == 0 && valid) {
-            float vfx = __fsub_rn(ax.s, ax.c), vfy = __fsub_rn(ay.s, ay.c), vfz = __fsub_rn(az.s, az.c);
-            float ve = __fsub_rn(ae.s, ae.c);
-            if (p.first) {
-                fx[i] = vfx;
-                fy[i] = vfy;
-                fz[i] = vfz;
-                pe[i] = ve;
-                vir[i] = av;
-            } else if (m) {
-                fx[i] += vfx;
-                fy[i] += vfy;
-                fz[i] += vfz;
-                pe[i] += ve;
-                vir[i] += av;
-            }
-        }
+        pair32_sum<LANES>(p, pack, nbr, ii, pi, ti, m, lane, ax, ay, az, ae, av, status);
+        if (lane == 0 && valid) pair32_store(p, i, m, ax, ay, az, ae, av, fx, fy, fz, pe, vir);
+    }
+}
+
+// The typed pair where the chip is full: a warp looks at 32 atoms with one
+// coalesced load each (type, mask), compacts those with a partner, and takes
+// them 32 / LANES at a time.  In the impact ensemble (1.47 M atoms, 256 Ar
+// atoms) LANES threads for every atom read every pack to find three thousand
+// rows: 122 us, now 20.
+template <int LANES>
+__global__ void __launch_bounds__(256) k_pair32_typed(PairParams p, const PosPack* __restrict__ pack,
+                                                      const int* __restrict__ type,
+                                                      const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
+                                                      float* __restrict__ fx, float* __restrict__ fy,
+                                                      float* __restrict__ fz, float* __restrict__ pe,
+                                                      float* __restrict__ vir, unsigned* status,
+                                                      const unsigned* __restrict__ nbmask) {
+    __shared__ int s_act[256];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, wl = threadIdx.x & 31;
+    const bool any = t < p.n && pair32_wanted(p, type[t], nbmask[t]);
+    const unsigned act = __ballot_sync(0xffffffffu, any);
+    int* const mine = s_act + (threadIdx.x & ~31);
+    if (any) mine[__popc(act & ((1u << wl) - 1u))] = t;
+    if (p.first && t < p.n && !any) fx[t] = fy[t] = fz[t] = pe[t] = vir[t] = 0.f;
+    __syncwarp();
+    const int lane = threadIdx.x & (LANES - 1), count = __popc(act);
+    for (int k = 0; k < count; k += 32 / LANES) {
+        const bool valid = k + wl / LANES < count;
+        const int i = mine[valid ? k + wl / LANES : 0];
+        const PosPack pi = pack[i];
+        const int m = valid ? nnb[i] : 0;
+        Kahan ax, ay, az, ae;
+        float av = 0.f;
+        pair32_sum<LANES>(p, pack, nbr, i, pi, pack_type(pi.hi), m, lane, ax, ay, az, ae, av, status);
+        if (lane == 0 && valid) pair32_store(p, i, m, ax, ay, az, ae, av, fx, fy, fz, pe, vir);
     }
 }
 
@@ -253,8 +303,17 @@ static void launch64(Context* c, const PairParams& p) {
     else launch64<32>(c, p);
 }
 
+constexpr int PAIR_TYPED_PER_SM = 256;  // atoms per SM from which typed pairs compact their rows
+
 template <int LANES>
 static void launch32(Context* c, const PairParams& p, int block) {
+    // below this a warp per 32 atoms would not fill the chip
+    if (!p.all_types && c->n >= PAIR_TYPED_PER_SM * c->num_sms) {
+        k_pair32_typed<LANES><<<grid_for(c->n, 256), 256, 0, c->stream>>>(
+            p, c->pack, c->type, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->fx, c->fy, c->fz, c->pe,
+            c->vir, c->d_status, c->nbmask);
+        return;
+    }
     int per_block = block / LANES;
     k_pair32<LANES><<<grid_for(c->n, per_block), block, 0, c->stream>>>(
         p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->fx, c->fy, c->fz, c->pe, c->vir,

@@ -169,3 +169,45 @@ def test_fp64_pair_below_the_first_knot(omdg_lib, gap, later):
             with pytest.raises(omdg_lib.OMDGError) as err:
                 ctx.compute_forces()
             assert err.value.code in (omdg_lib.OMDG_ERANGE, omdg_lib.OMDG_EOVERLAP)
+
+
+# Typed FP32 pairs in a box large enough for the compacted rows (256 atoms a
+# SM and more), dilute and half and half, one and two type pairs, a number of
+# atoms that leaves the last warp ragged, against the oracle.
+@pytest.mark.parametrize("share,pairs,lanes", [(0.001, [(0, 1)], 8), (0.5, [(0, 1), (1, 1)], 4),
+                                               (0.02, [(1, 1), (0, 1)], 32)])
+def test_typed_pair_in_a_large_box_matches_oracle(omdg_lib, oracle_lib, share, pairs, lanes):
+    from objectmd_gb300 import inputs
+
+    oc = oracle_lib
+    x, _, (lo, hi) = inputs.lj_argon(ncell=22)
+    x = inputs.perturb(x, 0.15, 9, lo, hi)[:-5]
+    n = len(x)
+    types = (np.random.default_rng(10).uniform(size=n) < share).astype(np.int32)
+    phi = oc.Table.from_file(LJ, "")
+    box = oc.make_box(lo, hi, (1, 1, 1))
+    nb = oc.neighbors(box, x, phi.max_range() + 0.3)
+    f, e, w = np.zeros((n, 3)), np.zeros(n), np.zeros(n)
+    for a, b in pairs:
+        oc.pair_table_typed(box, x, types, a, b, nb, phi, f, e, w)
+    with omdg_lib.Context(0) as ctx:
+        ctx.set_box(lo, hi)
+        ctx.set_atoms(x, types=types, masses=[inputs.md_mass("argon")] * 2, znum=[18.0] * 2)
+        for a, b in pairs:
+            ctx.add_pair_table(LJ, a, b)
+        ctx.set_neighbor(0.3, 1)
+        ctx.set_launch("pair_lanes", lanes)
+        ctx.compute_forces()
+        st = ctx.get_state()
+    assert np.linalg.norm(st["f"] - f) / np.linalg.norm(f) <= 1e-5
+    assert np.array_equal(np.abs(st["f"]).sum(1) == 0.0, np.abs(f).sum(1) == 0.0)
+    # the table ends in a jump (it is not shifted): a pair within FP32's
+    # rounding of the cutoff may fall on either side of it
+    off, j, code = nb
+    i = np.repeat(np.arange(n), np.diff(off))
+    shift = np.stack([code % 3 - 1, code // 3 % 3 - 1, code // 9 - 1], 1) * (np.asarray(hi) - lo)
+    r = np.linalg.norm(x[i] - x[j] - shift, axis=1)
+    clear = np.ones(n, dtype=bool)
+    clear[i[np.abs(r - phi.max_range()) < 4e-6]] = False
+    assert clear.mean() > 0.99
+    assert np.abs(st["pot"] - e)[clear].max() <= 2e-6
