@@ -25,7 +25,7 @@ int step_state_fetch(Context* c, unsigned* status, long long* step, int* row, do
 int step_state_rewind(Context* c);
 int step_clear_rebuild(Context* c);
 int step_flag_requested_replicas(Context* c);
-int launch_set_rebuild_cond(Context* c, cudaGraphConditionalHandle h);
+int launch_take_rebuild(Context* c);
 int threebody_prepare(Context* c);
 
 int set_error(Context* c, int code, const std::string& msg) {
@@ -929,9 +929,18 @@ static int build_list(Context* c) {
 int forces_compute(Context* c) {
     if (c->pots.empty()) return set_error(c, OMDG_ESTATE, "no force kernel");
     c->kick_fused = false;
+    c->gather_deferred = false;
+    if (!c->fuse_kick) c->wide_cleared = false;  // not a step's evaluation
     bool first = true;
+    // in a step the last slot gather joins the kick, unless a modify or the
+    // detector works on the forces in between
+    const Potential* last_slots = nullptr;
+    if (c->fuse_kick && !c->use_f64 && c->post_ops.empty() && !c->ttm)
+        for (auto& p : c->pots)
+            if (!p.fallback_only && (p.kind == POT_SW || p.kind == POT_TERSOFF || p.kind == POT_NN)) last_slots = &p;
     for (auto& p : c->pots) {
         if (p.fallback_only) continue;  // run by the potential that owns it
+        c->defer_gather = &p == last_slots;
         if (c->nrep > 0 && p.kind != POT_TERSOFF && p.kind != POT_ZBL && !(p.kind == POT_PAIR && !p.fp64))
             return set_error(c, OMDG_EINVAL, "replica mode evaluates Tersoff, ZBL and FP32 pair-table kernels only");
         int rc = OMDG_OK;
@@ -943,9 +952,11 @@ int forces_compute(Context* c) {
             case POT_ZBL: rc = zbl_launch(c, p, first); break;
             case POT_NN: rc = nn_launch(c, p, first); break;
         }
+        c->defer_gather = false;
         if (rc) return rc;
         first = false;
     }
+    c->wide_cleared = false;
     return post_force_modifies(c);  // MODIFY_POST_FORCE (integrator.cpp:215)
 }
 
@@ -992,18 +1003,18 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr)
     long l0 = c->launches, l1 = 0, l2 = 0;
     int rc = (c->ttm && ttm_active(c)) ? ttm_pre(c) : OMDG_OK;  // PreIntegration (TTM_Homogen_SCNA.h:352)
     if (!rc) rc = energy_source(c);                                 // PreIntegration (EnergySource.h:113)
-    if (!rc) rc = integrate_kick_drift(c, 0);
     cudaGraph_t g = nullptr;
     cudaStreamCaptureStatus cst;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
     cudaGraphConditionalHandle h = 0;
     if (!rc) {
+        // no rebuild unless the step's kick_drift asks for it
         e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, nullptr, nullptr, nullptr);
-        if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, 0);
+        if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
         if (e != cudaSuccess) rc = check_cuda(c, e, "conditional handle");
     }
-    if (!rc) rc = launch_set_rebuild_cond(c, h);
+    if (!rc) rc = integrate_kick_drift(c, &h);
     l1 = c->launches;
     cudaGraphNode_t cond_node = nullptr;
     if (!rc) {
@@ -1026,7 +1037,8 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr)
                 c->stream = gs.side;
                 c->build_in_step = true;
                 c->build_partial = c->nrep > 0;  // the flagged replicas only
-                rc = nlist_build(c);
+                rc = launch_take_rebuild(c);
+                if (!rc) rc = nlist_build(c);
                 c->build_partial = false;
                 c->build_in_step = false;
                 c->stream = s;
@@ -1041,10 +1053,11 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr)
     c->fuse_kick = true;
     if (!rc) rc = forces_compute(c);
     c->fuse_kick = false;
-    if (!rc && io) rc = branch(1, nullptr, nullptr, io[2]);
+    const bool f_after = c->gather_deferred;  // the kick completes the forces
+    if (!rc && io && !f_after) rc = branch(1, nullptr, nullptr, io[2]);
     if (!rc) rc = integrate_kick(c, 0);
     if (!rc && c->ttm) rc = thermo_detect(c, true);  // ExecuteDetectors (system.cpp:976)
-    if (!rc && io) rc = branch(2, nullptr, io[1], nullptr);
+    if (!rc && io) rc = branch(2, nullptr, io[1], f_after ? io[2] : nullptr);
     if (!rc && io_launches > 0) {  // join the branch
         e = cudaEventRecord(gs.io_ev[3], gs.io_side);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s, gs.io_ev[3], 0);
@@ -1371,7 +1384,7 @@ int omdg_step_async(omdg_ctx* c, int nsteps) {
         for (int k = 0; k < nsteps; k++) {
             if (c->ttm && ttm_active(c) && (rc = ttm_pre(c))) return rc;
             if ((rc = energy_source(c))) return rc;
-            if ((rc = integrate_kick_drift(c, k))) return rc;
+            if ((rc = integrate_kick_drift(c, nullptr))) return rc;
             c->build_in_step = true;
             rc = eager_maybe_rebuild(c);
             c->build_in_step = false;

@@ -21,6 +21,8 @@
 
 namespace omdg {
 
+constexpr int KICK_BLOCKS_SM = 6;
+
 __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __restrict__ x, double* __restrict__ y,
                                                     double* __restrict__ z, double* __restrict__ vx,
                                                     double* __restrict__ vy, double* __restrict__ vz,
@@ -29,10 +31,18 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __re
                                                     const int* __restrict__ type, PosPack* __restrict__ pack,
                                                     const float4* __restrict__ xref, unsigned* __restrict__ aflag,
                                                     StepState* st, const int* __restrict__ rep_of,
-                                                    int* __restrict__ rflag) {
+                                                    int* __restrict__ rflag, int* __restrict__ wide,
+                                                    cudaGraphConditionalHandle cond, int has_cond) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     __shared__ int moved;
-    if (threadIdx.x == 0) moved = 0;
+    bool asked = false;  // a rebuild requested before this step (periodic, a state upload)
+    if (threadIdx.x == 0) {
+        moved = 0;
+        if (blockIdx.x == 0) {
+            asked = has_cond && st->rebuild;
+            if (wide) *wide = 0;  // the three-body passes' queue of this step
+        }
+    }
     __syncthreads();
     bool self_moved = false;  // replica mode: flag this atom's replica
     unsigned fl = 1u;
@@ -102,30 +112,58 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __re
     }
     if (self_moved && rflag) rflag[rep_of[i]] = 1;
     __syncthreads();
-    if (threadIdx.x == 0 && moved) st->rebuild = 1;
+    if (threadIdx.x == 0) {
+        if (moved) st->rebuild = 1;
+        // the step graph's rebuild node runs (its default is not to); the
+        // body's first kernel takes the request (k_take_rebuild)
+        if (has_cond && (moved || asked) && !st->halted) cudaGraphSetConditional(cond, 1u);
+    }
 }
 
 
 // Second half kick v += dt/2 f/m (kick = 1) and the energy ledger: per
 // atom m v^2, the potential and the virial as FP32 pairs, a fixed xor tree
 // per warp and over the warps, FP32-pair block partials; the last block to
-// finish sums the partials in block order (finalize_block).
-__global__ void __launch_bounds__(RED_BLOCK, 2048 / RED_BLOCK) k_kick(IntParams p, FinParams f, double* __restrict__ vx,
-                                                    double* __restrict__ vy, double* __restrict__ vz,
-                                                    const float* __restrict__ fx, const float* __restrict__ fy,
-                                                    const float* __restrict__ fz, const double* __restrict__ f64,
-                                                    const int* __restrict__ type, const float* __restrict__ pe,
-                                                    const float* __restrict__ vir,
-                                                    const unsigned* __restrict__ aflag, BlockPartial* __restrict__ partial,
-                                                    double* __restrict__ ledger, StepState* st, int kick) {
-    const int i = blockIdx.x * RED_BLOCK + threadIdx.x;
+// finish sums the partials in block order (finalize_block).  A thread takes
+// every (grid's threads)-th atom, so that one tree (225 of the 580
+// instructions a warp needed for 32 atoms) serves several atoms and few
+// partials remain.
+// 1,048,576 EAM atoms 38.9 -> 30.7 us.
+// GATHER: the three-body kernels' slots are collected first (slot_sum), their
+// loads' latency beside the half-kick's FP64 work.  As two kernels and as one:
+// 512,000 Tersoff atoms 18.8 + 24.8 and 38.8 us, 194,184 Stillinger-Weber atoms
+// 22.3 + 20.0 and 34.4, 1.47 M atoms of the impact ensemble 57 + 54 and 85.
+template <bool GATHER>
+__global__ void __launch_bounds__(RED_BLOCK, KICK_BLOCKS_SM) k_kick(
+    IntParams p, FinParams f, SlotArgs ga, double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
+    float* __restrict__ fx, float* __restrict__ fy, float* __restrict__ fz, const double* __restrict__ f64,
+    const int* __restrict__ type, float* __restrict__ pe, float* __restrict__ vir,
+    const unsigned* __restrict__ aflag, BlockPartial* __restrict__ partial, double* __restrict__ ledger,
+    StepState* st, int kick) {
     F2 k = {0.f, 0.f}, e = {0.f, 0.f}, w = {0.f, 0.f};
     unsigned long long vmax = 0ull;  // bits of the largest squared speed
-    // inactive atoms: not integrated, not measured (system.cpp:1067, :1085)
-    if (i < p.n && (!aflag || (aflag[i] & 1u))) {
+    for (int i = blockIdx.x * RED_BLOCK + threadIdx.x; i < p.n; i += gridDim.x * RED_BLOCK) {
+        float gx, gy, gz, gp, gw;
+        if (!p.use_f64 || GATHER) {
+            gx = fx[i];
+            gy = fy[i];
+            gz = fz[i];
+            gp = pe[i];
+        }
+        gw = vir[i];
+        if (GATHER) {
+            slot_sum(ga, i, gx, gy, gz, gp);
+            fx[i] = gx;
+            fy[i] = gy;
+            fz[i] = gz;
+            pe[i] = gp;
+            if (ga.zero_virial) vir[i] = gw = 0.f;
+        }
+        // inactive atoms: not integrated, not measured (system.cpp:1067, :1085)
+        if (aflag && !(aflag[i] & 1u)) continue;
         const int t = type[i];
-        if (kick && !p.use_f64) {
-            kick_atom_terms(p, i, t, fx[i], fy[i], fz[i], pe[i], vir[i], st->hdtm[t], vx, vy, vz, k, e, w, vmax);
+        if (GATHER || (kick && !p.use_f64)) {
+            kick_atom_terms(p, i, t, gx, gy, gz, gp, gw, st->hdtm[t], vx, vy, vz, k, e, w, vmax);
         } else {
             double ux = vx[i], uy = vy[i], uz = vz[i];
             if (kick) {
@@ -139,15 +177,22 @@ __global__ void __launch_bounds__(RED_BLOCK, 2048 / RED_BLOCK) k_kick(IntParams 
             }
             const F2 sx = f2_from(ux), sy = f2_from(uy), sz = f2_from(uz);
             const F2 v2 = f2_add(f2_add(f2_mul(sx, sx), f2_mul(sy, sy)), f2_mul(sz, sz));
-            k = f2_mul(v2, F2{p.mh[t], p.ml[t]});
-            e = p.use_f64 ? f2_from(f64[3 * (size_t)p.n + i]) : F2{pe[i], 0.f};
-            w = F2{vir[i], 0.f};
+            k = f2_add(k, f2_mul(v2, F2{p.mh[t], p.ml[t]}));
+            e = f2_add(e, p.use_f64 ? f2_from(f64[3 * (size_t)p.n + i]) : F2{gp, 0.f});
+            w = f2_add(w, F2{gw, 0.f});
             if (p.need_vmax)  // sqrv = vx*vx + vy*vy + vz*vz (system.cpp:1086)
-                vmax = (unsigned long long)__double_as_longlong(
-                    __dadd_rn(__dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy)), __dmul_rn(uz, uz)));
+                vmax = max(vmax, (unsigned long long)__double_as_longlong(__dadd_rn(
+                                     __dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy)), __dmul_rn(uz, uz))));
         }
     }
     ledger_block(p, f, k, e, w, vmax, partial, ledger, st);
+}
+
+// Blocks of the kick: a whole number of atoms a thread, all blocks resident.
+static int kick_blocks(const Context* c) {
+    const int full = grid_for(c->n, RED_BLOCK);
+    const int per = grid_for(full, KICK_BLOCKS_SM * c->num_sms);
+    return grid_for(full, per);
 }
 
 struct GhostParams {
@@ -363,15 +408,19 @@ static IntParams int_params(Context* c) {
     return p;
 }
 
-int integrate_kick_drift(Context* c, int) {
+// cond: the step graph's rebuild node (capture only).  In a step the first
+// three-body pass finds its queue cleared here.
+int integrate_kick_drift(Context* c, const cudaGraphConditionalHandle* cond) {
     IntParams p = int_params(c);
+    c->wide_cleared = c->ters_wide != nullptr;
     prof_begin(c, "kick_drift");
     k_kick_drift<<<grid_for(c->n, 256), 256, 0, c->stream>>>(p, c->x, c->y, c->z, c->vx, c->vy, c->vz, c->fx, c->fy,
                                                              c->fz, c->f64, c->type, c->pack, c->xref,
                                                              c->flags_used ? c->aflag : nullptr,
                                                              reinterpret_cast<StepState*>(c->d_state),
                                                              c->nrep > 0 ? c->d_rep_of : nullptr,
-                                                             c->nrep > 0 ? c->d_rep_flag : nullptr);
+                                                             c->nrep > 0 ? c->d_rep_flag : nullptr, c->ters_wide,
+                                                             cond ? *cond : 0, cond ? 1 : 0);
     prof_end(c);
     c->launches++;
     return check_cuda(c, cudaGetLastError(), "kick_drift");
@@ -432,7 +481,7 @@ static int reduce_and_finalize(Context* c, int kick, int count_step) {
         return OMDG_OK;
     }
     IntParams p = int_params(c);
-    int nb = grid_for(c->n, RED_BLOCK);
+    int nb = kick_blocks(c);
     FinParams f = fin_params(c, p, count_step);
     if (c->thermo_count_ghosts && count_step && c->thermo_tau > 0.0) {
         // TempController::GetSystemTemperature divides by GetTotalAtom(), which
@@ -454,9 +503,13 @@ static int reduce_and_finalize(Context* c, int kick, int count_step) {
         c->launches += 2;
         f.ghosts = c->d_flags + 2;
     }
-    prof_begin(c, "kick");
-    k_kick<<<nb, RED_BLOCK, 0, c->stream>>>(p, f, c->vx, c->vy, c->vz, c->fx, c->fy, c->fz, c->f64, c->type, c->pe,
-                                            c->vir, c->flags_used ? c->aflag : nullptr,
+    const bool gather = kick && c->gather_deferred;
+    c->gather_deferred = false;
+    prof_begin(c, gather ? "gather_kick" : "kick");
+    auto kernel = gather ? k_kick<true> : k_kick<false>;
+    kernel<<<nb, RED_BLOCK, 0, c->stream>>>(p, f, slot_args(c, c->gather_zero_virial), c->vx, c->vy, c->vz, c->fx, c->fy,
+                                            c->fz, c->f64, c->type, c->pe, c->vir,
+                                            c->flags_used ? c->aflag : nullptr,
                                             reinterpret_cast<BlockPartial*>(c->d_red), c->d_ledger,
                                             reinterpret_cast<StepState*>(c->d_state), kick);
     prof_end(c);
@@ -724,29 +777,25 @@ int step_clear_rebuild(Context* c) {
     return check_cuda(c, cudaGetLastError(), "clear rebuild");
 }
 
-// Graph-side rebuild predicate: copies the request into the conditional
-// handle and clears it.
-// In replica mode a request for every replica sets every replica's flag
-// (the build then rebuilds the flagged replicas only).
-__global__ void k_set_rebuild_cond(StepState* st, cudaGraphConditionalHandle h, int nrep, int* rflag) {
-    const bool go = st->rebuild && !st->halted;
-    const bool all = st->rebuild_all != 0;
-    __syncthreads();
-    if (go && all && rflag)
+// The rebuild body's first kernel takes the request.  In replica mode a
+// request for every replica sets every replica's flag (the build then rebuilds
+// the flagged replicas only).
+__global__ void k_take_rebuild(StepState* st, int nrep, int* rflag) {
+    if (st->rebuild_all && rflag)
         for (int r = threadIdx.x; r < nrep; r += blockDim.x) rflag[r] = 1;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        cudaGraphSetConditional(h, go ? 1u : 0u);
-        if (go) st->nrebuild += 1;
+        st->nrebuild += 1;
         st->rebuild = 0;
-        if (go) st->rebuild_all = 0;
+        st->rebuild_all = 0;
     }
 }
 
-int launch_set_rebuild_cond(Context* c, cudaGraphConditionalHandle h) {
-    k_set_rebuild_cond<<<1, 256, 0, c->stream>>>(reinterpret_cast<StepState*>(c->d_state), h, c->nrep,
-                                                 c->nrep > 0 ? c->d_rep_flag : nullptr);
+int launch_take_rebuild(Context* c) {
+    k_take_rebuild<<<1, 256, 0, c->stream>>>(reinterpret_cast<StepState*>(c->d_state), c->nrep,
+                                             c->nrep > 0 ? c->d_rep_flag : nullptr);
     c->launches++;
-    return check_cuda(c, cudaGetLastError(), "rebuild predicate");
+    return check_cuda(c, cudaGetLastError(), "rebuild request");
 }
 
 __global__ void k_zero_f(int n, float* fx, float* fy, float* fz, double* f64) {

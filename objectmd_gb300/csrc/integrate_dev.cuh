@@ -174,6 +174,53 @@ static __device__ __noinline__ void finalize_block(const FinParams& p, int nbloc
     }
 }
 
+// The slots that point at atom i (three-body kernels): what its neighbours'
+// centre passes left for it, added to its own part.  Four entries' loads are
+// in flight at a time (entry and reverse slot, then the slots): the pass is
+// bound by their latency.
+struct SlotArgs {
+    int hshift, maxnb;
+    const unsigned* nbr;
+    const int* nnb;
+    const int* rev;
+    const float4* slot;
+    int zero_virial;  // the reference SW does not accumulate a virial (sw.cpp:238)
+};
+
+__device__ __forceinline__ void slot_sum(const SlotArgs& a, int i, float& fx, float& fy, float& fz, float& pe) {
+    Kahan gx, gy, gz, ge;
+    gx.add(fx);
+    gy.add(fy);
+    gz.add(fz);
+    ge.add(pe);
+    const int m = a.nnb[i];
+    for (int s0 = 0; s0 < m; s0 += 4) {
+        unsigned e[4];
+        int r[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const size_t at = nbr_at(i, min(s0 + k, m - 1), a.hshift, a.maxnb);
+            e[k] = __ldg(a.nbr + at);
+            r[k] = __ldg(a.rev + at);
+        }
+        float4 c[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) c[k] = __ldg(a.slot + nbr_at(nbr_index(e[k]), r[k], a.hshift, a.maxnb));
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (s0 + k < m) {
+                gx.add(c[k].x);
+                gy.add(c[k].y);
+                gz.add(c[k].z);
+                ge.add(c[k].w);
+            }
+    }
+    fx = gx.value();
+    fy = gy.value();
+    fz = gz.value();
+    pe = ge.value();
+}
+
 // One atom's second half-kick v += dt/2 f/m (velocity written back) and
 // its ledger terms: m v^2 and the potential and virial as FP32 pairs, the
 // squared speed's bits for DynamicTimeStep.  f is FP32 (the FP64 force path
@@ -275,6 +322,9 @@ struct KickArgs {
     int partial_cap;
     StepState* st;
 };
+
+// The slot gather's arguments (threebody.cu).
+SlotArgs slot_args(const Context* c, bool zero_virial);
 
 bool kick_fusable(const Context* c);
 void kick_args(Context* c, KickArgs& ka);

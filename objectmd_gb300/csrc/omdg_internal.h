@@ -198,6 +198,10 @@ struct Context {
     bool build_partial = false;          // the build being issued rebuilds only the flagged replicas
     bool fuse_kick = false;              // the forces being issued are a step's: the kick may join them
     bool kick_fused = false;             // the last force launch did the step's second half-kick
+    bool defer_gather = false;           // the slot gather being issued may join the step's kick
+    bool gather_deferred = false;        // ... and does: the kick collects the slots
+    bool gather_zero_virial = false;
+    bool wide_cleared = false;           // this step's kick_drift cleared the queue of wide centres
     int ncell_cap = 0;
     int* scan_partials = nullptr;
     int* cell_sorted = nullptr;
@@ -383,7 +387,7 @@ int tersoff_launch(Context* c, Potential& p, bool first);
 int zbl_launch(Context* c, Potential& p, bool first);
 
 // integrator (integrate.cu)
-int integrate_kick_drift(Context* c, int step_index);
+int integrate_kick_drift(Context* c, const cudaGraphConditionalHandle* cond);
 int integrate_kick(Context* c, int step_index);
 int integrate_pack(Context* c);
 int measure_energies(Context* c, int row);

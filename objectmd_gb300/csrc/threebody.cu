@@ -14,7 +14,7 @@
 // atom, V3/3 to each triplet member (sw.cpp:182-233); Tersoff: 1/2 V_ij to i.
 #include <cmath>
 
-#include "device_common.cuh"
+#include "integrate_dev.cuh"
 
 namespace omdg {
 
@@ -338,34 +338,18 @@ __global__ void __launch_bounds__(128) k_sw_wide(SWDev p, const PosPack* __restr
 }
 
 // Gathers what every neighbour's pass A left for i; clears no state.
-__global__ void __launch_bounds__(128) k_slot_gather(int n, int hshift, int maxnb, const unsigned* __restrict__ nbr,
-                                                     const int* __restrict__ nnb, const int* __restrict__ rev,
-                                                     const float4* __restrict__ slot, float* __restrict__ fx,
+__global__ void __launch_bounds__(128) k_slot_gather(int n, SlotArgs a, float* __restrict__ fx,
                                                      float* __restrict__ fy, float* __restrict__ fz,
-                                                     float* __restrict__ pe, float* __restrict__ vir,
-                                                     int zero_virial) {
+                                                     float* __restrict__ pe, float* __restrict__ vir) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    Kahan gx, gy, gz, ge;
-    gx.add(fx[i]);
-    gy.add(fy[i]);
-    gz.add(fz[i]);
-    ge.add(pe[i]);
-    const int m = nnb[i];
-    for (int s = 0; s < m; s++) {
-        const size_t at = nbr_at(i, s, hshift, maxnb);
-        const int j = nbr_index(nbr[at]);
-        const float4 c = slot[nbr_at(j, rev[at], hshift, maxnb)];
-        gx.add(c.x);
-        gy.add(c.y);
-        gz.add(c.z);
-        ge.add(c.w);
-    }
-    fx[i] = gx.value();
-    fy[i] = gy.value();
-    fz[i] = gz.value();
-    pe[i] = ge.value();
-    if (zero_virial) vir[i] = 0.f;  // the reference SW does not accumulate a virial (sw.cpp:238)
+    float gx = fx[i], gy = fy[i], gz = fz[i], ge = pe[i];
+    slot_sum(a, i, gx, gy, gz, ge);
+    fx[i] = gx;
+    fy[i] = gy;
+    fz[i] = gz;
+    pe[i] = ge;
+    if (a.zero_virial) vir[i] = 0.f;
 }
 
 // ------------------------------------------------------------------ Tersoff
@@ -730,14 +714,31 @@ __global__ void __launch_bounds__(128) k_zbl(ZBLDev p, const PosPack* __restrict
 // ------------------------------------------------------------------ host
 int threebody_prepare(Context* c) { return OMDG_OK; }
 
+SlotArgs slot_args(const Context* c, bool zero_virial) {
+    return SlotArgs{c->nbr_hshift, c->maxnb, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->rev, c->slot_buf,
+                    zero_virial ? 1 : 0};
+}
+
+// In a step the last gather before the kick joins it (forces_compute decides).
 int gather_slots(Context* c, bool zero_virial) {
+    if (c->defer_gather) {
+        c->gather_deferred = true;
+        c->gather_zero_virial = zero_virial;
+        return OMDG_OK;
+    }
     prof_begin(c, "slot_gather");
-    k_slot_gather<<<grid_for(c->n, 128), 128, 0, c->stream>>>(
-        c->n, c->nbr_hshift, c->maxnb, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->rev, c->slot_buf, c->fx,
-        c->fy, c->fz, c->pe, c->vir, zero_virial ? 1 : 0);
+    k_slot_gather<<<grid_for(c->n, 128), 128, 0, c->stream>>>(c->n, slot_args(c, zero_virial), c->fx, c->fy, c->fz,
+                                                              c->pe, c->vir);
     prof_end(c);
     c->launches++;
     return check_cuda(c, cudaGetLastError(), "slot gather");
+}
+
+// The queue of wide centres is empty: cleared by the step's kick_drift for the
+// first pass of a step, here for every other pass.
+static void clear_wide(Context* c) {
+    if (!c->wide_cleared) cudaMemsetAsync(c->ters_wide, 0, sizeof(int), c->stream);
+    c->wide_cleared = false;
 }
 
 int sw_launch(Context* c, Potential& pot, bool first) {
@@ -784,7 +785,7 @@ int sw_launch(Context* c, Potential& pot, bool first) {
     p.ze3 = (float)s.ze3;
     p.first = first ? 1 : 0;
     prof_begin(c, "sw_centre");
-    cudaMemsetAsync(c->ters_wide, 0, sizeof(int), c->stream);
+    clear_wide(c);
     k_sw_a<<<grid_for(c->n, 128), 128, 0, c->stream>>>(p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb,
                                                         c->slot_buf, c->fx, c->fy, c->fz, c->pe, c->d_status,
                                                         c->ters_wide);
@@ -834,7 +835,7 @@ int tersoff_centre(Context* c, Potential& pot, bool first, const int* mask, cons
     p.rc2 = p.rc * p.rc * 1.0001f;
     p.first = first ? 1 : 0;
     prof_begin(c, mask ? "tersoff_fallback" : "tersoff_centre");
-    cudaMemsetAsync(c->ters_wide, 0, sizeof(int), c->stream);
+    clear_wide(c);
     // a masked pass (the surrogate's fallback, usually for no centre at all)
     // takes the strided form: one resident grid, each block gone after
     // reading the count
