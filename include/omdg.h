@@ -203,9 +203,10 @@ int omdg_stats(omdg_ctx* ctx, long* rebuilds, long* launches);
 int omdg_replica_builds(omdg_ctx* ctx, int* builds, int nrep);
 /*
  * No reference counterpart (the reference has one scalar loop per potential).
- * Centres the last Stillinger-Weber or Tersoff force pass queued for the
- * dense second pass (k_sw_wide / k_tersoff_wide: more in-cutoff neighbours
- * than the register path holds, 8 for SW and 4 for Tersoff).  Synchronous.
+ * Centres of the last Stillinger-Weber or Tersoff force pass with more
+ * in-cutoff neighbours than the register path holds (8 for SW, 4 for Tersoff):
+ * eight lanes evaluate each of them, as they do every centre of a small
+ * system.  Synchronous.
  */
 int omdg_wide_centres(omdg_ctx* ctx, int* count);
 

@@ -340,6 +340,7 @@ int omdg_destroy(omdg_ctx* c) {
     cudaFree(c->nbr);
     cudaFree(c->rev);
     cudaFree(c->slot_buf);
+    cudaFree(c->row_hits);
     tile_release(c);
     cudaFree(c->cell_count);
     cudaFree(c->cell_start);
@@ -506,9 +507,11 @@ int omdg_set_atoms(omdg_ctx* c, int n, const double* x, const double* v, const i
     cudaFree(c->nbr);
     cudaFree(c->rev);
     cudaFree(c->slot_buf);
+    cudaFree(c->row_hits);
     c->nbr = nullptr;
     c->rev = nullptr;
     c->slot_buf = nullptr;
+    c->row_hits = nullptr;
     invalidate_graph(c);
     return integrate_pack(c);
 }
@@ -1948,9 +1951,11 @@ int omdg_set_launch(omdg_ctx* c, const char* key, int value) {
         cudaFree(c->nbr);
         cudaFree(c->rev);
         cudaFree(c->slot_buf);
+        cudaFree(c->row_hits);
         c->nbr = nullptr;
         c->rev = nullptr;
         c->slot_buf = nullptr;
+        c->row_hits = nullptr;
         if (m > 0) {
             int rc = nlist_reserve(c, m);
             if (rc) return rc;

@@ -130,9 +130,9 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __re
 // partials remain.
 // 1,048,576 EAM atoms 38.9 -> 30.7 us.
 // GATHER: the three-body kernels' slots are collected first (slot_sum), their
-// loads' latency beside the half-kick's FP64 work.  As two kernels and as one:
-// 512,000 Tersoff atoms 18.8 + 24.8 and 38.8 us, 194,184 Stillinger-Weber atoms
-// 22.3 + 20.0 and 34.4, 1.47 M atoms of the impact ensemble 57 + 54 and 85.
+// loads' latency beside the half-kick's FP64 work: 512,000 Tersoff atoms 32.9
+// us, 194,184 Stillinger-Weber atoms 27.0, 1.47 M atoms of the impact ensemble
+// 70 (as two kernels, over every slot of the list, 43.6, 42.3 and 111).
 template <bool GATHER>
 __global__ void __launch_bounds__(RED_BLOCK, KICK_BLOCKS_SM) k_kick(
     IntParams p, FinParams f, SlotArgs ga, double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,

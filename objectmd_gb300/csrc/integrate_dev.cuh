@@ -4,7 +4,7 @@
 // block partials and last-block finalisation.
 #pragma once
 
-#include "device_common.cuh"
+#include "rows.cuh"
 
 namespace omdg {
 
@@ -174,16 +174,16 @@ static __device__ __noinline__ void finalize_block(const FinParams& p, int nbloc
     }
 }
 
-// The slots that point at atom i (three-body kernels): what its neighbours'
-// centre passes left for it, added to its own part.  Four entries' loads are
-// in flight at a time (entry and reverse slot, then the slots): the pass is
-// bound by their latency.
+// What the neighbours' centre passes left for atom i (three-body kernels), in
+// the slots of its own row's hits, added to its own part.  Four slots' loads
+// are in flight at a time.  The row's other entries count as the zeros that
+// they are: one of them after a hit folds a compensation of just half a unit
+// in the last place into the sum (to even), and the rest change nothing.
 struct SlotArgs {
     int hshift, maxnb;
-    const unsigned* nbr;
     const int* nnb;
-    const int* rev;
     const float4* slot;
+    RowHits hits;
     int zero_virial;  // the reference SW does not accumulate a virial (sw.cpp:238)
 };
 
@@ -194,27 +194,37 @@ __device__ __forceinline__ void slot_sum(const SlotArgs& a, int i, float& fx, fl
     gz.add(fz);
     ge.add(pe);
     const int m = a.nnb[i];
-    for (int s0 = 0; s0 < m; s0 += 4) {
-        unsigned e[4];
-        int r[4];
+    int w0 = 0, s = -1;
+    do {
+        unsigned bits = a.hits.word(i, w0);
+        while (bits) {
+            float4 c[4];
+            bool gap[4];
+            int nk = 0;
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const size_t at = nbr_at(i, min(s0 + k, m - 1), a.hshift, a.maxnb);
-            e[k] = __ldg(a.nbr + at);
-            r[k] = __ldg(a.rev + at);
-        }
-        float4 c[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) c[k] = __ldg(a.slot + nbr_at(nbr_index(e[k]), r[k], a.hshift, a.maxnb));
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (s0 + k < m) {
-                gx.add(c[k].x);
-                gy.add(c[k].y);
-                gz.add(c[k].z);
-                ge.add(c[k].w);
+            for (int k = 0; k < 4; k++) {
+                if (bits) {
+                    const int next = w0 + __ffs(bits) - 1;
+                    gap[k] = next != s + 1;
+                    s = next;
+                    bits &= bits - 1u;
+                    nk++;
+                }
+                c[k] = __ldg(a.slot + nbr_at(i, s, a.hshift, a.maxnb));
             }
-    }
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k < nk) {
+                    if (gap[k]) gx.add(0.f), gy.add(0.f), gz.add(0.f), ge.add(0.f);
+                    gx.add(c[k].x);
+                    gy.add(c[k].y);
+                    gz.add(c[k].z);
+                    ge.add(c[k].w);
+                }
+        }
+        w0 += 32;
+    } while (w0 < m);
+    if (s + 1 < m) gx.add(0.f), gy.add(0.f), gz.add(0.f), ge.add(0.f);
     fx = gx.value();
     fy = gy.value();
     fz = gz.value();

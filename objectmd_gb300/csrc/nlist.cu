@@ -1098,14 +1098,18 @@ int nlist_reserve(Context* c, int maxnb) {
     cudaFree(c->nbr);
     cudaFree(c->rev);
     cudaFree(c->slot_buf);
+    cudaFree(c->row_hits);
     c->nbr = nullptr;
     c->rev = nullptr;
     c->slot_buf = nullptr;
+    c->row_hits = nullptr;
     if (cudaMalloc(&c->nbr, need) != cudaSuccess) return set_error(c, OMDG_ENOMEM, "neighbour list allocation");
     if (c->need_rev) {
         if (cudaMalloc(&c->rev, need) != cudaSuccess) return set_error(c, OMDG_ENOMEM, "reverse slot allocation");
         if (cudaMalloc(&c->slot_buf, nlist_slots(c, maxnb) * sizeof(float4)) != cudaSuccess)
             return set_error(c, OMDG_ENOMEM, "slot buffer allocation");
+        if (cudaMalloc(&c->row_hits, sizeof(unsigned) * (size_t)((maxnb + 31) / 32) * c->cap) != cudaSuccess)
+            return set_error(c, OMDG_ENOMEM, "row hits allocation");
     }
     c->maxnb = maxnb;
     c->nbr_bytes = (long)need;

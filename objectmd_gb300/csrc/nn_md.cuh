@@ -3,42 +3,39 @@
 // counterpart).
 #pragma once
 
-#include "device_common.cuh"
 #include "nn_desc.cuh"
+#include "rows.cuh"
 
 namespace omdg {
 
 struct NNMD {
     int n, hshift, maxnb, first;
     ShiftF L;
-    float rc2;
+    float t2;      // r2 < t2: inside the descriptor cutoff (r2_below)
+    float hit_t2;  // r2 < hit_t2: a hit of the row (the wider of the descriptors' and the fallback's cutoff)
+    RowHits hits;
 };
 
-// Neighbours of i inside the descriptor cutoff: vectors x_j - x_i, distances
-// and list slots.  Returns the count (capped at NN_MAXN, overflow flagged).
-__device__ __forceinline__ int nn_gather(const NNMD& q, const NNDescParams& p, int i, const PosPack& pi,
-                                         const PosPack* __restrict__ pack, const unsigned* __restrict__ nbr, int m,
-                                         float* vx, float* vy, float* vz, float* rr, int* sl, unsigned* status) {
+// Neighbours of i inside the descriptor cutoff: vectors x_j - x_i and
+// distances.  Returns the count (capped at NN_MAXN, overflow flagged) and
+// stores the row's hit bits, which the force kernel goes by.
+__device__ __forceinline__ int nn_gather(const NNMD& q, int i, const PosPack& pi, const PosPack* __restrict__ pack,
+                                         const unsigned* __restrict__ nbr, int m, float* vx, float* vy, float* vz,
+                                         float* rr, unsigned* status) {
     int nc = 0;
-    for (int s = 0; s < m; s++) {
-        const unsigned e = nbr[nbr_at(i, s, q.hshift, q.maxnb)];
-        const PosPack pj = pack[nbr_index(e)];
-        const float3 d = pair_delta(pi.hi, pi.lo, pj.hi, pj.lo, e, q.L);  // x_i - x_j
-        const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
-        if (!(r2 < q.rc2)) continue;
-        const float r = sqrtf(r2);
-        if (!(r < p.rc)) continue;
-        if (nc < NN_MAXN) {
-            vx[nc] = -d.x;
-            vy[nc] = -d.y;
-            vz[nc] = -d.z;
-            rr[nc] = r;
-            sl[nc] = s;
-            nc++;
-        } else {
-            atomicOr(status, ERR_NBR_OVERFLOW);
-        }
-    }
+    scan_row<true, false>(i, m, pi, q.L, q.hit_t2, -1, pack, nbr, nullptr, q.hshift, q.maxnb, q.hits,
+                   [&](int, int, int, const float3& d, float r2) {
+                       if (!(r2 < q.t2)) return;
+                       if (nc < NN_MAXN) {
+                           vx[nc] = -d.x;
+                           vy[nc] = -d.y;
+                           vz[nc] = -d.z;
+                           rr[nc] = sqrtf(r2);
+                           nc++;
+                       } else {
+                           atomicOr(status, ERR_NBR_OVERFLOW);
+                       }
+                   });
     return nc;
 }
 
@@ -49,8 +46,7 @@ __device__ __forceinline__ void nn_md_descriptors(const NNMD& q, const NNDescPar
                                                   const PosPack* __restrict__ pack, const unsigned* __restrict__ nbr,
                                                   int m, float* g, unsigned* status) {
     float vx[NN_MAXN], vy[NN_MAXN], vz[NN_MAXN], rr[NN_MAXN];
-    int sl[NN_MAXN];
-    const int nc = nn_gather(q, p, i, pack[i], pack, nbr, m, vx, vy, vz, rr, sl, status);
+    const int nc = nn_gather(q, i, pack[i], pack, nbr, m, vx, vy, vz, rr, status);
 #pragma unroll
     for (int k = 0; k < NN_DESC; k++) g[k] = 0.f;
     for (int a = 0; a < nc; a++) {

@@ -4,7 +4,7 @@
 //                  with a descriptor outside the training range is flagged
 //   k_nn_mlp       the network on the tensor cores: E_i and u_i = dE_i/dG_i
 //   k_nn_md_force  u_i contracted with the descriptor derivatives: the force
-//                  on each neighbour goes to i's slot, the rest to i
+//                  on each neighbour goes to its row's slot, the rest to i
 //   k_tersoff_a    (fallback) plain Tersoff for the flagged centres only
 //   k_slot_gather  every atom collects the slots that point at it
 // Flagged atoms take their energy and forces from Tersoff; all others from the
@@ -52,25 +52,54 @@ __global__ void __launch_bounds__(128) k_nn_md_desc(NNMD q, NNDescParams p, cons
     if (out) atomicAdd(count, 1);
 }
 
+// The neighbours inside the descriptor cutoff again, from the row's hits, with
+// the slots their forces go to; other hits get their zero.
+__device__ __forceinline__ int nn_hits(const NNMD& q, int i, const PosPack& pi, const PosPack* __restrict__ pack,
+                                       const unsigned* __restrict__ nbr, int m, SlotRows slot, float* vx,
+                                       float* vy, float* vz, float* rr, int2* to) {
+    int nc = 0;
+    for (int w0 = 0; w0 < m; w0 += 32)
+        for (unsigned bits = q.hits.word(i, w0); bits; bits &= bits - 1u) {
+            const int s = w0 + __ffs(bits) - 1;
+            const size_t at = nbr_at(i, s, q.hshift, q.maxnb);
+            const unsigned e = __ldg(nbr + at);
+            const int r = __ldg(slot.rev + at);
+            PosPack pj;
+            ldg256(pack + nbr_index(e), pj.hi, pj.lo);
+            const float3 d = pair_delta(pi.hi, pi.lo, pj.hi, pj.lo, e, q.L);  // x_i - x_j
+            const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
+            if (r2 < q.t2 && nc < NN_MAXN) {
+                vx[nc] = -d.x;
+                vy[nc] = -d.y;
+                vz[nc] = -d.z;
+                rr[nc] = sqrtf(r2);
+                to[nc] = make_int2(nbr_index(e), r);
+                nc++;
+            } else {
+                slot.at(nbr_index(e), r) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+    return nc;
+}
+
 // STD holds the shared powers of both bases: 80 registers at six blocks per
 // SM, where unbounded it takes 96 (five blocks)
 template <bool STD>
 __global__ void __launch_bounds__(128, STD ? 6 : 7) k_nn_md_force(NNMD q, NNDescParams p, const PosPack* __restrict__ pack,
                                                      const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
                                                      const float* __restrict__ E, const float* __restrict__ U,
-                                                     const int* __restrict__ flag, float4* __restrict__ slot,
+                                                     const int* __restrict__ flag, SlotRows slot,
                                                      float* __restrict__ fx, float* __restrict__ fy,
                                                      float* __restrict__ fz, float* __restrict__ pe,
                                                      float* __restrict__ vir, unsigned* status) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= q.n) return;
     const int m = nnb[i];
-    for (int s = 0; s < m; s++) slot[nbr_at(i, s, q.hshift, q.maxnb)] = make_float4(0.f, 0.f, 0.f, 0.f);
     float ox = 0.f, oy = 0.f, oz = 0.f, oe = 0.f, ow = 0.f;
     if (!flag[i]) {
         float vx[NN_MAXN], vy[NN_MAXN], vz[NN_MAXN], rr[NN_MAXN], tx[NN_MAXN], ty[NN_MAXN], tz[NN_MAXN];
-        int sl[NN_MAXN];
-        const int nc = nn_gather(q, p, i, pack[i], pack, nbr, m, vx, vy, vz, rr, sl, status);
+        int2 to[NN_MAXN];
+        const int nc = nn_hits(q, i, pack[i], pack, nbr, m, slot, vx, vy, vz, rr, to);
         float u[NN_DESC];
         const float4* src = reinterpret_cast<const float4*>(U + (size_t)i * NN_DESC);
 #pragma unroll
@@ -131,13 +160,17 @@ __global__ void __launch_bounds__(128, STD ? 6 : 7) k_nn_md_force(NNMD q, NNDesc
             }
         }
         for (int a = 0; a < nc; a++) {
-            slot[nbr_at(i, sl[a], q.hshift, q.maxnb)] = make_float4(-tx[a], -ty[a], -tz[a], 0.f);
+            slot.at(to[a].x, to[a].y) = make_float4(-tx[a], -ty[a], -tz[a], 0.f);
             ox += tx[a];
             oy += ty[a];
             oz += tz[a];
             ow -= vx[a] * tx[a] + vy[a] * ty[a] + vz[a] * tz[a];  // (x_i - x_j) . dE_i/dx_j
         }
         oe = E[i];
+    } else {  // the fallback writes the slots of its own hits
+        for (int w0 = 0; w0 < m; w0 += 32)
+            for (unsigned bits = q.hits.word(i, w0); bits; bits &= bits - 1u)
+                slot.put(i, w0 + __ffs(bits) - 1, make_float4(0.f, 0.f, 0.f, 0.f));
     }
     if (q.first) {
         fx[i] = ox;
@@ -186,7 +219,10 @@ int nn_launch(Context* c, Potential& pot, bool first) {
     q.maxnb = c->maxnb;
     q.first = first ? 1 : 0;
     q.L = make_shift(c->box);
-    q.rc2 = s.model.dp.rc * s.model.dp.rc * 1.0001f;
+    const float rc_nn = s.model.dp.rc;
+    q.t2 = r2_below(rc_nn, rc_nn * rc_nn * 1.0001f);
+    q.hit_t2 = s.fallback >= 0 ? std::max(q.t2, tersoff_t2(c->pots[s.fallback].ters)) : q.t2;
+    q.hits = row_hits(c);
     const unsigned grid = (unsigned)grid_for(c->n, 128);
     const unsigned* nbr = reinterpret_cast<const unsigned*>(c->nbr);
     cudaMemsetAsync(s.count, 0, sizeof(int), c->stream);
@@ -211,7 +247,7 @@ int nn_launch(Context* c, Potential& pot, bool first) {
     if (e != cudaSuccess) return check_cuda(c, e, "surrogate network");
     prof_begin(c, "nn_force");
     auto force = std_ang ? k_nn_md_force<true> : k_nn_md_force<false>;
-    force<<<grid, 128, 0, c->stream>>>(q, s.model.dp, c->pack, nbr, c->nnb, s.E, s.U, s.flag, c->slot_buf, c->fx,
+    force<<<grid, 128, 0, c->stream>>>(q, s.model.dp, c->pack, nbr, c->nnb, s.E, s.U, s.flag, slot_rows(c), c->fx,
                                        c->fy, c->fz, c->pe, c->vir, c->d_status);
     prof_end(c);
     c->launches += 3;

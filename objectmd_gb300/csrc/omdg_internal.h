@@ -240,7 +240,8 @@ struct Context {
     int nbr_capacity = 0;       // launch key: the first build's row capacity (0: from the density)
     long overflow_recoveries = 0;  // queued steps replayed after a row overflow
     int* rev = nullptr;       // slot of i in row j (three-body kernels)
-    float4* slot_buf = nullptr;  // per-slot force contributions (three-body kernels)
+    float4* slot_buf = nullptr;  // per-slot force contributions (three-body kernels), of the rows' hits only
+    unsigned* row_hits = nullptr;  // hit bits of every row (rows.cuh), cap words per 32 entries
     int* ters_wide = nullptr;    // Tersoff centres past the register path: [0] count, then their indices
     int maxnb = 0;
     long nbr_bytes = 0;
@@ -398,6 +399,7 @@ int resolve_thermostat(Context* c);
 int gather_slots(Context* c, bool zero_virial);
 // mask: only centres i with mask[i] != 0; mask_count: device count of them
 // (0: the pass does no work)
+float tersoff_t2(const TersoffParams& t);  // squared distance below which Tersoff takes a neighbour
 int tersoff_centre(Context* c, Potential& pot, bool first, const int* mask, const int* mask_count = nullptr);
 int nn_launch(Context* c, Potential& pot, bool first);
 int replica_prepare(Context* c);  // per-replica cell grids and shifts (host, before a build)

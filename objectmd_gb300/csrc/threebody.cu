@@ -5,9 +5,13 @@
 //           i's pairs and the triplets (SW, sw.cpp:166-236) or bonds
 //           (Tersoff) whose centre is i.  The force and energy a term gives
 //           to i accumulate in registers; what it gives to a neighbour j is
-//           written to j's slot in i's row of a per-slot buffer.
-//   pass B  for atom i: own part + sum over i's slots s of the buffer entry
-//           its neighbour j wrote for i (slot rev(i,s) of j's row).
+//           written to i's slot in j's row of a per-slot buffer (rows.cuh).
+//   pass B  for atom i: own part + the slots of i's own row's hits.
+//
+// Pass A has two forms: a thread a centre with the neighbours in registers,
+// and eight lanes a centre with up to TB_MAXN neighbours in shared memory.
+// The second takes the centres that do not fit the first (queued), and every
+// centre of a system too small to fill the chip with one thread each.
 //
 // FP32 arithmetic on relative vectors from the FP64 positions, Kahan sums in
 // pass B.  Per-atom energies follow the reference: each pair half to each
@@ -20,26 +24,87 @@ namespace omdg {
 
 constexpr int TB_MAXN = 24;  // neighbours within the cutoff one atom can hold
 
-// f(b) for the in-cutoff neighbours b < nc: fully unrolled over K (the
-// arrays f touches stay in registers), or a rolled loop over local arrays
-// (then the kernel's register count stays that of the unrolled path).
-template <int K, bool UNR, class F>
-__device__ __forceinline__ void for_nbrs(int nc, F&& f) {
-    if constexpr (UNR) {
-#pragma unroll
-        for (int b = 0; b < K; b++)
-            if (b < nc) f(b);
-    } else {
-#pragma unroll 1
-        for (int b = 0; b < nc; b++) f(b);
-    }
-}
+// Below this many atoms a SM every centre takes eight lanes.  Thread and lane
+// form, us with some 5 of launch: Tersoff 512 atoms 16.5, 11.7; 8,000 16.4,
+// 13.0; 17,576 16.6, 17.3; SW 512 19.0, 11.6; 32,768 24.8, 17.8; 64,000 28.1,
+// 26.2; 140,608 39.0, 42.7.
+constexpr int TERS_LANE_PER_SM = 96;
+constexpr int SW_LANE_PER_SM = 400;
+constexpr int TB_BLOCK = 128;  // thread-a-centre kernels
+constexpr int TB_LANES = 8;    // lanes a centre in the other form
+constexpr int TB_LBLOCK = 64;
+constexpr int TB_LGROUPS = TB_LBLOCK / TB_LANES;
 
+// One group's centre in the lane form: its place in the block's warp.
+struct LaneGroup {
+    int lane, shift;
+    unsigned mask;
+    __device__ __forceinline__ LaneGroup()
+        : lane(threadIdx.x & (TB_LANES - 1)), shift(threadIdx.x & 31 & ~(TB_LANES - 1)),
+          mask(((1u << TB_LANES) - 1u) << shift) {}
+    __device__ __forceinline__ float sum(float v) const {
+#pragma unroll
+        for (int o = TB_LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+};
+
+// The neighbours of centre i inside the cutoff, in row order: vectors to them
+// with their squared distance in v[], list slots in sl[]; returns their number
+// (those past TB_MAXN are reported and get a zero slot).  A queued centre's
+// row was scanned before (hits.w holds at least its hits); the others' bits
+// are stored here.
+template <bool QUEUED>
+__device__ __forceinline__ int lanes_collect(const LaneGroup& g, int i, int m, const PosPack& pi, const ShiftF& L,
+                                             float t2, int type, const PosPack* __restrict__ pack,
+                                             const unsigned* __restrict__ nbr, int hshift, int maxnb,
+                                             const RowHits& hits, const SlotRows& slot, float4* v, int* sl,
+                                             unsigned* status) {
+    int nc = 0;
+    int w0 = 0;
+    do {
+        const unsigned want = QUEUED ? hits.word(i, w0) : 0xffffffffu;
+        float4 d[4];
+        unsigned bits = 0u;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int b = j * TB_LANES + g.lane;
+            bool in = false;
+            if (w0 + b < m && ((want >> b) & 1u)) {
+                const unsigned e = __ldg(nbr + nbr_at(i, w0 + b, hshift, maxnb));
+                PosPack pj;
+                ldg256(pack + nbr_index(e), pj.hi, pj.lo);
+                const float3 x = pair_delta(pi.hi, pi.lo, pj.hi, pj.lo, e, L);
+                d[j] = make_float4(-x.x, -x.y, -x.z, fmaf(x.z, x.z, fmaf(x.y, x.y, x.x * x.x)));
+                in = d[j].w < t2 && (type < 0 || pack_type(pj.hi) == type);
+            }
+            bits |= ((__ballot_sync(g.mask, in) >> g.shift) & ((1u << TB_LANES) - 1u)) << (j * TB_LANES);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int b = j * TB_LANES + g.lane;
+            if (!((bits >> b) & 1u)) continue;
+            const int k = nc + __popc(bits & ((1u << b) - 1u));
+            if (k < TB_MAXN) {
+                v[k] = d[j];
+                sl[k] = w0 + b;
+            } else {
+                slot.put(i, w0 + b, make_float4(0.f, 0.f, 0.f, 0.f));
+                atomicOr(status, ERR_NBR_OVERFLOW);
+            }
+        }
+        nc += __popc(bits);
+        if (!QUEUED && g.lane == 0) hits.word(i, w0) = bits;
+        w0 += 32;
+    } while (w0 < m);
+    __syncwarp(g.mask);
+    return nc;
+}
 
 struct SWDev {
     int n, hshift, maxnb, single_type, ta;
     ShiftF L;
-    float rc, rc2;
+    float rc, t2;  // t2: r2 < t2 is "inside the cutoff" (r2_below); r == rc is outside, where 1/(r - rc) is infinite
     float A, B, p, q, sigma, eps;
     float c1, c2, c3, c4, c5, c6, c7, c8, c9, c10;
     int usezbl;
@@ -49,9 +114,8 @@ struct SWDev {
     int ip, iq;  // p and q as integers when they are (then r^-p by multiplication), else -1
 };
 
-// r^-k for a small non-negative integer k
-__device__ __forceinline__ float inv_ipow(float r, int k) {
-    const float ir = 1.0f / r;
+// r^-k for a small non-negative integer k, from ir = 1/r
+__device__ __forceinline__ float inv_ipow(float ir, int k) {
     float res = 1.0f, b = ir;
     while (k > 0) {
         if (k & 1) res *= b;
@@ -61,15 +125,14 @@ __device__ __forceinline__ float inv_ipow(float r, int k) {
     return res;
 }
 
-__device__ __forceinline__ void sw_two_body(const SWDev& p, float r, float& fr, float& half_e) {
+// One half of a pair at distance r; ir = 1/r, ira = 1/(r - rc).
+__device__ __forceinline__ void sw_two_body(const SWDev& p, float r, float ir, float ira, float& fr, float& half_e) {
     if (p.usezbl && r < p.sx0) {
         // sw.cpp:118-146
-        const float rinv = 1.0f / r;
         const float f0 = 0.1818f * expf(-p.ze0 * r), f1 = 0.5099f * expf(-p.ze1 * r);
         const float f2 = 0.2802f * expf(-p.ze2 * r), f3 = 0.02817f * expf(-p.ze3 * r);
-        const float fpot = (f0 + f1 + f2 + f3) * p.zc * rinv;
-        fr = ((rinv + p.ze0) * f0 + (rinv + p.ze1) * f1 + (rinv + p.ze2) * f2 + (rinv + p.ze3) * f3) * p.zc *
-             (rinv * rinv);
+        const float fpot = (f0 + f1 + f2 + f3) * p.zc * ir;
+        fr = ((ir + p.ze0) * f0 + (ir + p.ze1) * f1 + (ir + p.ze2) * f2 + (ir + p.ze3) * f3) * p.zc * (ir * ir);
         half_e = 0.5f * fpot;
     } else if (p.usezbl && r < p.sx1) {
         // sw.cpp:148-164 (force factor applied with the opposite sign)
@@ -78,133 +141,56 @@ __device__ __forceinline__ void sw_two_body(const SWDev& p, float r, float& fr, 
         half_e = 0.5f * (p.sa0 + f * r);
     } else {
         // sw.cpp:166-189
-        const float ira = 1.0f / (r - p.rc);
-        const float rp = p.ip >= 0 ? inv_ipow(r, p.ip) : powf(r, -p.p);
-        const float rq = p.iq >= 0 ? inv_ipow(r, p.iq) : powf(r, -p.q);
+        const float rp = p.ip >= 0 ? inv_ipow(ir, p.ip) : powf(r, -p.p);
+        const float rq = p.iq >= 0 ? inv_ipow(ir, p.iq) : powf(r, -p.q);
         const float fex = expf(p.sigma * ira);
-        fr = (p.c1 * rp - p.c2 * rq + (p.c3 * rp - p.c4 * rq) * ira * ira * r) * fex / (r * r);
+        fr = (p.c1 * rp - p.c2 * rq + (p.c3 * rp - p.c4 * rq) * ira * ira * r) * fex * (ir * ir);
         half_e = 0.5f * (p.c5 * rp - p.c6 * rq) * fex;
     }
 }
 
-// A centre with more in-cutoff neighbours than the register path holds:
-// up to TB_MAXN of them over local arrays (the two-body terms as well).
-__device__ __noinline__ void sw_centre_wide(const SWDev& p, int i, const PosPack* __restrict__ pack,
-                                            const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
-                                            float4* __restrict__ slot, float* __restrict__ fx, float* __restrict__ fy,
-                                            float* __restrict__ fz, float* __restrict__ pe, unsigned* status) {
-    const PosPack pi = pack[i];
-    const int ti = pack_type(pi.hi);
-    const bool mine = p.single_type || ti == p.ta;
-    const int m = nnb[i];
-    // neighbours inside the cutoff, vectors from i to the neighbour
-    float vx[TB_MAXN], vy[TB_MAXN], vz[TB_MAXN], rr[TB_MAXN];
-    int sl[TB_MAXN];
-    int nc = 0;
-    float ax = 0.f, ay = 0.f, az = 0.f, ae = 0.f;
-    for (int s = 0; s < m; s++) {
-        const size_t at = nbr_at(i, s, p.hshift, p.maxnb);
-        slot[at] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!mine) continue;
-        const unsigned e = nbr[at];
-        const int j = nbr_index(e);
-        const PosPack pj = pack[j];
-        if (!p.single_type && pack_type(pj.hi) != p.ta) continue;
-        const float3 d = pair_delta(pi.hi, pi.lo, pj.hi, pj.lo, e, p.L);  // x_i - x_j
-        const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
-        if (!(r2 < p.rc2)) continue;
-        const float r = sqrtf(r2);
-        // r2 just below rc^2 can round to r == rc, where 1/(r - rc) is infinite
-        // and 0 * inf gives NaN; every SW term is zero there, so drop the pair
-        if (!(r < p.rc)) continue;
-        float fr, he;
-        sw_two_body(p, r, fr, he);
-        ax += d.x * fr;
-        ay += d.y * fr;
-        az += d.z * fr;
-        ae += he;
-        if (nc < TB_MAXN) {
-            vx[nc] = -d.x;
-            vy[nc] = -d.y;
-            vz[nc] = -d.z;
-            rr[nc] = r;
-            sl[nc] = s;
-        } else {
-            atomicOr(status, ERR_NBR_OVERFLOW);
-        }
-        nc++;
+// A neighbour's own quantities: from (vector, squared distance) to (unit
+// vector, exp(c7/(r - rc))), with what its triplet sums are scaled by, and its
+// two-body half added to the centre.
+__device__ __forceinline__ void sw_neighbour(const SWDev& p, float4& v, float2& k, float& ax, float& ay, float& az,
+                                             float& ae) {
+    const float r = sqrtf(v.w), ir = 1.0f / r, ira = 1.0f / (r - p.rc), fira = p.c7 * ira;
+    float fr, he;
+    sw_two_body(p, r, ir, ira, fr, he);
+    ax -= v.x * fr;
+    ay -= v.y * fr;
+    az -= v.z * fr;
+    ae += he;
+    v = make_float4(v.x * ir, v.y * ir, v.z * ir, expf(fira));
+    k = make_float2(fira * ira, ir);
+}
+
+// The triplets of neighbour a (unit vector and factor ua) with b, summed over
+// b != a (sw.cpp:191-236): with w = e_b (cos - c10), the sums of w (cos -
+// c10), w cos and w u_b give the energy and the force of all of a's triplets
+// (sw_share), twelve instructions an ordered pair where one evaluated whole
+// took some sixty an unordered one.
+struct SWSums {
+    float s = 0.f, t = 0.f, x = 0.f, y = 0.f, z = 0.f;
+    __device__ __forceinline__ void add(const SWDev& p, const float4& ua, const float4& ub, bool self) {
+        const float c = fmaf(ua.z, ub.z, fmaf(ua.y, ub.y, ua.x * ub.x));
+        const float dc = c - p.c10, w = self ? 0.f : ub.w * dc;
+        s = fmaf(w, dc, s);
+        t = fmaf(w, c, t);
+        x = fmaf(w, ub.x, x);
+        y = fmaf(w, ub.y, y);
+        z = fmaf(w, ub.z, z);
     }
-    if (nc > TB_MAXN) nc = TB_MAXN;
-    // triplets centred on i (sw.cpp:191-236), each unordered pair (j, k) once;
-    // every neighbour's share is summed here and stored in its slot once.  The
-    // per-neighbour factors exp(c7 / (r - rc)), 1 / r and c7 / ((r - rc)^2 r)
-    // are computed once per neighbour instead of once per triplet.
-    float sjx[TB_MAXN], sjy[TB_MAXN], sjz[TB_MAXN], sje[TB_MAXN];
-    float ex[TB_MAXN], ir[TB_MAXN], gr[TB_MAXN];
-    for (int a = 0; a < nc; a++) {
-        sjx[a] = sjy[a] = sjz[a] = sje[a] = 0.f;
-        const float ira = 1.0f / (rr[a] - p.rc), fira = p.c7 * ira;
-        ex[a] = expf(fira);
-        ir[a] = 1.0f / rr[a];
-        gr[a] = fira * ira * ir[a];
-    }
-    for (int a = 0; a < nc; a++) {
-        const float dx1 = vx[a], dy1 = vy[a], dz1 = vz[a];
-        const float ex0 = ex[a], ir1 = ir[a], g0 = gr[a];
-        float gjx = 0.f, gjy = 0.f, gjz = 0.f, gje = 0.f;
-        for (int b = a + 1; b < nc; b++) {
-            const float dx2 = vx[b], dy2 = vy[b], dz2 = vz[b];
-            const float ir2 = ir[b];
-            const float ir1r2 = ir1 * ir2;
-            const float fex = ex0 * ex[b];
-            const float cs = (dx1 * dx2 + dy1 * dy2 + dz1 * dz2) * ir1r2;
-            const float dcos = cs - p.c10;
-            const float ftheta = p.c9 * fex * dcos;
-            const float ft12 = ir1r2 * ftheta;
-            const float fpot = p.c8 * fex * dcos * dcos;
-            const float fcos = cs * ftheta;
-            const float fr0 = fpot * g0, fr1 = fpot * gr[b];
-            const float ft0 = fcos * ir1 * ir1, ft1 = fcos * ir2 * ir2;
-            const float fx0 = dx1 * (fr0 + ft0) - dx2 * ft12, fx1 = dx2 * (fr1 + ft1) - dx1 * ft12;
-            const float fy0 = dy1 * (fr0 + ft0) - dy2 * ft12, fy1 = dy2 * (fr1 + ft1) - dy1 * ft12;
-            const float fz0 = dz1 * (fr0 + ft0) - dz2 * ft12, fz1 = dz2 * (fr1 + ft1) - dz1 * ft12;
-            ax -= fx0 + fx1;
-            ay -= fy0 + fy1;
-            az -= fz0 + fz1;
-            const float third = fpot * (1.0f / 3.0f);
-            ae += third;
-            gjx += fx0;
-            gjy += fy0;
-            gjz += fz0;
-            gje += third;
-            sjx[b] += fx1;
-            sjy[b] += fy1;
-            sjz[b] += fz1;
-            sje[b] += third;
-        }
-        sjx[a] += gjx;
-        sjy[a] += gjy;
-        sjz[a] += gjz;
-        sje[a] += gje;
-    }
-    for (int a = 0; a < nc; a++)
-        slot[nbr_at(i, sl[a], p.hshift, p.maxnb)] = make_float4(sjx[a], sjy[a], sjz[a], sje[a]);
-    if (p.first) {
-        fx[i] = ax;
-        fy[i] = ay;
-        fz[i] = az;
-        pe[i] = ae;
-    } else {
-        fx[i] += ax;
-        fy[i] += ay;
-        fz[i] += az;
-        pe[i] += ae;
-    }
+};
+
+// What the triplets give to neighbour a: the force, and a third of their
+// energy (sw.cpp:225-233).  Every triplet is in the sums of two neighbours.
+__device__ __forceinline__ float4 sw_share(const SWDev& p, const float4& ua, const float2& k, const SWSums& q) {
+    const float e = p.c8 * ua.w * q.s, g = p.c9 * ua.w * k.y, f = fmaf(k.x, e, g * q.t);
+    return make_float4(fmaf(ua.x, f, -g * q.x), fmaf(ua.y, f, -g * q.y), fmaf(ua.z, f, -g * q.z), e * (1.0f / 3.0f));
 }
 
 constexpr int SW_REG = 8;  // in-cutoff neighbours the register path holds (diamond: 4 + thermal second shell)
-// k_sw_a at six 128-thread blocks a SM (80 registers, 252 bytes spilled) ran
-// the Si 512k step faster than at its natural 121 registers (427 vs 458 us)
 
 __device__ __forceinline__ void sw_store(const SWDev& p, int i, float ax, float ay, float az, float ae,
                                          float* __restrict__ fx, float* __restrict__ fy, float* __restrict__ fz,
@@ -222,119 +208,130 @@ __device__ __forceinline__ void sw_store(const SWDev& p, int i, float ax, float 
     }
 }
 
-// Pass A of SW for centre i with up to SW_REG in-cutoff neighbours in
-// registers (fully unrolled loops, insertion by select); centres with more
-// are queued for k_sw_wide.  Same terms and summation order as the wide
-// path.
-__global__ void __launch_bounds__(128, 6) k_sw_a(SWDev p, const PosPack* __restrict__ pack,
-                                              const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
-                                              float4* __restrict__ slot, float* __restrict__ fx,
-                                              float* __restrict__ fy, float* __restrict__ fz, float* __restrict__ pe,
-                                              unsigned* status, int* __restrict__ wide) {
+// Pass A of SW, a thread a centre of up to SW_REG in-cutoff neighbours;
+// centres with more are queued.  The scan only collects the neighbours in
+// shared memory, so that the two-body term runs once for each of them with
+// most of the warp in it, and not at every row entry that any lane has a hit
+// at; the triplets then read them from registers.  194,184 atoms with some 7.5
+// neighbours each, both passes: 148 -> 61.6 us at five blocks a SM (two whole
+// waves; six leave an L1 of 64 KB to the gather: 70.0).
+__global__ void __launch_bounds__(TB_BLOCK, 5) k_sw_a(SWDev p, const PosPack* __restrict__ pack,
+                                                     const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
+                                                     RowHits hits, SlotRows slot, float* __restrict__ fx,
+                                                     float* __restrict__ fy, float* __restrict__ fz,
+                                                     float* __restrict__ pe, int* __restrict__ wide) {
     constexpr int K = SW_REG;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ float4 sv[K][TB_BLOCK];
+    __shared__ float2 sk[K][TB_BLOCK];
+    __shared__ int2 ss[K][TB_BLOCK];  // neighbour, the entry of its row that is i
+    const int t = threadIdx.x;
+    const int i = blockIdx.x * TB_BLOCK + t;
     if (i >= p.n) return;
     const PosPack pi = pack[i];
-    const int ti = pack_type(pi.hi);
-    const bool mine = p.single_type || ti == p.ta;
     const int m = nnb[i];
-    float vx[K], vy[K], vz[K], rr[K];
-    int sl[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) vx[k] = vy[k] = vz[k] = 0.f, rr[k] = 1.f, sl[k] = 0;
     int nc = 0;
+    if (p.single_type || pack_type(pi.hi) == p.ta) {
+        nc = scan_row<true, true>(i, m, pi, p.L, p.t2, p.single_type ? -1 : p.ta, pack, nbr, slot.rev, p.hshift, p.maxnb, hits,
+                            [&](int k, int j, int r, const float3& d, float r2) {
+                                if (k < K) sv[k][t] = make_float4(-d.x, -d.y, -d.z, r2), ss[k][t] = make_int2(j, r);
+                            });
+        if (nc > K) {
+            wide[1 + atomicAdd(wide, 1)] = i;
+            return;
+        }
+    } else {
+        no_hits(i, m, hits);
+    }
     float ax = 0.f, ay = 0.f, az = 0.f, ae = 0.f;
-    for (int s = 0; s < m; s++) {
-        const size_t at = nbr_at(i, s, p.hshift, p.maxnb);
-        slot[at] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!mine) continue;
-        const unsigned e = nbr[at];
-        const PosPack pj = pack[nbr_index(e)];
-        if (!p.single_type && pack_type(pj.hi) != p.ta) continue;
-        const float3 d = pair_delta(pi.hi, pi.lo, pj.hi, pj.lo, e, p.L);  // x_i - x_j
-        const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
-        if (!(r2 < p.rc2)) continue;
-        const float r = sqrtf(r2);
-        if (!(r < p.rc)) continue;  // r == rc: every SW term is zero (and 1/(r - rc) infinite)
-        float fr, he;
-        sw_two_body(p, r, fr, he);
-        ax += d.x * fr;
-        ay += d.y * fr;
-        az += d.z * fr;
-        ae += he;
+#pragma unroll 1
+    for (int a = 0; a < nc; a++) {
+        float4 v = sv[a][t];
+        float2 k;
+        sw_neighbour(p, v, k, ax, ay, az, ae);
+        sv[a][t] = v;
+        sk[a][t] = k;
+    }
+    float4 u[K];
 #pragma unroll
-        for (int k = 0; k < K; k++)
-            if (k == nc) vx[k] = -d.x, vy[k] = -d.y, vz[k] = -d.z, rr[k] = r, sl[k] = s;
-        nc++;
+    for (int b = 0; b < K; b++) u[b] = b < nc ? sv[b][t] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int a = 0; a < nc; a++) {
+        const float4 ua = sv[a][t];
+        SWSums q;
+#pragma unroll
+        for (int b = 0; b < K / 2; b++) q.add(p, ua, u[b], a == b);
+        if (nc > K / 2) {
+#pragma unroll
+            for (int b = K / 2; b < K; b++) q.add(p, ua, u[b], a == b);
+        }
+        const float4 f = sw_share(p, ua, sk[a][t], q);
+        slot.at(ss[a][t].x, ss[a][t].y) = f;
+        ax -= f.x;
+        ay -= f.y;
+        az -= f.z;
+        ae = fmaf(0.5f, f.w, ae);
     }
-    if (nc > K) {  // queued: k_sw_wide evaluates the whole centre
-        wide[1 + atomicAdd(wide, 1)] = i;
-        return;
-    }
-    // triplets centred on i (sw.cpp:191-236), each unordered pair (j, k) once
-    float sjx[K], sjy[K], sjz[K], sje[K], ex[K], ir[K], gr[K];
-    for_nbrs<K, true>(nc, [&](int a) {
-        sjx[a] = sjy[a] = sjz[a] = sje[a] = 0.f;
-        const float ira = 1.0f / (rr[a] - p.rc), fira = p.c7 * ira;
-        ex[a] = expf(fira);
-        ir[a] = 1.0f / rr[a];
-        gr[a] = fira * ira * ir[a];
-    });
-    for_nbrs<K, true>(nc, [&](int a) {
-        const float dx1 = vx[a], dy1 = vy[a], dz1 = vz[a];
-        const float ex0 = ex[a], ir1 = ir[a], g0 = gr[a];
-        float gjx = 0.f, gjy = 0.f, gjz = 0.f, gje = 0.f;
-        for_nbrs<K, true>(nc, [&](int b) {
-            if (b <= a) return;
-            const float dx2 = vx[b], dy2 = vy[b], dz2 = vz[b];
-            const float ir2 = ir[b];
-            const float ir1r2 = ir1 * ir2;
-            const float fex = ex0 * ex[b];
-            const float cs = (dx1 * dx2 + dy1 * dy2 + dz1 * dz2) * ir1r2;
-            const float dcos = cs - p.c10;
-            const float ftheta = p.c9 * fex * dcos;
-            const float ft12 = ir1r2 * ftheta;
-            const float fpot = p.c8 * fex * dcos * dcos;
-            const float fcos = cs * ftheta;
-            const float fr0 = fpot * g0, fr1 = fpot * gr[b];
-            const float ft0 = fcos * ir1 * ir1, ft1 = fcos * ir2 * ir2;
-            const float fx0 = dx1 * (fr0 + ft0) - dx2 * ft12, fx1 = dx2 * (fr1 + ft1) - dx1 * ft12;
-            const float fy0 = dy1 * (fr0 + ft0) - dy2 * ft12, fy1 = dy2 * (fr1 + ft1) - dy1 * ft12;
-            const float fz0 = dz1 * (fr0 + ft0) - dz2 * ft12, fz1 = dz2 * (fr1 + ft1) - dz1 * ft12;
-            ax -= fx0 + fx1;
-            ay -= fy0 + fy1;
-            az -= fz0 + fz1;
-            const float third = fpot * (1.0f / 3.0f);
-            ae += third;
-            gjx += fx0;
-            gjy += fy0;
-            gjz += fz0;
-            gje += third;
-            sjx[b] += fx1;
-            sjy[b] += fy1;
-            sjz[b] += fz1;
-            sje[b] += third;
-        });
-        sjx[a] += gjx;
-        sjy[a] += gjy;
-        sjz[a] += gjz;
-        sje[a] += gje;
-    });
-    for_nbrs<K, true>(nc, [&](int a) {
-        slot[nbr_at(i, sl[a], p.hshift, p.maxnb)] = make_float4(sjx[a], sjy[a], sjz[a], sje[a]);
-    });
     sw_store(p, i, ax, ay, az, ae, fx, fy, fz, pe);
 }
 
-// The queued centres (wide[0] of them, indices from wide[1]).
-__global__ void __launch_bounds__(128) k_sw_wide(SWDev p, const PosPack* __restrict__ pack,
-                                                 const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
-                                                 const int* __restrict__ wide, float4* __restrict__ slot,
-                                                 float* __restrict__ fx, float* __restrict__ fy,
-                                                 float* __restrict__ fz, float* __restrict__ pe, unsigned* status) {
-    const int cnt = wide[0];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x)
-        sw_centre_wide(p, wide[1 + k], pack, nbr, nnb, slot, fx, fy, fz, pe, status);
+// Pass A of SW, eight lanes a centre: the queued centres (wide[0] of them,
+// indices from wide[1]), or all of them (then the ones past the register path
+// are still counted).  A lane owns a neighbour, with all of its triplets.
+template <bool QUEUED>
+__global__ void __launch_bounds__(TB_LBLOCK) k_sw_lanes(SWDev p, const PosPack* __restrict__ pack,
+                                                       const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
+                                                       int* __restrict__ wide, RowHits hits,
+                                                       SlotRows slot, float* __restrict__ fx,
+                                                       float* __restrict__ fy, float* __restrict__ fz,
+                                                       float* __restrict__ pe, unsigned* status) {
+    __shared__ float4 gv[TB_LGROUPS][TB_MAXN];
+    __shared__ int gs[TB_LGROUPS][TB_MAXN];
+    const LaneGroup g;
+    float4* v = gv[threadIdx.x / TB_LANES];
+    int* sl = gs[threadIdx.x / TB_LANES];
+    const int total = QUEUED ? wide[0] : p.n;
+    for (int c = blockIdx.x * TB_LGROUPS + threadIdx.x / TB_LANES; c < total; c += gridDim.x * TB_LGROUPS) {
+        const int i = QUEUED ? wide[1 + c] : c;
+        const PosPack pi = pack[i];
+        const int m = nnb[i];
+        int nc = 0;
+        if (p.single_type || pack_type(pi.hi) == p.ta) {
+            nc = lanes_collect<QUEUED>(g, i, m, pi, p.L, p.t2, p.single_type ? -1 : p.ta, pack, nbr, p.hshift,
+                                       p.maxnb, hits, slot, v, sl, status);
+            if (!QUEUED && nc > SW_REG && g.lane == 0) wide[1 + atomicAdd(wide, 1)] = i;
+            nc = min(nc, TB_MAXN);
+        } else if (!QUEUED && g.lane == 0) {
+            no_hits(i, m, hits);
+        }
+        float ax = 0.f, ay = 0.f, az = 0.f, ae = 0.f;
+        float2 k[TB_MAXN / TB_LANES];
+#pragma unroll
+        for (int j = 0; j < TB_MAXN / TB_LANES; j++) {
+            const int a = j * TB_LANES + g.lane;
+            if (a < nc) sw_neighbour(p, v[a], k[j], ax, ay, az, ae);
+        }
+        __syncwarp(g.mask);
+#pragma unroll
+        for (int j = 0; j < TB_MAXN / TB_LANES; j++) {
+            const int a = j * TB_LANES + g.lane;
+            if (a >= nc) continue;
+            const float4 ua = v[a];
+            SWSums q;
+            for (int b = 0; b < nc; b++) q.add(p, ua, v[b], a == b);
+            const float4 f = sw_share(p, ua, k[j], q);
+            slot.put(i, sl[a], f);
+            ax -= f.x;
+            ay -= f.y;
+            az -= f.z;
+            ae = fmaf(0.5f, f.w, ae);
+        }
+        __syncwarp(g.mask);  // the group's neighbours are read: the next centre may overwrite them
+        ax = g.sum(ax);
+        ay = g.sum(ay);
+        az = g.sum(az);
+        ae = g.sum(ae);
+        if (g.lane == 0) sw_store(p, i, ax, ay, az, ae, fx, fy, fz, pe);
+    }
 }
 
 // Gathers what every neighbour's pass A left for i; clears no state.
@@ -358,7 +355,8 @@ struct TersDev {
     ShiftF L;
     const ShiftF* rep_L;  // replica mode: periodic lengths of each replica (else null)
     const int* rep_of;
-    float A, B, l1, l2, l3c, beta, nn, c2, d2, h, R, D, rc, rc2;
+    float A, B, l1, l2, l3c, beta, nn, c2, d2, h, R, D;
+    float t2;  // r2 < t2: inside the cutoff (r2_below)
     int first;
 };
 
@@ -401,30 +399,39 @@ __device__ __forceinline__ float ters_fc(const TersDev& p, float r, float& dfc) 
     return 0.f;
 }
 
-// The bonds centred on one atom, for its nc <= K in-cutoff neighbours
-// (unit vectors u from the centre, distances r).  Per neighbour the cutoff
-// f_c(r), f_c'(r) and 1/r are evaluated once; per triplet (a, b) the angular
-// and radial factors once, in the zeta sweep, with what the x_k gradient
-// needs kept for its sweep.
-template <int K, bool UNR>
+// f(b) for the in-cutoff neighbours b < nc, fully unrolled over K (the arrays
+// f touches stay in registers)
+template <int K, class F>
+__device__ __forceinline__ void for_nbrs(int nc, F&& f) {
+#pragma unroll
+    for (int b = 0; b < K; b++)
+        if (b < nc) f(b);
+}
+
+// The bonds centred on one atom, for its nc <= K in-cutoff neighbours in
+// registers (unit vectors u from the centre, distances r).  Per neighbour the
+// cutoff f_c(r), f_c'(r) and 1/r are evaluated once; per triplet (a, b) the
+// angular and radial factors once, in the zeta sweep, with what the x_k
+// gradient needs kept for its sweep.
+template <int K>
 __device__ __forceinline__ void ters_bonds(const TersDev& p, const int nc, const float (&ux)[K],
                                            const float (&uy)[K], const float (&uz)[K], const float (&rr)[K],
                                            float (&skx)[K], float (&sky)[K], float (&skz)[K], float& fix,
                                            float& fiy, float& fiz, float& ei, float& wi) {
     float fc[K], dfc[K], ir[K];
-    for_nbrs<K, UNR>(nc, [&](int b) {
+    for_nbrs<K>(nc, [&](int b) {
         fc[b] = ters_fc(p, rr[b], dfc[b]);
         ir[b] = 1.0f / rr[b];
         skx[b] = sky[b] = skz[b] = 0.f;
     });
     const float g0 = 1.f + p.c2 / p.d2;
-    for_nbrs<K, UNR>(nc, [&](int a) {
+    for_nbrs<K>(nc, [&](int a) {
         const float rij = rr[a];
         const float ex_ = ux[a], ey_ = uy[a], ez_ = uz[a];
         // zeta_ij and its gradient w.r.t. x_j; per k the x_k coefficients
         float zeta = 0.f, gjx = 0.f, gjy = 0.f, gjz = 0.f;
         float ck[K], cc[K], cs[K];
-        for_nbrs<K, UNR>(nc, [&](int b) {
+        for_nbrs<K>(nc, [&](int b) {
             if (b == a) return;
             const float c = ex_ * ux[b] + ey_ * uy[b] + ez_ * uz[b];
             const float hc = p.h - c;
@@ -458,7 +465,7 @@ __device__ __forceinline__ void ters_bonds(const TersDev& p, const int nc, const
         fiz += sjz;
         const float s = 0.5f * dv_dz;
         // x_k parts
-        for_nbrs<K, UNR>(nc, [&](int b) {
+        for_nbrs<K>(nc, [&](int b) {
             if (b == a) return;
             const float kx = s * (ck[b] * ux[b] + cc[b] * (ex_ - cs[b] * ux[b]));
             const float ky = s * (ck[b] * uy[b] + cc[b] * (ey_ - cs[b] * uy[b]));
@@ -479,22 +486,6 @@ __device__ __forceinline__ void ters_bonds(const TersDev& p, const int nc, const
     });
 }
 
-// Relative vector from centre i to its list entry at `at`, when the pair is
-// one this potential evaluates and lies within the cutoff.
-__device__ __forceinline__ bool ters_neighbor(const TersDev& p, const PosPack& pi, const ShiftF& L,
-                                              const PosPack* __restrict__ pack, unsigned e, float3& u, float& r) {
-    const PosPack pj = pack[nbr_index(e)];
-    if (!p.single_type && pack_type(pj.hi) != p.ta) return false;
-    const float3 d = pair_delta(pi.hi, pi.lo, pj.hi, pj.lo, e, L);
-    const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
-    if (!(r2 < p.rc2)) return false;
-    r = sqrtf(r2);
-    if (!(r < p.rc)) return false;
-    const float ri = 1.0f / r;
-    u = make_float3(-d.x * ri, -d.y * ri, -d.z * ri);  // unit vector from i to the neighbour
-    return true;
-}
-
 __device__ __forceinline__ void ters_store(const TersDev& p, int i, float fix, float fiy, float fiz, float ei,
                                            float wi, float* __restrict__ fx, float* __restrict__ fy,
                                            float* __restrict__ fz, float* __restrict__ pe, float* __restrict__ vir) {
@@ -513,131 +504,243 @@ __device__ __forceinline__ void ters_store(const TersDev& p, int i, float fix, f
     }
 }
 
-// A centre with more in-cutoff neighbours than the register path holds (a
-// collision cascade): up to TB_MAXN of them over local arrays.
-__device__ __noinline__ void ters_centre_wide(const TersDev& p, int i, const PosPack pi, const ShiftF L,
-                                              const PosPack* __restrict__ pack, const unsigned* __restrict__ nbr,
-                                              int m, float4* __restrict__ slot, float* __restrict__ fx,
-                                              float* __restrict__ fy, float* __restrict__ fz, float* __restrict__ pe,
-                                              float* __restrict__ vir, unsigned* status) {
-    float ux[TB_MAXN], uy[TB_MAXN], uz[TB_MAXN], rr[TB_MAXN];
-    int sl[TB_MAXN];
-    int nc = 0;
-    for (int s = 0; s < m; s++) {
-        const size_t at = nbr_at(i, s, p.hshift, p.maxnb);
-        float3 u;
-        float r;
-        if (!ters_neighbor(p, pi, L, pack, nbr[at], u, r)) continue;
-        if (nc < TB_MAXN) {
-            ux[nc] = u.x;
-            uy[nc] = u.y;
-            uz[nc] = u.z;
-            rr[nc] = r;
-            sl[nc] = s;
-        } else {
-            atomicOr(status, ERR_NBR_OVERFLOW);
-        }
-        nc++;
-    }
-    if (nc > TB_MAXN) nc = TB_MAXN;
-    float fix = 0.f, fiy = 0.f, fiz = 0.f, ei = 0.f, wi = 0.f;
-    float skx[TB_MAXN], sky[TB_MAXN], skz[TB_MAXN];
-    ters_bonds<TB_MAXN, false>(p, nc, ux, uy, uz, rr, skx, sky, skz, fix, fiy, fiz, ei, wi);
-    for (int a = 0; a < nc; a++)
-        slot[nbr_at(i, sl[a], p.hshift, p.maxnb)] = make_float4(skx[a], sky[a], skz[a], 0.f);
-    ters_store(p, i, fix, fiy, fiz, ei, wi, fx, fy, fz, pe, vir);
-}
-
 constexpr int TERS_REG = 4;  // in-cutoff neighbours the register path holds (diamond: 4)
 
+// A masked pass (mask[i] != 0: the centre is evaluated) finds the hit bits of
+// the pass that made the mask, and leaves them.
+template <bool MASKED>
 __device__ __forceinline__ void ters_reg_centre(const TersDev& p, int i, const PosPack* __restrict__ pack,
                                                 const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
-                                                float4* __restrict__ slot, float* __restrict__ fx,
-                                                float* __restrict__ fy, float* __restrict__ fz,
-                                                float* __restrict__ pe, float* __restrict__ vir,
-                                                const int* __restrict__ mask, int* __restrict__ wide);
+                                                const RowHits& hits, const SlotRows& slot,
+                                                float* __restrict__ fx, float* __restrict__ fy,
+                                                float* __restrict__ fz, float* __restrict__ pe,
+                                                float* __restrict__ vir, int* __restrict__ wide) {
+    __shared__ float4 sv[TERS_REG][TB_BLOCK];
+    __shared__ int2 ss[TERS_REG][TB_BLOCK];  // neighbour, the entry of its row that is i
+    const int t = threadIdx.x;
+    const PosPack pi = pack[i];
+    const ShiftF L = p.rep_L ? p.rep_L[p.rep_of[i]] : p.L;
+    const int m = nnb[i];
+    int nc = 0;
+    if (p.single_type || pack_type(pi.hi) == p.ta) {
+        nc = scan_row<!MASKED, true>(i, m, pi, L, p.t2, p.single_type ? -1 : p.ta, pack, nbr, slot.rev, p.hshift, p.maxnb, hits,
+                               [&](int k, int j, int r, const float3& d, float r2) {
+                                   if (k < TERS_REG)
+                                       sv[k][t] = make_float4(-d.x, -d.y, -d.z, r2), ss[k][t] = make_int2(j, r);
+                               });
+        if (nc > TERS_REG) {  // queued, so its warp does not wait on it
+            wide[1 + atomicAdd(wide, 1)] = i;
+            return;
+        }
+    } else if (!MASKED) {
+        no_hits(i, m, hits);
+    }
+    float ux[TERS_REG], uy[TERS_REG], uz[TERS_REG], rr[TERS_REG];
+#pragma unroll
+    for (int k = 0; k < TERS_REG; k++) {
+        ux[k] = uy[k] = uz[k] = rr[k] = 0.f;
+        if (k >= nc) continue;
+        const float4 v = sv[k][t];
+        rr[k] = sqrtf(v.w);
+        const float ri = 1.0f / rr[k];
+        ux[k] = __fmul_rn(v.x, ri);
+        uy[k] = __fmul_rn(v.y, ri);
+        uz[k] = __fmul_rn(v.z, ri);
+    }
+    float fix = 0.f, fiy = 0.f, fiz = 0.f, ei = 0.f, wi = 0.f;
+    float skx[TERS_REG], sky[TERS_REG], skz[TERS_REG];
+    ters_bonds<TERS_REG>(p, nc, ux, uy, uz, rr, skx, sky, skz, fix, fiy, fiz, ei, wi);
+#pragma unroll
+    for (int a = 0; a < TERS_REG; a++)
+        if (a < nc) slot.at(ss[a][t].x, ss[a][t].y) = make_float4(skx[a], sky[a], skz[a], 0.f);
+    ters_store(p, i, fix, fiy, fiz, ei, wi, fx, fy, fz, pe, vir);
+}
 
 // One thread per centre.  Launched with fewer threads than centres (the
 // persistent form: one resident grid over the flattened atoms of every
 // replica), each thread strides over the centres.
-constexpr int TERS_CTAS_PER_SM = 8;  // 64 registers: the Si 512k register pass 54.8 -> 51.6 us against 6 (80)
+// 72 registers and an L1 of 160 KB: 512,000 atoms take 50.4, 49.7, 53.1 and 69.4
+// us (with the queue's pass) at six, seven, eight and ten blocks a SM.
+constexpr int TERS_CTAS_PER_SM = 7;
 
-template <bool PERSISTENT>
-__global__ void __launch_bounds__(128, TERS_CTAS_PER_SM) k_tersoff_a(TersDev p, const PosPack* __restrict__ pack,
-                                                   const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
-                                                   float4* __restrict__ slot, float* __restrict__ fx,
-                                                   float* __restrict__ fy, float* __restrict__ fz,
-                                                   float* __restrict__ pe, float* __restrict__ vir, unsigned* status,
-                                                   const int* __restrict__ mask, int* __restrict__ wide,
-                                                   const int* __restrict__ nmask) {
-    if (nmask && *nmask == 0) return;  // a mask with no centre in it
+template <bool PERSISTENT, bool MASKED>
+__global__ void __launch_bounds__(TB_BLOCK, TERS_CTAS_PER_SM) k_tersoff_a(
+    TersDev p, const PosPack* __restrict__ pack, const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
+    RowHits hits, SlotRows slot, float* __restrict__ fx, float* __restrict__ fy, float* __restrict__ fz,
+    float* __restrict__ pe, float* __restrict__ vir, int* __restrict__ wide, const int* __restrict__ mask,
+    const int* __restrict__ nmask) {
+    if (MASKED && nmask && *nmask == 0) return;  // a mask with no centre in it
+    int i = blockIdx.x * TB_BLOCK + threadIdx.x;
     if (PERSISTENT) {
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += gridDim.x * blockDim.x)
-            ters_reg_centre(p, i, pack, nbr, nnb, slot, fx, fy, fz, pe, vir, mask, wide);
+        for (; i < p.n; i += gridDim.x * TB_BLOCK)
+            if (!MASKED || mask[i])
+                ters_reg_centre<MASKED>(p, i, pack, nbr, nnb, hits, slot, fx, fy, fz, pe, vir, wide);
     } else {
-        const int i = blockIdx.x * blockDim.x + threadIdx.x;
-        if (i < p.n) ters_reg_centre(p, i, pack, nbr, nnb, slot, fx, fy, fz, pe, vir, mask, wide);
+        if (i < p.n && (!MASKED || mask[i]))
+            ters_reg_centre<MASKED>(p, i, pack, nbr, nnb, hits, slot, fx, fy, fz, pe, vir, wide);
     }
 }
 
-__device__ __forceinline__ void ters_reg_centre(const TersDev& p, int i, const PosPack* __restrict__ pack,
-                                                const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
-                                                float4* __restrict__ slot, float* __restrict__ fx,
-                                                float* __restrict__ fy, float* __restrict__ fz,
-                                                float* __restrict__ pe, float* __restrict__ vir,
-                                                const int* __restrict__ mask, int* __restrict__ wide) {
-    if (mask && !mask[i]) return;  // centres another potential evaluates
-    const PosPack pi = pack[i];
-    const bool mine = p.single_type || pack_type(pi.hi) == p.ta;
-    const ShiftF L = p.rep_L ? p.rep_L[p.rep_of[i]] : p.L;
-    const int m = nnb[i];
-    // the in-cutoff neighbours go to registers by select; every other slot
-    // of the row gets its zero here
-    float ux[TERS_REG], uy[TERS_REG], uz[TERS_REG], rr[TERS_REG];
-    int sl[TERS_REG];
-#pragma unroll
-    for (int k = 0; k < TERS_REG; k++) ux[k] = uy[k] = uz[k] = rr[k] = 0.f, sl[k] = 0;
-    int nc = 0;
-    for (int s = 0; s < m; s++) {
-        const size_t at = nbr_at(i, s, p.hshift, p.maxnb);
-        float3 u;
-        float r;
-        if (mine && ters_neighbor(p, pi, L, pack, nbr[at], u, r)) {
-#pragma unroll
-            for (int k = 0; k < TERS_REG; k++)
-                if (k == nc) ux[k] = u.x, uy[k] = u.y, uz[k] = u.z, rr[k] = r, sl[k] = s;
-            nc++;
-        } else {
-            slot[at] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
-    if (nc > TERS_REG) {  // queued for k_tersoff_wide, so its warp does not wait on it
-        wide[1 + atomicAdd(wide, 1)] = i;
-        return;
-    }
-    float fix = 0.f, fiy = 0.f, fiz = 0.f, ei = 0.f, wi = 0.f;
-    float skx[TERS_REG], sky[TERS_REG], skz[TERS_REG];
-    ters_bonds<TERS_REG, true>(p, nc, ux, uy, uz, rr, skx, sky, skz, fix, fiy, fiz, ei, wi);
-#pragma unroll
-    for (int a = 0; a < TERS_REG; a++)
-        if (a < nc) slot[nbr_at(i, sl[a], p.hshift, p.maxnb)] = make_float4(skx[a], sky[a], skz[a], 0.f);
-    ters_store(p, i, fix, fiy, fiz, ei, wi, fx, fy, fz, pe, vir);
-}
+// a b + c d rounded as the compiler contracts it in ters_bonds
+__device__ __forceinline__ float fma2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
 
-// The queued centres (wide[0] of them, indices from wide[1]): a grid-stride
-// loop, so the few centres of a collision cascade run in dense warps.
-__global__ void __launch_bounds__(128) k_tersoff_wide(TersDev p, const PosPack* __restrict__ pack,
-                                                      const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
-                                                      const int* __restrict__ wide, float4* __restrict__ slot,
-                                                      float* __restrict__ fx, float* __restrict__ fy,
-                                                      float* __restrict__ fz, float* __restrict__ pe,
-                                                      float* __restrict__ vir, unsigned* status) {
-    const int cnt = wide[0];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
-        const int i = wide[1 + k];
+// Eight lanes a centre: the queued centres (wide[0] of them, indices from
+// wide[1]), or all of them (then the ones past the register path are still
+// counted).  A lane owns a neighbour: its bond's zeta and gradient first, then
+// what each bond in turn gives to it as its third atom, for which the factors
+// of the triplet are evaluated again (some 30 instructions).  The centre's sums
+// are taken bond by bond in the register path's order, and the products that
+// join a sum are the ones that do there: both forms give the same bits, and a
+// trajectory does not depend on which took a centre.  The queue was one thread a centre over local
+// arrays, a chain of some 190,000 cycles: 0.7 % of the 1.47 M
+// atoms of the impact ensemble, both passes 199 -> 141 us.
+template <bool QUEUED>
+__global__ void __launch_bounds__(TB_LBLOCK) k_tersoff_lanes(
+    TersDev p, const PosPack* __restrict__ pack, const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
+    int* __restrict__ wide, RowHits hits, SlotRows slot, float* __restrict__ fx, float* __restrict__ fy,
+    float* __restrict__ fz, float* __restrict__ pe, float* __restrict__ vir, unsigned* status) {
+    __shared__ float4 gu[TB_LGROUPS][TB_MAXN];  // vector and squared distance, then unit vector and distance
+    __shared__ float4 gf[TB_LGROUPS][TB_MAXN];  // f_c, f_c', 1/r, half the bond's dV/dzeta
+    __shared__ float4 gx[TB_LGROUPS][TB_MAXN];  // one bond's gradients by its neighbours
+    __shared__ float2 ge[TB_LGROUPS][TB_MAXN];  // a bond's energy and its derivative by r
+    __shared__ int gs[TB_LGROUPS][TB_MAXN];
+    constexpr int NJ = TB_MAXN / TB_LANES;
+    const LaneGroup g;
+    float4* u = gu[threadIdx.x / TB_LANES];
+    float4* f = gf[threadIdx.x / TB_LANES];
+    float4* x = gx[threadIdx.x / TB_LANES];
+    float2* ve = ge[threadIdx.x / TB_LANES];
+    int* sl = gs[threadIdx.x / TB_LANES];
+    const float g0 = 1.f + p.c2 / p.d2;
+    const int total = QUEUED ? wide[0] : p.n;
+    for (int c0 = blockIdx.x * TB_LGROUPS + threadIdx.x / TB_LANES; c0 < total; c0 += gridDim.x * TB_LGROUPS) {
+        const int i = QUEUED ? wide[1 + c0] : c0;
         const PosPack pi = pack[i];
         const ShiftF L = p.rep_L ? p.rep_L[p.rep_of[i]] : p.L;
-        ters_centre_wide(p, i, pi, L, pack, nbr, nnb[i], slot, fx, fy, fz, pe, vir, status);
+        const int m = nnb[i];
+        int nc = 0;
+        if (p.single_type || pack_type(pi.hi) == p.ta) {
+            nc = lanes_collect<QUEUED>(g, i, m, pi, L, p.t2, p.single_type ? -1 : p.ta, pack, nbr, p.hshift,
+                                       p.maxnb, hits, slot, u, sl, status);
+            if (!QUEUED && nc > TERS_REG && g.lane == 0) wide[1 + atomicAdd(wide, 1)] = i;
+            nc = min(nc, TB_MAXN);
+        } else if (!QUEUED && g.lane == 0) {
+            no_hits(i, m, hits);
+        }
+        for (int a = g.lane; a < nc; a += TB_LANES) {
+            const float4 v = u[a];
+            const float r = sqrtf(v.w), ri = 1.0f / r;
+            float dfc;
+            const float fc = ters_fc(p, r, dfc);
+            u[a] = make_float4(v.x * ri, v.y * ri, v.z * ri, r);
+            f[a] = make_float4(fc, dfc, ri, 0.f);
+        }
+        __syncwarp(g.mask);
+        float sjx[NJ], sjy[NJ], sjz[NJ], dz[NJ];
+#pragma unroll
+        for (int j = 0; j < NJ; j++) {
+            const int a = j * TB_LANES + g.lane;
+            if (a >= nc) continue;
+            const float4 ua = u[a], fa = f[a];
+            float zeta = 0.f, gjx = 0.f, gjy = 0.f, gjz = 0.f;
+            for (int b = 0; b < nc; b++) {
+                if (b == a) continue;
+                const float4 ub = u[b];
+                const float fb = f[b].x;
+                const float c = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
+                const float hc = p.h - c;
+                const float rden = __fdividef(1.f, p.d2 + hc * hc);
+                const float g = g0 - p.c2 * rden;
+                const float dg = -2.f * p.c2 * hc * rden * rden;
+                const float dr = ua.w - ub.w;
+                const float ex = __expf(p.l3c * dr * dr * dr);
+                const float dex = 3.f * p.l3c * dr * dr * ex;
+                zeta += fb * g * ex;
+                const float cj = fb * dg * ex * fa.z, cu = fb * g * dex;
+                gjx = __fadd_rn(gjx, fma2(cu, ua.x, cj, fmaf(-c, ua.x, ub.x)));
+                gjy = __fadd_rn(gjy, fma2(cu, ua.y, cj, fmaf(-c, ua.y, ub.y)));
+                gjz = __fadd_rn(gjz, fma2(cu, ua.z, cj, fmaf(-c, ua.z, ub.z)));
+            }
+            const float fR = p.A * __expf(-p.l1 * ua.w), fA = p.B * __expf(-p.l2 * ua.w);
+            float bij, dbdz;
+            ters_bond_order(p, zeta, bij, dbdz);
+            const float vij = fa.x * (fR - bij * fA);
+            const float dv_dr = fma2(fa.y, fmaf(-bij, fA, fR), fa.x, fma2(bij * p.l2, fA, -p.l1, fR));
+            const float dv_dz = -fa.x * fA * dbdz;
+            sjx[j] = 0.5f * fma2(dv_dr, ua.x, dv_dz, gjx);
+            sjy[j] = 0.5f * fma2(dv_dr, ua.y, dv_dz, gjy);
+            sjz[j] = 0.5f * fma2(dv_dr, ua.z, dv_dz, gjz);
+            dz[j] = 0.5f * dv_dz;
+            ve[a] = make_float2(vij, dv_dr);
+        }
+        __syncwarp(g.mask);
+#pragma unroll
+        for (int j = 0; j < NJ; j++) {
+            const int a = j * TB_LANES + g.lane;
+            if (a < nc) f[a].w = dz[j];
+        }
+        __syncwarp(g.mask);
+        float skx[NJ], sky[NJ], skz[NJ];
+#pragma unroll
+        for (int j = 0; j < NJ; j++) skx[j] = sky[j] = skz[j] = 0.f;
+        float own = 0.f;  // lane 0 to 4: the centre's x, y, z, energy and virial, in the register path's order
+        for (int a = 0; a < nc; a++) {
+            const float4 ua = u[a];
+            const float s = f[a].w;
+#pragma unroll
+            for (int j = 0; j < NJ; j++) {
+                const int k = j * TB_LANES + g.lane;
+                if (k >= nc) continue;
+                if (k == a) {
+                    x[k] = make_float4(sjx[j], sjy[j], sjz[j], 0.f);
+                    skx[j] -= sjx[j];
+                    sky[j] -= sjy[j];
+                    skz[j] -= sjz[j];
+                    continue;
+                }
+                const float4 uk = u[k], fk = f[k];
+                const float c = ua.x * uk.x + ua.y * uk.y + ua.z * uk.z;
+                const float hc = p.h - c;
+                const float rden = __fdividef(1.f, p.d2 + hc * hc);
+                const float g = g0 - p.c2 * rden;
+                const float dg = -2.f * p.c2 * hc * rden * rden;
+                const float dr = ua.w - uk.w;
+                const float ex = __expf(p.l3c * dr * dr * dr);
+                const float dex = 3.f * p.l3c * dr * dr * ex;
+                const float ck = fma2(fk.y * g, ex, -fk.x * g, dex);
+                const float cc = fk.x * dg * ex * fk.z;
+                const float kx = fma2(ck, uk.x, cc, fmaf(-c, uk.x, ua.x));
+                const float ky = fma2(ck, uk.y, cc, fmaf(-c, uk.y, ua.y));
+                const float kz = fma2(ck, uk.z, cc, fmaf(-c, uk.z, ua.z));
+                x[k] = make_float4(kx, ky, kz, 0.f);
+                // force on k = -gradient
+                skx[j] = fmaf(-s, kx, skx[j]);
+                sky[j] = fmaf(-s, ky, sky[j]);
+                skz[j] = fmaf(-s, kz, skz[j]);
+            }
+            __syncwarp(g.mask);
+            if (g.lane < 3) {
+                const float* xc = &x[0].x + g.lane;
+                own += xc[4 * a];  // the x_i gradient is minus the sum of the others
+                for (int b = 0; b < nc; b++)
+                    if (b != a) own = fmaf(s, xc[4 * b], own);
+            } else if (g.lane == 3) {
+                own += 0.5f * ve[a].x;
+            } else if (g.lane == 4) {
+                own += 0.5f * ve[a].y * ua.w;
+            }
+            __syncwarp(g.mask);
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; j++) {
+            const int k = j * TB_LANES + g.lane;
+            if (k < nc) slot.put(i, sl[k], make_float4(skx[j], sky[j], skz[j], 0.f));
+        }
+        __syncwarp(g.mask);  // the group's neighbours are read: the next centre may overwrite them
+        if (g.lane < 5) {
+            float* out = g.lane == 0 ? fx : g.lane == 1 ? fy : g.lane == 2 ? fz : g.lane == 3 ? pe : vir;
+            out[i] = p.first ? own : out[i] + own;
+        }
     }
 }
 
@@ -714,10 +817,22 @@ __global__ void __launch_bounds__(128) k_zbl(ZBLDev p, const PosPack* __restrict
 // ------------------------------------------------------------------ host
 int threebody_prepare(Context* c) { return OMDG_OK; }
 
-SlotArgs slot_args(const Context* c, bool zero_virial) {
-    return SlotArgs{c->nbr_hshift, c->maxnb, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->rev, c->slot_buf,
-                    zero_virial ? 1 : 0};
+RowHits row_hits(const Context* c) { return RowHits{c->row_hits, (size_t)c->cap}; }
+
+SlotRows slot_rows(const Context* c) {
+    return SlotRows{c->slot_buf, reinterpret_cast<const unsigned*>(c->nbr), c->rev, c->nbr_hshift, c->maxnb};
 }
+
+SlotArgs slot_args(const Context* c, bool zero_virial) {
+    return SlotArgs{c->nbr_hshift, c->maxnb, c->nnb, c->slot_buf, row_hits(c), zero_virial ? 1 : 0};
+}
+
+// All centres in the lane form?
+static bool all_by_lanes(const Context* c, int per_sm) { return c->n < per_sm * c->num_sms; }
+
+// Blocks of the queue's pass: its length is on the device, so one resident
+// set of groups that stride over it.
+static unsigned queue_blocks(const Context* c) { return 8u * (unsigned)c->num_sms; }
 
 // In a step the last gather before the kick joins it (forces_compute decides).
 int gather_slots(Context* c, bool zero_virial) {
@@ -752,7 +867,7 @@ int sw_launch(Context* c, Potential& pot, bool first) {
     p.ta = pot.ta;
     p.L = make_shift(c->box);
     p.rc = (float)s.rc;
-    p.rc2 = (float)(s.rc * s.rc);
+    p.t2 = r2_below(p.rc, (float)(s.rc * s.rc));
     p.A = (float)s.A;
     p.B = (float)s.B;
     p.p = (float)s.p;
@@ -786,14 +901,20 @@ int sw_launch(Context* c, Potential& pot, bool first) {
     p.first = first ? 1 : 0;
     prof_begin(c, "sw_centre");
     clear_wide(c);
-    k_sw_a<<<grid_for(c->n, 128), 128, 0, c->stream>>>(p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb,
-                                                        c->slot_buf, c->fx, c->fy, c->fz, c->pe, c->d_status,
-                                                        c->ters_wide);
-    k_sw_wide<<<2 * c->num_sms, 128, 0, c->stream>>>(p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb,
-                                                     c->ters_wide, c->slot_buf, c->fx, c->fy, c->fz, c->pe,
-                                                     c->d_status);
+    const unsigned* nbr = reinterpret_cast<const unsigned*>(c->nbr);
+    if (all_by_lanes(c, SW_LANE_PER_SM)) {
+        k_sw_lanes<false><<<grid_for(c->n, TB_LGROUPS), TB_LBLOCK, 0, c->stream>>>(
+            p, c->pack, nbr, c->nnb, c->ters_wide, row_hits(c), slot_rows(c), c->fx, c->fy, c->fz, c->pe, c->d_status);
+    } else {
+        k_sw_a<<<grid_for(c->n, TB_BLOCK), TB_BLOCK, 0, c->stream>>>(p, c->pack, nbr, c->nnb, row_hits(c), slot_rows(c),
+                                                                     c->fx, c->fy, c->fz, c->pe, c->ters_wide);
+        k_sw_lanes<true><<<queue_blocks(c), TB_LBLOCK, 0, c->stream>>>(p, c->pack, nbr, c->nnb, c->ters_wide,
+                                                                       row_hits(c), slot_rows(c), c->fx, c->fy, c->fz,
+                                                                       c->pe, c->d_status);
+        c->launches++;
+    }
     prof_end(c);
-    c->launches += 2;
+    c->launches++;
     int rc = check_cuda(c, cudaGetLastError(), "sw");
     if (rc) return rc;
     return gather_slots(c, first);
@@ -803,6 +924,11 @@ int tersoff_launch(Context* c, Potential& pot, bool first) {
     int rc = tersoff_centre(c, pot, first, nullptr);
     if (rc) return rc;
     return gather_slots(c, false);
+}
+
+float tersoff_t2(const TersoffParams& t) {
+    const float rc = (float)(t.R + t.D);
+    return r2_below(rc, rc * rc * 1.0001f);
 }
 
 // Pass A of Tersoff: bond gradients of every centre (or of the centres with
@@ -831,27 +957,33 @@ int tersoff_centre(Context* c, Potential& pot, bool first, const int* mask, cons
     p.h = (float)t.h;
     p.R = (float)t.R;
     p.D = (float)t.D;
-    p.rc = (float)(t.R + t.D);
-    p.rc2 = p.rc * p.rc * 1.0001f;
+    p.t2 = tersoff_t2(t);
     p.first = first ? 1 : 0;
     prof_begin(c, mask ? "tersoff_fallback" : "tersoff_centre");
     clear_wide(c);
-    // a masked pass (the surrogate's fallback, usually for no centre at all)
-    // takes the strided form: one resident grid, each block gone after
-    // reading the count
-    if (c->tb_persistent || mask_count)
-        k_tersoff_a<true><<<std::min(grid_for(c->n, 128), TERS_CTAS_PER_SM * c->num_sms), 128, 0, c->stream>>>(
-            p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->slot_buf, c->fx, c->fy, c->fz, c->pe,
-            c->vir, c->d_status, mask, c->ters_wide, mask_count);
-    else
-        k_tersoff_a<false><<<grid_for(c->n, 128), 128, 0, c->stream>>>(
-            p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->slot_buf, c->fx, c->fy, c->fz, c->pe,
-            c->vir, c->d_status, mask, c->ters_wide, mask_count);
-    k_tersoff_wide<<<2 * c->num_sms, 128, 0, c->stream>>>(p, c->pack, reinterpret_cast<const unsigned*>(c->nbr),
-                                                          c->nnb, c->ters_wide, c->slot_buf, c->fx, c->fy, c->fz,
-                                                          c->pe, c->vir, c->d_status);
+    const unsigned* nbr = reinterpret_cast<const unsigned*>(c->nbr);
+    const RowHits hits = row_hits(c);
+    if (!mask && all_by_lanes(c, TERS_LANE_PER_SM)) {
+        k_tersoff_lanes<false><<<grid_for(c->n, TB_LGROUPS), TB_LBLOCK, 0, c->stream>>>(
+            p, c->pack, nbr, c->nnb, c->ters_wide, hits, slot_rows(c), c->fx, c->fy, c->fz, c->pe, c->vir,
+            c->d_status);
+    } else {
+        // a masked pass (the surrogate's fallback, usually for no centre at
+        // all) takes the strided form: one resident grid, each block gone
+        // after reading the count
+        const unsigned all = grid_for(c->n, TB_BLOCK);
+        const unsigned resident = std::min(all, (unsigned)(TERS_CTAS_PER_SM * c->num_sms));
+        auto pass = mask ? k_tersoff_a<true, true> : c->tb_persistent ? k_tersoff_a<true, false> : k_tersoff_a<false, false>;
+        pass<<<mask || c->tb_persistent ? resident : all, TB_BLOCK, 0, c->stream>>>(
+            p, c->pack, nbr, c->nnb, hits, slot_rows(c), c->fx, c->fy, c->fz, c->pe, c->vir, c->ters_wide, mask,
+            mask_count);
+        k_tersoff_lanes<true><<<queue_blocks(c), TB_LBLOCK, 0, c->stream>>>(p, c->pack, nbr, c->nnb, c->ters_wide,
+                                                                            hits, slot_rows(c), c->fx, c->fy, c->fz,
+                                                                            c->pe, c->vir, c->d_status);
+        c->launches++;
+    }
     prof_end(c);
-    c->launches += 2;
+    c->launches++;
     return check_cuda(c, cudaGetLastError(), "tersoff");
 }
 

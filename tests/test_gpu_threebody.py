@@ -134,6 +134,63 @@ def test_dense_centres_take_the_wide_kernel(omdg_lib, oracle_lib, kind):
     check(st["f"], fref, st["pot"], eref, etol=etol)
 
 
+@pytest.mark.parametrize("kind,ncell,skin", [("sw", 6, 3.0), ("sw", 20, 0.3), ("sw", 20, 3.0), ("tersoff", 6, 3.0),
+                                             ("tersoff", 13, 0.3), ("tersoff", 13, 3.0)])
+def test_both_forms_over_long_rows(omdg_lib, oracle_lib, kind, ncell, skin):
+    """Eight lanes for every centre (1,731 atoms), and a thread a centre with
+    eight lanes for the queued ones (17,579 Tersoff and 64,003 SW atoms), over
+    rows of one word of hit bits and of three (a skin of 3 A: some 65 and 45
+    entries, up to 90)."""
+    oc = oracle_lib
+    x, v, lo, hi = interstitial_silicon(ncell, 71)
+    box = oc.make_box(lo, hi, (1, 1, 1))
+    if kind == "sw":
+        p = oc.SWParam(eps=2.1683, A=7.049556277, B=0.6022245584, p=4, q=0, sigma=2.0951, a=1.80, lam=21.0,
+                       gamma=1.2, icos0=-3.0, usezbl=1, sx0=1.2107, sx1=1.8456, sa0=335.0594, sa1=-492.3905,
+                       sa2=244.5280, sa3=-41.2347, z1=14, z2=14)
+        fref, eref, _ = oc.sw(box, x, oc.neighbors(box, x, 2.0951 * 1.8 + 0.3), p)
+        etol = 2e-5
+    else:
+        p = oc.TersoffParam(A=3264.7, B=95.373, lambda1=3.2394, lambda2=1.3258, lambda3=1.3258, beta=0.33675,
+                            n=22.956, c=4.8381, d=2.0417, h=0.0, R=2.7, D=0.15)
+        fref, eref, _ = oc.tersoff(box, x, oc.neighbors(box, x, 2.85 + 0.3), p)
+        etol = 5e-6
+    with si_context(omdg_lib, x, v, lo, hi, kind) as ctx:
+        ctx.set_neighbor(skin, 1)
+        ctx.compute_forces()
+        st = ctx.get_state()
+        wide = ctx.wide_centres()
+        ctx.compute_forces()
+        again = ctx.get_state()
+    assert wide >= 3, wide
+    check(st["f"], fref, st["pot"], eref, etol=etol)
+    assert np.array_equal(st["f"], again["f"]) and np.array_equal(st["pot"], again["pot"])
+
+
+def test_tersoff_forms_agree_on_a_repeated_cell(omdg_lib):
+    """8,112 atoms (eight lanes a centre) and the same cell three times along z
+    (24,336 atoms, a thread a centre).  A relative vector is the FP32 rounding
+    of the same difference but for 1e-14, so a component may be off by a unit
+    in its last place (2.4e-7 A): with four bonds of at most 50 eV/A^2 a force
+    moves by 5e-5 eV/A at most, and an energy, with bond forces of at most 10
+    eV/A, by 1e-5 eV."""
+    from objectmd_gb300 import inputs
+
+    a, n = 5.431, (13, 13, 6)
+    x, lo, hi = inputs.diamond(n, a)
+    x = inputs.perturb(x, 0.05, 5, lo, hi, (True, True, True))
+    up = np.array([0.0, 0.0, hi[2] - lo[2]])
+    out = []
+    for y, top in ((x, np.array(hi)), (np.vstack([x, x + up, x + 2 * up]), np.array(hi) + 2 * up)):
+        with si_context(omdg_lib, y, np.zeros_like(y), lo, top, "tersoff") as ctx:
+            ctx.compute_forces()
+            out.append(ctx.get_state())
+    for k in range(3):
+        part = slice(k * len(x), (k + 1) * len(x))
+        assert np.abs(out[1]["f"][part] - out[0]["f"]).max() <= 5e-5
+        assert np.abs(out[1]["pot"][part] - out[0]["pot"]).max() <= 1e-5
+
+
 def test_tersoff_nve_conserves_energy(omdg_lib):
     from objectmd_gb300 import inputs
 
