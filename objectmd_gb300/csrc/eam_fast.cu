@@ -371,7 +371,7 @@ __global__ void EAMF_BOUNDS(STAGED) k_eamf_force(EAMFast p, const PosPack* __res
                 F2 kk = s_kk[kslot], ke = s_ke[kslot], kw = s_kw[kslot];
                 unsigned long long kv = s_kv[kslot];
                 // one type on this path; the finalising block changes hdtm only after every block read it
-                kick_atom_terms(ka.p, i, 0, vfx, vfy, vfz, ve, av, ka.st->hdtm[0], vx, vy, vz, kk, ke, kw, kv);
+                kick_atom_terms(ka.p, i, 0, vfx, vfy, vfz, ve, av, ka.st->hdtm[0], vx[i], vy[i], vz[i], vx, vy, vz, kk, ke, kw, kv);
                 s_kk[kslot] = kk;
                 s_ke[kslot] = ke;
                 s_kw[kslot] = kw;

@@ -21,7 +21,7 @@
 
 namespace omdg {
 
-constexpr int KICK_BLOCKS_SM = 6;
+constexpr int KICK_BLOCKS_SM = 4;
 
 __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __restrict__ x, double* __restrict__ y,
                                                     double* __restrict__ z, double* __restrict__ vx,
@@ -122,17 +122,15 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __re
 
 
 // Second half kick v += dt/2 f/m (kick = 1) and the energy ledger: per
-// atom m v^2, the potential and the virial as FP32 pairs, a fixed xor tree
-// per warp and over the warps, FP32-pair block partials; the last block to
-// finish sums the partials in block order (finalize_block).  A thread takes
-// every (grid's threads)-th atom, so that one tree (225 of the 580
-// instructions a warp needed for 32 atoms) serves several atoms and few
-// partials remain.
-// 1,048,576 EAM atoms 38.9 -> 30.7 us.
+// atom m v^2, the potential and the virial as FP32 pairs, then the block's sums
+// and the last block's (ledger_block).  A thread takes every (grid's
+// threads)-th atom, all blocks resident at four a SM: 64 registers, so that an
+// atom's loads are in flight together (at six, 40 registers, 1,048,576 EAM atoms
+// took 29.0 us, at four 24.8).
 // GATHER: the three-body kernels' slots are collected first (slot_sum), their
-// loads' latency beside the half-kick's FP64 work: 512,000 Tersoff atoms 32.9
-// us, 194,184 Stillinger-Weber atoms 27.0, 1.47 M atoms of the impact ensemble
-// 70 (as two kernels, over every slot of the list, 43.6, 42.3 and 111).
+// loads' latency beside the half-kick's: 512,000 Tersoff atoms 32.9 us at six
+// blocks a SM and 24.4 at four, 194,184 Stillinger-Weber atoms 27.0 and 20.8,
+// 1.47 M atoms of the impact ensemble 70 and 56.
 template <bool GATHER>
 __global__ void __launch_bounds__(RED_BLOCK, KICK_BLOCKS_SM) k_kick(
     IntParams p, FinParams f, SlotArgs ga, double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
@@ -151,7 +149,10 @@ __global__ void __launch_bounds__(RED_BLOCK, KICK_BLOCKS_SM) k_kick(
             gp = pe[i];
         }
         gw = vir[i];
-        if (GATHER) {
+        const int t = type[i];
+        const double h = st->hdtm[t];
+        double ux = vx[i], uy = vy[i], uz = vz[i];
+        if (GATHER) {  // (the loads above are in flight beside the slots')
             slot_sum(ga, i, gx, gy, gz, gp);
             fx[i] = gx;
             fy[i] = gy;
@@ -161,13 +162,10 @@ __global__ void __launch_bounds__(RED_BLOCK, KICK_BLOCKS_SM) k_kick(
         }
         // inactive atoms: not integrated, not measured (system.cpp:1067, :1085)
         if (aflag && !(aflag[i] & 1u)) continue;
-        const int t = type[i];
         if (GATHER || (kick && !p.use_f64)) {
-            kick_atom_terms(p, i, t, gx, gy, gz, gp, gw, st->hdtm[t], vx, vy, vz, k, e, w, vmax);
+            kick_atom_terms(p, i, t, gx, gy, gz, gp, gw, h, ux, uy, uz, vx, vy, vz, k, e, w, vmax);
         } else {
-            double ux = vx[i], uy = vy[i], uz = vz[i];
             if (kick) {
-                const double h = st->hdtm[t];
                 ux = fma(f64[3 * (size_t)i], h, ux);
                 uy = fma(f64[3 * (size_t)i + 1], h, uy);
                 uz = fma(f64[3 * (size_t)i + 2], h, uz);
@@ -432,8 +430,8 @@ static FinParams fin_params(Context* c, const IntParams& p, int count_step) {
     f.ledger_cap = c->ledger_cap;
     f.count_step = count_step;
     f.tau = c->thermo_tau;
-    f.tset = c->thermo_T;
-    f.temp_factor = 2.0 / 3.0 / 8.61734279e-05;
+    f.inv_tau = 1.0 / c->thermo_tau;
+    f.kin_set = c->thermo_T / (2.0 / 3.0 / 8.61734279e-05);
     f.ghosts = nullptr;
     f.status = c->d_status;
     f.ticket = reinterpret_cast<unsigned*>(c->d_flags + 4);
@@ -467,7 +465,8 @@ void kick_args(Context* c, KickArgs& ka) {
 
 __global__ void __launch_bounds__(1024) k_ledger_finalize(FinParams f, int nparts, const BlockPartial* partial,
                                                           double* ledger, StepState* st) {
-    finalize_block(f, nparts, partial, ledger, st);
+    __shared__ LedgerSums<1024> s;
+    finalize_block<1024>(s, f, nparts, partial, ledger, st);
 }
 
 void launch_ledger_finalize(Context* c, const KickArgs& ka, int nparts) {
@@ -481,7 +480,6 @@ static int reduce_and_finalize(Context* c, int kick, int count_step) {
         return OMDG_OK;
     }
     IntParams p = int_params(c);
-    int nb = kick_blocks(c);
     FinParams f = fin_params(c, p, count_step);
     if (c->thermo_count_ghosts && count_step && c->thermo_tau > 0.0) {
         // TempController::GetSystemTemperature divides by GetTotalAtom(), which
@@ -505,6 +503,7 @@ static int reduce_and_finalize(Context* c, int kick, int count_step) {
     }
     const bool gather = kick && c->gather_deferred;
     c->gather_deferred = false;
+    const int nb = kick_blocks(c);
     prof_begin(c, gather ? "gather_kick" : "kick");
     auto kernel = gather ? k_kick<true> : k_kick<false>;
     kernel<<<nb, RED_BLOCK, 0, c->stream>>>(p, f, slot_args(c, c->gather_zero_virial), c->vx, c->vy, c->vz, c->fx, c->fy,

@@ -46,8 +46,8 @@ struct FinParams {
     const int* ghosts;    // reference compatibility: periodic images added to the atom count (or null)
     unsigned* status;     // ERR_NONFINITE when a total is NaN or infinite
     unsigned* ticket;     // blocks done (the last one resets it)
-    double tau, tset;     // thermostat (tau <= 0: off)
-    double temp_factor;   // 2/3/k_B (unit.h:66-104)
+    double tau, inv_tau;  // thermostat (tau <= 0: off)
+    double kin_set;       // kinetic energy of an atom at Tset: Tset / (2/3/k_B) (unit.h:66-104)
     int need_vmax;        // SqrMaxVelocity from the block partials
     int dyn_update;       // DynamicTimeStep period (0: off; DynamicTimeStep.h:58-70)
     int dyn_apply;        // this measurement precedes a step's PreIntegration
@@ -68,110 +68,137 @@ __device__ __forceinline__ unsigned long long vmax_bits(const float4& wv) {
     return ((unsigned long long)__float_as_uint(wv.w) << 32) | __float_as_uint(wv.z);
 }
 
-// Ledger row, thermostat factor and step counter from the block partials
-// (one block; each thread sums a contiguous run of partials, then a fixed
-// xor tree per warp and over the warps, all on FP32 pairs; FP64 only for
-// the totals).  Partials are read through L2: other blocks wrote them.
-static __device__ __noinline__ void finalize_block(const FinParams& p, int nblocks, const BlockPartial* partial, double* ledger,
-                               StepState* st) {
-    __shared__ F2 sk[32], se[32], sw[32];
-    __shared__ unsigned long long sv[32];
-    const int nwarps = blockDim.x >> 5;  // a power of two
-    F2 kf = {0.f, 0.f}, ef = {0.f, 0.f}, wf = {0.f, 0.f};
-    unsigned long long vb = 0ull;
-    const int per = (nblocks + (int)blockDim.x - 1) / (int)blockDim.x;
-    const int b0 = threadIdx.x * per, b1 = min(nblocks, b0 + per);
-#pragma unroll 4
-    for (int b = b0; b < b1; b++) {
-        const float4 ke = __ldcg(&partial[b].ke), wv = __ldcg(&partial[b].wv);
-        kf = f2_add(kf, F2{ke.x, ke.y});
-        ef = f2_add(ef, F2{ke.z, ke.w});
-        wf = f2_add(wf, F2{wv.x, wv.y});
-        if (p.need_vmax) vb = max(vb, vmax_bits(wv));
-    }
-    // fixed xor tree within each warp, then over the warps in warp 0
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int o = 16; o > 0; o >>= 1) {
-        kf = f2_add(kf, f2_shfl_xor(kf, o));
-        ef = f2_add(ef, f2_shfl_xor(ef, o));
-        wf = f2_add(wf, f2_shfl_xor(wf, o));
-        if (p.need_vmax) vb = max(vb, __shfl_xor_sync(0xffffffffu, vb, o));
-    }
-    if (lane == 0) {
-        sk[warp] = kf;
-        se[warp] = ef;
-        sw[warp] = wf;
-        sv[warp] = vb;
-    }
-    __syncthreads();
-    if (warp != 0) return;
-    const F2 z = {0.f, 0.f};
-    kf = lane < nwarps ? sk[lane] : z;
-    ef = lane < nwarps ? se[lane] : z;
-    wf = lane < nwarps ? sw[lane] : z;
-    vb = lane < nwarps ? sv[lane] : 0ull;
-    for (int o = nwarps / 2; o > 0; o >>= 1) {
-        kf = f2_add(kf, f2_shfl_xor(kf, o));
-        ef = f2_add(ef, f2_shfl_xor(ef, o));
-        wf = f2_add(wf, f2_shfl_xor(wf, o));
-        if (p.need_vmax) vb = max(vb, __shfl_xor_sync(0xffffffffu, vb, o));
-    }
-    const double k = f2_to_double(kf), e = f2_to_double(ef), w = f2_to_double(wf);
-    const double vm = __longlong_as_double((long long)vb);
-    if (threadIdx.x == 0) {
-        double kinetic = 0.5 * k;
-        if (!(isfinite(kinetic) && isfinite(e))) atomicOr(p.status, ERR_NONFINITE);
-        int row = st->row;
-        int slot = row % p.ledger_cap;  // ring buffer between host reads
-        double* row_out = ledger + LEDGER_W * (size_t)slot;
-        row_out[0] = kinetic;
-        row_out[1] = e;
-        row_out[2] = 0.5 * w;
-        row_out[4] = (double)st->step;  // SysMonitor's Step, ElapsedTime and TimeStep of this step
-        row_out[5] = st->elapsed;
-        row_out[6] = st->dt;
-        row_out[7] = 0.0;
-        double lam = 1.0;
-        if (p.count_step && p.tau > 0.0 && st->step != 0) {
-            // TempController::PostIntegration: T from the system kinetic energy
-            const double count = (double)p.natoms + (p.ghosts ? (double)*p.ghosts : 0.0);
-            double T = p.temp_factor * kinetic / count;
-            if (T > 0.0) lam = sqrt(1. + st->dt / p.tau * (p.tset / T - 1.));
+// A block's sums of the three ledger terms of its T threads, and the largest
+// squared speed, in shared memory: one warp for each sum adds T / 32 terms a
+// lane and then a fixed xor tree (450 instructions for 256 threads; a tree in
+// every warp took 1,800).  Ends with a barrier.
+template <int T>
+struct LedgerSums {
+    F2 terms[3][T], sums[3];
+    unsigned long long vmax[T / 32];
+    // what the last block reads of the step's state, and what follows from it
+    int slot, row, rebuild, dyn, thermo;
+    long long step;
+    double elapsed, dt, a, b;
+
+    __device__ __forceinline__ void add(F2 k, F2 e, F2 w, unsigned long long vm, int need_vmax) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        terms[0][threadIdx.x] = k;
+        terms[1][threadIdx.x] = e;
+        terms[2][threadIdx.x] = w;
+        if (need_vmax) {
+            for (int o = 16; o > 0; o >>= 1) vm = max(vm, __shfl_xor_sync(0xffffffffu, vm, o));
+            if (lane == 0) vmax[warp] = vm;
         }
-        row_out[3] = lam;
-        if (p.need_vmax) st->sqrmaxv = vm;
+        __syncthreads();
+        if (warp < 3) {
+            F2 q = terms[warp][lane];
+#pragma unroll 8
+            for (int j = 1; j < T / 32; j++) q = f2_add(q, terms[warp][32 * j + lane]);
+            for (int o = 16; o > 0; o >>= 1) q = f2_add(q, f2_shfl_xor(q, o));
+            if (lane == 0) sums[warp] = q;
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ unsigned long long largest(int need_vmax) const {
+        unsigned long long v = 0ull;
+        if (need_vmax)
+            for (int q = 0; q < T / 32; q++) v = max(v, vmax[q]);
+        return v;
+    }
+    // By one thread outside the summing warps, beside them: the state's loads
+    // and what does not wait for the sums.
+    __device__ __forceinline__ void prepare(const FinParams& p, const StepState* st) {
+        step = st->step;
+        row = st->row;
+        slot = row % p.ledger_cap;  // ring buffer between host reads
+        elapsed = st->elapsed;
+        dt = st->dt;
+        const long long after = step + (p.count_step ? 1 : 0);
+        const int every = st->rebuild_every;
+        rebuild = p.count_step && every > 0 && after % every == 0;
+        dyn = p.dyn_update > 0 && p.dyn_apply && after % p.dyn_update == 0;
+        thermo = p.count_step && p.tau > 0.0 && step != 0;
+        if (thermo) {
+            const double count = (double)p.natoms + (p.ghosts ? (double)*p.ghosts : 0.0);
+            a = dt * p.inv_tau;
+            b = p.kin_set * count;
+        }
+    }
+    // By one thread: ledger row, thermostat factor and step counter.
+    __device__ __forceinline__ void finish(const FinParams& p, double* __restrict__ ledger, StepState* st) const {
+        const double kinetic = 0.5 * f2_to_double(sums[0]), e = f2_to_double(sums[1]), w = f2_to_double(sums[2]);
+        if (!(isfinite(kinetic) && isfinite(e))) atomicOr(p.status, ERR_NONFINITE);
+        double* out = ledger + LEDGER_W * (size_t)slot;
+        out[0] = kinetic;
+        out[1] = e;
+        out[2] = 0.5 * w;
+        out[4] = (double)step;  // SysMonitor's Step, ElapsedTime and TimeStep of this step
+        out[5] = elapsed;
+        out[6] = dt;
+        out[7] = 0.0;
+        double lam = 1.0;
+        // TempController::PostIntegration: lambda^2 = 1 + dt/tau (Tset/T - 1),
+        // with Tset/T as the quotient of the kinetic energies
+        if (thermo && kinetic > 0.0) lam = sqrt(1. + a * (b / kinetic - 1.));
+        out[3] = lam;
+        const double sqrmaxv = __longlong_as_double((long long)largest(p.need_vmax));
+        if (p.need_vmax) st->sqrmaxv = sqrmaxv;
         if (p.count_step) {
+            const double now = elapsed + dt;  // ElapsedTime += TimeStep; Step++ (system.cpp:979-980)
             st->lambda = lam;
-            st->elapsed += st->dt;  // ElapsedTime += TimeStep; Step++ (system.cpp:979-980)
-            st->step += 1;
+            st->elapsed = now;
+            st->step = step + 1;
             st->row = row + 1;
-            if (st->rebuild_every > 0 && (st->step % st->rebuild_every) == 0) {
+            if (rebuild) {
                 st->rebuild = 1;
                 st->rebuild_all = 1;
             }
             if (p.src_on) {  // EnergySource::PreIntegration of the next step
                 int scale = 0;
-                if (st->elapsed >= p.src_start) {
+                if (now >= p.src_start) {
                     if (st->src_first) st->src_first = 0;  // firstcall: return
-                    else scale = st->elapsed < p.src_stop ? 1 : 0;
+                    else scale = now < p.src_stop ? 1 : 0;
                 }
                 st->src_scale = scale;
             }
         }
-        if (p.dyn_update > 0 && p.dyn_apply && (st->step % p.dyn_update) == 0) {
+        if (dyn) {
             // DynamicTimeStep::PreIntegration of the next step
-            double ndt;
-            if (st->sqrmaxv > 0.0) {
-                ndt = p.dyn_maxpath / (sqrt(st->sqrmaxv) * 1.10);
+            const double v2 = p.need_vmax ? sqrmaxv : st->sqrmaxv;
+            double ndt = p.dyn_maxdt;
+            if (v2 > 0.0) {
+                ndt = p.dyn_maxpath / (sqrt(v2) * 1.10);
                 if (ndt > p.dyn_maxdt) ndt = p.dyn_maxdt;
-            } else {
-                ndt = p.dyn_maxdt;
             }
             st->dt = ndt;
             for (int t = 0; t < MAX_TYPES; t++) st->hdtm[t] = p.mass[t] > 0 ? (0.5 * ndt) / p.mass[t] : 0.0;
         }
         *p.ticket = 0u;
     }
+};
+
+constexpr int LEDGER_PREPARE = 96;  // the thread that prepares: the first one outside the summing warps
+
+// Ledger row, thermostat factor and step counter from the block partials, by
+// one block of T threads (FP32 pairs; FP64 only for the totals).  Partials are
+// read through L2: other blocks wrote them.
+template <int T>
+__device__ __forceinline__ void finalize_block(LedgerSums<T>& s, const FinParams& p, int nblocks,
+                                               const BlockPartial* partial, double* ledger, StepState* st) {
+    if (threadIdx.x == LEDGER_PREPARE) s.prepare(p, st);
+    F2 k = {0.f, 0.f}, e = {0.f, 0.f}, w = {0.f, 0.f};
+    unsigned long long vm = 0ull;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < nblocks; b += T) {
+        const float4 ke = __ldcg(&partial[b].ke), wv = __ldcg(&partial[b].wv);
+        k = f2_add(k, F2{ke.x, ke.y});
+        e = f2_add(e, F2{ke.z, ke.w});
+        w = f2_add(w, F2{wv.x, wv.y});
+        if (p.need_vmax) vm = max(vm, vmax_bits(wv));
+    }
+    s.add(k, e, w, vm, p.need_vmax);
+    if (threadIdx.x == 0) s.finish(p, ledger, st);
 }
 
 // What the neighbours' centre passes left for atom i (three-body kernels), in
@@ -231,17 +258,18 @@ __device__ __forceinline__ void slot_sum(const SlotArgs& a, int i, float& fx, fl
     pe = ge.value();
 }
 
-// One atom's second half-kick v += dt/2 f/m (velocity written back) and
+// One atom's second half-kick v += dt/2 f/m (from ux, uy, uz, written back) and
 // its ledger terms: m v^2 and the potential and virial as FP32 pairs, the
 // squared speed's bits for DynamicTimeStep.  f is FP32 (the FP64 force path
 // does not fuse).
 __device__ __forceinline__ void kick_atom_terms(const IntParams& p, int i, int t, float fxi, float fyi, float fzi,
-                                                float pei, float viri, double h, double* __restrict__ vx,
-                                                double* __restrict__ vy, double* __restrict__ vz, F2& k, F2& e,
-                                                F2& w, unsigned long long& vmax) {
-    double ux = fma(f2d_exact(fxi), h, vx[i]);
-    double uy = fma(f2d_exact(fyi), h, vy[i]);
-    double uz = fma(f2d_exact(fzi), h, vz[i]);
+                                                float pei, float viri, double h, double ux, double uy, double uz,
+                                                double* __restrict__ vx, double* __restrict__ vy,
+                                                double* __restrict__ vz, F2& k, F2& e, F2& w,
+                                                unsigned long long& vmax) {
+    ux = fma(f2d_exact(fxi), h, ux);
+    uy = fma(f2d_exact(fyi), h, uy);
+    uz = fma(f2d_exact(fzi), h, uz);
     vx[i] = ux;
     vy[i] = uy;
     vz[i] = uz;
@@ -255,56 +283,31 @@ __device__ __forceinline__ void kick_atom_terms(const IntParams& p, int i, int t
                              __dadd_rn(__dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy)), __dmul_rn(uz, uz))));
 }
 
-// The block's ledger partial from every thread's terms (a fixed xor tree per
-// warp and over the warps); the last block to finish sums the partials in
-// block order and writes the ledger row (finalize_block).  Every thread of
-// the block calls it.
+// The block's ledger partial from every thread's terms; the last block to
+// finish sums the partials and writes the ledger row (finalize_block).  Every
+// thread of a block of RED_BLOCK calls it.  What comes after the atoms is a
+// chain of latencies in one block, the same for 512 atoms and a million: 12,000
+// cycles with a tree in every warp, fences around the ticket, the state's loads
+// and three FP64 divisions in the thread that had the sums; some 7,500 now, a
+// third of them the quotient and the root of a thermostat.
 __device__ __forceinline__ void ledger_block(const IntParams& p, const FinParams& f, F2 k, F2 e, F2 w,
                                              unsigned long long vmax, BlockPartial* __restrict__ partial,
                                              double* __restrict__ ledger, StepState* st) {
-    if (p.need_vmax)
-        for (int o = 16; o > 0; o >>= 1) vmax = max(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-    for (int o = 16; o > 0; o >>= 1) {
-        k = f2_add(k, f2_shfl_xor(k, o));
-        e = f2_add(e, f2_shfl_xor(e, o));
-        w = f2_add(w, f2_shfl_xor(w, o));
-    }
-    __shared__ F2 wk[32], we[32], ww[32];
-    __shared__ unsigned long long wv[32];
+    __shared__ LedgerSums<RED_BLOCK> s;
     __shared__ bool last;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    if (lane == 0) {
-        wk[warp] = k;
-        we[warp] = e;
-        ww[warp] = w;
-        wv[warp] = vmax;
+    s.add(k, e, w, vmax, p.need_vmax);
+    if (threadIdx.x == 0) {
+        const unsigned long long bv = s.largest(p.need_vmax);
+        partial[blockIdx.x].ke = make_float4(s.sums[0].hi, s.sums[0].lo, s.sums[1].hi, s.sums[1].lo);
+        partial[blockIdx.x].wv = make_float4(s.sums[2].hi, s.sums[2].lo, __uint_as_float((unsigned)bv),
+                                             __uint_as_float((unsigned)(bv >> 32)));
+        // releases this partial, and acquires all others in the last block
+        unsigned done;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(done) : "l"(f.ticket) : "memory");
+        last = done == gridDim.x - 1;
     }
     __syncthreads();
-    if (warp == 0) {
-        const F2 z = {0.f, 0.f};
-        k = lane < nwarps ? wk[lane] : z;
-        e = lane < nwarps ? we[lane] : z;
-        w = lane < nwarps ? ww[lane] : z;
-        for (int o = nwarps / 2; o > 0; o >>= 1) {
-            k = f2_add(k, f2_shfl_xor(k, o));
-            e = f2_add(e, f2_shfl_xor(e, o));
-            w = f2_add(w, f2_shfl_xor(w, o));
-        }
-        if (lane == 0) {
-            unsigned long long bv = 0ull;
-            if (p.need_vmax)
-                for (int q = 0; q < nwarps; q++) bv = max(bv, wv[q]);
-            partial[blockIdx.x].ke = make_float4(k.hi, k.lo, e.hi, e.lo);
-            partial[blockIdx.x].wv = make_float4(w.hi, w.lo, __uint_as_float((unsigned)bv),
-                                                 __uint_as_float((unsigned)(bv >> 32)));
-            __threadfence();
-            last = atomicAdd(f.ticket, 1u) == gridDim.x - 1;
-        }
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    finalize_block(f, gridDim.x, partial, ledger, st);
+    if (last) finalize_block<RED_BLOCK>(s, f, gridDim.x, partial, ledger, st);
 }
 
 // One warp's ledger partial (the per-warp half of ledger_block): lane 0
