@@ -1011,16 +1011,22 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr)
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
     cudaGraphConditionalHandle h = 0;
-    if (!rc) {
+    const bool on_request = small_sort(c);  // the rebuild's kernels are the step's own, and look for the request
+    if (!rc && !on_request) {
         // no rebuild unless the step's kick_drift asks for it
         e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, nullptr, nullptr, nullptr);
         if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
         if (e != cudaSuccess) rc = check_cuda(c, e, "conditional handle");
     }
-    if (!rc) rc = integrate_kick_drift(c, &h);
+    if (!rc) rc = integrate_kick_drift(c, on_request ? nullptr : &h);
     l1 = c->launches;
     cudaGraphNode_t cond_node = nullptr;
-    if (!rc) {
+    if (!rc && on_request) {
+        c->build_in_step = true;
+        rc = nlist_build(c, true);
+        c->build_in_step = false;
+        l1 = c->launches;
+    } else if (!rc) {
         e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, &deps, nullptr, &ndeps);
         cudaGraphNodeParams cp = {};
         cp.type = cudaGraphNodeTypeConditional;

@@ -607,6 +607,7 @@ __global__ void k_rewind(StepState* st, int rebuild_every) {
 // that fill columns of the current row).
 const int* step_state_row(Context* c) { return &reinterpret_cast<StepState*>(c->d_state)->row; }
 int* step_state_halted(Context* c) { return &reinterpret_cast<StepState*>(c->d_state)->halted; }
+int* step_state_building(Context* c) { return &reinterpret_cast<StepState*>(c->d_state)->building; }
 
 int step_state_rewind(Context* c) {
     k_rewind<<<1, 1, 0, c->stream>>>(reinterpret_cast<StepState*>(c->d_state), c->rebuild_every);

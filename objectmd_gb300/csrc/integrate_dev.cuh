@@ -23,6 +23,7 @@ struct StepState {
     int src_scale;           // EnergySource: scale velocities at the next PreIntegration
     int halted;              // a rebuild overflowed its rows: later rebuilds are skipped until omdg_sync recovers
     int rebuild_all;         // replica mode: the request covers every replica (periodic rebuild, state upload)
+    int building;            // small boxes: this step's rebuild kernels run (k_sort_small)
 };
 
 struct IntParams {

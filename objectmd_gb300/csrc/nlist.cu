@@ -18,7 +18,9 @@
 
 #include <climits>
 
-#include "device_common.cuh"
+#include <cooperative_groups.h>
+
+#include "integrate_dev.cuh"
 
 namespace omdg {
 
@@ -75,24 +77,27 @@ __device__ __forceinline__ int axis_cell_of(double& p, int periodic, double lo, 
     return k < 0 ? 0 : (k >= nc ? nc - 1 : k);
 }
 
+// Wraps atom i's position into the box and returns its cell.
+__device__ __forceinline__ int cell_of(int i, double* p, const CellGeom& g, unsigned* status) {
+    const int cx = axis_cell_of(p[0], g.periodic[0], g.lo[0], g.L[0], g.org[0], g.inv_h[0], g.nc[0]);
+    const int cy = axis_cell_of(p[1], g.periodic[1], g.lo[1], g.L[1], g.org[1], g.inv_h[1], g.nc[1]);
+    const int cz = axis_cell_of(p[2], g.periodic[2], g.lo[2], g.L[2], g.org[2], g.inv_h[2], g.nc[2]);
+    if (isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2])) return (cz * g.nc[1] + cy) * g.nc[0] + cx;
+    // spread non-finite atoms over the cells so that the per-cell work stays
+    // bounded; the run is already invalid and the status word says so
+    atomicOr(status, ERR_NONFINITE);
+    return i % (g.nc[0] * g.nc[1] * g.nc[2]);
+}
+
 __global__ void k_cell_assign(int n, double* __restrict__ x, double* __restrict__ y, double* __restrict__ z,
                               CellGeom g, int* __restrict__ cell, int* __restrict__ count, unsigned* status) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double p[3] = {x[i], y[i], z[i]};
-    const int cx = axis_cell_of(p[0], g.periodic[0], g.lo[0], g.L[0], g.org[0], g.inv_h[0], g.nc[0]);
-    const int cy = axis_cell_of(p[1], g.periodic[1], g.lo[1], g.L[1], g.org[1], g.inv_h[1], g.nc[1]);
-    const int cz = axis_cell_of(p[2], g.periodic[2], g.lo[2], g.L[2], g.org[2], g.inv_h[2], g.nc[2]);
+    const int c = cell_of(i, p, g, status);
     x[i] = p[0];
     y[i] = p[1];
     z[i] = p[2];
-    int c = (cz * g.nc[1] + cy) * g.nc[0] + cx;
-    if (!(isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2]))) {
-        // spread non-finite atoms over the cells so that the per-cell work stays
-        // bounded; the run is already invalid and the status word says so
-        atomicOr(status, ERR_NONFINITE);
-        c = i % (g.nc[0] * g.nc[1] * g.nc[2]);
-    }
     cell[i] = c;
     atomicAdd(&count[c], 1);
 }
@@ -389,6 +394,38 @@ struct PackFrame {
 };
 
 // loc: the position rounded to FP32, which the list build screens (w: the type)
+// One atom's packs; returns its share of umax.
+__device__ __forceinline__ float pack_atom(int i, double X, double Y, double Z, int type, bool active,
+                                           const PackFrame& f, PosPack* __restrict__ pack, float4* __restrict__ xref,
+                                           float4* __restrict__ loc) {
+    PosPack p;
+    pack_coord(X, f.Qh[0], f.Ql[0], p.hi.x, p.lo.x);
+    pack_coord(Y, f.Qh[1], f.Ql[1], p.hi.y, p.lo.y);
+    pack_coord(Z, f.Qh[2], f.Ql[2], p.hi.z, p.lo.z);
+    p.hi.w = __int_as_float(type);
+    p.lo.w = 0.f;
+    pack[i] = p;
+    if (xref) xref[i] = make_float4(p.hi.x, p.hi.y, p.hi.z, 0.f);
+    if (!loc) return 0.f;
+    if (!active) {
+        // inactive (SetActive false): far from every centre, so no list takes
+        // it, and outside the band's max |x|
+        loc[i] = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f);
+        return 0.f;
+    }
+    const float ux = f2_from(X).hi, uy = f2_from(Y).hi, uz = f2_from(Z).hi;
+    loc[i] = make_float4(ux, uy, uz, p.hi.w);
+    const float m = fmaxf(fabsf(ux), fmaxf(fabsf(uy), fabsf(uz)));
+    return m <= 3.0e38f ? m : 3.0e38f;  // non-finite: flagged by the cell assignment
+}
+
+// The largest |x| sets the width of the screening band.  Whole warps.
+__device__ __forceinline__ void pack_umax(float m, unsigned* umax) {
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+    if ((threadIdx.x & 31) == 0 && m > 0.f && __float_as_uint(m) > *(volatile unsigned*)umax)
+        atomicMax(umax, __float_as_uint(m));
+}
+
 __global__ void k_pack(int n, const double* __restrict__ x, const double* __restrict__ y,
                        const double* __restrict__ z, const int* __restrict__ type, PackFrame f,
                        PosPack* __restrict__ pack, float4* __restrict__ xref, const int* __restrict__ rep_of,
@@ -396,35 +433,9 @@ __global__ void k_pack(int n, const double* __restrict__ x, const double* __rest
                        const int* __restrict__ rflag) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float m = 0.f;
-    if (i < n && (!rflag || rflag[rep_of[i]])) {
-        PosPack p;
-        const double X = x[i], Y = y[i], Z = z[i];
-        pack_coord(X, f.Qh[0], f.Ql[0], p.hi.x, p.lo.x);
-        pack_coord(Y, f.Qh[1], f.Ql[1], p.hi.y, p.lo.y);
-        pack_coord(Z, f.Qh[2], f.Ql[2], p.hi.z, p.lo.z);
-        p.hi.w = __int_as_float(type[i]);
-        p.lo.w = 0.f;
-        pack[i] = p;
-        if (xref) xref[i] = make_float4(p.hi.x, p.hi.y, p.hi.z, 0.f);
-        if (loc) {
-            if (aflag && !(aflag[i] & 1u)) {
-                // inactive (SetActive false): far from every centre, so no
-                // list takes it, and outside the band's max |x|
-                loc[i] = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f);
-            } else {
-                const float ux = f2_from(X).hi, uy = f2_from(Y).hi, uz = f2_from(Z).hi;
-                loc[i] = make_float4(ux, uy, uz, p.hi.w);
-                m = fmaxf(fabsf(ux), fmaxf(fabsf(uy), fabsf(uz)));
-                if (!(m <= 3.0e38f)) m = 3.0e38f;  // non-finite: flagged by the cell assignment
-            }
-        }
-    }
-    if (loc) {
-        // the largest |x| sets the width of the screening band
-        m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-        if ((threadIdx.x & 31) == 0 && m > 0.f && __float_as_uint(m) > *(volatile unsigned*)umax)
-            atomicMax(umax, __float_as_uint(m));
-    }
+    if (i < n && (!rflag || rflag[rep_of[i]]))
+        m = pack_atom(i, x[i], y[i], z[i], type[i], !aflag || (aflag[i] & 1u), f, pack, xref, loc);
+    if (loc) pack_umax(m, umax);
 }
 
 // EAM cell tiles: besides the list entry, the build writes each entry's
@@ -442,6 +453,7 @@ struct TileOut {
 };
 
 struct BuildParams {
+    const int* on;  // build only if set (a small box's step; else null)
     TileOut to;
     int n, maxnb, hshift;
     int cap;              // LANES = 1: row entries a thread keeps in shared memory
@@ -617,6 +629,7 @@ __global__ void __launch_bounds__(BUILD_THREADS, 7) k_build(
     unsigned* __restrict__ nbr, int* __restrict__ nnb, unsigned* status, int* need, const int* __restrict__ rflag,
     unsigned* __restrict__ nbmask) {
     extern __shared__ unsigned s_row[];
+    if (p.on && !*p.on) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = t / LANES, lane = t % LANES;
     if (i >= p.n) return;  // LANES = 8: whole groups leave together
@@ -863,7 +876,9 @@ constexpr int REV_LANES = 4;
 
 __global__ void k_reverse(int n, int hshift, int maxnb, const unsigned* __restrict__ nbr,
                           const int* __restrict__ nnb, int* __restrict__ rev, unsigned* status,
-                          const int* __restrict__ rep_of, const int* __restrict__ rflag) {
+                          const int* __restrict__ rep_of, const int* __restrict__ rflag,
+                          const int* __restrict__ on) {
+    if (on && !*on) return;
     const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
     const int i = (int)(t / REV_LANES), lane = (int)(t % REV_LANES);
     if (i >= n) return;
@@ -1086,6 +1101,254 @@ void tile_release(Context* c) {
     c->tile_valid = false;
 }
 
+PackFrame pack_frame(const Context* c) {
+    PackFrame f;
+    for (int d = 0; d < 3; d++) {
+        const double Q = c->box.P[d] - c->box.org[d];
+        f.Qh[d] = (float)Q;
+        f.Ql[d] = (float)(Q - (double)f.Qh[d]);
+    }
+    return f;
+}
+
+// The whole re-sort of a small box in one kernel, PER atoms a thread, one
+// cluster: snapshot, wrap, count, scan, order, permute and pack.  An atom stays
+// in its thread's registers from the first phase to the last, so the permutation needs no staging; a barrier of the
+// cluster stands where the general path ends a kernel (14 of them).  Both with
+// the pack, us with some 5 and 10 of launch: 512 atoms 15.2 and 58.6, 4,096 19.1
+// and 64.2, 13,824 25.3 and 65.5, 32,768 42.1 and 65.9.  Same order as there: by cell, then by the old
+// index; a cell of more than CELL_SORT_MAX atoms stays as it came.
+// With `on_request` the kernel is part of every step and returns unless the
+// step's kick_drift asked for a rebuild; the list kernels after it go by
+// st->building: three launches that return cost less than a conditional node
+// that is not taken.  A step of 512 Tersoff atoms, us: 23.5 and 28.4, of 8,000
+// 26.5 and 31.1, of 32,768 31.1 and 36.0.
+constexpr int SORT_THREADS = 1024, SORT_CTAS = 8;
+constexpr int SORT_PER = 4, SORT_CELLS = 4;  // atoms a thread moves, and cells it scans, at most
+
+struct SortArgs {
+    int n, m, on_request, st_bytes;
+    CellGeom g;
+    PackFrame f;
+    StepState* st;
+    unsigned* status;
+    int* taken;
+    AtomArrays a, snap;  // snap.x null: no snapshot
+    unsigned char* st_snap;
+    int *count, *start, *perm, *cell, *inv;
+    const unsigned* aflag;  // null: every atom is active
+    PosPack* pack;
+    float4 *xref, *loc;
+    unsigned* umax;
+};
+
+template <int PER>
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
+    static_assert(sizeof(StepState) <= SORT_THREADS, "a block copies the step state");
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    __shared__ int warp_sum[SORT_THREADS / 32], total;
+    const int rank = (int)cl.block_rank(), t = threadIdx.x, lane = t & 31;
+    const int threads = (int)cl.num_blocks() * SORT_THREADS;
+    const int i = rank * SORT_THREADS + t;
+    if (a.on_request) {
+        // a build that overflowed its rows halts the queued steps' later ones
+        const bool halted = a.st->halted || (a.st->building && (*a.status & ERR_NBR_OVERFLOW));
+        const bool go = !halted && a.st->rebuild;
+        cl.sync();  // every thread has read the same words before one changes them
+        if (!go) {
+            if (i == 0) {
+                a.st->building = 0;
+                if (halted) a.st->halted = 1;
+            }
+            return;
+        }
+    }
+    const bool snap = a.snap.x && !a.st->halted && !*a.taken;
+    double p[PER][3], v[PER][3];
+    int type[PER], id[PER], c[PER], slot[PER];
+    unsigned flag[PER];
+#pragma unroll
+    for (int w = 0; w < PER; w++) {
+        const int j = w * threads + i;
+        if (j >= a.n) continue;
+        p[w][0] = a.a.x[j];
+        p[w][1] = a.a.y[j];
+        p[w][2] = a.a.z[j];
+        v[w][0] = a.a.vx[j];
+        v[w][1] = a.a.vy[j];
+        v[w][2] = a.a.vz[j];
+        type[w] = a.a.type[j];
+        id[w] = a.a.id[j];
+        flag[w] = a.a.flag[j];
+        if (snap) {
+            a.snap.x[j] = p[w][0];
+            a.snap.y[j] = p[w][1];
+            a.snap.z[j] = p[w][2];
+            a.snap.vx[j] = v[w][0];
+            a.snap.vy[j] = v[w][1];
+            a.snap.vz[j] = v[w][2];
+            a.snap.type[j] = type[w];
+            a.snap.id[j] = id[w];
+            a.snap.flag[j] = flag[w];
+        }
+    }
+    for (int q = i; q < a.m; q += threads) a.count[q] = 0;
+    if (i == 0) *a.umax = 0u;
+    cl.sync();  // the counts are zero, and `taken` read
+    if (rank == 0) {
+        if (t == 0 && a.on_request) {
+            a.st->nrebuild += 1;
+            a.st->rebuild = 0;
+            a.st->rebuild_all = 0;
+            a.st->building = 1;
+        }
+        if (snap) {  // the state as it is after the request was taken
+            __syncthreads();
+            if (t < a.st_bytes) a.st_snap[t] = reinterpret_cast<const unsigned char*>(a.st)[t];
+            if (t == 0) *a.taken = 1;
+        }
+    }
+#pragma unroll
+    for (int w = 0; w < PER; w++) {
+        const int j = w * threads + i;
+        if (j >= a.n) continue;
+        c[w] = cell_of(j, p[w], a.g, a.status);
+        slot[w] = atomicAdd(&a.count[c[w]], 1);
+    }
+    cl.sync();
+    // exclusive scan: a thread's run of cells, the block's threads, the blocks
+    const int per = (a.m + threads - 1) / threads;
+    const int q0 = min(a.m, i * per), q1 = min(a.m, q0 + per);
+    int cells[SORT_CELLS], sum = 0;
+#pragma unroll
+    for (int k = 0; k < SORT_CELLS; k++) {
+        cells[k] = q0 + k < q1 ? a.count[q0 + k] : 0;
+        sum += cells[k];
+    }
+    int run = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += u;
+    }
+    if (lane == 31) warp_sum[t >> 5] = run;
+    __syncthreads();
+    if (t < 32) {
+        int w = warp_sum[t];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += u;
+        }
+        warp_sum[t] = w;
+        if (t == 31) total = w;
+    }
+    cl.sync();
+    run += (t >= 32 ? warp_sum[(t >> 5) - 1] : 0) - sum;
+    for (int r = 0; r < rank; r++) run += *cl.map_shared_rank(&total, r);
+#pragma unroll
+    for (int k = 0; k < SORT_CELLS; k++)
+        if (q0 + k < q1) {
+            a.start[q0 + k] = run;
+            run += cells[k];
+        }
+    if (i == 0) a.start[a.m] = a.n;
+    cl.sync();
+#pragma unroll
+    for (int w = 0; w < PER; w++)
+        if (w * threads + i < a.n) a.perm[a.start[c[w]] + slot[w]] = w * threads + i;
+    cl.sync();
+    float u = 0.f;
+#pragma unroll
+    for (int w = 0; w < PER; w++) {
+        const int j = w * threads + i;
+        if (j >= a.n) continue;
+        const int base = a.start[c[w]], in_cell = a.start[c[w] + 1] - base;
+        if (in_cell <= CELL_SORT_MAX) {
+            slot[w] = 0;
+            for (int q = 0; q < in_cell; q++) slot[w] += a.perm[base + q] < j;
+        }
+        const int k = slot[w] = base + slot[w];
+        a.a.x[k] = p[w][0];
+        a.a.y[k] = p[w][1];
+        a.a.z[k] = p[w][2];
+        a.a.vx[k] = v[w][0];
+        a.a.vy[k] = v[w][1];
+        a.a.vz[k] = v[w][2];
+        a.a.type[k] = type[w];
+        a.a.id[k] = id[w];
+        a.a.flag[k] = flag[w];
+        a.cell[k] = c[w];
+        a.inv[id[w]] = k;
+        u = fmaxf(u, pack_atom(k, p[w][0], p[w][1], p[w][2], type[w], !a.aflag || (flag[w] & 1u), a.f, a.pack, a.xref,
+                               a.loc));
+    }
+    pack_umax(u, a.umax);
+    for (int q = 0; q < a.a.extra_n; q++) {
+        double* x = a.a.extra + (size_t)q * a.n;
+        double keep[PER];
+#pragma unroll
+        for (int w = 0; w < PER; w++) keep[w] = w * threads + i < a.n ? x[w * threads + i] : 0.0;
+        cl.sync();
+#pragma unroll
+        for (int w = 0; w < PER; w++)
+            if (w * threads + i < a.n) x[slot[w]] = keep[w];
+    }
+}
+
+static int cells_of(const Context* c) { return c->box.nc[0] * c->box.nc[1] * c->box.nc[2]; }
+
+bool small_sort(const Context* c) {
+    return c->nrep == 0 && !c->tile_want && c->n <= SORT_CTAS * SORT_THREADS * SORT_PER &&
+           (long)c->box.nc[0] * c->box.nc[1] * c->box.nc[2] <= SORT_CTAS * SORT_THREADS * SORT_CELLS;
+}
+
+static int launch_sort_small(Context* c, const CellGeom& g, int m, bool on_request, unsigned* umax) {
+    SortArgs a;
+    a.n = c->n;
+    a.m = m;
+    a.on_request = on_request ? 1 : 0;
+    a.st_bytes = (int)step_state_bytes();
+    a.g = g;
+    a.f = pack_frame(c);
+    a.st = reinterpret_cast<StepState*>(c->d_state);
+    a.status = c->d_status;
+    a.taken = c->d_flags + 6;
+    a.a = AtomArrays{c->x, c->y, c->z, c->vx, c->vy, c->vz, c->type, c->id, c->aflag, c->extra, c->extra_n};
+    a.snap = AtomArrays{};
+    if (c->build_in_step && c->snap_d)
+        a.snap = AtomArrays{c->snap_d, c->snap_d + c->cap, c->snap_d + 2 * (size_t)c->cap, c->snap_d + 3 * (size_t)c->cap,
+                            c->snap_d + 4 * (size_t)c->cap, c->snap_d + 5 * (size_t)c->cap, c->snap_i,
+                            c->snap_i + c->cap, reinterpret_cast<unsigned*>(c->snap_i + 2 * (size_t)c->cap), nullptr, 0};
+    a.st_snap = static_cast<unsigned char*>(c->snap_state);
+    a.count = c->cell_count;
+    a.start = c->cell_start;
+    a.perm = c->perm;
+    a.cell = c->cell_sorted;
+    a.inv = c->inv;
+    a.aflag = c->flags_used ? c->aflag : nullptr;
+    a.pack = c->pack;
+    a.xref = c->xref;
+    a.loc = c->loc;
+    a.umax = umax;
+    int blocks = 1;
+    while (blocks < SORT_CTAS && (blocks * SORT_THREADS < c->n || blocks * SORT_THREADS * SORT_CELLS < m)) blocks *= 2;
+    const int per = grid_for(c->n, blocks * SORT_THREADS);
+    auto kernel = per <= 1 ? k_sort_small<1> : per <= 2 ? k_sort_small<2> : k_sort_small<4>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(SORT_THREADS);
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    c->launches++;
+    return check_cuda(c, cudaLaunchKernelEx(&cfg, kernel, a), "small sort");
+}
+
 size_t nlist_slots(const Context* c, int maxnb) {
     size_t H = (size_t)1 << c->nbr_hshift;
     size_t slices = ((size_t)c->cap + H - 1) / H;
@@ -1136,16 +1399,6 @@ static int ensure_cells(Context* c, int m) {
     return OMDG_OK;
 }
 
-PackFrame pack_frame(const Context* c) {
-    PackFrame f;
-    for (int d = 0; d < 3; d++) {
-        const double Q = c->box.P[d] - c->box.org[d];
-        f.Qh[d] = (float)Q;
-        f.Ql[d] = (float)(Q - (double)f.Qh[d]);
-    }
-    return f;
-}
-
 int integrate_pack(Context* c) {
     if (c->n == 0) return OMDG_OK;
     // xref keeps the positions of the last build (the displacement reference)
@@ -1155,84 +1408,91 @@ int integrate_pack(Context* c) {
     return check_cuda(c, cudaGetLastError(), "pack");
 }
 
-int nlist_build(Context* c) {
+// on_request: the kernels look for the step's request themselves (small_sort
+// boxes, inside a captured step).
+int nlist_build(Context* c, bool on_request) {
     int n = c->n;
     if (n == 0) return OMDG_OK;
     CellGeom g = cell_geom(c);
     const bool reps = c->nrep > 0;
-    int m = reps ? c->rep_cells : g.nc[0] * g.nc[1] * g.nc[2];
+    int m = reps ? c->rep_cells : cells_of(c);
     int rc = ensure_cells(c, m);
     if (rc) return rc;
     cudaStream_t s = c->stream;
-    prof_begin(c, "cell_sort");
-    if (c->build_in_step && c->snap_d) {
-        AtomArrays cur0{c->x, c->y, c->z, c->vx, c->vy, c->vz, c->type, c->id, c->aflag, nullptr, 0};
-        AtomArrays snap{c->snap_d, c->snap_d + c->cap, c->snap_d + 2 * (size_t)c->cap, c->snap_d + 3 * (size_t)c->cap,
-                        c->snap_d + 4 * (size_t)c->cap, c->snap_d + 5 * (size_t)c->cap, c->snap_i,
-                        c->snap_i + c->cap, reinterpret_cast<unsigned*>(c->snap_i + 2 * (size_t)c->cap), nullptr, 0};
-        const int sb = (int)step_state_bytes();
-        int* taken = c->d_flags + 6;
-        k_snapshot<<<grid_for(std::max(n, sb), 256), 256, 0, s>>>(
-            n, step_state_halted(c), taken, cur0, snap, static_cast<const unsigned char*>(c->d_state),
-            static_cast<unsigned char*>(c->snap_state), sb);
-        k_set_one<<<1, 1, 0, s>>>(taken);
-        c->launches += 2;
-    }
+    unsigned* umax = reinterpret_cast<unsigned*>(c->d_flags + 3);
+    const RepGeom* rg = reps ? static_cast<const RepGeom*>(c->d_rep_geom) : nullptr;
+    int* cell_sorted = c->cell_sorted;
     // a partial build (replica mode, inside a step): only the replicas whose
     // atoms moved past skin/2 are re-sorted and re-listed; every replica keeps
     // its index range and cell range, so the others' arrays stay valid
     const int* rflag = (reps && c->build_partial) ? c->d_rep_flag : nullptr;
-    if (rflag)
-        k_zero_cells_rep<<<grid_for(m + 1, 256), 256, 0, s>>>(m, c->cell_count, c->cell_fill, c->d_cell_rep, rflag);
-    else
-        k_zero_ints<<<grid_for(m + 1, 256), 256, 0, s>>>(m + 1, c->cell_count, c->cell_fill);
-    if (reps)
-        k_cell_assign_rep<<<grid_for(n, 256), 256, 0, s>>>(n, c->x, c->y, c->z, c->d_rep_of,
-                                                             static_cast<const RepGeom*>(c->d_rep_geom), c->cell,
-                                                             c->cell_count, c->d_status, rflag);
-    else
-        k_cell_assign<<<grid_for(n, 256), 256, 0, s>>>(n, c->x, c->y, c->z, g, c->cell, c->cell_count,
-                                                         c->d_status);
-    const int ntiles = (m + SCAN_TILE - 1) / SCAN_TILE;
-    k_scan_tiles<<<ntiles, SCAN_THREADS, 0, s>>>(m, c->cell_count, c->cell_start, c->cell_tile_sum);
-    k_scan_totals<<<1, 1024, 0, s>>>(ntiles, m, c->cell_tile_sum, c->cell_start);
-    k_scan_add<<<grid_for(m, 256), 256, 0, s>>>(m, c->cell_start, c->cell_tile_sum);
-    k_scatter<<<grid_for(n, 256), 256, 0, s>>>(n, c->cell, c->cell_start, c->cell_fill, c->perm, c->d_rep_of, rflag);
-    // most cells of a sparse grid (replica margins, vacuum) hold 0 or 1 atoms:
-    // a bounded grid of warps strides over the cells instead of one warp each
-    // sparse grids (a few atoms per cell) sort most cells a thread each;
-    // dense ones (EAM: ~20 atoms per cell) leave every cell to the warps
-    const bool sparse = n < 8 * m;
-    int* big = nullptr;  // the queue of cells for the warps: the cell_fill array, free again after the scatter
-    if (sparse) {
-        big = c->cell_fill;
-        k_zero_ints<<<1, 32, 0, s>>>(1, big, big);
-        k_cell_sort_small<<<grid_for(m, 256), 256, 0, s>>>(m, c->cell_start, c->perm, c->d_cell_rep, rflag, big);
+    prof_begin(c, "cell_sort");
+    if (small_sort(c)) {
+        if ((rc = launch_sort_small(c, g, m, on_request, umax))) return rc;
+        prof_end(c);
+    } else {
+        if (c->build_in_step && c->snap_d) {
+            AtomArrays cur0{c->x, c->y, c->z, c->vx, c->vy, c->vz, c->type, c->id, c->aflag, nullptr, 0};
+            AtomArrays snap{c->snap_d, c->snap_d + c->cap, c->snap_d + 2 * (size_t)c->cap, c->snap_d + 3 * (size_t)c->cap,
+                            c->snap_d + 4 * (size_t)c->cap, c->snap_d + 5 * (size_t)c->cap, c->snap_i,
+                            c->snap_i + c->cap, reinterpret_cast<unsigned*>(c->snap_i + 2 * (size_t)c->cap), nullptr, 0};
+            const int sb = (int)step_state_bytes();
+            int* taken = c->d_flags + 6;
+            k_snapshot<<<grid_for(std::max(n, sb), 256), 256, 0, s>>>(
+                n, step_state_halted(c), taken, cur0, snap, static_cast<const unsigned char*>(c->d_state),
+                static_cast<unsigned char*>(c->snap_state), sb);
+            k_set_one<<<1, 1, 0, s>>>(taken);
+            c->launches += 2;
+        }
+        if (rflag)
+            k_zero_cells_rep<<<grid_for(m + 1, 256), 256, 0, s>>>(m, c->cell_count, c->cell_fill, c->d_cell_rep, rflag);
+        else
+            k_zero_ints<<<grid_for(m + 1, 256), 256, 0, s>>>(m + 1, c->cell_count, c->cell_fill);
+        if (reps)
+            k_cell_assign_rep<<<grid_for(n, 256), 256, 0, s>>>(n, c->x, c->y, c->z, c->d_rep_of,
+                                                                 static_cast<const RepGeom*>(c->d_rep_geom), c->cell,
+                                                                 c->cell_count, c->d_status, rflag);
+        else
+            k_cell_assign<<<grid_for(n, 256), 256, 0, s>>>(n, c->x, c->y, c->z, g, c->cell, c->cell_count,
+                                                             c->d_status);
+        const int ntiles = (m + SCAN_TILE - 1) / SCAN_TILE;
+        k_scan_tiles<<<ntiles, SCAN_THREADS, 0, s>>>(m, c->cell_count, c->cell_start, c->cell_tile_sum);
+        k_scan_totals<<<1, 1024, 0, s>>>(ntiles, m, c->cell_tile_sum, c->cell_start);
+        k_scan_add<<<grid_for(m, 256), 256, 0, s>>>(m, c->cell_start, c->cell_tile_sum);
+        k_scatter<<<grid_for(n, 256), 256, 0, s>>>(n, c->cell, c->cell_start, c->cell_fill, c->perm, c->d_rep_of, rflag);
+        // most cells of a sparse grid (replica margins, vacuum) hold 0 or 1 atoms:
+        // a bounded grid of warps strides over the cells instead of one warp each
+        // sparse grids (a few atoms per cell) sort most cells a thread each;
+        // dense ones (EAM: ~20 atoms per cell) leave every cell to the warps
+        const bool sparse = n < 8 * m;
+        int* big = nullptr;  // the queue of cells for the warps: the cell_fill array, free again after the scatter
+        if (sparse) {
+            big = c->cell_fill;
+            k_zero_ints<<<1, 32, 0, s>>>(1, big, big);
+            k_cell_sort_small<<<grid_for(m, 256), 256, 0, s>>>(m, c->cell_start, c->perm, c->d_cell_rep, rflag, big);
+            c->launches += 2;
+        }
+        k_cell_sort_warp<<<std::min(grid_for(m, 8), 16 * c->num_sms), 256, 0, s>>>(
+            m, c->cell_start, c->perm, sparse ? CELL_SORT_SMALL : 1, c->d_cell_rep, rflag, big);
+        c->launches += 7;
+        AtomArrays cur{c->x, c->y, c->z, c->vx, c->vy, c->vz, c->type, c->id, c->aflag, c->extra, c->extra_n};
+        AtomArrays stg{c->stage_d, c->stage_d + c->cap, c->stage_d + 2 * (size_t)c->cap, c->stage_d + 3 * (size_t)c->cap,
+                       c->stage_d + 4 * (size_t)c->cap, c->stage_d + 5 * (size_t)c->cap, c->stage_i,
+                       c->stage_i + c->cap, reinterpret_cast<unsigned*>(c->stage_i + 2 * (size_t)c->cap),
+                       c->stage_extra, c->extra_n};
+        k_permute_gather<<<grid_for(n, 256), 256, 0, s>>>(n, c->perm, cur, stg, c->cell, cell_sorted, c->inv,
+                                                          c->d_rep_of, rflag);
+        k_permute_copyback<<<grid_for(n, 256), 256, 0, s>>>(n, stg, cur, c->d_rep_of, rflag);
         c->launches += 2;
+        prof_end(c);
+        prof_begin(c, "pack");
+        k_zero_ints<<<1, 32, 0, s>>>(1, c->d_flags + 3, c->d_flags + 3);
+        k_pack<<<grid_for(n, 256), 256, 0, s>>>(n, c->x, c->y, c->z, c->type, pack_frame(c), c->pack, c->xref,
+                                                reps ? c->d_rep_of : nullptr, c->flags_used ? c->aflag : nullptr, c->loc,
+                                                umax, rflag);
+        c->launches += 2;
+        prof_end(c);
     }
-    k_cell_sort_warp<<<std::min(grid_for(m, 8), 16 * c->num_sms), 256, 0, s>>>(
-        m, c->cell_start, c->perm, sparse ? CELL_SORT_SMALL : 1, c->d_cell_rep, rflag, big);
-    c->launches += 7;
-    AtomArrays cur{c->x, c->y, c->z, c->vx, c->vy, c->vz, c->type, c->id, c->aflag, c->extra, c->extra_n};
-    AtomArrays stg{c->stage_d, c->stage_d + c->cap, c->stage_d + 2 * (size_t)c->cap, c->stage_d + 3 * (size_t)c->cap,
-                   c->stage_d + 4 * (size_t)c->cap, c->stage_d + 5 * (size_t)c->cap, c->stage_i,
-                   c->stage_i + c->cap, reinterpret_cast<unsigned*>(c->stage_i + 2 * (size_t)c->cap),
-                   c->stage_extra, c->extra_n};
-    int* cell_sorted = c->cell_sorted;
-    k_permute_gather<<<grid_for(n, 256), 256, 0, s>>>(n, c->perm, cur, stg, c->cell, cell_sorted, c->inv,
-                                                      c->d_rep_of, rflag);
-    k_permute_copyback<<<grid_for(n, 256), 256, 0, s>>>(n, stg, cur, c->d_rep_of, rflag);
-    c->launches += 2;
-    prof_end(c);
-    prof_begin(c, "pack");
-    const RepGeom* rg = reps ? static_cast<const RepGeom*>(c->d_rep_geom) : nullptr;
-    unsigned* umax = reinterpret_cast<unsigned*>(c->d_flags + 3);
-    k_zero_ints<<<1, 32, 0, s>>>(1, c->d_flags + 3, c->d_flags + 3);
-    k_pack<<<grid_for(n, 256), 256, 0, s>>>(n, c->x, c->y, c->z, c->type, pack_frame(c), c->pack, c->xref,
-                                            reps ? c->d_rep_of : nullptr, c->flags_used ? c->aflag : nullptr, c->loc,
-                                            umax, rflag);
-    c->launches += 2;
-    prof_end(c);
 
     BuildParams bp;
     bp.to = TileOut{};
@@ -1270,6 +1530,7 @@ int nlist_build(Context* c) {
         bp.to.cap = c->tile_cap;
     }
     c->tile_valid = tiles;
+    bp.on = on_request ? step_state_building(c) : nullptr;
     bp.n = n;
     bp.maxnb = c->maxnb;
     bp.hshift = c->nbr_hshift;
@@ -1311,7 +1572,7 @@ int nlist_build(Context* c) {
         else one ? launch(k_build<1, false, false, true>) : launch(k_build<1, false, false, false>);
     }
     c->launches++;
-    if (c->build_in_step) {
+    if (c->build_in_step && !on_request) {  // (k_sort_small looks for itself)
         k_halt_on_overflow<<<1, 1, 0, s>>>(c->d_status, step_state_halted(c));
         c->launches++;
     }
@@ -1321,7 +1582,7 @@ int nlist_build(Context* c) {
         prof_begin(c, "nlist_reverse");
         k_reverse<<<grid_for(n, 128 / REV_LANES), 128, 0, s>>>(n, c->nbr_hshift, c->maxnb,
                                                    reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->rev,
-                                                   c->d_status, c->d_rep_of, rflag);
+                                                   c->d_status, c->d_rep_of, rflag, bp.on);
         c->launches++;
         prof_end(c);
     }

@@ -368,7 +368,7 @@ void prof_end(Context* c);
 void prof_collect(Context* c);
 
 // neighbour list (nlist.cu)
-int nlist_build(Context* c);
+int nlist_build(Context* c, bool on_request = false);
 void nlist_prepare_geometry(Context* c);
 int nlist_reserve(Context* c, int maxnb);
 size_t nlist_slots(const Context* c, int maxnb);
@@ -406,6 +406,8 @@ int replica_prepare(Context* c);  // per-replica cell grids and shifts (host, be
 int thermo_detect(Context* c, bool after_step);  // local thermodynamics (ttm.cu); after_step: the step advanced the ledger row
 const int* step_state_row(Context* c);           // device address of the ledger row counter (integrate.cu)
 int* step_state_halted(Context* c);              // device address of the step state's halt flag
+int* step_state_building(Context* c);            // and of "this step's rebuild kernels run"
+bool small_sort(const Context* c);               // the one-kernel sort takes this box (nlist.cu)
 size_t step_state_bytes();
 double thermo_ercut(const Context* c);  // the detector's cutoff (its own, else the largest force cutoff); -1: off
 int ttm_pre(Context* c);          // electron temperature step and rescaling before a step

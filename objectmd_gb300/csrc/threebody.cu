@@ -25,10 +25,10 @@ namespace omdg {
 constexpr int TB_MAXN = 24;  // neighbours within the cutoff one atom can hold
 
 // Below this many atoms a SM every centre takes eight lanes.  Thread and lane
-// form, us with some 5 of launch: Tersoff 512 atoms 16.5, 11.7; 8,000 16.4,
-// 13.0; 17,576 16.6, 17.3; SW 512 19.0, 11.6; 32,768 24.8, 17.8; 64,000 28.1,
+// form, us with some 5 of launch: Tersoff 512 atoms 16.5, 13.7; 8,000 16.4,
+// 15.1; 13,824 16.6, 21.1; SW 512 19.0, 11.6; 32,768 24.8, 17.8; 64,000 28.1,
 // 26.2; 140,608 39.0, 42.7.
-constexpr int TERS_LANE_PER_SM = 96;
+constexpr int TERS_LANE_PER_SM = 64;
 constexpr int SW_LANE_PER_SM = 400;
 constexpr int TB_BLOCK = 128;  // thread-a-centre kernels
 constexpr int TB_LANES = 8;    // lanes a centre in the other form

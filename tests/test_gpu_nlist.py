@@ -109,3 +109,37 @@ def test_rows_past_the_shared_columns(omdg_lib, oracle_lib, n, side, ntypes):
             ctx.set_launch("build_lanes", mode)
             ctx.build_neighbors()
             assert nbr_set(*ctx.neighbors()) == ref, mode
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 8192, 8193, 16384, 16385, 32768, 32769])
+def test_small_sort_edges(omdg_lib, oracle_lib, n):
+    """The one-kernel sort at the edges of its blocks and of the atoms a thread
+    moves, and the general path one atom past it: the list is the oracle's, and
+    after steps that each rebuild (the sort looks for their request) so is the
+    list of the new positions, with every atom still under its own id."""
+    from objectmd_gb300 import inputs
+
+    oc = oracle_lib
+    side = max(3, int(np.ceil((n / 8) ** (1.0 / 3.0))))
+    x, v, (lo, hi) = inputs.diamond_silicon(ncell=side, a=5.431, sigma=0.05, temp=600.0, seed_pos=3, seed_vel=4)
+    pick = np.random.default_rng(n).permutation(len(x))[:n]  # vacancies, and an order that is not the cells'
+    x, v = x[pick], v[pick]
+    box = oc.make_box(lo, hi, (1, 1, 1))
+    rv = 2.85 + SKIN
+    with omdg_lib.Context(0) as ctx:
+        ctx.set_box(lo, hi)
+        ctx.set_atoms(x, v, masses=[inputs.md_mass("silicon")], znum=[14.0])
+        ctx.add_tersoff(os.path.join(TABLES, "tersoff.silicon27"))
+        ctx.set_neighbor(SKIN, 1)
+        ctx.compute_forces()
+        assert nbr_set(*ctx.neighbors()) == nbr_set(*oc.neighbors(box, x, rv))
+        ctx.set_timestep(0.001)
+        b0 = ctx.stats()["rebuilds"]
+        ctx.step(3)
+        assert ctx.stats()["rebuilds"] - b0 >= 3
+        st = ctx.get_state()
+        ctx.compute_forces()
+        assert nbr_set(*ctx.neighbors()) == nbr_set(*oc.neighbors(box, st["x"], rv))
+    d = st["x"] - x
+    d -= (np.asarray(hi) - np.asarray(lo)) * np.round(d / (np.asarray(hi) - np.asarray(lo)))
+    assert np.abs(d).max() < 0.5  # three femtoseconds: no atom took another's place
