@@ -262,6 +262,11 @@ struct GraphState {
     cudaGraph_t graph = nullptr;
     cudaStream_t side = nullptr;
     bool valid = false;
+    // GRAPH_STEPS steps in one graph, once enough steps were replayed one by one
+    cudaGraphExec_t many_exec = nullptr;
+    cudaGraph_t many_graph = nullptr;
+    bool many_valid = false;
+    long replayed = 0;
     // the same step with download branches into pinned host arrays
     // (omdg_step_io), keyed by the x, v, f output pointers
     cudaGraphExec_t io_exec = nullptr;
@@ -281,11 +286,14 @@ void invalidate_graph(Context* c) {
     GraphState& gs = it->second;
     if (gs.exec) cudaGraphExecDestroy(gs.exec);
     if (gs.graph) cudaGraphDestroy(gs.graph);
+    if (gs.many_exec) cudaGraphExecDestroy(gs.many_exec);
+    if (gs.many_graph) cudaGraphDestroy(gs.many_graph);
     if (gs.io_exec) cudaGraphExecDestroy(gs.io_exec);
     if (gs.io_graph) cudaGraphDestroy(gs.io_graph);
-    gs.exec = gs.io_exec = nullptr;
-    gs.graph = gs.io_graph = nullptr;
-    gs.valid = gs.io_valid = false;
+    gs.exec = gs.many_exec = gs.io_exec = nullptr;
+    gs.graph = gs.many_graph = gs.io_graph = nullptr;
+    gs.valid = gs.many_valid = gs.io_valid = false;
+    gs.replayed = 0;
 }
 }  // namespace omdg
 
@@ -984,7 +992,16 @@ static int eager_maybe_rebuild(Context* c) {
 // any rebuild's order) are final, f once the forces are, and v after the
 // kick, while the force and kick kernels run; the branch joins before the
 // step ends.
-static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr) {
+//
+// steps > 1: that many steps one after the other in one graph.  A replay
+// boundary costs the device 3.5 us (three small kernels a step and a
+// conditional node, us a step: 14.4 in graphs of one, 11.3 of four, 11.0 of
+// eight; without the node 6.2, 2.6, 2.6), a capture and instantiation some 0.1
+// to 1 ms, so the graph is made once a run has replayed GRAPH_AFTER steps of
+// the same context one by one.
+constexpr int GRAPH_STEPS = 8;
+constexpr long GRAPH_AFTER = 64;
+static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr, int steps = 1) {
     cudaStream_t s = c->stream;
     if (!gs.side) cudaStreamCreateWithFlags(&gs.side, cudaStreamNonBlocking);
     if (io && !gs.io_side) {
@@ -1003,81 +1020,86 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr)
     };
     cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return check_cuda(c, e, "capture begin");
-    long l0 = c->launches, l1 = 0, l2 = 0;
-    int rc = (c->ttm && ttm_active(c)) ? ttm_pre(c) : OMDG_OK;  // PreIntegration (TTM_Homogen_SCNA.h:352)
-    if (!rc) rc = energy_source(c);                                 // PreIntegration (EnergySource.h:113)
-    cudaGraph_t g = nullptr;
-    cudaStreamCaptureStatus cst;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    cudaGraphConditionalHandle h = 0;
-    const bool on_request = small_sort(c);  // the rebuild's kernels are the step's own, and look for the request
-    if (!rc && !on_request) {
-        // no rebuild unless the step's kick_drift asks for it
-        e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, nullptr, nullptr, nullptr);
-        if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
-        if (e != cudaSuccess) rc = check_cuda(c, e, "conditional handle");
-    }
-    if (!rc) rc = integrate_kick_drift(c, on_request ? nullptr : &h);
-    l1 = c->launches;
-    cudaGraphNode_t cond_node = nullptr;
-    if (!rc && on_request) {
-        c->build_in_step = true;
-        rc = nlist_build(c, true);
-        c->build_in_step = false;
+    const long launches0 = c->launches;
+    long l0 = 0, l1 = 0, l2 = 0, l3 = 0;
+    int rc = OMDG_OK;
+    for (int k = 0; k < steps && !rc; k++) {
+        l0 = c->launches;
+        rc = (c->ttm && ttm_active(c)) ? ttm_pre(c) : OMDG_OK;  // PreIntegration (TTM_Homogen_SCNA.h:352)
+        if (!rc) rc = energy_source(c);                                 // PreIntegration (EnergySource.h:113)
+        cudaGraph_t g = nullptr;
+        cudaStreamCaptureStatus cst;
+        const cudaGraphNode_t* deps = nullptr;
+        size_t ndeps = 0;
+        cudaGraphConditionalHandle h = 0;
+        const bool on_request = small_sort(c);  // the rebuild's kernels are the step's own, and look for the request
+        if (!rc && !on_request) {
+            // no rebuild unless the step's kick_drift asks for it
+            e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, nullptr, nullptr, nullptr);
+            if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
+            if (e != cudaSuccess) rc = check_cuda(c, e, "conditional handle");
+        }
+        if (!rc) rc = integrate_kick_drift(c, on_request ? nullptr : &h);
         l1 = c->launches;
-    } else if (!rc) {
-        e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, &deps, nullptr, &ndeps);
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = h;
-        cp.conditional.type = cudaGraphCondTypeIf;
-        cp.conditional.size = 1;
-        if (e == cudaSuccess) e = cudaGraphAddNode(&cond_node, g, deps, nullptr, ndeps, &cp);
-        if (e == cudaSuccess)
-            e = cudaStreamUpdateCaptureDependencies(s, &cond_node, nullptr, 1, cudaStreamSetCaptureDependencies);
-        if (e != cudaSuccess) rc = check_cuda(c, e, "conditional node");
-        if (!rc) {
-            // populate the body: the rebuild pipeline, captured on a side stream
-            cudaGraph_t body = cp.conditional.phGraph_out[0];
-            e = cudaStreamBeginCaptureToGraph(gs.side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-            if (e != cudaSuccess) rc = check_cuda(c, e, "body capture");
+        cudaGraphNode_t cond_node = nullptr;
+        if (!rc && on_request) {
+            c->build_in_step = true;
+            rc = nlist_build(c, true);
+            c->build_in_step = false;
+            l1 = c->launches;
+        } else if (!rc) {
+            e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, &deps, nullptr, &ndeps);
+            cudaGraphNodeParams cp = {};
+            cp.type = cudaGraphNodeTypeConditional;
+            cp.conditional.handle = h;
+            cp.conditional.type = cudaGraphCondTypeIf;
+            cp.conditional.size = 1;
+            if (e == cudaSuccess) e = cudaGraphAddNode(&cond_node, g, deps, nullptr, ndeps, &cp);
+            if (e == cudaSuccess)
+                e = cudaStreamUpdateCaptureDependencies(s, &cond_node, nullptr, 1, cudaStreamSetCaptureDependencies);
+            if (e != cudaSuccess) rc = check_cuda(c, e, "conditional node");
             if (!rc) {
-                c->stream = gs.side;
-                c->build_in_step = true;
-                c->build_partial = c->nrep > 0;  // the flagged replicas only
-                rc = launch_take_rebuild(c);
-                if (!rc) rc = nlist_build(c);
-                c->build_partial = false;
-                c->build_in_step = false;
-                c->stream = s;
-                cudaGraph_t body_out = nullptr;
-                e = cudaStreamEndCapture(gs.side, &body_out);
-                if (!rc && e != cudaSuccess) rc = check_cuda(c, e, "body capture end");
+                // populate the body: the rebuild pipeline, captured on a side stream
+                cudaGraph_t body = cp.conditional.phGraph_out[0];
+                e = cudaStreamBeginCaptureToGraph(gs.side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+                if (e != cudaSuccess) rc = check_cuda(c, e, "body capture");
+                if (!rc) {
+                    c->stream = gs.side;
+                    c->build_in_step = true;
+                    c->build_partial = c->nrep > 0;  // the flagged replicas only
+                    rc = launch_take_rebuild(c);
+                    if (!rc) rc = nlist_build(c);
+                    c->build_partial = false;
+                    c->build_in_step = false;
+                    c->stream = s;
+                    cudaGraph_t body_out = nullptr;
+                    e = cudaStreamEndCapture(gs.side, &body_out);
+                    if (!rc && e != cudaSuccess) rc = check_cuda(c, e, "body capture end");
+                }
             }
         }
+        l2 = c->launches;
+        if (!rc && io) rc = branch(0, io[0], nullptr, nullptr);
+        c->fuse_kick = true;
+        if (!rc) rc = forces_compute(c);
+        c->fuse_kick = false;
+        const bool f_after = c->gather_deferred;  // the kick completes the forces
+        if (!rc && io && !f_after) rc = branch(1, nullptr, nullptr, io[2]);
+        if (!rc) rc = integrate_kick(c, 0);
+        if (!rc && c->ttm) rc = thermo_detect(c, true);  // ExecuteDetectors (system.cpp:976)
+        if (!rc && io) rc = branch(2, nullptr, io[1], f_after ? io[2] : nullptr);
+        if (!rc && io_launches > 0) {  // join the branch
+            e = cudaEventRecord(gs.io_ev[3], gs.io_side);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(s, gs.io_ev[3], 0);
+            if (e != cudaSuccess) rc = check_cuda(c, e, "download join");
+        }
+        l3 = c->launches;
+        c->captured_builds += 1;
     }
-    l2 = c->launches;
-    if (!rc && io) rc = branch(0, io[0], nullptr, nullptr);
-    c->fuse_kick = true;
-    if (!rc) rc = forces_compute(c);
-    c->fuse_kick = false;
-    const bool f_after = c->gather_deferred;  // the kick completes the forces
-    if (!rc && io && !f_after) rc = branch(1, nullptr, nullptr, io[2]);
-    if (!rc) rc = integrate_kick(c, 0);
-    if (!rc && c->ttm) rc = thermo_detect(c, true);  // ExecuteDetectors (system.cpp:976)
-    if (!rc && io) rc = branch(2, nullptr, io[1], f_after ? io[2] : nullptr);
-    if (!rc && io_launches > 0) {  // join the branch
-        e = cudaEventRecord(gs.io_ev[3], gs.io_side);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, gs.io_ev[3], 0);
-        if (e != cudaSuccess) rc = check_cuda(c, e, "download join");
-    }
-    long l3 = c->launches;
     // captured launches are counted when the graph replays, not here
     c->graph_step_kernels = (l1 - l0) + (l3 - l2);
     c->graph_body_kernels = l2 - l1;
-    c->launches = l0;
-    c->captured_builds += 1;
+    c->launches = launches0;
     cudaGraph_t graph = nullptr;
     e = cudaStreamEndCapture(s, &graph);
     if (rc) {
@@ -1097,6 +1119,10 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr)
         gs.io_valid = true;
         for (int k = 0; k < 3; k++) gs.io_key[k] = io[k];
         gs.io_kernels = io_launches;
+    } else if (steps > 1) {
+        gs.many_graph = graph;
+        gs.many_exec = exec;
+        gs.many_valid = true;
     } else {
         gs.graph = graph;
         gs.exec = exec;
@@ -1411,10 +1437,16 @@ int omdg_step_async(omdg_ctx* c, int nsteps) {
         if (!gs.valid) {
             if ((rc = capture_step(c, gs))) return rc;
         }
-        for (int k = 0; k < nsteps; k++) {
-            cudaError_t e = cudaGraphLaunch(gs.exec, c->stream);
+        if (!gs.many_valid && nsteps >= GRAPH_STEPS && gs.replayed >= GRAPH_AFTER &&
+            (rc = capture_step(c, gs, nullptr, GRAPH_STEPS)))
+            return rc;
+        for (int k = 0; k < nsteps;) {
+            const bool many = gs.many_valid && nsteps - k >= GRAPH_STEPS;
+            cudaError_t e = cudaGraphLaunch(many ? gs.many_exec : gs.exec, c->stream);
             if (e != cudaSuccess) return check_cuda(c, e, "graph launch");
+            k += many ? GRAPH_STEPS : 1;
         }
+        gs.replayed += nsteps;
         c->graph_steps += nsteps;
     }
     c->async_steps += nsteps;

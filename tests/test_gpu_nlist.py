@@ -143,3 +143,30 @@ def test_small_sort_edges(omdg_lib, oracle_lib, n):
     d = st["x"] - x
     d -= (np.asarray(hi) - np.asarray(lo)) * np.round(d / (np.asarray(hi) - np.asarray(lo)))
     assert np.abs(d).max() < 0.5  # three femtoseconds: no atom took another's place
+
+
+@pytest.mark.parametrize("ncell", [4, 17])
+def test_steps_in_one_graph(omdg_lib, ncell):
+    """Steps taken one call at a time, and in calls long enough for the graph
+    of several steps (with single ones left over), are the same trajectory and
+    ledger bit for bit; 512 atoms (the rebuild's kernels look for its request)
+    and 39,304 (the conditional node)."""
+    from objectmd_gb300 import inputs
+
+    x, v, (lo, hi) = inputs.diamond_silicon(ncell=ncell, a=5.431, sigma=0.05, temp=1500.0, seed_pos=3, seed_vel=4)
+    out = []
+    for calls in ([1] * 131, [70, 61], [65, 8, 9, 7, 42]):
+        with omdg_lib.Context(0) as ctx:
+            ctx.set_box(lo, hi)
+            ctx.set_atoms(x, v, masses=[inputs.md_mass("silicon")], znum=[14.0])
+            ctx.add_tersoff(os.path.join(TABLES, "tersoff.silicon27"))
+            ctx.set_neighbor(SKIN, 0)
+            ctx.set_timestep(0.001)
+            ctx.set_thermostat(1200.0, 0.1)
+            for k in calls:
+                ctx.step(k)
+            st = ctx.get_state()
+            out.append((st["x"], st["v"], st["f"], ctx.ledger()["energy"], ctx.stats()["rebuilds"]))
+    assert out[0][4] > 5
+    for o in out[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(o, out[0]))
