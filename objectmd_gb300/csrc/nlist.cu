@@ -453,6 +453,7 @@ struct TileOut {
 };
 
 struct BuildParams {
+    const int *list, *list_n;  // partial replica build: the rebuilt atoms (else null)
     const int* on;  // build only if set (a small box's step; else null)
     TileOut to;
     int n, maxnb, hshift;
@@ -621,20 +622,17 @@ __device__ __forceinline__ void build_run(const float4* __restrict__ u, int left
 // REP: the centre's replica supplies the grid and lengths.  TILES (LANES = 1):
 // the rows also go out as EAM tile slots.  ONE: a single atom type (no type
 // mask).
+constexpr int BUILD_CTAS_PER_SM = 7;
+
 template <int LANES, bool REP, bool TILES, bool ONE>
-__global__ void __launch_bounds__(BUILD_THREADS, 7) k_build(
-    BuildParams p, const RepGeom* __restrict__ rg, const int* __restrict__ rep_of, const float4* __restrict__ loc,
-    const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
-    const int* __restrict__ cell, const int* __restrict__ start, const unsigned* __restrict__ umax,
-    unsigned* __restrict__ nbr, int* __restrict__ nnb, unsigned* status, int* need, const int* __restrict__ rflag,
+__device__ __forceinline__ void build_centre(
+    const BuildParams& p, int i, int lane, const RepGeom* __restrict__ rg, const int* __restrict__ rep_of,
+    const float4* __restrict__ loc, const double* __restrict__ x, const double* __restrict__ y,
+    const double* __restrict__ z, const int* __restrict__ cell, const int* __restrict__ start,
+    const unsigned* __restrict__ umax, unsigned* __restrict__ nbr, int* __restrict__ nnb, unsigned* status, int* need,
     unsigned* __restrict__ nbmask) {
     extern __shared__ unsigned s_row[];
-    if (p.on && !*p.on) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / LANES, lane = t % LANES;
-    if (i >= p.n) return;  // LANES = 8: whole groups leave together
     const RepGeom* g = REP ? rg + rep_of[i] : nullptr;
-    if (REP && rflag && !rflag[rep_of[i]]) return;  // the replica keeps its list
     const float4 ui = loc[i];
     if (ui.x == 3.0e38f) {  // inactive centre (k_pack): an empty row
         if (lane == 0) {
@@ -767,6 +765,31 @@ __global__ void __launch_bounds__(BUILD_THREADS, 7) k_build(
     nbmask[i] = ONE ? (cnt > 0 ? 1u : 0u) : tmask;
 }
 
+// A partial replica build goes over p.list (the atoms of the rebuilt replicas,
+// p.list_n of them) with a resident grid.
+template <int LANES, bool REP, bool TILES, bool ONE>
+__global__ void __launch_bounds__(BUILD_THREADS, BUILD_CTAS_PER_SM) k_build(
+    BuildParams p, const RepGeom* __restrict__ rg, const int* __restrict__ rep_of, const float4* __restrict__ loc,
+    const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+    const int* __restrict__ cell, const int* __restrict__ start, const unsigned* __restrict__ umax,
+    unsigned* __restrict__ nbr, int* __restrict__ nnb, unsigned* status, int* need, const int* __restrict__ rflag,
+    unsigned* __restrict__ nbmask) {
+    if (p.on && !*p.on) return;
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (REP && p.list) {
+        const int total = *p.list_n;
+        for (; t / LANES < total; t += gridDim.x * blockDim.x)  // LANES = 8: whole groups go on together
+            build_centre<LANES, REP, TILES, ONE>(p, p.list[t / LANES], t % LANES, rg, rep_of, loc, x, y, z, cell,
+                                                 start, umax, nbr, nnb, status, need, nbmask);
+        return;
+    }
+    const int i = t / LANES;
+    if (i >= p.n) return;  // LANES = 8: whole groups leave together
+    if (REP && rflag && !rflag[rep_of[i]]) return;  // the replica keeps its list
+    build_centre<LANES, REP, TILES, ONE>(p, i, t % LANES, rg, rep_of, loc, x, y, z, cell, start, umax, nbr, nnb,
+                                         status, need, nbmask);
+}
+
 // ------------------------------------------------------------------ EAM cell tiles
 
 struct TilePrep {
@@ -874,15 +897,9 @@ __global__ void k_cell_assign_rep(int n, double* __restrict__ x, double* __restr
 // flight).
 constexpr int REV_LANES = 4;
 
-__global__ void k_reverse(int n, int hshift, int maxnb, const unsigned* __restrict__ nbr,
-                          const int* __restrict__ nnb, int* __restrict__ rev, unsigned* status,
-                          const int* __restrict__ rep_of, const int* __restrict__ rflag,
-                          const int* __restrict__ on) {
-    if (on && !*on) return;
-    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    const int i = (int)(t / REV_LANES), lane = (int)(t % REV_LANES);
-    if (i >= n) return;
-    if (rflag && !rflag[rep_of[i]]) return;  // the replica kept its rows, and so their reverse slots
+__device__ __forceinline__ void reverse_centre(int i, int lane, int hshift, int maxnb,
+                                               const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
+                                               int* __restrict__ rev, unsigned* status) {
     int m = nnb[i];
     for (int s = lane; s < m; s += REV_LANES) {
         unsigned e = nbr[nbr_at(i, s, hshift, maxnb)];
@@ -897,6 +914,25 @@ __global__ void k_reverse(int n, int hshift, int maxnb, const unsigned* __restri
         if (found < 0) atomicOr(status, ERR_NBR_OVERFLOW);
         rev[nbr_at(i, s, hshift, maxnb)] = found < 0 ? 0 : found;
     }
+}
+
+__global__ void k_reverse(int n, int hshift, int maxnb, const unsigned* __restrict__ nbr,
+                          const int* __restrict__ nnb, int* __restrict__ rev, unsigned* status,
+                          const int* __restrict__ rep_of, const int* __restrict__ rflag,
+                          const int* __restrict__ on, const int* __restrict__ list,
+                          const int* __restrict__ list_n) {
+    if (on && !*on) return;
+    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (list) {  // a partial replica build (k_build)
+        const int total = *list_n;
+        for (long q = t; q / REV_LANES < total; q += gridDim.x * (long)blockDim.x)
+            reverse_centre(list[q / REV_LANES], (int)(q % REV_LANES), hshift, maxnb, nbr, nnb, rev, status);
+        return;
+    }
+    const int i = (int)(t / REV_LANES), lane = (int)(t % REV_LANES);
+    if (i >= n) return;
+    if (rflag && !rflag[rep_of[i]]) return;  // the replica kept its rows, and so their reverse slots
+    reverse_centre(i, lane, hshift, maxnb, nbr, nnb, rev, status);
 }
 
 // ---------------------------------------------------------------- host side
@@ -976,6 +1012,11 @@ int replica_prepare(Context* c) {
     }
     c->rep_cells = base;
     c->rep_lmax = lmax;
+    c->rep_max_atoms = c->rep_max_cells = 0;
+    for (int r = 0; r < c->nrep; r++) {
+        c->rep_max_atoms = std::max(c->rep_max_atoms, c->rep_start[r + 1] - c->rep_start[r]);
+        c->rep_max_cells = std::max(c->rep_max_cells, (r + 1 < c->nrep ? rg[r + 1].cell_base : base) - rg[r].cell_base);
+    }
     // The step graph holds these pointers: allocate once (omdg_set_replicas
     // frees them) and reallocate only for a larger atom capacity, dropping
     // the graph then.  Contents are rewritten in place.
@@ -1123,8 +1164,13 @@ PackFrame pack_frame(const Context* c) {
 // st->building: three launches that return cost less than a conditional node
 // that is not taken.  A step of 512 Tersoff atoms, us: 23.5 and 28.4, of 8,000
 // 26.5 and 31.1, of 32,768 31.1 and 36.0.
+// Replicas: a cluster each, and those that keep their rows return at once,
+// where the general path's eleven kernels went over every atom and cell; the
+// list kernels go over the rebuilt atoms only.  A step of the impact ensemble
+// (1.47 M atoms in 256 replicas, some of them rebuilt in every step), us: sort
+// and pack 116 -> 66, build 74 -> 63, reverse 33 -> 18.
 constexpr int SORT_THREADS = 1024, SORT_CTAS = 8;
-constexpr int SORT_PER = 4, SORT_CELLS = 4;  // atoms a thread moves, and cells it scans, at most
+constexpr int SORT_PER = 4, SORT_CELLS = 8;  // atoms a thread moves, and cells it scans, at most
 
 struct SortArgs {
     int n, m, on_request, st_bytes;
@@ -1137,19 +1183,46 @@ struct SortArgs {
     unsigned char* st_snap;
     int *count, *start, *perm, *cell, *inv;
     const unsigned* aflag;  // null: every atom is active
+    // replica mode: a cluster a replica, of those flagged (rflag null: of all)
+    const RepGeom* rg;
+    const int *rep_start, *rflag;
+    int *list, *list_n;
     PosPack* pack;
     float4 *xref, *loc;
     unsigned* umax;
 };
 
-template <int PER>
+template <int PER, bool REP>
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
     static_assert(sizeof(StepState) <= SORT_THREADS, "a block copies the step state");
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-    __shared__ int warp_sum[SORT_THREADS / 32], total;
+    __shared__ int warp_sum[SORT_THREADS / 32], total, list_at;
+    __shared__ CellGeom sg;
     const int rank = (int)cl.block_rank(), t = threadIdx.x, lane = t & 31;
     const int threads = (int)cl.num_blocks() * SORT_THREADS;
     const int i = rank * SORT_THREADS + t;
+    // this cluster's atoms [a0, a0 + n) and cells [c0, c0 + m)
+    int a0 = 0, n = a.n, c0 = 0, m = a.m;
+    if (REP) {
+        const int r = blockIdx.x / cl.num_blocks();
+        if (a.rflag && !a.rflag[r]) return;  // the replica keeps its order and rows
+        const RepGeom& g = a.rg[r];
+        a0 = a.rep_start[r];
+        n = a.rep_start[r + 1] - a0;
+        c0 = g.cell_base;
+        m = g.nc[0] * g.nc[1] * g.nc[2];
+        if (t < 3) {
+            sg.nc[t] = g.nc[t];
+            sg.org[t] = g.cell_org[t];
+            sg.h[t] = g.cell_h[t];
+            sg.inv_h[t] = g.inv_h[t];
+            sg.periodic[t] = g.periodic[t];
+            sg.lo[t] = g.lo[t];
+            sg.L[t] = g.L[t];
+        }
+        if (rank == 0 && t == 0 && a.rflag) list_at = atomicAdd(a.list_n, n);
+    }
+    const CellGeom& geom = REP ? sg : a.g;
     if (a.on_request) {
         // a build that overflowed its rows halts the queued steps' later ones
         const bool halted = a.st->halted || (a.st->building && (*a.status & ERR_NBR_OVERFLOW));
@@ -1163,14 +1236,14 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
             return;
         }
     }
-    const bool snap = a.snap.x && !a.st->halted && !*a.taken;
+    const bool snap = !REP && a.snap.x && !a.st->halted && !*a.taken;
     double p[PER][3], v[PER][3];
     int type[PER], id[PER], c[PER], slot[PER];
     unsigned flag[PER];
 #pragma unroll
     for (int w = 0; w < PER; w++) {
-        const int j = w * threads + i;
-        if (j >= a.n) continue;
+        const int j = a0 + w * threads + i;
+        if (j >= a0 + n) continue;
         p[w][0] = a.a.x[j];
         p[w][1] = a.a.y[j];
         p[w][2] = a.a.z[j];
@@ -1192,10 +1265,10 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
             a.snap.flag[j] = flag[w];
         }
     }
-    for (int q = i; q < a.m; q += threads) a.count[q] = 0;
-    if (i == 0) *a.umax = 0u;
+    for (int q = i; q < m; q += threads) a.count[c0 + q] = 0;
+    if (!REP && i == 0) *a.umax = 0u;
     cl.sync();  // the counts are zero, and `taken` read
-    if (rank == 0) {
+    if (!REP && rank == 0) {
         if (t == 0 && a.on_request) {
             a.st->nrebuild += 1;
             a.st->rebuild = 0;
@@ -1210,19 +1283,19 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
     }
 #pragma unroll
     for (int w = 0; w < PER; w++) {
-        const int j = w * threads + i;
-        if (j >= a.n) continue;
-        c[w] = cell_of(j, p[w], a.g, a.status);
+        const int j = a0 + w * threads + i;
+        if (j >= a0 + n) continue;
+        c[w] = c0 + cell_of(j, p[w], geom, a.status);
         slot[w] = atomicAdd(&a.count[c[w]], 1);
     }
     cl.sync();
     // exclusive scan: a thread's run of cells, the block's threads, the blocks
-    const int per = (a.m + threads - 1) / threads;
-    const int q0 = min(a.m, i * per), q1 = min(a.m, q0 + per);
+    const int per = (m + threads - 1) / threads;
+    const int q0 = min(m, i * per), q1 = min(m, q0 + per);
     int cells[SORT_CELLS], sum = 0;
 #pragma unroll
     for (int k = 0; k < SORT_CELLS; k++) {
-        cells[k] = q0 + k < q1 ? a.count[q0 + k] : 0;
+        cells[k] = q0 + k < q1 ? a.count[c0 + q0 + k] : 0;
         sum += cells[k];
     }
     int run = sum;
@@ -1244,26 +1317,31 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
         if (t == 31) total = w;
     }
     cl.sync();
-    run += (t >= 32 ? warp_sum[(t >> 5) - 1] : 0) - sum;
+    run += a0 + (t >= 32 ? warp_sum[(t >> 5) - 1] : 0) - sum;
     for (int r = 0; r < rank; r++) run += *cl.map_shared_rank(&total, r);
 #pragma unroll
     for (int k = 0; k < SORT_CELLS; k++)
         if (q0 + k < q1) {
-            a.start[q0 + k] = run;
+            a.start[c0 + q0 + k] = run;
             run += cells[k];
         }
-    if (i == 0) a.start[a.m] = a.n;
+    if (i == 0 && a0 + n == a.n) a.start[c0 + m] = a.n;
+    if (REP && a.rflag) {  // the rebuilt atoms, for the list kernels
+        const int at = *cl.map_shared_rank(&list_at, 0);
+        for (int q = i; q < n; q += threads) a.list[at + q] = a0 + q;
+    }
     cl.sync();
 #pragma unroll
     for (int w = 0; w < PER; w++)
-        if (w * threads + i < a.n) a.perm[a.start[c[w]] + slot[w]] = w * threads + i;
+        if (w * threads + i < n) a.perm[a.start[c[w]] + slot[w]] = a0 + w * threads + i;
     cl.sync();
     float u = 0.f;
 #pragma unroll
     for (int w = 0; w < PER; w++) {
-        const int j = w * threads + i;
-        if (j >= a.n) continue;
-        const int base = a.start[c[w]], in_cell = a.start[c[w] + 1] - base;
+        const int j = a0 + w * threads + i;
+        if (j >= a0 + n) continue;
+        const int base = a.start[c[w]];
+        const int in_cell = (c[w] + 1 < c0 + m ? a.start[c[w] + 1] : a0 + n) - base;
         if (in_cell <= CELL_SORT_MAX) {
             slot[w] = 0;
             for (int q = 0; q < in_cell; q++) slot[w] += a.perm[base + q] < j;
@@ -1288,22 +1366,28 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
         double* x = a.a.extra + (size_t)q * a.n;
         double keep[PER];
 #pragma unroll
-        for (int w = 0; w < PER; w++) keep[w] = w * threads + i < a.n ? x[w * threads + i] : 0.0;
+        for (int w = 0; w < PER; w++) keep[w] = w * threads + i < n ? x[a0 + w * threads + i] : 0.0;
         cl.sync();
 #pragma unroll
         for (int w = 0; w < PER; w++)
-            if (w * threads + i < a.n) x[slot[w]] = keep[w];
+            if (w * threads + i < n) x[slot[w]] = keep[w];
     }
 }
 
 static int cells_of(const Context* c) { return c->box.nc[0] * c->box.nc[1] * c->box.nc[2]; }
 
-bool small_sort(const Context* c) {
-    return c->nrep == 0 && !c->tile_want && c->n <= SORT_CTAS * SORT_THREADS * SORT_PER &&
-           (long)c->box.nc[0] * c->box.nc[1] * c->box.nc[2] <= SORT_CTAS * SORT_THREADS * SORT_CELLS;
+// One cluster's share: its atoms and cells.
+static bool sort_fits(long atoms, long cells) {
+    return atoms <= SORT_CTAS * SORT_THREADS * SORT_PER && cells <= SORT_CTAS * SORT_THREADS * SORT_CELLS;
 }
 
-static int launch_sort_small(Context* c, const CellGeom& g, int m, bool on_request, unsigned* umax) {
+bool small_sort(const Context* c) {
+    return c->nrep == 0 && !c->tile_want &&
+           sort_fits(c->n, (long)c->box.nc[0] * c->box.nc[1] * c->box.nc[2]);
+}
+
+static int launch_sort_small(Context* c, const CellGeom& g, int m, bool on_request, unsigned* umax, const int* rflag,
+                             int* list_n) {
     SortArgs a;
     a.n = c->n;
     a.m = m;
@@ -1331,12 +1415,24 @@ static int launch_sort_small(Context* c, const CellGeom& g, int m, bool on_reque
     a.xref = c->xref;
     a.loc = c->loc;
     a.umax = umax;
+    a.rg = static_cast<const RepGeom*>(c->d_rep_geom);
+    a.rep_start = c->d_rep_start;
+    a.rflag = rflag;
+    a.list = c->cell;  // (the general path's cell numbers)
+    a.list_n = list_n;
+    // a replica's cluster is as small as four atoms a thread allow: many run
+    // beside each other
+    const bool reps = c->nrep > 0;
+    const int atoms = reps ? c->rep_max_atoms : c->n, cells = reps ? c->rep_max_cells : m;
+    const int most = reps ? SORT_PER : 1;
     int blocks = 1;
-    while (blocks < SORT_CTAS && (blocks * SORT_THREADS < c->n || blocks * SORT_THREADS * SORT_CELLS < m)) blocks *= 2;
-    const int per = grid_for(c->n, blocks * SORT_THREADS);
-    auto kernel = per <= 1 ? k_sort_small<1> : per <= 2 ? k_sort_small<2> : k_sort_small<4>;
+    while (blocks < SORT_CTAS && (blocks * SORT_THREADS * most < atoms || blocks * SORT_THREADS * SORT_CELLS < cells))
+        blocks *= 2;
+    const int per = grid_for(atoms, blocks * SORT_THREADS);
+    auto kernel = reps ? (per <= 1 ? k_sort_small<1, true> : per <= 2 ? k_sort_small<2, true> : k_sort_small<4, true>)
+                       : (per <= 1 ? k_sort_small<1, false> : per <= 2 ? k_sort_small<2, false> : k_sort_small<4, false>);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
+    cfg.gridDim = dim3(blocks * (reps ? c->nrep : 1));
     cfg.blockDim = dim3(SORT_THREADS);
     cfg.stream = c->stream;
     cudaLaunchAttribute at;
@@ -1427,23 +1523,32 @@ int nlist_build(Context* c, bool on_request) {
     // its index range and cell range, so the others' arrays stay valid
     const int* rflag = (reps && c->build_partial) ? c->d_rep_flag : nullptr;
     prof_begin(c, "cell_sort");
-    if (small_sort(c)) {
-        if ((rc = launch_sort_small(c, g, m, on_request, umax))) return rc;
+    // a replica's cluster cannot see the others': the snapshot of all atoms is
+    // taken before
+    const bool small_reps = reps && sort_fits(c->rep_max_atoms, c->rep_max_cells);
+    const bool small_one = small_sort(c);
+    int* list_n = c->d_flags + 5;
+    if (!small_one && c->build_in_step && c->snap_d) {
+        AtomArrays cur0{c->x, c->y, c->z, c->vx, c->vy, c->vz, c->type, c->id, c->aflag, nullptr, 0};
+        AtomArrays snap{c->snap_d, c->snap_d + c->cap, c->snap_d + 2 * (size_t)c->cap, c->snap_d + 3 * (size_t)c->cap,
+                        c->snap_d + 4 * (size_t)c->cap, c->snap_d + 5 * (size_t)c->cap, c->snap_i,
+                        c->snap_i + c->cap, reinterpret_cast<unsigned*>(c->snap_i + 2 * (size_t)c->cap), nullptr, 0};
+        const int sb = (int)step_state_bytes();
+        int* taken = c->d_flags + 6;
+        k_snapshot<<<grid_for(std::max(n, sb), 256), 256, 0, s>>>(
+            n, step_state_halted(c), taken, cur0, snap, static_cast<const unsigned char*>(c->d_state),
+            static_cast<unsigned char*>(c->snap_state), sb);
+        k_set_one<<<1, 1, 0, s>>>(taken);
+        c->launches += 2;
+    }
+    if (small_one || small_reps) {
+        if (small_reps) {
+            k_zero_ints<<<1, 32, 0, s>>>(1, c->d_flags + 3, list_n);
+            c->launches++;
+        }
+        if ((rc = launch_sort_small(c, g, m, on_request, umax, rflag, list_n))) return rc;
         prof_end(c);
     } else {
-        if (c->build_in_step && c->snap_d) {
-            AtomArrays cur0{c->x, c->y, c->z, c->vx, c->vy, c->vz, c->type, c->id, c->aflag, nullptr, 0};
-            AtomArrays snap{c->snap_d, c->snap_d + c->cap, c->snap_d + 2 * (size_t)c->cap, c->snap_d + 3 * (size_t)c->cap,
-                            c->snap_d + 4 * (size_t)c->cap, c->snap_d + 5 * (size_t)c->cap, c->snap_i,
-                            c->snap_i + c->cap, reinterpret_cast<unsigned*>(c->snap_i + 2 * (size_t)c->cap), nullptr, 0};
-            const int sb = (int)step_state_bytes();
-            int* taken = c->d_flags + 6;
-            k_snapshot<<<grid_for(std::max(n, sb), 256), 256, 0, s>>>(
-                n, step_state_halted(c), taken, cur0, snap, static_cast<const unsigned char*>(c->d_state),
-                static_cast<unsigned char*>(c->snap_state), sb);
-            k_set_one<<<1, 1, 0, s>>>(taken);
-            c->launches += 2;
-        }
         if (rflag)
             k_zero_cells_rep<<<grid_for(m + 1, 256), 256, 0, s>>>(m, c->cell_count, c->cell_fill, c->d_cell_rep, rflag);
         else
@@ -1531,6 +1636,8 @@ int nlist_build(Context* c, bool on_request) {
     }
     c->tile_valid = tiles;
     bp.on = on_request ? step_state_building(c) : nullptr;
+    bp.list = small_reps && rflag ? c->cell : nullptr;
+    bp.list_n = list_n;
     bp.n = n;
     bp.maxnb = c->maxnb;
     bp.hshift = c->nbr_hshift;
@@ -1559,7 +1666,8 @@ int nlist_build(Context* c, bool on_request) {
     const int lanes = small && !tiles ? 8 : 1;  // only the one-thread form writes tile slots
     const size_t smem = sizeof(unsigned) * BUILD_THREADS * (lanes == 1 ? bp.cap : BUILD_RUN);
     const auto launch = [&](auto kernel) {
-        kernel<<<grid_for(n, BUILD_THREADS / lanes), BUILD_THREADS, smem, s>>>(
+        const int all = grid_for(n, BUILD_THREADS / lanes);
+        kernel<<<bp.list ? std::min(all, BUILD_CTAS_PER_SM * c->num_sms) : all, BUILD_THREADS, smem, s>>>(
             bp, rg, c->d_rep_of, c->loc, c->x, c->y, c->z, cell_sorted, c->cell_start, umax,
             reinterpret_cast<unsigned*>(c->nbr), c->nnb, c->d_status, c->d_flags + 1, rflag, c->nbmask);
     };
@@ -1580,9 +1688,10 @@ int nlist_build(Context* c, bool on_request) {
     prof_end(c);
     if (c->need_rev) {
         prof_begin(c, "nlist_reverse");
-        k_reverse<<<grid_for(n, 128 / REV_LANES), 128, 0, s>>>(n, c->nbr_hshift, c->maxnb,
+        const int all = grid_for(n, 128 / REV_LANES);
+        k_reverse<<<bp.list ? std::min(all, 16 * c->num_sms) : all, 128, 0, s>>>(n, c->nbr_hshift, c->maxnb,
                                                    reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->rev,
-                                                   c->d_status, c->d_rep_of, rflag, bp.on);
+                                                   c->d_status, c->d_rep_of, rflag, bp.on, bp.list, bp.list_n);
         c->launches++;
         prof_end(c);
     }

@@ -183,6 +183,7 @@ struct Context {
     std::vector<double> rep_lo, rep_hi;  // nrep x 3
     int rep_periodic[3] = {1, 1, 0};
     int rep_cells = 0;                   // cells over all replicas
+    int rep_max_atoms = 0, rep_max_cells = 0;  // of the largest replica
     double rep_lmax = 0.0;               // largest periodic replica length (list screening band)
     int rep_cells_cap = 0;               // entries of d_cell_rep
     int* d_rep_of = nullptr;             // replica of each atom (index order)
@@ -327,7 +328,8 @@ struct Context {
     unsigned* d_status = nullptr;   // error bits
     int* d_flags = nullptr;         // [0] rebuild request, [1] row length needed, [2] ghost count,
                                     // [3] largest coordinate of the last build (float bits),
-                                    // [4] blocks done in the current kick (reset by the last block)
+                                    // [4] blocks done in the current kick (reset by the last block),
+                                    // [5] atoms of the replicas a partial build takes, [6] snapshot taken
     double* d_red = nullptr;        // block partials
     int red_cap = 0;
     double* d_ledger = nullptr;     // per step LEDGER_W doubles: kinetic, potential, virial, lambda,

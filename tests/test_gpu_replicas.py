@@ -148,3 +148,44 @@ def test_persistent_tersoff_pass_is_the_same(omdg_lib, ensemble):
             out.append((st["x"], st["f"], st["pot"]))
     for a, b_ in zip(*out):
         assert np.array_equal(a, b_)
+
+
+@pytest.mark.parametrize("sizes", [(1, 1024, 1025, 4096), (4097, 5, 16385, 700), (32769, 300)])
+def test_sort_of_replicas_at_its_edges(omdg_lib, sizes):
+    """Replicas at the edges of the one-kernel sort's threads and blocks (and,
+    with 32,769 atoms in one, the general path): after steps in which some
+    rebuild and some do not, each is where it is as the only replica (to the
+    1e-5 A that FP32 forces in another frame leave, as above)."""
+    from objectmd_gb300 import inputs
+
+    rng = np.random.default_rng(5)
+    xs, vs, los, his = [], [], [], []
+    for k, n in enumerate(sizes):
+        side = max(3, int(np.ceil((n / 8) ** (1.0 / 3.0))))
+        x, v, (lo, hi) = inputs.diamond_silicon(ncell=side, a=5.431, sigma=0.05, temp=300.0 * (k + 1), seed_pos=k,
+                                                seed_vel=9 + k)
+        pick = rng.permutation(len(x))[:n]
+        xs.append(x[pick])
+        vs.append(v[pick])
+        los.append(lo)
+        his.append(hi)
+
+    def run(group):
+        with omdg_lib.Context(0) as ctx:
+            ctx.set_replicas([len(xs[k]) for k in group], [los[k] for k in group], [his[k] for k in group], (1, 1, 1))
+            ctx.set_atoms(np.vstack([xs[k] for k in group]), np.vstack([vs[k] for k in group]),
+                          masses=[inputs.md_mass("silicon")], znum=[14.0])
+            ctx.add_tersoff(TERSOFF)
+            ctx.set_neighbor(0.3, 0)
+            ctx.set_timestep(0.001)
+            ctx.step(60)
+            return ctx.get_state()["x"], ctx.replica_builds(len(group))
+
+    whole, builds = run(range(len(sizes)))
+    assert max(builds) > min(builds)  # partial rebuilds took place
+    at = 0
+    for k, n in enumerate(sizes):
+        L = np.asarray(his[k]) - np.asarray(los[k])
+        d = whole[at:at + n] - run([k])[0]
+        assert np.abs(d - L * np.round(d / L)).max() <= 1e-5, k
+        at += n
