@@ -9,6 +9,8 @@
 //     interleaved (phi, rho) knot are one 256-bit load each,
 //   - the periodic image comes from a 64-entry shared table of split shift
 //     vectors indexed by the entry's 6 image bits,
+//   - boxes three list ranges long read fixed-point positions instead
+//     (fixed_density_sum), and need no shift,
 //   - the knot index is clamped instead of branched (r <= rc keeps it below
 //     n-1; the reference's x == n-1 rule selects the same segment),
 //   - forces use Kahan sums, the per-pair energy and virial plain FP32 sums.
@@ -42,7 +44,31 @@ struct EAMFast {
     int stage_k0, stage_n;
     int first;
     int src_phi, src_rho, src_emb;  // table ids for error reports (DevTable::src)
+    float qh[3], ql[3];             // fixed-point step (FixFrame)
 };
+
+// 128-bit coherent load: the density pass writes the w words beside it.
+__device__ __forceinline__ int4 ld_ipos(const int4* p) {
+    int4 v;
+    asm volatile("ld.global.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// x_i - x_j of the nearest images from the fixed-point positions (fix_coord).
+// The step's low part keeps its rounding from scaling every length alike.
+__device__ __forceinline__ float3 fix_delta(const EAMFast& p, const int4& a, const int4& b) {
+    const float x = (float)(a.x - b.x), y = (float)(a.y - b.y), z = (float)(a.z - b.z);
+    return make_float3(fmaf(x, p.qh[0], x * p.ql[0]), fmaf(y, p.qh[1], y * p.ql[1]), fmaf(z, p.qh[2], z * p.ql[2]));
+}
+
+// r and 1/r from r2: the approximate root with one Newton step each.
+__device__ __forceinline__ float root(float r2, float& rinv) {
+    rinv = rsqrtf(r2);
+    float r = r2 * rinv;
+    r = fmaf(fmaf(-r, r, r2), 0.5f * rinv, r);
+    rinv = fmaf(fmaf(-r, rinv, 1.f), rinv, rinv);
+    return r;
+}
 
 __device__ __forceinline__ void build_shift_table(const EAMFast& p, float4* s_hi, float4* s_lo) {
     for (int k = threadIdx.x; k < 64; k += blockDim.x) {
@@ -85,7 +111,7 @@ __device__ __forceinline__ float plain_reduce(float v) {
     return v;
 }
 
-// Entries a lane prefetches into registers per pass over its row.
+// Entries a lane prefetches into registers per pass over its row (packs).
 template <int LANES>
 struct Prefetch {
     static constexpr int N = LANES >= 4 ? 64 / LANES : 16;
@@ -93,7 +119,7 @@ struct Prefetch {
 
 // Staged variants hold the knot window in shared memory (up to ~110 KB) and
 // run two 512-thread CTAs per SM, so 32 warps hide the gathers' latency.
-#define EAMF_BOUNDS(STAGED) __launch_bounds__((STAGED) ? 512 : 256, (STAGED) ? 2 : 4)
+#define EAMF_BOUNDS(STAGED, N) __launch_bounds__((STAGED) ? 512 : 256, (STAGED) ? 2 : (N))
 
 // Index of the rho knot below r, or -1 when r is closer than the first knot
 // (outside every tabulated range here).
@@ -155,9 +181,69 @@ __device__ __forceinline__ void gather_density_sum(const EAMFast& p, const PosPa
     }
 }
 
+// The same from the fixed-point positions: half the bytes a neighbour (from the
+// packs both passes were at 75 % of the L1's data path) and no image shift to
+// look up or add.  What bounds them now is the latency of the chain from entry
+// to position to knot: a lane holds few entries ahead, so that more warps fit
+// (density, 256,000 atoms: 16 entries and four blocks a SM 64.1 us, 16 and six
+// 59.2, four and six 54.3; force: 16 and four 69.7, eight and four 65.1, eight
+// and five 69.6).  Packs and fixed point, us, 256,000 atoms: density 72.5 and
+// 55.7, force 85.7 and 66.8; 1,048,576 (two lanes an atom): 264 and 189, 329
+// and 243.  One Newton step each for the root and its reciprocal leaves the
+// forces nearer to FP64 than the packs with the bare approximation did.
+constexpr int FIX_AHEAD_DENSITY = 4, FIX_CTAS_DENSITY = 6;
+constexpr int FIX_AHEAD_FORCE = 8, FIX_CTAS_FORCE = 4;
+constexpr int FIX_TWO_LANES_PER_SM = 3000;
+// Below this many atoms a SM launches and latency are all, and the packs serve
+// as well (both passes, us: 16,384 atoms 28.1 and 27.4, 32,000 34.8 and 30.6,
+// 55,296 52.5 and 40.1).
+constexpr int FIX_PER_SM = 128;
+
+template <int LANES>
+__device__ __forceinline__ void fixed_density_sum(const EAMFast& p, const int4* ipos, const unsigned* __restrict__ nbr,
+                                                  int ii, int m, int lane, Kahan& acc, unsigned* status) {
+    constexpr int PF = FIX_AHEAD_DENSITY;
+    const int step = LANES << p.hshift;
+    const float rc2 = p.rc_rho * p.rc_rho * 1.0001f;
+    const float offdr = p.off * p.inv_dr;
+    const int4 xi = ld_ipos(ipos + ii);
+    const unsigned* rp = nbr + nbr_at(ii, lane, p.hshift, p.maxnb);
+    bool bad = false;
+    for (int s0 = lane; s0 < m; s0 += PF * LANES, rp += PF * step) {
+        unsigned ent[PF];
+#pragma unroll
+        for (int k = 0; k < PF; k++) ent[k] = (s0 + k * LANES < m) ? __ldg(rp + k * step) & (unsigned)INDEX_MASK : 0u;
+        int4 xj = ld_ipos(ipos + ent[0]);
+#pragma unroll
+        for (int k = 0; k < PF; k++) {
+            if (s0 + k * LANES >= m) break;
+            int4 xn;
+            if (k + 1 < PF && s0 + (k + 1) * LANES < m) xn = ld_ipos(ipos + ent[k + 1]);
+            const float3 d = fix_delta(p, xi, xj);
+            xj = xn;
+            const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
+            if (r2 > rc2) continue;
+            float rinv;
+            const float r = root(r2, rinv);
+            if (!(r <= p.rc_rho)) continue;
+            float dx;
+            const int x = knot_of(p, r, offdr, dx);
+            if (x < 0) {
+                if (!bad) report_range(status, r, p.src_rho);
+                bad = true;
+                continue;
+            }
+            const float4 cf = __ldg(&p.coef2[2 * (size_t)x + 1]);
+            float v = fmaf(dx, fmaf(dx, fmaf(dx, cf.x, cf.y), cf.z), cf.w);
+            if (p.rmult_rho) v = v / r;
+            acc.add(v);
+        }
+    }
+}
+
 // F(rho), F'(rho) for atom i (TableReader::read on the EMBED section); F'
 // also travels with the position for the force pass.
-__device__ __forceinline__ void density_finish(const EAMFast& p, int i, float rho, PosPack* pack, float* fp,
+__device__ __forceinline__ void density_finish(const EAMFast& p, int i, float rho, float* spare, float* fp,
                                                float* femb, unsigned* status) {
     const float rval = rho - p.e_off;
     int x = __float2int_rz(rval * p.e_inv_dr);
@@ -181,19 +267,19 @@ __device__ __forceinline__ void density_finish(const EAMFast& p, int i, float rh
     }
     fp[i] = dF;
     femb[i] = F;
-    pack[i].lo.w = dF;
+    *spare = dF;
 }
 
-template <int LANES, bool STAGED>
-__global__ void EAMF_BOUNDS(STAGED) k_eamf_density(EAMFast p, PosPack* pack, const unsigned* __restrict__ nbr,
+template <int LANES, bool STAGED, bool FIXED>
+__global__ void EAMF_BOUNDS(STAGED, FIXED ? FIX_CTAS_DENSITY : 4) k_eamf_density(EAMFast p, PosPack* pack, int4* ipos, const unsigned* __restrict__ nbr,
                                                    const int* __restrict__ nnb, float* __restrict__ fp,
                                                    float* __restrict__ femb, unsigned* status) {
-    __shared__ float4 s_hi[64], s_lo[64];
+    __shared__ float4 s_hi[FIXED ? 1 : 64], s_lo[FIXED ? 1 : 64];
     extern __shared__ float4 s_rho[];
-    build_shift_table(p, s_hi, s_lo);
+    if (!FIXED) build_shift_table(p, s_hi, s_lo);
     if (STAGED)
         for (int k = threadIdx.x; k < p.stage_n; k += blockDim.x) s_rho[k] = p.coef2[2 * (size_t)(p.stage_k0 + k) + 1];
-    __syncthreads();
+    if (!FIXED) __syncthreads();
     const int lane = threadIdx.x & (LANES - 1);
     const int per_block = blockDim.x / LANES;
     for (int base = blockIdx.x * per_block; base < p.n; base += gridDim.x * per_block) {
@@ -202,10 +288,11 @@ __global__ void EAMF_BOUNDS(STAGED) k_eamf_density(EAMFast p, PosPack* pack, con
         const int ii = valid ? i : p.n - 1;
         const int m = valid ? nnb[ii] : 0;
         Kahan acc;
-        gather_density_sum<LANES, STAGED>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_rho, acc, status);
+        if (FIXED) fixed_density_sum<LANES>(p, ipos, nbr, ii, m, lane, acc, status);
+        else gather_density_sum<LANES, STAGED>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_rho, acc, status);
         float sum = acc.s, comp = acc.c;
         twosum_reduce<LANES>(sum, comp);
-        if (lane == 0 && valid) density_finish(p, i, __fsub_rn(sum, comp), pack, fp, femb, status);
+        if (lane == 0 && valid) density_finish(p, i, __fsub_rn(sum, comp), FIXED ? reinterpret_cast<float*>(&ipos[i].w) : &pack[i].lo.w, fp, femb, status);
     }
 }
 
@@ -291,6 +378,56 @@ __device__ __forceinline__ void gather_force_sum(const EAMFast& p, const PosPack
     }
 }
 
+// The same from the fixed-point positions (fixed_density_sum).
+template <int LANES>
+__device__ __forceinline__ void fixed_force_sum(const EAMFast& p, const int4* __restrict__ ipos,
+                                                const unsigned* __restrict__ nbr, int ii, int m, int lane, Kahan& ax,
+                                                Kahan& ay, Kahan& az, float& ae, float& av, unsigned* status) {
+    constexpr int PF = FIX_AHEAD_FORCE;
+    const int step = LANES << p.hshift;
+    const float offdr = p.off * p.inv_dr;
+    const int4 xi = __ldg(ipos + ii);
+    const float fpi = __int_as_float(xi.w);
+    const unsigned* rp = nbr + nbr_at(ii, lane, p.hshift, p.maxnb);
+    bool bad = false;
+    for (int s0 = lane; s0 < m; s0 += PF * LANES, rp += PF * step) {
+        unsigned ent[PF];
+#pragma unroll
+        for (int k = 0; k < PF; k++) ent[k] = (s0 + k * LANES < m) ? __ldg(rp + k * step) & (unsigned)INDEX_MASK : 0u;
+        int4 xj = __ldg(ipos + ent[0]);
+#pragma unroll
+        for (int k = 0; k < PF; k++) {
+            if (s0 + k * LANES >= m) break;
+            int4 xn;
+            if (k + 1 < PF && s0 + (k + 1) * LANES < m) xn = __ldg(ipos + ent[k + 1]);
+            const float3 d = fix_delta(p, xi, xj);
+            const float fpj = __int_as_float(xj.w);  // F'(rho_j) from the density pass
+            xj = xn;
+            const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
+            if (r2 > p.rc2) continue;
+            float rinv;
+            const float r = root(r2, rinv);
+            if (!(r <= p.rc_phi)) continue;
+            float dx;
+            const int x = knot_of(p, r, offdr, dx);
+            if (x < 0) {
+                if (!bad) report_range(status, r, p.src_phi);
+                bad = true;
+                continue;
+            }
+            float4 cp, cr;
+            ldg256(&p.coef2[2 * (size_t)x], cp, cr);
+            float fr, eh;
+            eam_pair_terms(p, r2, fpi + fpj, cp, cr, dx, r, rinv, fr, eh);
+            ax.add(d.x * fr);
+            ay.add(d.y * fr);
+            az.add(d.z * fr);
+            ae += eh;
+            av = fmaf(fr, r2, av);
+        }
+    }
+}
+
 // Lane reductions of one atom's force sums (every lane holds the totals).
 template <int LANES>
 __device__ __forceinline__ void force_reduce(Kahan& ax, Kahan& ay, Kahan& az, float& ae, float& av) {
@@ -321,8 +458,9 @@ __device__ __forceinline__ void force_store(const EAMFast& p, int i, float vfx, 
 // KICK: the step's second half-kick and its ledger terms in the epilogue (the
 // force is final here: one potential, no force modifies), as k_kick does
 // them, one ledger partial per warp.
-template <int LANES, bool STAGED, bool KICK>
-__global__ void EAMF_BOUNDS(STAGED) k_eamf_force(EAMFast p, const PosPack* __restrict__ pack,
+template <int LANES, bool STAGED, bool KICK, bool FIXED>
+__global__ void EAMF_BOUNDS(STAGED, FIXED ? FIX_CTAS_FORCE : 4) k_eamf_force(EAMFast p, const PosPack* __restrict__ pack,
+                                                       const int4* __restrict__ ipos,
                                                        const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
                                                        const float* __restrict__ femb, float* __restrict__ fx,
                                                        float* __restrict__ fy, float* __restrict__ fz,
@@ -341,16 +479,16 @@ __global__ void EAMF_BOUNDS(STAGED) k_eamf_force(EAMFast p, const PosPack* __res
         s_kk[kslot] = s_ke[kslot] = s_kw[kslot] = F2{0.f, 0.f};
         s_kv[kslot] = 0ull;
     }
-    __shared__ float4 s_hi[64], s_lo[64];
+    __shared__ float4 s_hi[FIXED ? 1 : 64], s_lo[FIXED ? 1 : 64];
     extern __shared__ float4 s_tab[];  // phi knots [k0, k0+ns), then rho knots (separate arrays: a warp's
                                        // random knots spread over all eight 16-byte bank groups)
-    build_shift_table(p, s_hi, s_lo);
+    if (!FIXED) build_shift_table(p, s_hi, s_lo);
     if (STAGED)
         for (int k = threadIdx.x; k < 2 * p.stage_n; k += blockDim.x) {
             const int kk = k < p.stage_n ? k : k - p.stage_n;
             s_tab[k] = p.coef2[2 * (size_t)(p.stage_k0 + kk) + (k < p.stage_n ? 0 : 1)];
         }
-    __syncthreads();
+    if (!FIXED) __syncthreads();
     const int lane = threadIdx.x & (LANES - 1);
     const int per_block = blockDim.x / LANES;
     for (int base = blockIdx.x * per_block; base < p.n; base += gridDim.x * per_block) {
@@ -360,7 +498,8 @@ __global__ void EAMF_BOUNDS(STAGED) k_eamf_force(EAMFast p, const PosPack* __res
         const int m = valid ? nnb[ii] : 0;
         Kahan ax, ay, az;
         float ae = 0.f, av = 0.f;
-        gather_force_sum<LANES, STAGED>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_tab, ax, ay, az, ae, av, status);
+        if (FIXED) fixed_force_sum<LANES>(p, ipos, nbr, ii, m, lane, ax, ay, az, ae, av, status);
+        else gather_force_sum<LANES, STAGED>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_tab, ax, ay, az, ae, av, status);
         force_reduce<LANES>(ax, ay, az, ae, av);
         if (lane == 0 && valid) {
             const float vfx = __fsub_rn(ax.s, ax.c), vfy = __fsub_rn(ay.s, ay.c), vfz = __fsub_rn(az.s, az.c);
@@ -590,7 +729,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) k_eamt_density(EAMFast p, EAM
         }
         float sum = acc.s, comp = acc.c;
         twosum_reduce<LANES>(sum, comp);
-        if (lane == 0 && valid) density_finish(p, i, __fsub_rn(sum, comp), pack, fp, femb, status);
+        if (lane == 0 && valid) density_finish(p, i, __fsub_rn(sum, comp), &pack[i].lo.w, fp, femb, status);
     }
 }
 
@@ -697,33 +836,33 @@ static void launch_tiles(Context* c, const EAMFast& p, const EAMTileArgs& a) {
     prof_end(c);
 }
 
-template <int LANES, bool STAGED>
+template <int LANES, bool STAGED, bool FIXED>
 static void launch_fast(Context* c, const EAMFast& p, int grid, int block, size_t smem1, size_t smem2,
                         const KickArgs* ka) {
     static bool attr = false;
     if (!attr) {
-        cudaFuncSetAttribute(k_eamf_density<LANES, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_eamf_density<LANES, STAGED, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, false, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              200 * 1024);
-        cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, true, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              200 * 1024);
         attr = true;
     }
     prof_begin(c, "eam_density");
-    k_eamf_density<LANES, STAGED><<<grid, block, smem1, c->stream>>>(
-        p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->fp, c->femb, c->d_status);
+    k_eamf_density<LANES, STAGED, FIXED><<<grid, block, smem1, c->stream>>>(
+        p, c->pack, c->ipos, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->fp, c->femb, c->d_status);
     prof_end(c);
     const unsigned* aflag = c->flags_used ? c->aflag : nullptr;
     if (ka) {
         prof_begin(c, "eam_force_kick");
-        k_eamf_force<LANES, STAGED, true><<<grid, block, smem2, c->stream>>>(
-            p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->femb, c->fx, c->fy, c->fz, c->pe,
+        k_eamf_force<LANES, STAGED, true, FIXED><<<grid, block, smem2, c->stream>>>(
+            p, c->pack, c->ipos, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->femb, c->fx, c->fy, c->fz, c->pe,
             c->vir, c->d_status, *ka, c->vx, c->vy, c->vz, aflag, c->d_ledger);
         launch_ledger_finalize(c, *ka, grid * (block >> 5));
     } else {
         prof_begin(c, "eam_force");
-        k_eamf_force<LANES, STAGED, false><<<grid, block, smem2, c->stream>>>(
-            p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->femb, c->fx, c->fy, c->fz, c->pe,
+        k_eamf_force<LANES, STAGED, false, FIXED><<<grid, block, smem2, c->stream>>>(
+            p, c->pack, c->ipos, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->femb, c->fx, c->fy, c->fz, c->pe,
             c->vir, c->d_status, KickArgs{}, nullptr, nullptr, nullptr, nullptr, nullptr);
     }
     prof_end(c);
@@ -744,6 +883,13 @@ bool tiles_apply(const Context* c) {
     return p.kind == POT_EAM && eam_fast_shape(c, p);
 }
 
+bool eam_uses_fixed(const Context* c) {
+    if (c->use_f64 || c->eam_stage || c->n < FIX_PER_SM * c->num_sms) return false;
+    for (const Potential& p : c->pots)
+        if (p.kind == POT_EAM && eam_fast_shape(c, p)) return true;
+    return false;
+}
+
 bool eam_fast_ok(const Context* c, const Potential& pot) { return pot.d_coef2 && eam_fast_shape(c, pot); }
 
 int eam_fast_launch(Context* c, Potential& pot, bool first) {
@@ -754,6 +900,8 @@ int eam_fast_launch(Context* c, Potential& pot, bool first) {
     for (int d = 0; d < 3; d++) {
         p.Lh[d] = c->box.Lh[d];
         p.Ll[d] = c->box.Ll[d];
+        p.qh[d] = c->fix.qh[d];
+        p.ql[d] = c->fix.ql[d];
     }
     p.coef2 = pot.d_coef2;
     p.emb = pot.dt[2].coef;
@@ -790,7 +938,12 @@ int eam_fast_launch(Context* c, Potential& pot, bool first) {
     }
     p.stage_k0 = k0;
     p.stage_n = ns;
+    const bool fixed = c->fix.on && c->ipos && ns == 0;
     int block = c->eam_block > 256 ? 256 : c->eam_block, lanes = c->eam_lanes;
+    // a large box fills the chip with two lanes an atom, and reduces less:
+    // density and force of 1,048,576 atoms 197 and 252 us with four, 188 and 236
+    // with two; of 256,000 54 and 65, 58 and 64
+    if (fixed && !c->eam_lanes_set && c->n >= FIX_TWO_LANES_PER_SM * c->num_sms) lanes = 2;
     int per_block = block / lanes;
     int grid = grid_for(c->n, per_block);
     if (ns > 0) {
@@ -844,8 +997,9 @@ int eam_fast_launch(Context* c, Potential& pot, bool first) {
         return check_cuda(c, cudaGetLastError(), "eam tiles");
     }
 #define OMDG_EAMF(L)                                                 \
-    (st ? launch_fast<L, true>(c, p, grid, block, smem1, smem2, kap) \
-        : launch_fast<L, false>(c, p, grid, block, smem1, smem2, kap))
+    (st      ? launch_fast<L, true, false>(c, p, grid, block, smem1, smem2, kap) \
+     : fixed ? launch_fast<L, false, true>(c, p, grid, block, smem1, smem2, kap) \
+             : launch_fast<L, false, false>(c, p, grid, block, smem1, smem2, kap))
     switch (lanes) {
         case 1: OMDG_EAMF(1); break;
         case 2: OMDG_EAMF(2); break;

@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __re
         pk.hi.w = __int_as_float(t);
         pk.lo.w = 0.f;
         pack[i] = pk;
+        if (p.ipos) p.ipos[i] = fix_pos(X, Y, Z, p.fix);
         float4 r0 = xref[i];
         float dx = (pk.hi.x - r0.x) + pk.lo.x, dy = (pk.hi.y - r0.y) + pk.lo.y, dz = (pk.hi.z - r0.z) + pk.lo.z;
         if (!(dx * dx + dy * dy + dz * dz <= p.half_skin2)) {  // NaN counts as moved
@@ -397,6 +398,8 @@ static IntParams int_params(Context* c) {
     }
     float hs = (float)(0.5 * c->skin);
     p.half_skin2 = hs * hs;
+    p.fix = c->fix;
+    p.ipos = c->fix.on ? c->ipos : nullptr;
     p.use_f64 = c->use_f64 ? 1 : 0;
     for (int d = 0; d < 3; d++) {
         p.Q[d] = c->box.P[d] - c->box.org[d];
@@ -734,6 +737,7 @@ __global__ void __launch_bounds__(IO_BLOCK) k_upload_state(IntParams p, const in
             pk.hi.w = __int_as_float(type[i]);
             pk.lo.w = 0.f;
             pack[i] = pk;
+            if (p.ipos) p.ipos[i] = fix_pos(X, Y, Z, p.fix);
             const float4 r0 = xref[i];
             const float dx = (pk.hi.x - r0.x) + pk.lo.x, dy = (pk.hi.y - r0.y) + pk.lo.y,
                         dz = (pk.hi.z - r0.z) + pk.lo.z;

@@ -379,3 +379,45 @@ def test_kick_in_the_force_epilogue_is_the_same_step(omdg_lib):
         assert np.array_equal(a[k], b[k]), k
     np.testing.assert_allclose(ka, kb, rtol=1e-6)
     np.testing.assert_allclose(pa, pb, rtol=1e-7)
+
+
+@pytest.mark.parametrize("case", ["three_ranges", "below", "above", "far", "offset", "lanes2"])
+def test_fixed_point_positions(omdg_lib, oracle_lib, case):
+    """The passes over fixed-point positions, at the shortest box they take and
+    one part in 10^9 below (the packs), with free atoms past the range of the
+    direct conversion, a box far from the origin, and two lanes an atom."""
+    from objectmd_gb300 import inputs
+
+    oc = oracle_lib
+    phi = oc.Table.from_file(EAM_TABLE, "PAIR")
+    ed = oc.Table.from_file(EAM_TABLE, "EDENS")
+    em = oc.Table.from_file(EAM_TABLE, "EMBED")
+    rv = phi.max_range() + 0.3
+    edge = {"three_ranges": 3 * rv, "below": 3 * rv * (1 - 1e-9), "above": 3 * rv * (1 + 1e-9)}
+    n = int(round(3 * rv / 4.05)) if case in edge else int(np.ceil(3 * rv / 4.05))
+    side = edge.get(case, n * 4.05)
+    cells = (n, n, 24000 // (4 * n * n))  # over the line by size (128 atoms a SM)
+    x, lo, hi = inputs.fcc(cells, side / n)
+    x = inputs.perturb(x, 0.08, 15, lo, hi)
+    v = np.zeros_like(x)
+    lo, hi = np.asarray(lo, dtype=np.float64), np.asarray(hi, dtype=np.float64)
+    periodic = (1, 1, 1)
+    if case == "far":
+        periodic = (1, 1, 0)
+        x = np.vstack([x, [[3.0, 4.0, 3.0e5], [4.0, 5.0, 3.0e5 + 2.4], [9.0, 9.0, -2.7e5], [9.5, 11.5, -2.7e5]]])
+        v = np.zeros_like(x)
+    if case == "offset":
+        shift = np.array([-1000.5, 3.0e4, 17.25])
+        x, lo, hi = x + shift, lo + shift, hi + shift
+    box = oc.make_box(lo, hi, periodic)
+    fref, eref, vref, _ = oc.eam(box, x, oc.neighbors(box, x, rv), phi, ed, em)
+    with omdg_lib.Context(0) as ctx:
+        ctx.set_box(lo, hi, tuple(bool(p) for p in periodic))
+        ctx.set_atoms(x, v, masses=[inputs.md_mass("aluminum")], znum=[13.0])
+        ctx.add_eam(EAM_TABLE)
+        ctx.set_neighbor(0.3, 1)
+        if case == "lanes2":
+            ctx.set_launch("eam_lanes", 2)
+        ctx.compute_forces()
+        st = ctx.get_state()
+    check_forces(st["f"], fref, st["pot"], eref)
