@@ -70,9 +70,18 @@ inline bool nn_std_angular(const NNDescParams& p) {
     return true;
 }
 
+// ... and one eta for each of its two groups of eight.
+inline bool nn_grouped_angular(const NNDescParams& p) {
+    for (int m = 0; m < NN_ANG; m++)
+        if (p.eta_a[m] != p.eta_a[m & 8]) return false;
+    return nn_std_angular(p);
+}
+
 // Angular term m of the neighbour pair (a, b): the value and its derivatives
 // with respect to r_a, r_b and cos(theta); ex = exp(-eta_a[m] (r_a^2 + r_b^2)).
-template <bool STD = false>
+// GROUPED: one eta for each group of eight, so what does not depend on the term
+// is formed once a group.
+template <bool STD = false, bool GROUPED = false>
 __device__ __forceinline__ void nn_angular(const NNDescParams& p, int m, float ra, float rb, float cs, float fa,
                                            float dfa, float fb, float dfb, float ex, float& val, float& d_ra,
                                            float& d_rb, float& d_cs) {
@@ -82,10 +91,10 @@ __device__ __forceinline__ void nn_angular(const NNDescParams& p, int m, float r
     const int z = STD ? nn_std_zeta(m) : p.zeta[m];
     const float pm1 = nn_ipow(base, z - 1);
     const float pw = pm1 * base;
-    const float k = p.pref[m] * ex;
+    const float k = p.pref[m] * ex, eta = p.eta_a[GROUPED ? m & 8 : m];
     val = k * pw * fa * fb;
-    d_ra = k * pw * fb * (dfa - 2.f * p.eta_a[m] * ra * fa);
-    d_rb = k * pw * fa * (dfb - 2.f * p.eta_a[m] * rb * fb);
+    d_ra = k * pw * fb * (dfa - 2.f * eta * ra * fa);
+    d_rb = k * pw * fa * (dfb - 2.f * eta * rb * fb);
     d_cs = base > 0.f ? k * (float)z * pm1 * lam * fa * fb : 0.f;
 }
 

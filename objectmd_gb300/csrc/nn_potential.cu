@@ -82,8 +82,14 @@ __device__ __forceinline__ int nn_hits(const NNMD& q, int i, const PosPack& pi, 
     return nc;
 }
 
-// STD holds the shared powers of both bases: 80 registers at six blocks per
-// SM, where unbounded it takes 96 (five blocks)
+// STD: the default angular layout with one eta a group (nn_grouped_angular).  It
+// holds the shared powers of both bases: 80 registers at six blocks per SM,
+// where unbounded it takes 96 (five blocks).  Bound by its instructions: the
+// cutoffs of a neighbour once instead of once a pair, and what depends on eta
+// once a group, 512,000 atoms 112 -> 103 us with the same bits.  (Sums over the
+// powers first and the three derivatives of a pair from them take 78 us, but
+// the other rounding moves enough descriptors across a BF16 step to move the
+// forces by 2e-5 in ten steps.)
 template <bool STD>
 __global__ void __launch_bounds__(128, STD ? 6 : 7) k_nn_md_force(NNMD q, NNDescParams p, const PosPack* __restrict__ pack,
                                                      const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
@@ -110,10 +116,13 @@ __global__ void __launch_bounds__(128, STD ? 6 : 7) k_nn_md_force(NNMD q, NNDesc
             u[k + 2] = w.z;
             u[k + 3] = w.w;
         }
+        float fcut[NN_MAXN], dfcut[NN_MAXN], inv[NN_MAXN];
         // radial: dE/dx_j = (sum_k u_k dG_k/dr) e_j
         for (int a = 0; a < nc; a++) {
             float dfc;
             const float fc = nn_fc(p, rr[a], dfc);
+            fcut[a] = fc;
+            dfcut[a] = dfc;
             float c = 0.f;
 #pragma unroll
             for (int k = 0; k < NN_RAD; k++) {
@@ -122,20 +131,17 @@ __global__ void __launch_bounds__(128, STD ? 6 : 7) k_nn_md_force(NNMD q, NNDesc
                 c = fmaf(u[k], ddr, c);
             }
             const float ir = 1.f / rr[a];
+            inv[a] = ir;
             tx[a] = c * vx[a] * ir;
             ty[a] = c * vy[a] * ir;
             tz[a] = c * vz[a] * ir;
         }
         // angular: through r_a, r_b and cos(theta)
         for (int a = 0; a < nc; a++) {
-            float dfa;
-            const float fa = nn_fc(p, rr[a], dfa);
-            const float ia = 1.f / rr[a];
+            const float fa = fcut[a], dfa = dfcut[a], ia = inv[a];
             const float ea[3] = {vx[a] * ia, vy[a] * ia, vz[a] * ia};
             for (int b = a + 1; b < nc; b++) {
-                float dfb;
-                const float fb = nn_fc(p, rr[b], dfb);
-                const float ib = 1.f / rr[b];
+                const float fb = fcut[b], dfb = dfcut[b], ib = inv[b];
                 const float eb[3] = {vx[b] * ib, vy[b] * ib, vz[b] * ib};
                 const float cs = ea[0] * eb[0] + ea[1] * eb[1] + ea[2] * eb[2];
                 float cra = 0.f, crb = 0.f, ccs = 0.f;
@@ -144,7 +150,7 @@ __global__ void __launch_bounds__(128, STD ? 6 : 7) k_nn_md_force(NNMD q, NNDesc
 #pragma unroll
                 for (int mm = 0; mm < NN_ANG; mm++) {
                     float v, d_ra, d_rb, d_cs;
-                    nn_angular<STD>(p, mm, rr[a], rr[b], cs, fa, dfa, fb, dfb, ex.get(p.eta_a[mm], s2), v, d_ra,
+                    nn_angular<STD, STD>(p, mm, rr[a], rr[b], cs, fa, dfa, fb, dfb, ex.get(p.eta_a[STD ? mm & 8 : mm], s2), v, d_ra,
                                     d_rb, d_cs);
                     const float w = u[NN_RAD + mm];
                     cra = fmaf(w, d_ra, cra);
@@ -246,7 +252,7 @@ int nn_launch(Context* c, Potential& pot, bool first) {
     }
     if (e != cudaSuccess) return check_cuda(c, e, "surrogate network");
     prof_begin(c, "nn_force");
-    auto force = std_ang ? k_nn_md_force<true> : k_nn_md_force<false>;
+    auto force = nn_grouped_angular(s.model.dp) ? k_nn_md_force<true> : k_nn_md_force<false>;
     force<<<grid, 128, 0, c->stream>>>(q, s.model.dp, c->pack, nbr, c->nnb, s.E, s.U, s.flag, slot_rows(c), c->fx,
                                        c->fy, c->fz, c->pe, c->vir, c->d_status);
     prof_end(c);
