@@ -150,28 +150,42 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(int m, const int* _
 }
 
 // One block: tile totals -> exclusive tile offsets; start[m] = total.
-__global__ void k_scan_totals(int ntiles, int m, int* __restrict__ tile_sum, int* __restrict__ start) {
-    __shared__ int sums[1024];
-    const int t = threadIdx.x, nt = blockDim.x;
+// (and clears umax for the permutation, which packs)
+__global__ void k_scan_totals(int ntiles, int m, int* __restrict__ tile_sum, int* __restrict__ start,
+                              unsigned* umax) {
+    __shared__ int warp_sum[32];
+    const int t = threadIdx.x, nt = blockDim.x, lane = t & 31;
+    if (t == 0) *umax = 0u;
     const int chunk = (ntiles + nt - 1) / nt;
     const int b = t * chunk, e = min(ntiles, b + chunk);
     int s = 0;
     for (int k = b; k < e; k++) s += tile_sum[k];
-    sums[t] = s;
-    __syncthreads();
-    for (int off = 1; off < nt; off <<= 1) {
-        const int y = t >= off ? sums[t - off] : 0;
-        __syncthreads();
-        sums[t] += y;
-        __syncthreads();
+    int run = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += u;
     }
-    int run = sums[t] - s;
+    if (lane == 31) warp_sum[t >> 5] = run;
+    __syncthreads();
+    if (t < 32) {
+        int w = t < (nt >> 5) ? warp_sum[t] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += u;
+        }
+        warp_sum[t] = w;
+    }
+    __syncthreads();
+    if (t >= 32) run += warp_sum[(t >> 5) - 1];
+    if (t == nt - 1) start[m] = run;
+    run -= s;
     for (int k = b; k < e; k++) {
         const int c = tile_sum[k];
         tile_sum[k] = run;
         run += c;
     }
-    if (t == nt - 1) start[m] = sums[t];
 }
 
 __global__ void k_scan_add(int m, int* __restrict__ start, const int* __restrict__ tile_off) {
@@ -281,27 +295,81 @@ struct AtomArrays {
     int extra_n;
 };
 
+// The pack coordinate is X = x + Q with Q = P - org, formed as FP32 hi + lo
+// by pack_coord (the integrator refreshes the pack with the same function).
+struct PackFrame {
+    float Qh[3], Ql[3];
+    FixFrame fix;
+    int4* ipos;  // null: not kept
+};
+
+// loc: the position rounded to FP32, which the list build screens (w: the type)
+// One atom's packs; returns its share of umax.
+__device__ __forceinline__ float pack_atom(int i, double X, double Y, double Z, int type, bool active,
+                                           const PackFrame& f, PosPack* __restrict__ pack, float4* __restrict__ xref,
+                                           float4* __restrict__ loc) {
+    PosPack p;
+    pack_coord(X, f.Qh[0], f.Ql[0], p.hi.x, p.lo.x);
+    pack_coord(Y, f.Qh[1], f.Ql[1], p.hi.y, p.lo.y);
+    pack_coord(Z, f.Qh[2], f.Ql[2], p.hi.z, p.lo.z);
+    p.hi.w = __int_as_float(type);
+    p.lo.w = 0.f;
+    pack[i] = p;
+    if (f.ipos) f.ipos[i] = fix_pos(X, Y, Z, f.fix);
+    if (xref) xref[i] = make_float4(p.hi.x, p.hi.y, p.hi.z, 0.f);
+    if (!loc) return 0.f;
+    if (!active) {
+        // inactive (SetActive false): far from every centre, so no list takes
+        // it, and outside the band's max |x|
+        loc[i] = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f);
+        return 0.f;
+    }
+    const float ux = f2_from(X).hi, uy = f2_from(Y).hi, uz = f2_from(Z).hi;
+    loc[i] = make_float4(ux, uy, uz, p.hi.w);
+    const float m = fmaxf(fabsf(ux), fmaxf(fabsf(uy), fabsf(uz)));
+    return m <= 3.0e38f ? m : 3.0e38f;  // non-finite: flagged by the cell assignment
+}
+
+// The largest |x| sets the width of the screening band.  Whole warps.
+__device__ __forceinline__ void pack_umax(float m, unsigned* umax) {
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+    if ((threadIdx.x & 31) == 0 && m > 0.f && __float_as_uint(m) > *(volatile unsigned*)umax)
+        atomicMax(umax, __float_as_uint(m));
+}
+
 // Also writes the sorted atoms' cells and the caller-to-sorted map (the new
 // position k of caller atom id[o]).
+// The permutation into the staging arrays, and the packs while the position is
+// at hand (a pass of its own read it back: sort and pack of 512,000 atoms 112.7
+// -> 99.5 us).
 __global__ void k_permute_gather(int n, const int* __restrict__ perm, AtomArrays a, AtomArrays st,
                                  const int* __restrict__ cell_old, int* __restrict__ cell_new,
                                  int* __restrict__ inv, const int* __restrict__ rep_of,
-                                 const int* __restrict__ rflag) {
+                                 const int* __restrict__ rflag, PackFrame f, const unsigned* __restrict__ aflag,
+                                 PosPack* __restrict__ pack, float4* __restrict__ xref, float4* __restrict__ loc,
+                                 unsigned* umax) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n || !rep_on(rflag, rep_of, k)) return;  // a replica's atoms stay in its index range
-    int o = perm[k];
-    cell_new[k] = cell_old[o];
-    inv[a.id[o]] = k;
-    st.x[k] = a.x[o];
-    st.y[k] = a.y[o];
-    st.z[k] = a.z[o];
-    st.vx[k] = a.vx[o];
-    st.vy[k] = a.vy[o];
-    st.vz[k] = a.vz[o];
-    st.type[k] = a.type[o];
-    st.id[k] = a.id[o];
-    st.flag[k] = a.flag[o];
-    for (int q = 0; q < a.extra_n; q++) st.extra[(size_t)q * n + k] = a.extra[(size_t)q * n + o];
+    float u = 0.f;
+    if (k < n && rep_on(rflag, rep_of, k)) {  // a replica's atoms stay in its index range
+        int o = perm[k];
+        cell_new[k] = cell_old[o];
+        inv[a.id[o]] = k;
+        const double X = a.x[o], Y = a.y[o], Z = a.z[o];
+        const int type = a.type[o];
+        const unsigned flag = a.flag[o];
+        st.x[k] = X;
+        st.y[k] = Y;
+        st.z[k] = Z;
+        st.vx[k] = a.vx[o];
+        st.vy[k] = a.vy[o];
+        st.vz[k] = a.vz[o];
+        st.type[k] = type;
+        st.id[k] = a.id[o];
+        st.flag[k] = flag;
+        for (int q = 0; q < a.extra_n; q++) st.extra[(size_t)q * n + k] = a.extra[(size_t)q * n + o];
+        u = pack_atom(k, X, Y, Z, type, !aflag || (flag & 1u), f, pack, xref, loc);
+    }
+    pack_umax(u, umax);
 }
 
 // The state a rebuild reorders, copied before the rebuild of a step (unless
@@ -387,58 +455,11 @@ struct RepGeom {
     ShiftF S;
 };
 
-// The pack coordinate is X = x + Q with Q = P - org, formed as FP32 hi + lo
-// by pack_coord (the integrator refreshes the pack with the same function).
-struct PackFrame {
-    float Qh[3], Ql[3];
-    FixFrame fix;
-    int4* ipos;  // null: not kept
-};
-
-// loc: the position rounded to FP32, which the list build screens (w: the type)
-// One atom's packs; returns its share of umax.
-__device__ __forceinline__ float pack_atom(int i, double X, double Y, double Z, int type, bool active,
-                                           const PackFrame& f, PosPack* __restrict__ pack, float4* __restrict__ xref,
-                                           float4* __restrict__ loc) {
-    PosPack p;
-    pack_coord(X, f.Qh[0], f.Ql[0], p.hi.x, p.lo.x);
-    pack_coord(Y, f.Qh[1], f.Ql[1], p.hi.y, p.lo.y);
-    pack_coord(Z, f.Qh[2], f.Ql[2], p.hi.z, p.lo.z);
-    p.hi.w = __int_as_float(type);
-    p.lo.w = 0.f;
-    pack[i] = p;
-    if (f.ipos) f.ipos[i] = fix_pos(X, Y, Z, f.fix);
-    if (xref) xref[i] = make_float4(p.hi.x, p.hi.y, p.hi.z, 0.f);
-    if (!loc) return 0.f;
-    if (!active) {
-        // inactive (SetActive false): far from every centre, so no list takes
-        // it, and outside the band's max |x|
-        loc[i] = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f);
-        return 0.f;
-    }
-    const float ux = f2_from(X).hi, uy = f2_from(Y).hi, uz = f2_from(Z).hi;
-    loc[i] = make_float4(ux, uy, uz, p.hi.w);
-    const float m = fmaxf(fabsf(ux), fmaxf(fabsf(uy), fabsf(uz)));
-    return m <= 3.0e38f ? m : 3.0e38f;  // non-finite: flagged by the cell assignment
-}
-
-// The largest |x| sets the width of the screening band.  Whole warps.
-__device__ __forceinline__ void pack_umax(float m, unsigned* umax) {
-    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-    if ((threadIdx.x & 31) == 0 && m > 0.f && __float_as_uint(m) > *(volatile unsigned*)umax)
-        atomicMax(umax, __float_as_uint(m));
-}
-
 __global__ void k_pack(int n, const double* __restrict__ x, const double* __restrict__ y,
                        const double* __restrict__ z, const int* __restrict__ type, PackFrame f,
-                       PosPack* __restrict__ pack, float4* __restrict__ xref, const int* __restrict__ rep_of,
-                       const unsigned* __restrict__ aflag, float4* __restrict__ loc, unsigned* umax,
-                       const int* __restrict__ rflag) {
+                       PosPack* __restrict__ pack) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float m = 0.f;
-    if (i < n && (!rflag || rflag[rep_of[i]]))
-        m = pack_atom(i, x[i], y[i], z[i], type[i], !aflag || (aflag[i] & 1u), f, pack, xref, loc);
-    if (loc) pack_umax(m, umax);
+    if (i < n) pack_atom(i, x[i], y[i], z[i], type[i], true, f, pack, nullptr, nullptr);
 }
 
 // EAM cell tiles: besides the list entry, the build writes each entry's
@@ -897,7 +918,9 @@ __global__ void k_cell_assign_rep(int n, double* __restrict__ x, double* __restr
 // For every list entry (i, s) -> j, the slot of i in row j: REV_LANES
 // threads per centre, each searching for every REV_LANES-th entry (the
 // searches are independent chains of loads; lanes keep more of them in
-// flight).
+// flight).  A search finds both entries of a pair, so only the lower atom
+// searches: 194,184 Stillinger-Weber atoms 45.0 -> 36.4 us, 512,000 Tersoff
+// atoms 22.5 -> 20.8.
 constexpr int REV_LANES = 4;
 
 __device__ __forceinline__ void reverse_centre(int i, int lane, int hshift, int maxnb,
@@ -907,6 +930,7 @@ __device__ __forceinline__ void reverse_centre(int i, int lane, int hshift, int 
     for (int s = lane; s < m; s += REV_LANES) {
         unsigned e = nbr[nbr_at(i, s, hshift, maxnb)];
         int j = nbr_index(e);
+        if (j < i) continue;  // j's search finds both
         unsigned want = nbr_encode(i, -nbr_sx(e), -nbr_sy(e), -nbr_sz(e));
         int mj = nnb[j], found = -1;
         for (int u = 0; u < mj; u++)
@@ -915,6 +939,7 @@ __device__ __forceinline__ void reverse_centre(int i, int lane, int hshift, int 
                 break;
             }
         if (found < 0) atomicOr(status, ERR_NBR_OVERFLOW);
+        else rev[nbr_at(j, found, hshift, maxnb)] = s;
         rev[nbr_at(i, s, hshift, maxnb)] = found < 0 ? 0 : found;
     }
 }
@@ -1505,6 +1530,8 @@ int nlist_reserve(Context* c, int maxnb) {
     if (cudaMalloc(&c->nbr, need) != cudaSuccess) return set_error(c, OMDG_ENOMEM, "neighbour list allocation");
     if (c->need_rev) {
         if (cudaMalloc(&c->rev, need) != cudaSuccess) return set_error(c, OMDG_ENOMEM, "reverse slot allocation");
+        // a row that overflows can leave an entry without its reverse: it stays a valid slot
+        cudaMemsetAsync(c->rev, 0, need, c->stream);
         if (cudaMalloc(&c->slot_buf, nlist_slots(c, maxnb) * sizeof(float4)) != cudaSuccess)
             return set_error(c, OMDG_ENOMEM, "slot buffer allocation");
         if (cudaMalloc(&c->row_hits, sizeof(unsigned) * (size_t)((maxnb + 31) / 32) * c->cap) != cudaSuccess)
@@ -1538,8 +1565,7 @@ static int ensure_cells(Context* c, int m) {
 int integrate_pack(Context* c) {
     if (c->n == 0) return OMDG_OK;
     // xref keeps the positions of the last build (the displacement reference)
-    k_pack<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->x, c->y, c->z, c->type, pack_frame(c), c->pack,
-                                                       nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+    k_pack<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->x, c->y, c->z, c->type, pack_frame(c), c->pack);
     c->launches++;
     return check_cuda(c, cudaGetLastError(), "pack");
 }
@@ -1602,7 +1628,7 @@ int nlist_build(Context* c, bool on_request) {
                                                              c->d_status);
         const int ntiles = (m + SCAN_TILE - 1) / SCAN_TILE;
         k_scan_tiles<<<ntiles, SCAN_THREADS, 0, s>>>(m, c->cell_count, c->cell_start, c->cell_tile_sum);
-        k_scan_totals<<<1, 1024, 0, s>>>(ntiles, m, c->cell_tile_sum, c->cell_start);
+        k_scan_totals<<<1, 1024, 0, s>>>(ntiles, m, c->cell_tile_sum, c->cell_start, umax);
         k_scan_add<<<grid_for(m, 256), 256, 0, s>>>(m, c->cell_start, c->cell_tile_sum);
         k_scatter<<<grid_for(n, 256), 256, 0, s>>>(n, c->cell, c->cell_start, c->cell_fill, c->perm, c->d_rep_of, rflag);
         // most cells of a sparse grid (replica margins, vacuum) hold 0 or 1 atoms:
@@ -1626,15 +1652,10 @@ int nlist_build(Context* c, bool on_request) {
                        c->stage_i + c->cap, reinterpret_cast<unsigned*>(c->stage_i + 2 * (size_t)c->cap),
                        c->stage_extra, c->extra_n};
         k_permute_gather<<<grid_for(n, 256), 256, 0, s>>>(n, c->perm, cur, stg, c->cell, cell_sorted, c->inv,
-                                                          c->d_rep_of, rflag);
+                                                          c->d_rep_of, rflag, pack_frame(c),
+                                                          c->flags_used ? c->aflag : nullptr, c->pack, c->xref, c->loc,
+                                                          umax);
         k_permute_copyback<<<grid_for(n, 256), 256, 0, s>>>(n, stg, cur, c->d_rep_of, rflag);
-        c->launches += 2;
-        prof_end(c);
-        prof_begin(c, "pack");
-        k_zero_ints<<<1, 32, 0, s>>>(1, c->d_flags + 3, c->d_flags + 3);
-        k_pack<<<grid_for(n, 256), 256, 0, s>>>(n, c->x, c->y, c->z, c->type, pack_frame(c), c->pack, c->xref,
-                                                reps ? c->d_rep_of : nullptr, c->flags_used ? c->aflag : nullptr, c->loc,
-                                                umax, rflag);
         c->launches += 2;
         prof_end(c);
     }
