@@ -132,16 +132,18 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __re
 // loads' latency beside the half-kick's: 512,000 Tersoff atoms 32.9 us at six
 // blocks a SM and 24.4 at four, 194,184 Stillinger-Weber atoms 27.0 and 20.8,
 // 1.47 M atoms of the impact ensemble 70 and 56.
-template <bool GATHER>
-__global__ void __launch_bounds__(RED_BLOCK, KICK_BLOCKS_SM) k_kick(
+template <bool GATHER, int T>
+__global__ void __launch_bounds__(T, T == RED_BLOCK ? KICK_BLOCKS_SM : 1) k_kick(
     IntParams p, FinParams f, SlotArgs ga, double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
     float* __restrict__ fx, float* __restrict__ fy, float* __restrict__ fz, const double* __restrict__ f64,
     const int* __restrict__ type, float* __restrict__ pe, float* __restrict__ vir,
     const unsigned* __restrict__ aflag, BlockPartial* __restrict__ partial, double* __restrict__ ledger,
     StepState* st, int kick) {
+    __shared__ LedgerSums<T> sums;
+    if (threadIdx.x == LEDGER_PREPARE) sums.prepare(f, st);
     F2 k = {0.f, 0.f}, e = {0.f, 0.f}, w = {0.f, 0.f};
     unsigned long long vmax = 0ull;  // bits of the largest squared speed
-    for (int i = blockIdx.x * RED_BLOCK + threadIdx.x; i < p.n; i += gridDim.x * RED_BLOCK) {
+    for (int i = blockIdx.x * T + threadIdx.x; i < p.n; i += gridDim.x * T) {
         float gx, gy, gz, gp, gw;
         if (!p.use_f64 || GATHER) {
             gx = fx[i];
@@ -184,7 +186,7 @@ __global__ void __launch_bounds__(RED_BLOCK, KICK_BLOCKS_SM) k_kick(
                                      __dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy)), __dmul_rn(uz, uz))));
         }
     }
-    ledger_block(p, f, k, e, w, vmax, partial, ledger, st);
+    ledger_block<T>(sums, p, f, k, e, w, vmax, partial, ledger, st);
 }
 
 // Blocks of the kick: a whole number of atoms a thread, all blocks resident.
@@ -469,6 +471,7 @@ void kick_args(Context* c, KickArgs& ka) {
 __global__ void __launch_bounds__(1024) k_ledger_finalize(FinParams f, int nparts, const BlockPartial* partial,
                                                           double* ledger, StepState* st) {
     __shared__ LedgerSums<1024> s;
+    if (threadIdx.x == LEDGER_PREPARE) s.prepare(f, st);
     finalize_block<1024>(s, f, nparts, partial, ledger, st);
 }
 
@@ -508,12 +511,16 @@ static int reduce_and_finalize(Context* c, int kick, int count_step) {
     c->gather_deferred = false;
     const int nb = kick_blocks(c);
     prof_begin(c, gather ? "gather_kick" : "kick");
-    auto kernel = gather ? k_kick<true> : k_kick<false>;
-    kernel<<<nb, RED_BLOCK, 0, c->stream>>>(p, f, slot_args(c, c->gather_zero_virial), c->vx, c->vy, c->vz, c->fx, c->fy,
-                                            c->fz, c->f64, c->type, c->pe, c->vir,
-                                            c->flags_used ? c->aflag : nullptr,
-                                            reinterpret_cast<BlockPartial*>(c->d_red), c->d_ledger,
-                                            reinterpret_cast<StepState*>(c->d_state), kick);
+    // up to 1,024 atoms in one block: no ticket, no partials (a step of 512
+    // Tersoff atoms 30.1 us with two blocks of 256, 28.9 with one of 512)
+    const int threads = c->n <= RED_BLOCK || c->n > 1024 ? RED_BLOCK : c->n <= 512 ? 512 : 1024;
+    auto kernel = threads == 512    ? (gather ? k_kick<true, 512> : k_kick<false, 512>)
+                  : threads == 1024 ? (gather ? k_kick<true, 1024> : k_kick<false, 1024>)
+                                    : (gather ? k_kick<true, RED_BLOCK> : k_kick<false, RED_BLOCK>);
+    kernel<<<threads == RED_BLOCK ? nb : 1, threads, 0, c->stream>>>(
+        p, f, slot_args(c, c->gather_zero_virial), c->vx, c->vy, c->vz, c->fx, c->fy, c->fz, c->f64, c->type, c->pe,
+        c->vir, c->flags_used ? c->aflag : nullptr, reinterpret_cast<BlockPartial*>(c->d_red), c->d_ledger,
+        reinterpret_cast<StepState*>(c->d_state), kick);
     prof_end(c);
     c->launches += 1;
     return check_cuda(c, cudaGetLastError(), "kick");

@@ -71,6 +71,20 @@ __device__ __forceinline__ unsigned long long vmax_bits(const float4& wv) {
     return ((unsigned long long)__float_as_uint(wv.w) << 32) | __float_as_uint(wv.z);
 }
 
+// sqrt(1 + a (b / k - 1)) as N / sqrt(N k) with N = k + a (b - k): one root's
+// estimate and a third-order step (Householder; the estimate is good to 2^-20)
+// in place of a division, a root and what lies between them (2,660 cycles from
+// the sums to the factor in one thread, 2,050 now: FP64 latency).  Outside the estimate's safe range
+// the plain form.
+__device__ __forceinline__ double thermo_factor(double a, double b, double k) {
+    const double N = fma(a, b - k, k), M = N * k;
+    if (!(M > 1e-280 && M < 1e280)) return sqrt(1. + a * (b / k - 1.));
+    double w;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(w) : "d"(M));
+    const double err = fma(-(M * w), w, 1.0);
+    return N * fma(fma(0.375, err, 0.5), w * err, w);
+}
+
 // A block's sums of the three ledger terms of its T threads, and the largest
 // squared speed, in shared memory: one warp for each sum adds T / 32 terms a
 // lane and then a fixed xor tree (450 instructions for 256 threads; a tree in
@@ -109,8 +123,8 @@ struct LedgerSums {
             for (int q = 0; q < T / 32; q++) v = max(v, vmax[q]);
         return v;
     }
-    // By one thread outside the summing warps, beside them: the state's loads
-    // and what does not wait for the sums.
+    // By one thread, ahead of the sums: the state's loads and what follows from
+    // them alone.
     __device__ __forceinline__ void prepare(const FinParams& p, const StepState* st) {
         step = st->step;
         row = st->row;
@@ -143,7 +157,7 @@ struct LedgerSums {
         double lam = 1.0;
         // TempController::PostIntegration: lambda^2 = 1 + dt/tau (Tset/T - 1),
         // with Tset/T as the quotient of the kinetic energies
-        if (thermo && kinetic > 0.0) lam = sqrt(1. + a * (b / kinetic - 1.));
+        if (thermo && kinetic > 0.0) lam = thermo_factor(a, b, kinetic);
         out[3] = lam;
         const double sqrmaxv = __longlong_as_double((long long)largest(p.need_vmax));
         if (p.need_vmax) st->sqrmaxv = sqrmaxv;
@@ -184,12 +198,11 @@ struct LedgerSums {
 constexpr int LEDGER_PREPARE = 96;  // the thread that prepares: the first one outside the summing warps
 
 // Ledger row, thermostat factor and step counter from the block partials, by
-// one block of T threads (FP32 pairs; FP64 only for the totals).  Partials are
-// read through L2: other blocks wrote them.
+// one block of T threads (FP32 pairs; FP64 only for the totals), which has
+// prepared.  Partials are read through L2: other blocks wrote them.
 template <int T>
 __device__ __forceinline__ void finalize_block(LedgerSums<T>& s, const FinParams& p, int nblocks,
                                                const BlockPartial* partial, double* ledger, StepState* st) {
-    if (threadIdx.x == LEDGER_PREPARE) s.prepare(p, st);
     F2 k = {0.f, 0.f}, e = {0.f, 0.f}, w = {0.f, 0.f};
     unsigned long long vm = 0ull;
 #pragma unroll 4
@@ -287,18 +300,23 @@ __device__ __forceinline__ void kick_atom_terms(const IntParams& p, int i, int t
 }
 
 // The block's ledger partial from every thread's terms; the last block to
-// finish sums the partials and writes the ledger row (finalize_block).  Every
-// thread of a block of RED_BLOCK calls it.  What comes after the atoms is a
-// chain of latencies in one block, the same for 512 atoms and a million: 12,000
-// cycles with a tree in every warp, fences around the ticket, the state's loads
-// and three FP64 divisions in the thread that had the sums; some 7,500 now, a
-// third of them the quotient and the root of a thermostat.
-__device__ __forceinline__ void ledger_block(const IntParams& p, const FinParams& f, F2 k, F2 e, F2 w,
-                                             unsigned long long vmax, BlockPartial* __restrict__ partial,
+// finish sums the partials and writes the ledger row (finalize_block); a block
+// alone has the sums.  Every thread of a block of T calls it, and its
+// LEDGER_PREPARE-th has prepared.  What comes after the atoms is a chain of
+// latencies in one block, the same for 512 atoms and a million: 12,000 cycles
+// with a tree in every warp, fences around the ticket, the state's loads and
+// three FP64 divisions in the thread that had the sums; some 6,500 now with the
+// ticket and the partials, 3,800 without (one block).
+template <int T>
+__device__ __forceinline__ void ledger_block(LedgerSums<T>& s, const IntParams& p, const FinParams& f, F2 k, F2 e,
+                                             F2 w, unsigned long long vmax, BlockPartial* __restrict__ partial,
                                              double* __restrict__ ledger, StepState* st) {
-    __shared__ LedgerSums<RED_BLOCK> s;
     __shared__ bool last;
     s.add(k, e, w, vmax, p.need_vmax);
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) s.finish(f, ledger, st);
+        return;
+    }
     if (threadIdx.x == 0) {
         const unsigned long long bv = s.largest(p.need_vmax);
         partial[blockIdx.x].ke = make_float4(s.sums[0].hi, s.sums[0].lo, s.sums[1].hi, s.sums[1].lo);
@@ -310,7 +328,7 @@ __device__ __forceinline__ void ledger_block(const IntParams& p, const FinParams
         last = done == gridDim.x - 1;
     }
     __syncthreads();
-    if (last) finalize_block<RED_BLOCK>(s, f, gridDim.x, partial, ledger, st);
+    if (last) finalize_block<T>(s, f, gridDim.x, partial, ledger, st);
 }
 
 // One warp's ledger partial (the per-warp half of ledger_block): lane 0

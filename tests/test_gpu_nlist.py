@@ -170,3 +170,26 @@ def test_steps_in_one_graph(omdg_lib, ncell):
     assert out[0][4] > 5
     for o in out[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(o, out[0]))
+
+
+@pytest.mark.parametrize("n", [255, 256, 257, 512, 513, 1024, 1025])
+def test_ledger_of_one_block_and_several(omdg_lib, n):
+    """The kick's ledger row at the edges of its one-block forms: kinetic and
+    potential energy against FP64 sums over the atoms (their own FP32 parts:
+    2^-40 relative)."""
+    from objectmd_gb300 import inputs
+
+    x, v, (lo, hi) = inputs.diamond_silicon(ncell=6, a=5.431, sigma=0.05, temp=900.0, seed_pos=3, seed_vel=4)
+    x, v = x[:n], v[:n]
+    mass = inputs.md_mass("silicon")
+    with omdg_lib.Context(0) as ctx:
+        ctx.set_box(lo, hi)
+        ctx.set_atoms(x, v, masses=[mass], znum=[14.0])
+        ctx.add_tersoff(os.path.join(TABLES, "tersoff.silicon27"))
+        ctx.set_neighbor(SKIN, 0)
+        ctx.set_timestep(0.001)
+        ctx.step(2)
+        st = ctx.get_state()
+        k, p = ctx.ledger_history(2)
+    assert abs(k[-1] - 0.5 * mass * (st["v"] ** 2).sum()) <= 2.0 ** -40 * abs(k[-1])
+    assert abs(p[-1] - st["pot"].astype(np.float64).sum()) <= 2.0 ** -40 * abs(p[-1])
