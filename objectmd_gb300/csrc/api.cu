@@ -267,6 +267,7 @@ struct GraphState {
     cudaGraphExec_t many_exec = nullptr;
     cudaGraph_t many_graph = nullptr;
     bool many_valid = false;
+    int many_joined = 0;  // kernels fewer than as many single steps have
     long replayed = 0;
     // the same step with download branches into pinned host arrays
     // (omdg_step_io), keyed by the x, v, f output pointers
@@ -1025,6 +1026,19 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
     const long launches0 = c->launches;
     long l0 = 0, l1 = 0, l2 = 0, l3 = 0;
     int rc = OMDG_OK;
+    bool drifted = false;  // the step's kick_drift was in the last one's kick
+    int joined = 0;
+    cudaGraphConditionalHandle h = 0;
+    const bool on_request = small_sort(c);  // the rebuild's kernels are the step's own, and look for the request
+    const auto new_handle = [&]() -> int {
+        if (on_request) return OMDG_OK;
+        // no rebuild unless the step's drift asks for it
+        cudaStreamCaptureStatus st;
+        cudaGraph_t cg = nullptr;
+        cudaError_t e2 = cudaStreamGetCaptureInfo(s, &st, nullptr, &cg, nullptr, nullptr, nullptr);
+        if (e2 == cudaSuccess) e2 = cudaGraphConditionalHandleCreate(&h, cg, 0, cudaGraphCondAssignDefault);
+        return e2 == cudaSuccess ? OMDG_OK : check_cuda(c, e2, "conditional handle");
+    };
     for (int k = 0; k < steps && !rc; k++) {
         l0 = c->launches;
         rc = (c->ttm && ttm_active(c)) ? ttm_pre(c) : OMDG_OK;  // PreIntegration (TTM_Homogen_SCNA.h:352)
@@ -1033,15 +1047,11 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
         cudaStreamCaptureStatus cst;
         const cudaGraphNode_t* deps = nullptr;
         size_t ndeps = 0;
-        cudaGraphConditionalHandle h = 0;
-        const bool on_request = small_sort(c);  // the rebuild's kernels are the step's own, and look for the request
-        if (!rc && !on_request) {
-            // no rebuild unless the step's kick_drift asks for it
-            e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &g, nullptr, nullptr, nullptr);
-            if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
-            if (e != cudaSuccess) rc = check_cuda(c, e, "conditional handle");
+        if (!rc && !drifted) {
+            rc = new_handle();
+            if (!rc) rc = integrate_kick_drift(c, on_request ? nullptr : &h);
         }
-        if (!rc) rc = integrate_kick_drift(c, on_request ? nullptr : &h);
+        drifted = false;
         l1 = c->launches;
         cudaGraphNode_t cond_node = nullptr;
         if (!rc && on_request) {
@@ -1087,7 +1097,14 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
         c->fuse_kick = false;
         const bool f_after = c->gather_deferred;  // the kick completes the forces
         if (!rc && io && !f_after) rc = branch(1, nullptr, nullptr, io[2]);
-        if (!rc) rc = integrate_kick(c, 0);
+        if (!rc && k + 1 < steps && drift_joins(c)) {
+            rc = new_handle();
+            if (!rc) rc = integrate_kick_and_drift(c, on_request ? nullptr : &h);
+            drifted = true;
+            joined++;
+        } else if (!rc) {
+            rc = integrate_kick(c, 0);
+        }
         if (!rc && c->ttm) rc = thermo_detect(c, true);  // ExecuteDetectors (system.cpp:976)
         if (!rc && io) rc = branch(2, nullptr, io[1], f_after ? io[2] : nullptr);
         if (!rc && io_launches > 0) {  // join the branch
@@ -1099,8 +1116,10 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
         c->captured_builds += 1;
     }
     // captured launches are counted when the graph replays, not here
-    c->graph_step_kernels = (l1 - l0) + (l3 - l2);
-    c->graph_body_kernels = l2 - l1;
+    if (steps == 1) {
+        c->graph_step_kernels = (l1 - l0) + (l3 - l2);
+        c->graph_body_kernels = l2 - l1;
+    }
     c->launches = launches0;
     cudaGraph_t graph = nullptr;
     e = cudaStreamEndCapture(s, &graph);
@@ -1125,6 +1144,7 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
         gs.many_graph = graph;
         gs.many_exec = exec;
         gs.many_valid = true;
+        gs.many_joined = joined;
     } else {
         gs.graph = graph;
         gs.exec = exec;
@@ -1447,6 +1467,7 @@ int omdg_step_async(omdg_ctx* c, int nsteps) {
             cudaError_t e = cudaGraphLaunch(many ? gs.many_exec : gs.exec, c->stream);
             if (e != cudaSuccess) return check_cuda(c, e, "graph launch");
             k += many ? GRAPH_STEPS : 1;
+            if (many) c->launches -= gs.many_joined;
         }
         gs.replayed += nsteps;
         c->graph_steps += nsteps;

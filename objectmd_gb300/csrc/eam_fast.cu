@@ -510,7 +510,11 @@ __global__ void EAMF_BOUNDS(STAGED, FIXED ? FIX_CTAS_FORCE : 4) k_eamf_force(EAM
                 F2 kk = s_kk[kslot], ke = s_ke[kslot], kw = s_kw[kslot];
                 unsigned long long kv = s_kv[kslot];
                 // one type on this path; the finalising block changes hdtm only after every block read it
-                kick_atom_terms(ka.p, i, 0, vfx, vfy, vfz, ve, av, ka.st->hdtm[0], vx[i], vy[i], vz[i], vx, vy, vz, kk, ke, kw, kv);
+                double ux = vx[i], uy = vy[i], uz = vz[i];
+                kick_atom_terms(ka.p, i, 0, vfx, vfy, vfz, ve, av, ka.st->hdtm[0], ux, uy, uz, kk, ke, kw, kv);
+                vx[i] = ux;
+                vy[i] = uy;
+                vz[i] = uz;
                 s_kk[kslot] = kk;
                 s_ke[kslot] = ke;
                 s_kw[kslot] = kw;

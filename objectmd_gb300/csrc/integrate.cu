@@ -23,24 +23,61 @@ namespace omdg {
 
 constexpr int KICK_BLOCKS_SM = 4;
 
-__global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __restrict__ x, double* __restrict__ y,
-                                                    double* __restrict__ z, double* __restrict__ vx,
+// Where a step's first half-kick and drift leave the positions, their packs and
+// the request for a rebuild.
+struct DriftArgs {
+    double *x, *y, *z;
+    PosPack* pack;
+    const float4* xref;
+    const int* rep_of;
+    int* rflag;
+    int* wide;  // the three-body passes' queue, cleared for the step
+    cudaGraphConditionalHandle cond;  // the step's rebuild node in a graph (has_cond)
+    int has_cond;
+};
+
+// Atom i at its new position: stored, packed, and whether it moved past skin/2
+// since the list was built (NaN counts as moved).
+__device__ __forceinline__ bool drift_store(const IntParams& p, const DriftArgs& d, int i, int t, double X, double Y,
+                                            double Z) {
+    d.x[i] = X;
+    d.y[i] = Y;
+    d.z[i] = Z;
+    PosPack pk;
+    pack_coord(X, p.Qh[0], p.Ql[0], pk.hi.x, pk.lo.x);
+    pack_coord(Y, p.Qh[1], p.Ql[1], pk.hi.y, pk.lo.y);
+    pack_coord(Z, p.Qh[2], p.Ql[2], pk.hi.z, pk.lo.z);
+    pk.hi.w = __int_as_float(t);
+    pk.lo.w = 0.f;
+    d.pack[i] = pk;
+    if (p.ipos) p.ipos[i] = fix_pos(X, Y, Z, p.fix);
+    const float4 r0 = d.xref[i];
+    const float dx = (pk.hi.x - r0.x) + pk.lo.x, dy = (pk.hi.y - r0.y) + pk.lo.y, dz = (pk.hi.z - r0.z) + pk.lo.z;
+    return !(dx * dx + dy * dy + dz * dz <= p.half_skin2);
+}
+
+// A block's request for the step's rebuild (one thread).
+__device__ __forceinline__ void drift_request(const DriftArgs& d, StepState* st, bool moved, bool asked) {
+    if (moved) st->rebuild = 1;
+    // the step graph's rebuild node runs (its default is not to); the body's
+    // first kernel takes the request (k_take_rebuild)
+    if (d.has_cond && (moved || asked) && !st->halted) cudaGraphSetConditional(d.cond, 1u);
+}
+
+__global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, DriftArgs d, double* __restrict__ vx,
                                                     double* __restrict__ vy, double* __restrict__ vz,
                                                     const float* __restrict__ fx, const float* __restrict__ fy,
                                                     const float* __restrict__ fz, const double* __restrict__ f64,
-                                                    const int* __restrict__ type, PosPack* __restrict__ pack,
-                                                    const float4* __restrict__ xref, unsigned* __restrict__ aflag,
-                                                    StepState* st, const int* __restrict__ rep_of,
-                                                    int* __restrict__ rflag, int* __restrict__ wide,
-                                                    cudaGraphConditionalHandle cond, int has_cond) {
+                                                    const int* __restrict__ type, unsigned* __restrict__ aflag,
+                                                    StepState* st) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     __shared__ int moved;
     bool asked = false;  // a rebuild requested before this step (periodic, a state upload)
     if (threadIdx.x == 0) {
         moved = 0;
         if (blockIdx.x == 0) {
-            asked = has_cond && st->rebuild;
-            if (wide) *wide = 0;  // the three-body passes' queue of this step
+            asked = d.has_cond && st->rebuild;
+            if (d.wide) *d.wide = 0;
         }
     }
     __syncthreads();
@@ -52,7 +89,7 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __re
         // unchanged since): a group atom beyond box -/+ border is deactivated,
         // and the list is rebuilt without it
         if (p.range_on && (fl & 1u) && (fl & p.range_group)) {
-            const double X0 = x[i], Y0 = y[i], Z0 = z[i];
+            const double X0 = d.x[i], Y0 = d.y[i], Z0 = d.z[i];
             if (X0 < p.range_lo[0] || X0 > p.range_hi[0] || Y0 < p.range_lo[1] || Y0 > p.range_hi[1] ||
                 Z0 < p.range_lo[2] || Z0 > p.range_hi[2]) {
                 fl &= ~1u;
@@ -87,38 +124,17 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __re
         ux = fma(ax, h, ux);
         uy = fma(ay, h, uy);
         uz = fma(az, h, uz);
-        double X = fma(dt, ux, x[i]);
-        double Y = fma(dt, uy, y[i]);
-        double Z = fma(dt, uz, z[i]);
         vx[i] = ux;
         vy[i] = uy;
         vz[i] = uz;
-        x[i] = X;
-        y[i] = Y;
-        z[i] = Z;
-        PosPack pk;
-        pack_coord(X, p.Qh[0], p.Ql[0], pk.hi.x, pk.lo.x);
-        pack_coord(Y, p.Qh[1], p.Ql[1], pk.hi.y, pk.lo.y);
-        pack_coord(Z, p.Qh[2], p.Ql[2], pk.hi.z, pk.lo.z);
-        pk.hi.w = __int_as_float(t);
-        pk.lo.w = 0.f;
-        pack[i] = pk;
-        if (p.ipos) p.ipos[i] = fix_pos(X, Y, Z, p.fix);
-        float4 r0 = xref[i];
-        float dx = (pk.hi.x - r0.x) + pk.lo.x, dy = (pk.hi.y - r0.y) + pk.lo.y, dz = (pk.hi.z - r0.z) + pk.lo.z;
-        if (!(dx * dx + dy * dy + dz * dz <= p.half_skin2)) {  // NaN counts as moved
+        if (drift_store(p, d, i, t, fma(dt, ux, d.x[i]), fma(dt, uy, d.y[i]), fma(dt, uz, d.z[i]))) {
             moved = 1;
             self_moved = true;
         }
     }
-    if (self_moved && rflag) rflag[rep_of[i]] = 1;
+    if (self_moved && d.rflag) d.rflag[d.rep_of[i]] = 1;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        if (moved) st->rebuild = 1;
-        // the step graph's rebuild node runs (its default is not to); the
-        // body's first kernel takes the request (k_take_rebuild)
-        if (has_cond && (moved || asked) && !st->halted) cudaGraphSetConditional(cond, 1u);
-    }
+    if (threadIdx.x == 0) drift_request(d, st, moved, asked);
 }
 
 
@@ -132,15 +148,33 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, double* __re
 // loads' latency beside the half-kick's: 512,000 Tersoff atoms 32.9 us at six
 // blocks a SM and 24.4 at four, 194,184 Stillinger-Weber atoms 27.0 and 20.8,
 // 1.47 M atoms of the impact ensemble 70 and 56.
-template <bool GATHER, int T>
+// DRIFT: the next step's first half-kick and drift follow at once (same force,
+// and no thermostat factor or new time step in between), so the velocity is read
+// and written once, and the force not at all: for the steps inside one graph.
+// A step of eight in a graph with the kernels apart and joined, us: 256,000 EAM
+// atoms 178.8 and 175.7, 194,184 Stillinger-Weber atoms 108.9 and 104.8, 512,000
+// Tersoff atoms 114.3 and 111.6, the impact ensemble 400.6 and 382.7.
+template <bool GATHER, bool DRIFT, int T>
 __global__ void __launch_bounds__(T, T == RED_BLOCK ? KICK_BLOCKS_SM : 1) k_kick(
-    IntParams p, FinParams f, SlotArgs ga, double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
+    IntParams p, FinParams f, SlotArgs ga, DriftArgs d, double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
     float* __restrict__ fx, float* __restrict__ fy, float* __restrict__ fz, const double* __restrict__ f64,
     const int* __restrict__ type, float* __restrict__ pe, float* __restrict__ vir,
     const unsigned* __restrict__ aflag, BlockPartial* __restrict__ partial, double* __restrict__ ledger,
     StepState* st, int kick) {
     __shared__ LedgerSums<T> sums;
     if (threadIdx.x == LEDGER_PREPARE) sums.prepare(f, st);
+    __shared__ int moved;
+    bool asked = false;
+    if (DRIFT) {
+        if (threadIdx.x == 0) {
+            moved = 0;
+            if (blockIdx.x == 0) {
+                asked = d.has_cond && st->rebuild;
+                if (d.wide) *d.wide = 0;
+            }
+        }
+        __syncthreads();
+    }
     F2 k = {0.f, 0.f}, e = {0.f, 0.f}, w = {0.f, 0.f};
     unsigned long long vmax = 0ull;  // bits of the largest squared speed
     for (int i = blockIdx.x * T + threadIdx.x; i < p.n; i += gridDim.x * T) {
@@ -155,26 +189,32 @@ __global__ void __launch_bounds__(T, T == RED_BLOCK ? KICK_BLOCKS_SM : 1) k_kick
         const int t = type[i];
         const double h = st->hdtm[t];
         double ux = vx[i], uy = vy[i], uz = vz[i];
+        double X, Y, Z;
+        if (DRIFT) {
+            X = d.x[i];
+            Y = d.y[i];
+            Z = d.z[i];
+        }
         if (GATHER) {  // (the loads above are in flight beside the slots')
             slot_sum(ga, i, gx, gy, gz, gp);
-            fx[i] = gx;
-            fy[i] = gy;
-            fz[i] = gz;
-            pe[i] = gp;
-            if (ga.zero_virial) vir[i] = gw = 0.f;
+            if (ga.zero_virial) gw = 0.f;
+            if (!DRIFT) {
+                fx[i] = gx;
+                fy[i] = gy;
+                fz[i] = gz;
+                pe[i] = gp;
+                if (ga.zero_virial) vir[i] = 0.f;
+            }
         }
         // inactive atoms: not integrated, not measured (system.cpp:1067, :1085)
         if (aflag && !(aflag[i] & 1u)) continue;
         if (GATHER || (kick && !p.use_f64)) {
-            kick_atom_terms(p, i, t, gx, gy, gz, gp, gw, h, ux, uy, uz, vx, vy, vz, k, e, w, vmax);
+            kick_atom_terms(p, i, t, gx, gy, gz, gp, gw, h, ux, uy, uz, k, e, w, vmax);
         } else {
             if (kick) {
                 ux = fma(f64[3 * (size_t)i], h, ux);
                 uy = fma(f64[3 * (size_t)i + 1], h, uy);
                 uz = fma(f64[3 * (size_t)i + 2], h, uz);
-                vx[i] = ux;
-                vy[i] = uy;
-                vz[i] = uz;
             }
             const F2 sx = f2_from(ux), sy = f2_from(uy), sz = f2_from(uz);
             const F2 v2 = f2_add(f2_add(f2_mul(sx, sx), f2_mul(sy, sy)), f2_mul(sz, sz));
@@ -185,9 +225,31 @@ __global__ void __launch_bounds__(T, T == RED_BLOCK ? KICK_BLOCKS_SM : 1) k_kick
                 vmax = max(vmax, (unsigned long long)__double_as_longlong(__dadd_rn(
                                      __dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy)), __dmul_rn(uz, uz))));
         }
+        if (DRIFT) {
+            const bool s64 = !GATHER && p.use_f64;
+            ux = fma(s64 ? f64[3 * (size_t)i] : f2d_exact(gx), h, ux);
+            uy = fma(s64 ? f64[3 * (size_t)i + 1] : f2d_exact(gy), h, uy);
+            uz = fma(s64 ? f64[3 * (size_t)i + 2] : f2d_exact(gz), h, uz);
+            const double dt = st->dt;
+            if (drift_store(p, d, i, t, fma(dt, ux, X), fma(dt, uy, Y), fma(dt, uz, Z))) {
+                moved = 1;
+                if (d.rflag) d.rflag[d.rep_of[i]] = 1;
+            }
+        }
+        if (kick) {
+            vx[i] = ux;
+            vy[i] = uy;
+            vz[i] = uz;
+        }
     }
-    ledger_block<T>(sums, p, f, k, e, w, vmax, partial, ledger, st);
+    if (DRIFT) {
+        __syncthreads();
+        if (threadIdx.x == 0) drift_request(d, st, moved, asked);
+    }
+    const bool periodic = ledger_block<T>(sums, p, f, k, e, w, vmax, partial, ledger, st);
+    if (DRIFT && periodic) drift_request(d, st, false, true);
 }
+
 
 // Blocks of the kick: a whole number of atoms a thread, all blocks resident.
 static int kick_blocks(const Context* c) {
@@ -411,22 +473,30 @@ static IntParams int_params(Context* c) {
     return p;
 }
 
-// cond: the step graph's rebuild node (capture only).  In a step the first
-// three-body pass finds its queue cleared here.
+static DriftArgs drift_args(Context* c, const cudaGraphConditionalHandle* cond) {
+    c->wide_cleared = c->ters_wide != nullptr;  // in a step the first three-body pass finds its queue cleared
+    const bool reps = c->nrep > 0;
+    return DriftArgs{c->x, c->y, c->z, c->pack, c->xref, reps ? c->d_rep_of : nullptr, reps ? c->d_rep_flag : nullptr,
+                     c->ters_wide, cond ? *cond : 0, cond ? 1 : 0};
+}
+
+// cond: the step graph's rebuild node (capture only).
 int integrate_kick_drift(Context* c, const cudaGraphConditionalHandle* cond) {
     IntParams p = int_params(c);
-    c->wide_cleared = c->ters_wide != nullptr;
+    const DriftArgs d = drift_args(c, cond);
     prof_begin(c, "kick_drift");
-    k_kick_drift<<<grid_for(c->n, 256), 256, 0, c->stream>>>(p, c->x, c->y, c->z, c->vx, c->vy, c->vz, c->fx, c->fy,
-                                                             c->fz, c->f64, c->type, c->pack, c->xref,
-                                                             c->flags_used ? c->aflag : nullptr,
-                                                             reinterpret_cast<StepState*>(c->d_state),
-                                                             c->nrep > 0 ? c->d_rep_of : nullptr,
-                                                             c->nrep > 0 ? c->d_rep_flag : nullptr, c->ters_wide,
-                                                             cond ? *cond : 0, cond ? 1 : 0);
+    k_kick_drift<<<grid_for(c->n, 256), 256, 0, c->stream>>>(p, d, c->vx, c->vy, c->vz, c->fx, c->fy, c->fz, c->f64,
+                                                             c->type, c->flags_used ? c->aflag : nullptr,
+                                                             reinterpret_cast<StepState*>(c->d_state));
     prof_end(c);
     c->launches++;
     return check_cuda(c, cudaGetLastError(), "kick_drift");
+}
+
+// Nothing acts between a step's kick and the next one's drift.
+bool drift_joins(const Context* c) {
+    return c->thermo_tau <= 0.0 && c->dyn_update <= 0 && !c->src_on && !c->range_on && !c->ttm && c->post_ops.empty() &&
+           !c->kick_fused;
 }
 
 static FinParams fin_params(Context* c, const IntParams& p, int count_step) {
@@ -480,7 +550,7 @@ void launch_ledger_finalize(Context* c, const KickArgs& ka, int nparts) {
     c->launches++;
 }
 
-static int reduce_and_finalize(Context* c, int kick, int count_step) {
+static int reduce_and_finalize(Context* c, int kick, int count_step, const DriftArgs* drift = nullptr) {
     if (kick && count_step && c->kick_fused) {  // the force kernel's epilogue took it
         c->kick_fused = false;
         return OMDG_OK;
@@ -514,19 +584,37 @@ static int reduce_and_finalize(Context* c, int kick, int count_step) {
     // up to 1,024 atoms in one block: no ticket, no partials (a step of 512
     // Tersoff atoms 30.1 us with two blocks of 256, 28.9 with one of 512)
     const int threads = c->n <= RED_BLOCK || c->n > 1024 ? RED_BLOCK : c->n <= 512 ? 512 : 1024;
-    auto kernel = threads == 512    ? (gather ? k_kick<true, 512> : k_kick<false, 512>)
-                  : threads == 1024 ? (gather ? k_kick<true, 1024> : k_kick<false, 1024>)
-                                    : (gather ? k_kick<true, RED_BLOCK> : k_kick<false, RED_BLOCK>);
-    kernel<<<threads == RED_BLOCK ? nb : 1, threads, 0, c->stream>>>(
-        p, f, slot_args(c, c->gather_zero_virial), c->vx, c->vy, c->vz, c->fx, c->fy, c->fz, c->f64, c->type, c->pe,
-        c->vir, c->flags_used ? c->aflag : nullptr, reinterpret_cast<BlockPartial*>(c->d_red), c->d_ledger,
-        reinterpret_cast<StepState*>(c->d_state), kick);
+    const int blocks = threads == RED_BLOCK ? nb : 1;
+    const auto launch = [&](auto kernel) {
+        kernel<<<blocks, threads, 0, c->stream>>>(
+            p, f, slot_args(c, c->gather_zero_virial), drift ? *drift : DriftArgs{}, c->vx, c->vy, c->vz, c->fx, c->fy,
+            c->fz, c->f64, c->type, c->pe, c->vir, c->flags_used ? c->aflag : nullptr,
+            reinterpret_cast<BlockPartial*>(c->d_red), c->d_ledger, reinterpret_cast<StepState*>(c->d_state), kick);
+    };
+    const auto sized = [&](auto g, auto dr) {
+        constexpr bool G = decltype(g)::value, DR = decltype(dr)::value;
+        if (threads == 512) launch(k_kick<G, DR, 512>);
+        else if (threads == 1024) launch(k_kick<G, DR, 1024>);
+        else launch(k_kick<G, DR, RED_BLOCK>);
+    };
+    const auto joined = [&](auto g) {
+        if (drift) sized(g, std::true_type{});
+        else sized(g, std::false_type{});
+    };
+    if (gather) joined(std::true_type{});
+    else joined(std::false_type{});
     prof_end(c);
     c->launches += 1;
     return check_cuda(c, cudaGetLastError(), "kick");
 }
 
 int integrate_kick(Context* c, int) { return reduce_and_finalize(c, 1, 1); }
+
+// The kick and the next step's kick_drift (drift_joins).
+int integrate_kick_and_drift(Context* c, const cudaGraphConditionalHandle* cond) {
+    const DriftArgs d = drift_args(c, cond);
+    return reduce_and_finalize(c, 1, 1, &d);
+}
 
 int measure_energies(Context* c, int) { return reduce_and_finalize(c, 0, 0); }
 

@@ -274,21 +274,16 @@ __device__ __forceinline__ void slot_sum(const SlotArgs& a, int i, float& fx, fl
     pe = ge.value();
 }
 
-// One atom's second half-kick v += dt/2 f/m (from ux, uy, uz, written back) and
+// One atom's second half-kick v += dt/2 f/m (of ux, uy, uz) and
 // its ledger terms: m v^2 and the potential and virial as FP32 pairs, the
 // squared speed's bits for DynamicTimeStep.  f is FP32 (the FP64 force path
 // does not fuse).
 __device__ __forceinline__ void kick_atom_terms(const IntParams& p, int i, int t, float fxi, float fyi, float fzi,
-                                                float pei, float viri, double h, double ux, double uy, double uz,
-                                                double* __restrict__ vx, double* __restrict__ vy,
-                                                double* __restrict__ vz, F2& k, F2& e, F2& w,
-                                                unsigned long long& vmax) {
+                                                float pei, float viri, double h, double& ux, double& uy, double& uz,
+                                                F2& k, F2& e, F2& w, unsigned long long& vmax) {
     ux = fma(f2d_exact(fxi), h, ux);
     uy = fma(f2d_exact(fyi), h, uy);
     uz = fma(f2d_exact(fzi), h, uz);
-    vx[i] = ux;
-    vy[i] = uy;
-    vz[i] = uz;
     const F2 sx = f2_from(ux), sy = f2_from(uy), sz = f2_from(uz);
     const F2 v2 = f2_add(f2_add(f2_mul(sx, sx), f2_mul(sy, sy)), f2_mul(sz, sz));
     k = f2_add(k, f2_mul(v2, F2{p.mh[t], p.ml[t]}));
@@ -307,15 +302,16 @@ __device__ __forceinline__ void kick_atom_terms(const IntParams& p, int i, int t
 // with a tree in every warp, fences around the ticket, the state's loads and
 // three FP64 divisions in the thread that had the sums; some 6,500 now with the
 // ticket and the partials, 3,800 without (one block).
+// True in the thread that finished, when that asked for a periodic rebuild.
 template <int T>
-__device__ __forceinline__ void ledger_block(LedgerSums<T>& s, const IntParams& p, const FinParams& f, F2 k, F2 e,
+__device__ __forceinline__ bool ledger_block(LedgerSums<T>& s, const IntParams& p, const FinParams& f, F2 k, F2 e,
                                              F2 w, unsigned long long vmax, BlockPartial* __restrict__ partial,
                                              double* __restrict__ ledger, StepState* st) {
     __shared__ bool last;
     s.add(k, e, w, vmax, p.need_vmax);
     if (gridDim.x == 1) {
         if (threadIdx.x == 0) s.finish(f, ledger, st);
-        return;
+        return threadIdx.x == 0 && s.rebuild;
     }
     if (threadIdx.x == 0) {
         const unsigned long long bv = s.largest(p.need_vmax);
@@ -329,6 +325,7 @@ __device__ __forceinline__ void ledger_block(LedgerSums<T>& s, const IntParams& 
     }
     __syncthreads();
     if (last) finalize_block<T>(s, f, gridDim.x, partial, ledger, st);
+    return last && threadIdx.x == 0 && s.rebuild;
 }
 
 // One warp's ledger partial (the per-warp half of ledger_block): lane 0

@@ -405,6 +405,8 @@ int zbl_launch(Context* c, Potential& p, bool first);
 
 // integrator (integrate.cu)
 int integrate_kick_drift(Context* c, const cudaGraphConditionalHandle* cond);
+bool drift_joins(const Context* c);  // the kick may take the next step's kick_drift
+int integrate_kick_and_drift(Context* c, const cudaGraphConditionalHandle* cond);
 int integrate_kick(Context* c, int step_index);
 int integrate_pack(Context* c);
 int measure_energies(Context* c, int row);

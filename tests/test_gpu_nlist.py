@@ -193,3 +193,39 @@ def test_ledger_of_one_block_and_several(omdg_lib, n):
         k, p = ctx.ledger_history(2)
     assert abs(k[-1] - 0.5 * mass * (st["v"] ** 2).sum()) <= 2.0 ** -40 * abs(k[-1])
     assert abs(p[-1] - st["pot"].astype(np.float64).sum()) <= 2.0 ** -40 * abs(p[-1])
+
+
+@pytest.mark.parametrize("kind,ncell,every", [("tersoff", 4, 0), ("tersoff", 17, 0), ("tersoff", 4, 5), ("tersoff", 17, 5),
+                                              ("sw", 5, 0), ("eam", 6, 0), ("eam", 22, 4)])
+def test_kick_and_drift_in_one_kernel(omdg_lib, kind, ncell, every):
+    """Without a thermostat the steps inside one graph join a step's kick and the
+    next one's drift: the same trajectory and ledger, bit for bit, as single
+    steps, with displacement and periodic rebuilds, in boxes of both forms."""
+    from objectmd_gb300 import inputs
+
+    if kind == "eam":
+        x, v, (lo, hi) = inputs.eam_aluminium(ncell=ncell, a=4.05, sigma=0.05, temp=900.0, seed_pos=3, seed_vel=4)
+    else:
+        x, v, (lo, hi) = inputs.diamond_silicon(ncell=ncell, a=5.431, sigma=0.05, temp=1500.0, seed_pos=3, seed_vel=4)
+    out = []
+    for calls in ([1] * 110, [70, 40], [66, 9, 8, 27]):
+        with omdg_lib.Context(0) as ctx:
+            ctx.set_box(lo, hi)
+            ctx.set_atoms(x, v, masses=[inputs.md_mass("aluminum" if kind == "eam" else "silicon")],
+                          znum=[13.0 if kind == "eam" else 14.0])
+            if kind == "eam":
+                ctx.add_eam(EAM_TABLE)
+            elif kind == "sw":
+                ctx.add_sw(os.path.join(TABLES, "sw.silicon"))
+            else:
+                ctx.add_tersoff(os.path.join(TABLES, "tersoff.silicon27"))
+            ctx.set_neighbor(SKIN, every)
+            ctx.set_timestep(0.001)
+            for k in calls:
+                ctx.step(k)
+            st = ctx.get_state()
+            out.append((st["x"], st["v"], st["f"], st["pot"], ctx.ledger()["energy"], ctx.ledger()["virial"],
+                        ctx.stats()["rebuilds"]))
+    assert out[0][-1] > 3
+    for o in out[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(o, out[0]))
