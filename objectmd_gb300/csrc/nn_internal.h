@@ -82,9 +82,9 @@ cudaError_t nn_mlp_launch(const NNDevNet& net, const float* gt, int rows, float*
                           int num_sms, cudaStream_t s);
 // The same network with each row's descriptors computed in the kernel from
 // the Verlet list (MD): flags atoms outside the training range and counts them.
-// std_ang: the descriptor set has the default angular layout.
+// layout: nn_layout of the descriptor set.
 struct NNMD;
-cudaError_t nn_mlp_md_launch(const NNDevNet& net, const NNMD& q, const NNDescParams& dp, bool std_ang,
+cudaError_t nn_mlp_md_launch(const NNDevNet& net, const NNMD& q, const NNDescParams& dp, int layout,
                              const PosPack* pack, const unsigned* nbr, const int* nnb, int* flag, int* count,
                              float* E, float* u, unsigned* status, int num_sms, cudaStream_t s);
 

@@ -27,8 +27,7 @@ struct NNState {
     int fallback = -1;     // index of the Tersoff potential in ctx->pots
 };
 
-// STD: the default angular layout (zeta and lambda constants of the term loop)
-template <bool STD>
+template <int LAYOUT>
 __global__ void __launch_bounds__(128) k_nn_md_desc(NNMD q, NNDescParams p, const PosPack* __restrict__ pack,
                                                     const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
                                                     float* __restrict__ Gt, int* __restrict__ flag, int* count,
@@ -36,7 +35,7 @@ __global__ void __launch_bounds__(128) k_nn_md_desc(NNMD q, NNDescParams p, cons
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= q.n) return;
     float g[NN_DESC];
-    nn_md_descriptors<STD>(q, p, i, pack, nbr, nnb[i], g, status);
+    nn_md_descriptors<LAYOUT>(q, p, i, pack, nbr, nnb[i], g, status);
     float4* dst = reinterpret_cast<float4*>(Gt + (size_t)i * NN_DESC);
 #pragma unroll
     for (int k = 0; k < NN_DESC; k += 4) {
@@ -82,16 +81,15 @@ __device__ __forceinline__ int nn_hits(const NNMD& q, int i, const PosPack& pi, 
     return nc;
 }
 
-// STD: the default angular layout with one eta a group (nn_grouped_angular).  It
-// holds the shared powers of both bases: 80 registers at six blocks per SM,
+// The default layout (NN_STD, NN_GROUPED) holds the shared powers of both bases: 80 registers at six blocks per SM,
 // where unbounded it takes 96 (five blocks).  Bound by its instructions: the
 // cutoffs of a neighbour once instead of once a pair, and what depends on eta
 // once a group, 512,000 atoms 112 -> 103 us with the same bits.  (Sums over the
 // powers first and the three derivatives of a pair from them take 78 us, but
 // the other rounding moves enough descriptors across a BF16 step to move the
 // forces by 2e-5 in ten steps.)
-template <bool STD>
-__global__ void __launch_bounds__(128, STD ? 6 : 7) k_nn_md_force(NNMD q, NNDescParams p, const PosPack* __restrict__ pack,
+template <int LAYOUT>
+__global__ void __launch_bounds__(128, LAYOUT != NN_ANY ? 6 : 7) k_nn_md_force(NNMD q, NNDescParams p, const PosPack* __restrict__ pack,
                                                      const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
                                                      const float* __restrict__ E, const float* __restrict__ U,
                                                      const int* __restrict__ flag, SlotRows slot,
@@ -150,7 +148,7 @@ __global__ void __launch_bounds__(128, STD ? 6 : 7) k_nn_md_force(NNMD q, NNDesc
 #pragma unroll
                 for (int mm = 0; mm < NN_ANG; mm++) {
                     float v, d_ra, d_rb, d_cs;
-                    nn_angular<STD, STD>(p, mm, rr[a], rr[b], cs, fa, dfa, fb, dfb, ex.get(p.eta_a[STD ? mm & 8 : mm], s2), v, d_ra,
+                    nn_angular<LAYOUT>(p, mm, rr[a], rr[b], cs, fa, dfa, fb, dfb, ex.get(nn_eta_a<LAYOUT>(p, mm), s2), v, d_ra,
                                     d_rb, d_cs);
                     const float w = u[NN_RAD + mm];
                     cra = fmaf(w, d_ra, cra);
@@ -232,18 +230,20 @@ int nn_launch(Context* c, Potential& pot, bool first) {
     const unsigned grid = (unsigned)grid_for(c->n, 128);
     const unsigned* nbr = reinterpret_cast<const unsigned*>(c->nbr);
     cudaMemsetAsync(s.count, 0, sizeof(int), c->stream);
-    const bool std_ang = nn_std_angular(s.model.dp);
+    const int layout = nn_layout(s.model.dp);
     cudaError_t e;
     if (c->nn_fused) {
         // descriptors computed by the network kernel's own threads
         prof_begin(c, "nn_desc_mlp");
-        e = nn_mlp_md_launch(s.net, q, s.model.dp, std_ang, c->pack, nbr, c->nnb, s.flag, s.count, s.E, s.U,
+        e = nn_mlp_md_launch(s.net, q, s.model.dp, layout, c->pack, nbr, c->nnb, s.flag, s.count, s.E, s.U,
                              c->d_status, c->num_sms, c->stream);
         prof_end(c);
         c->launches -= 1;
     } else {
         prof_begin(c, "nn_descriptors");
-        auto desc = std_ang ? k_nn_md_desc<true> : k_nn_md_desc<false>;
+        auto desc = layout == NN_GROUPED ? k_nn_md_desc<NN_GROUPED>
+                    : layout == NN_STD   ? k_nn_md_desc<NN_STD>
+                                         : k_nn_md_desc<NN_ANY>;
         desc<<<grid, 128, 0, c->stream>>>(q, s.model.dp, c->pack, nbr, c->nnb, s.Gt, s.flag, s.count, c->d_status);
         prof_end(c);
         prof_begin(c, "nn_mlp");
@@ -252,7 +252,9 @@ int nn_launch(Context* c, Potential& pot, bool first) {
     }
     if (e != cudaSuccess) return check_cuda(c, e, "surrogate network");
     prof_begin(c, "nn_force");
-    auto force = nn_grouped_angular(s.model.dp) ? k_nn_md_force<true> : k_nn_md_force<false>;
+    auto force = layout == NN_GROUPED ? k_nn_md_force<NN_GROUPED>
+                 : layout == NN_STD   ? k_nn_md_force<NN_STD>
+                                      : k_nn_md_force<NN_ANY>;
     force<<<grid, 128, 0, c->stream>>>(q, s.model.dp, c->pack, nbr, c->nnb, s.E, s.U, s.flag, slot_rows(c), c->fx,
                                        c->fy, c->fz, c->pe, c->vir, c->d_status);
     prof_end(c);
