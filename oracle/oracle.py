@@ -41,8 +41,8 @@ def build(force: bool = False) -> str:
 
 def build_reference(ref_root: str) -> bool:
     """Compile the reference sources found under ``ref_root`` (the Object-MD
-    source tree) into oracle/_ref; False where that tree is absent."""
-    if not ref_root or not os.path.isdir(ref_root):
+    source tree) into oracle/_ref; False where that tree is absent or empty."""
+    if not ref_root or not os.path.isdir(os.path.join(ref_root, "include")):
         return False
     subprocess.check_call(["make", "-s", "-C", os.path.join(HERE, "ref"), "REF=" + ref_root, "-j8"])
     return os.path.exists(REF_DRIVER)
