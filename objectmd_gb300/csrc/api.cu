@@ -266,7 +266,7 @@ struct GraphState {
     // GRAPH_STEPS steps in one graph, once enough steps were replayed one by one
     cudaGraphExec_t many_exec = nullptr;
     cudaGraph_t many_graph = nullptr;
-    bool many_valid = false;
+    bool many_valid = false, many_failed = false;
     int many_joined = 0;  // kernels fewer than as many single steps have
     long replayed = 0;
     // the same step with download branches into pinned host arrays
@@ -295,6 +295,7 @@ void invalidate_graph(Context* c) {
     gs.exec = gs.many_exec = gs.io_exec = nullptr;
     gs.graph = gs.many_graph = gs.io_graph = nullptr;
     gs.valid = gs.many_valid = gs.io_valid = false;
+    gs.many_failed = false;
     gs.replayed = 0;
 }
 }  // namespace omdg
@@ -1459,9 +1460,13 @@ int omdg_step_async(omdg_ctx* c, int nsteps) {
         if (!gs.valid) {
             if ((rc = capture_step(c, gs))) return rc;
         }
-        if (!gs.many_valid && nsteps >= GRAPH_STEPS && gs.replayed >= GRAPH_AFTER &&
-            (rc = capture_step(c, gs, nullptr, GRAPH_STEPS)))
-            return rc;
+        const std::string said = c->last_error;
+        if (!gs.many_valid && !gs.many_failed && nsteps >= GRAPH_STEPS && gs.replayed >= GRAPH_AFTER &&
+            capture_step(c, gs, nullptr, GRAPH_STEPS)) {
+            gs.many_failed = true;  // no room for it, say: the single steps go on
+            cudaGetLastError();
+            c->last_error = said;
+        }
         for (int k = 0; k < nsteps;) {
             const bool many = gs.many_valid && nsteps - k >= GRAPH_STEPS;
             cudaError_t e = cudaGraphLaunch(many ? gs.many_exec : gs.exec, c->stream);
