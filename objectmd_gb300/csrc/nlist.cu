@@ -9,10 +9,11 @@
 //   2 scan          exclusive scan of the counts -> cell starts
 //   3 scatter       atom -> slot in its cell
 //   4 cell_sort     sort each cell's slots by previous index (deterministic order)
-//   5 permute       reorder every per-atom array into cell order
-//   6 pack          FP32 hi/lo position packs + displacement reference
-//   7 build         full list, slot-major nbr[s*n+i]; FP32 screen, FP64 tie-break
-//   8 reverse       (three-body kernels) slot of i in each neighbour's row
+//   5 permute       reorder every per-atom array into cell order; position
+//                   packs, displacement reference, screening positions
+//                   (1 to 5 are k_sort_small in a small box or replica)
+//   6 build         full list, slot-major nbr[s*n+i]; FP32 screen, FP64 tie-break
+//   7 reverse       (three-body kernels) slot of i in each neighbour's row
 #include <algorithm>
 #include <cmath>
 
