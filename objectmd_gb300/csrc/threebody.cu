@@ -584,6 +584,144 @@ __global__ void __launch_bounds__(TB_BLOCK, TERS_CTAS_PER_SM) k_tersoff_a(
 // a b + c d rounded as the compiler contracts it in ters_bonds
 __device__ __forceinline__ float fma2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
 
+// The bonds of one centre in the lane form, NJ neighbours a lane: the slots are
+// written, and lane 0 to 4 return the centre's sums.  wide: more neighbours than
+// the register path holds; two of the sums are then rounded as a loop over arrays
+// contracts them, so that a trajectory through a collision stays the one that
+// such a loop gave.  With one neighbour a lane (a small box, where the chain of
+// one centre is all the time there is) the gradients of all bonds are kept, and
+// added up once at the end: centre pass of 512 atoms 11.9 -> 11.3 us with some 5
+// of launch.
+template <int NJ>
+__device__ __forceinline__ float ters_lanes_bonds(const TersDev& p, const LaneGroup& g, int i, int nc, bool wide,
+                                                  float g0, const float4* u, float4* f, float4* x, float2* ve,
+                                                  const int* sl, const SlotRows& slot) {
+    int2 to[NJ];  // the slots that the neighbours' forces go to, loaded beside the bonds
+#pragma unroll
+    for (int j = 0; j < NJ; j++) {
+        const int k = j * TB_LANES + g.lane;
+        if (k >= nc) continue;
+        const size_t at = nbr_at(i, sl[k], p.hshift, p.maxnb);
+        to[j] = make_int2(nbr_index(__ldg(slot.nbr + at)), __ldg(slot.rev + at));
+    }
+    float sjx[NJ], sjy[NJ], sjz[NJ], dz[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; j++) {
+        const int a = j * TB_LANES + g.lane;
+        if (a >= nc) continue;
+        const float4 ua = u[a], fa = f[a];
+        float zeta = 0.f, gjx = 0.f, gjy = 0.f, gjz = 0.f;
+#pragma unroll (NJ == 1 ? 4 : 1)
+        for (int b = 0; b < nc; b++) {
+            if (b == a) continue;
+            const float4 ub = u[b];
+            const float fb = f[b].x;
+            const float c = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
+            const float hc = p.h - c;
+            const float rden = __fdividef(1.f, p.d2 + hc * hc);
+            const float g = g0 - p.c2 * rden;
+            const float dg = -2.f * p.c2 * hc * rden * rden;
+            const float dr = ua.w - ub.w;
+            const float ex = __expf(p.l3c * dr * dr * dr);
+            const float dex = 3.f * p.l3c * dr * dr * ex;
+            zeta += fb * g * ex;
+            const float cj = fb * dg * ex * fa.z, cu = fb * g * dex;
+            gjx = __fadd_rn(gjx, wide ? fma2(cj, fmaf(-c, ua.x, ub.x), cu, ua.x)
+                                      : fma2(cu, ua.x, cj, fmaf(-c, ua.x, ub.x)));
+            gjy = __fadd_rn(gjy, wide ? fma2(cj, fmaf(-c, ua.y, ub.y), cu, ua.y)
+                                      : fma2(cu, ua.y, cj, fmaf(-c, ua.y, ub.y)));
+            gjz = __fadd_rn(gjz, wide ? fma2(cj, fmaf(-c, ua.z, ub.z), cu, ua.z)
+                                      : fma2(cu, ua.z, cj, fmaf(-c, ua.z, ub.z)));
+        }
+        const float fR = p.A * __expf(-p.l1 * ua.w), fA = p.B * __expf(-p.l2 * ua.w);
+        float bij, dbdz;
+        ters_bond_order(p, zeta, bij, dbdz);
+        const float vij = fa.x * (fR - bij * fA);
+        const float dv_dr = fma2(fa.y, fmaf(-bij, fA, fR), fa.x, fma2(bij * p.l2, fA, -p.l1, fR));
+        const float dv_dz = -fa.x * fA * dbdz;
+        sjx[j] = 0.5f * (wide ? fma2(dv_dz, gjx, dv_dr, ua.x) : fma2(dv_dr, ua.x, dv_dz, gjx));
+        sjy[j] = 0.5f * (wide ? fma2(dv_dz, gjy, dv_dr, ua.y) : fma2(dv_dr, ua.y, dv_dz, gjy));
+        sjz[j] = 0.5f * (wide ? fma2(dv_dz, gjz, dv_dr, ua.z) : fma2(dv_dr, ua.z, dv_dz, gjz));
+        dz[j] = 0.5f * dv_dz;
+        ve[a] = make_float2(vij, dv_dr);
+    }
+    __syncwarp(g.mask);
+#pragma unroll
+    for (int j = 0; j < NJ; j++) {
+        const int a = j * TB_LANES + g.lane;
+        if (a < nc) f[a].w = dz[j];
+    }
+    __syncwarp(g.mask);
+    float skx[NJ], sky[NJ], skz[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; j++) skx[j] = sky[j] = skz[j] = 0.f;
+    float own = 0.f;  // lane 0 to 4: the centre's x, y, z, energy and virial, in the register path's order
+    const auto add = [&](int a, float s, const float4* row) {
+        if (g.lane < 3) {
+            const float* xc = &row[0].x + g.lane;
+            own += xc[4 * a];  // the x_i gradient is minus the sum of the others
+            for (int b = 0; b < nc; b++)
+                if (b != a) own = fmaf(s, xc[4 * b], own);
+        } else if (g.lane == 3) {
+            own += 0.5f * ve[a].x;
+        } else if (g.lane == 4) {
+            own += 0.5f * ve[a].y * u[a].w;
+        }
+    };
+#pragma unroll (NJ == 1 ? 2 : 1)
+    for (int a = 0; a < nc; a++) {
+        float4* const row = NJ == 1 ? x + a * TB_LANES : x;
+        const float4 ua = u[a];
+        const float s = f[a].w;
+#pragma unroll
+        for (int j = 0; j < NJ; j++) {
+            const int k = j * TB_LANES + g.lane;
+            if (k >= nc) continue;
+            if (k == a) {
+                row[k] = make_float4(sjx[j], sjy[j], sjz[j], 0.f);
+                skx[j] -= sjx[j];
+                sky[j] -= sjy[j];
+                skz[j] -= sjz[j];
+                continue;
+            }
+            const float4 uk = u[k], fk = f[k];
+            const float c = ua.x * uk.x + ua.y * uk.y + ua.z * uk.z;
+            const float hc = p.h - c;
+            const float rden = __fdividef(1.f, p.d2 + hc * hc);
+            const float g = g0 - p.c2 * rden;
+            const float dg = -2.f * p.c2 * hc * rden * rden;
+            const float dr = ua.w - uk.w;
+            const float ex = __expf(p.l3c * dr * dr * dr);
+            const float dex = 3.f * p.l3c * dr * dr * ex;
+            const float ck = fma2(fk.y * g, ex, -fk.x * g, dex);
+            const float cc = fk.x * dg * ex * fk.z;
+            const float kx = fma2(ck, uk.x, cc, fmaf(-c, uk.x, ua.x));
+            const float ky = fma2(ck, uk.y, cc, fmaf(-c, uk.y, ua.y));
+            const float kz = fma2(ck, uk.z, cc, fmaf(-c, uk.z, ua.z));
+            row[k] = make_float4(kx, ky, kz, 0.f);
+            // force on k = -gradient
+            skx[j] = fmaf(-s, kx, skx[j]);
+            sky[j] = fmaf(-s, ky, sky[j]);
+            skz[j] = fmaf(-s, kz, skz[j]);
+        }
+        if (NJ > 1) {
+            __syncwarp(g.mask);
+            add(a, s, row);
+            __syncwarp(g.mask);
+        }
+    }
+    if (NJ == 1) {
+        __syncwarp(g.mask);
+        for (int a = 0; a < nc; a++) add(a, f[a].w, x + a * TB_LANES);
+    }
+#pragma unroll
+    for (int j = 0; j < NJ; j++) {
+        const int k = j * TB_LANES + g.lane;
+        if (k < nc) slot.at(to[j].x, to[j].y) = make_float4(skx[j], sky[j], skz[j], 0.f);
+    }
+    return own;
+}
+
 // Eight lanes a centre: the queued centres (wide[0] of them, indices from
 // wide[1]), or all of them (then the ones past the register path are still
 // counted).  A lane owns a neighbour: its bond's zeta and gradient first, then
@@ -601,10 +739,9 @@ __global__ void __launch_bounds__(TB_LBLOCK) k_tersoff_lanes(
     float* __restrict__ fz, float* __restrict__ pe, float* __restrict__ vir, unsigned* status) {
     __shared__ float4 gu[TB_LGROUPS][TB_MAXN];  // vector and squared distance, then unit vector and distance
     __shared__ float4 gf[TB_LGROUPS][TB_MAXN];  // f_c, f_c', 1/r, half the bond's dV/dzeta
-    __shared__ float4 gx[TB_LGROUPS][TB_MAXN];  // one bond's gradients by its neighbours
+    __shared__ float4 gx[TB_LGROUPS][QUEUED ? TB_MAXN : TB_LANES * TB_LANES];  // the bonds' gradients by the neighbours
     __shared__ float2 ge[TB_LGROUPS][TB_MAXN];  // a bond's energy and its derivative by r
     __shared__ int gs[TB_LGROUPS][TB_MAXN];
-    constexpr int NJ = TB_MAXN / TB_LANES;
     const LaneGroup g;
     float4* u = gu[threadIdx.x / TB_LANES];
     float4* f = gf[threadIdx.x / TB_LANES];
@@ -636,106 +773,9 @@ __global__ void __launch_bounds__(TB_LBLOCK) k_tersoff_lanes(
             f[a] = make_float4(fc, dfc, ri, 0.f);
         }
         __syncwarp(g.mask);
-        float sjx[NJ], sjy[NJ], sjz[NJ], dz[NJ];
-#pragma unroll
-        for (int j = 0; j < NJ; j++) {
-            const int a = j * TB_LANES + g.lane;
-            if (a >= nc) continue;
-            const float4 ua = u[a], fa = f[a];
-            float zeta = 0.f, gjx = 0.f, gjy = 0.f, gjz = 0.f;
-            for (int b = 0; b < nc; b++) {
-                if (b == a) continue;
-                const float4 ub = u[b];
-                const float fb = f[b].x;
-                const float c = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
-                const float hc = p.h - c;
-                const float rden = __fdividef(1.f, p.d2 + hc * hc);
-                const float g = g0 - p.c2 * rden;
-                const float dg = -2.f * p.c2 * hc * rden * rden;
-                const float dr = ua.w - ub.w;
-                const float ex = __expf(p.l3c * dr * dr * dr);
-                const float dex = 3.f * p.l3c * dr * dr * ex;
-                zeta += fb * g * ex;
-                const float cj = fb * dg * ex * fa.z, cu = fb * g * dex;
-                gjx = __fadd_rn(gjx, fma2(cu, ua.x, cj, fmaf(-c, ua.x, ub.x)));
-                gjy = __fadd_rn(gjy, fma2(cu, ua.y, cj, fmaf(-c, ua.y, ub.y)));
-                gjz = __fadd_rn(gjz, fma2(cu, ua.z, cj, fmaf(-c, ua.z, ub.z)));
-            }
-            const float fR = p.A * __expf(-p.l1 * ua.w), fA = p.B * __expf(-p.l2 * ua.w);
-            float bij, dbdz;
-            ters_bond_order(p, zeta, bij, dbdz);
-            const float vij = fa.x * (fR - bij * fA);
-            const float dv_dr = fma2(fa.y, fmaf(-bij, fA, fR), fa.x, fma2(bij * p.l2, fA, -p.l1, fR));
-            const float dv_dz = -fa.x * fA * dbdz;
-            sjx[j] = 0.5f * fma2(dv_dr, ua.x, dv_dz, gjx);
-            sjy[j] = 0.5f * fma2(dv_dr, ua.y, dv_dz, gjy);
-            sjz[j] = 0.5f * fma2(dv_dr, ua.z, dv_dz, gjz);
-            dz[j] = 0.5f * dv_dz;
-            ve[a] = make_float2(vij, dv_dr);
-        }
-        __syncwarp(g.mask);
-#pragma unroll
-        for (int j = 0; j < NJ; j++) {
-            const int a = j * TB_LANES + g.lane;
-            if (a < nc) f[a].w = dz[j];
-        }
-        __syncwarp(g.mask);
-        float skx[NJ], sky[NJ], skz[NJ];
-#pragma unroll
-        for (int j = 0; j < NJ; j++) skx[j] = sky[j] = skz[j] = 0.f;
-        float own = 0.f;  // lane 0 to 4: the centre's x, y, z, energy and virial, in the register path's order
-        for (int a = 0; a < nc; a++) {
-            const float4 ua = u[a];
-            const float s = f[a].w;
-#pragma unroll
-            for (int j = 0; j < NJ; j++) {
-                const int k = j * TB_LANES + g.lane;
-                if (k >= nc) continue;
-                if (k == a) {
-                    x[k] = make_float4(sjx[j], sjy[j], sjz[j], 0.f);
-                    skx[j] -= sjx[j];
-                    sky[j] -= sjy[j];
-                    skz[j] -= sjz[j];
-                    continue;
-                }
-                const float4 uk = u[k], fk = f[k];
-                const float c = ua.x * uk.x + ua.y * uk.y + ua.z * uk.z;
-                const float hc = p.h - c;
-                const float rden = __fdividef(1.f, p.d2 + hc * hc);
-                const float g = g0 - p.c2 * rden;
-                const float dg = -2.f * p.c2 * hc * rden * rden;
-                const float dr = ua.w - uk.w;
-                const float ex = __expf(p.l3c * dr * dr * dr);
-                const float dex = 3.f * p.l3c * dr * dr * ex;
-                const float ck = fma2(fk.y * g, ex, -fk.x * g, dex);
-                const float cc = fk.x * dg * ex * fk.z;
-                const float kx = fma2(ck, uk.x, cc, fmaf(-c, uk.x, ua.x));
-                const float ky = fma2(ck, uk.y, cc, fmaf(-c, uk.y, ua.y));
-                const float kz = fma2(ck, uk.z, cc, fmaf(-c, uk.z, ua.z));
-                x[k] = make_float4(kx, ky, kz, 0.f);
-                // force on k = -gradient
-                skx[j] = fmaf(-s, kx, skx[j]);
-                sky[j] = fmaf(-s, ky, sky[j]);
-                skz[j] = fmaf(-s, kz, skz[j]);
-            }
-            __syncwarp(g.mask);
-            if (g.lane < 3) {
-                const float* xc = &x[0].x + g.lane;
-                own += xc[4 * a];  // the x_i gradient is minus the sum of the others
-                for (int b = 0; b < nc; b++)
-                    if (b != a) own = fmaf(s, xc[4 * b], own);
-            } else if (g.lane == 3) {
-                own += 0.5f * ve[a].x;
-            } else if (g.lane == 4) {
-                own += 0.5f * ve[a].y * ua.w;
-            }
-            __syncwarp(g.mask);
-        }
-#pragma unroll
-        for (int j = 0; j < NJ; j++) {
-            const int k = j * TB_LANES + g.lane;
-            if (k < nc) slot.put(i, sl[k], make_float4(skx[j], sky[j], skz[j], 0.f));
-        }
+        const float own = !QUEUED && nc <= TB_LANES
+                              ? ters_lanes_bonds<1>(p, g, i, nc, nc > TERS_REG, g0, u, f, x, ve, sl, slot)
+                              : ters_lanes_bonds<TB_MAXN / TB_LANES>(p, g, i, nc, true, g0, u, f, x, ve, sl, slot);
         __syncwarp(g.mask);  // the group's neighbours are read: the next centre may overwrite them
         if (g.lane < 5) {
             float* out = g.lane == 0 ? fx : g.lane == 1 ? fy : g.lane == 2 ? fz : g.lane == 3 ? pe : vir;
