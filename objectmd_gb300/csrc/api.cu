@@ -947,12 +947,14 @@ int forces_compute(Context* c) {
     c->gather_deferred = false;
     if (!c->fuse_kick) c->wide_cleared = false;  // not a step's evaluation
     bool first = true;
-    // in a step the last slot gather joins the kick, unless a modify or the
-    // detector works on the forces in between
+    // in a step the last potential's slot gather joins the kick, unless a modify
+    // or the detector works on the forces in between (a potential after it would
+    // be added before the slots instead of after them: another rounding)
     const Potential* last_slots = nullptr;
     if (c->fuse_kick && !c->use_f64 && c->post_ops.empty() && !c->ttm)
         for (auto& p : c->pots)
-            if (!p.fallback_only && (p.kind == POT_SW || p.kind == POT_TERSOFF || p.kind == POT_NN)) last_slots = &p;
+            if (!p.fallback_only)
+                last_slots = p.kind == POT_SW || p.kind == POT_TERSOFF || p.kind == POT_NN ? &p : nullptr;
     for (auto& p : c->pots) {
         if (p.fallback_only) continue;  // run by the potential that owns it
         c->defer_gather = &p == last_slots;

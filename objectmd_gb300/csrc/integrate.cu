@@ -146,14 +146,13 @@ __global__ void __launch_bounds__(256, 8) k_kick_drift(IntParams p, DriftArgs d,
 // took 29.0 us, at four 24.8).
 // GATHER: the three-body kernels' slots are collected first (slot_sum), their
 // loads' latency beside the half-kick's: 512,000 Tersoff atoms 32.9 us at six
-// blocks a SM and 24.4 at four, 194,184 Stillinger-Weber atoms 27.0 and 20.8,
-// 1.47 M atoms of the impact ensemble 70 and 56.
+// blocks a SM and 24.4 at four, 194,184 Stillinger-Weber atoms 27.0 and 20.8.
 // DRIFT: the next step's first half-kick and drift follow at once (same force,
 // and no thermostat factor or new time step in between), so the velocity is read
 // and written once, and the force not at all: for the steps inside one graph.
 // A step of eight in a graph with the kernels apart and joined, us: 256,000 EAM
 // atoms 178.8 and 175.7, 194,184 Stillinger-Weber atoms 108.9 and 104.8, 512,000
-// Tersoff atoms 114.3 and 111.6, the impact ensemble 400.6 and 382.7.
+// Tersoff atoms 114.3 and 111.6.
 template <bool GATHER, bool DRIFT, int T>
 __global__ void __launch_bounds__(T, T == RED_BLOCK ? KICK_BLOCKS_SM : 1) k_kick(
     IntParams p, FinParams f, SlotArgs ga, DriftArgs d, double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,

@@ -586,8 +586,8 @@ __device__ __forceinline__ float fma2(float a, float b, float c, float d) { retu
 
 // The bonds of one centre in the lane form, NJ neighbours a lane: the slots are
 // written, and lane 0 to 4 return the centre's sums.  wide: more neighbours than
-// the register path holds; two of the sums are then rounded as a loop over arrays
-// contracts them, so that a trajectory through a collision stays the one that
+// the register path holds; gjx and the neighbour's part are then rounded as a loop
+// over arrays contracts them, so that a trajectory through a collision stays the one that
 // such a loop gave.  With one neighbour a lane (a small box, where the chain of
 // one centre is all the time there is) the gradients of all bonds are kept, and
 // added up once at the end: centre pass of 512 atoms 11.9 -> 11.3 us with some 5
@@ -628,10 +628,8 @@ __device__ __forceinline__ float ters_lanes_bonds(const TersDev& p, const LaneGr
             const float cj = fb * dg * ex * fa.z, cu = fb * g * dex;
             gjx = __fadd_rn(gjx, wide ? fma2(cj, fmaf(-c, ua.x, ub.x), cu, ua.x)
                                       : fma2(cu, ua.x, cj, fmaf(-c, ua.x, ub.x)));
-            gjy = __fadd_rn(gjy, wide ? fma2(cj, fmaf(-c, ua.y, ub.y), cu, ua.y)
-                                      : fma2(cu, ua.y, cj, fmaf(-c, ua.y, ub.y)));
-            gjz = __fadd_rn(gjz, wide ? fma2(cj, fmaf(-c, ua.z, ub.z), cu, ua.z)
-                                      : fma2(cu, ua.z, cj, fmaf(-c, ua.z, ub.z)));
+            gjy = __fadd_rn(gjy, fma2(cu, ua.y, cj, fmaf(-c, ua.y, ub.y)));
+            gjz = __fadd_rn(gjz, fma2(cu, ua.z, cj, fmaf(-c, ua.z, ub.z)));
         }
         const float fR = p.A * __expf(-p.l1 * ua.w), fA = p.B * __expf(-p.l2 * ua.w);
         float bij, dbdz;
