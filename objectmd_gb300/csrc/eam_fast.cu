@@ -54,20 +54,19 @@ __device__ __forceinline__ int4 ld_ipos(const int4* p) {
     return v;
 }
 
-// x_i - x_j of the nearest images from the fixed-point positions (fix_coord).
-// The step's low part keeps its rounding from scaling every length alike.
-__device__ __forceinline__ float3 fix_delta(const EAMFast& p, const int4& a, const int4& b) {
-    const float x = (float)(a.x - b.x), y = (float)(a.y - b.y), z = (float)(a.z - b.z);
-    return make_float3(fmaf(x, p.qh[0], x * p.ql[0]), fmaf(y, p.qh[1], y * p.ql[1]), fmaf(z, p.qh[2], z * p.ql[2]));
+// steps q of an axis as a length, rounded once: both halves of q are exact in
+// FP32, and the step is an FP32 pair (one number would scale all lengths alike).
+// The result is the FP32 rounding of the difference, as pair_delta's is but where
+// the quantisation, a hundredth of that rounding, moves it across.
+__device__ __forceinline__ float fix_length(int q, float qh, float ql) {
+    const float h = (float)(q & ~0xfff), l = (float)(q & 0xfff);
+    return fmaf(h, qh, fmaf(l, qh, h * ql));
 }
 
-// r and 1/r from r2: the approximate root with one Newton step each.
-__device__ __forceinline__ float root(float r2, float& rinv) {
-    rinv = rsqrtf(r2);
-    float r = r2 * rinv;
-    r = fmaf(fmaf(-r, r, r2), 0.5f * rinv, r);
-    rinv = fmaf(fmaf(-r, rinv, 1.f), rinv, rinv);
-    return r;
+// x_i - x_j of the nearest images from the fixed-point positions (fix_coord).
+__device__ __forceinline__ float3 fix_delta(const EAMFast& p, const int4& a, const int4& b) {
+    return make_float3(fix_length(a.x - b.x, p.qh[0], p.ql[0]), fix_length(a.y - b.y, p.qh[1], p.ql[1]),
+                       fix_length(a.z - b.z, p.qh[2], p.ql[2]));
 }
 
 __device__ __forceinline__ void build_shift_table(const EAMFast& p, float4* s_hi, float4* s_lo) {
@@ -184,19 +183,20 @@ __device__ __forceinline__ void gather_density_sum(const EAMFast& p, const PosPa
 // The same from the fixed-point positions: half the bytes a neighbour (from the
 // packs both passes were at 75 % of the L1's data path) and no image shift to
 // look up or add.  What bounds them now is the latency of the chain from entry
-// to position to knot: a lane holds few entries ahead, so that more warps fit
-// (density, 256,000 atoms: 16 entries and four blocks a SM 64.1 us, 16 and six
-// 59.2, four and six 54.3; force: 16 and four 69.7, eight and four 65.1, eight
-// and five 69.6).  Packs and fixed point, us, 256,000 atoms: density 72.5 and
-// 55.7, force 85.7 and 66.8; 1,048,576 (two lanes an atom): 264 and 189, 329
-// and 243.  One Newton step each for the root and its reciprocal leaves the
-// forces nearer to FP64 than the packs with the bare approximation did.
+// to position to knot, and issue: a lane holds few entries ahead, so that more
+// warps fit (density, 256,000 atoms: four entries ahead and six blocks a SM
+// 58.6 us, five blocks 64.3; force: eight and four 70.6, four and four 74.6, eight
+// and five 75.2).  Packs and fixed point, us, 256,000 atoms: density 72.5 and
+// 58.6, force 85.7 and 70.6; 1,048,576 (two lanes an atom): 264 and 207, 329
+// and 256.  (Lengths rounded twice and a Newton step for the root take 55.7 and
+// 66.8, with a smaller error, but leave a trajectory four times as far from the
+// packs'.)
 constexpr int FIX_AHEAD_DENSITY = 4, FIX_CTAS_DENSITY = 6;
 constexpr int FIX_AHEAD_FORCE = 8, FIX_CTAS_FORCE = 4;
 constexpr int FIX_TWO_LANES_PER_SM = 3000;
 // Below this many atoms a SM launches and latency are all, and the packs serve
 // as well (both passes, us: 16,384 atoms 28.1 and 27.4, 32,000 34.8 and 30.6,
-// 55,296 52.5 and 40.1).
+// 55,296 52.5 and 40.1, before the lengths' second half).
 constexpr int FIX_PER_SM = 128;
 
 template <int LANES>
@@ -223,8 +223,7 @@ __device__ __forceinline__ void fixed_density_sum(const EAMFast& p, const int4* 
             xj = xn;
             const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
             if (r2 > rc2) continue;
-            float rinv;
-            const float r = root(r2, rinv);
+            const float r = r2 * rsqrtf(r2);
             if (!(r <= p.rc_rho)) continue;
             float dx;
             const int x = knot_of(p, r, offdr, dx);
@@ -405,8 +404,8 @@ __device__ __forceinline__ void fixed_force_sum(const EAMFast& p, const int4* __
             xj = xn;
             const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
             if (r2 > p.rc2) continue;
-            float rinv;
-            const float r = root(r2, rinv);
+            const float rinv = rsqrtf(r2);
+            const float r = r2 * rinv;
             if (!(r <= p.rc_phi)) continue;
             float dx;
             const int x = knot_of(p, r, offdr, dx);
@@ -946,7 +945,7 @@ int eam_fast_launch(Context* c, Potential& pot, bool first) {
     int block = c->eam_block > 256 ? 256 : c->eam_block, lanes = c->eam_lanes;
     // a large box fills the chip with two lanes an atom, and reduces less:
     // density and force of 1,048,576 atoms 197 and 252 us with four, 188 and 236
-    // with two; of 256,000 54 and 65, 58 and 64
+    // with two; of 256,000 54 and 65, 58 and 64 (before the lengths' second half)
     if (fixed && !c->eam_lanes_set && c->n >= FIX_TWO_LANES_PER_SM * c->num_sms) lanes = 2;
     int per_block = block / lanes;
     int grid = grid_for(c->n, per_block);
