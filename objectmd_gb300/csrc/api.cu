@@ -184,7 +184,7 @@ static void free_atoms(Context* c) {
                     c->id,   c->inv,   c->fp,     c->femb,   c->cell,        c->perm,        c->stage_d,
                     c->stage_i, c->f64, c->extra, c->stage_extra, c->nnb, c->d_red, c->aflag,
                     c->snap_d, c->snap_i,
-                    c->ters_wide, c->nbmask, c->cell_sorted, c->ipos};
+                    c->ters_wide, c->nbmask, c->cell_sorted};
     for (void* p : ptrs) cudaFree(p);
     c->x = c->y = c->z = c->vx = c->vy = c->vz = nullptr;
     c->fx = c->fy = c->fz = c->pe = c->vir = nullptr;
@@ -193,7 +193,6 @@ static void free_atoms(Context* c) {
     c->loc = nullptr;
     c->nbmask = nullptr;
     c->cell_sorted = nullptr;
-    c->ipos = nullptr;
     c->type = c->id = c->inv = c->ters_wide = nullptr;
     c->fp = c->femb = nullptr;
     c->cell = c->perm = nullptr;
@@ -891,7 +890,6 @@ static int build_list(Context* c) {
     if (c->pots.empty()) return set_error(c, OMDG_ESTATE, "no force kernel (integrator.cpp:79)");
     nlist_prepare_geometry(c);
     if (int rt = tile_prepare(c)) return rt;
-    fix_prepare(c);
     if (c->nrep > 0) {
         if (c->rep_start.back() != c->n) return set_error(c, OMDG_ESTATE, "replica atom counts do not sum to n");
         int rc = replica_prepare(c);
@@ -2002,10 +2000,6 @@ int omdg_set_launch(omdg_ctx* c, const char* key, int value) {
     int* p = launch_knob(c, k);
     if (!p) return set_error(c, OMDG_EINVAL, "unknown launch key " + k);
     if (!valid_knob(k, value)) return set_error(c, OMDG_EINVAL, "invalid value for " + k);
-    if (k == "eam_lanes" && !c->eam_lanes_set) {  // the default gives way to a rule by size
-        c->eam_lanes_set = true;
-        invalidate_graph(c);
-    }
     if (*p == value) return OMDG_OK;
     *p = value;
     // the build writes tile slots for the tile shape and capacity it sees
@@ -2093,7 +2087,6 @@ int omdg_autotune(omdg_ctx* c, int reps, double* best_ms) {
         while ((1 << hs) * cd.lanes < 32 && hs < 5) hs++;
         if (eam) {
             c->eam_lanes = cd.lanes;
-            c->eam_lanes_set = true;
             c->eam_block = cd.block;
             c->eam_stage = cd.stage;
             c->eam_ctas_per_sm = cd.block >= 512 ? 2 : 4;
@@ -2123,7 +2116,6 @@ int omdg_autotune(omdg_ctx* c, int reps, double* best_ms) {
     while ((1 << hs) * win.lanes < 32 && hs < 5) hs++;
     if (eam) {
         c->eam_lanes = win.lanes;
-        c->eam_lanes_set = true;
         c->eam_block = win.block;
         c->eam_stage = win.stage;
         c->eam_ctas_per_sm = win.block >= 512 ? 2 : 4;

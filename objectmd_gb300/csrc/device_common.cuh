@@ -320,23 +320,6 @@ __device__ __forceinline__ void pack_coord(double x, float qh, float ql, float& 
     lo = __fsub_rn(t, __fsub_rn(hi, s.hi));
 }
 
-// A position as a multiple of (period / 2^32), modulo the period: the
-// difference of two such words, as a signed 32-bit number, is the separation
-// of the nearest images, with no image shift to look up or add.  The period is
-// a whole fraction of a periodic axis' length (any on a free axis) of at least
-// twice the list range, so nearest is the listed image; the step, at most
-// range / 10^9, is a hundredth of the FP32 rounding of a bond's length.
-// x S + C puts the integer into the low mantissa bits (C holds 1.5 2^52).
-__device__ __forceinline__ int fix_coord(double x, double S, double C, double range) {
-    if ((__double2hiint(x) & 0x7fffffff) >= 0x41100000) x -= range * rint(x / range);  // |x| >= 2^18: keep |x S| small
-    return __double2loint(fma(x, S, C));
-}
-
-__device__ __forceinline__ int4 fix_pos(double x, double y, double z, const FixFrame& f) {
-    return make_int4(fix_coord(x, f.S[0], f.C[0], f.range[0]), fix_coord(y, f.S[1], f.C[1], f.range[1]),
-                     fix_coord(z, f.S[2], f.C[2], f.range[2]), 0);
-}
-
 __device__ __forceinline__ F2 f2_from(double x) {
     F2 r;
     split_bits(x, r.hi, r.lo);

@@ -8,9 +8,7 @@
 //   - a neighbour's position pack (with F'(rho) in its spare word) and an
 //     interleaved (phi, rho) knot are one 256-bit load each,
 //   - the periodic image comes from a 64-entry shared table of split shift
-//     vectors indexed by the entry's 6 image bits,
-//   - boxes three list ranges long read fixed-point positions instead
-//     (fixed_density_sum), and need no shift,
+//     vectors indexed by the entry's 6 image bits (where they name one),
 //   - the knot index is clamped instead of branched (r <= rc keeps it below
 //     n-1; the reference's x == n-1 rule selects the same segment),
 //   - forces use Kahan sums, the per-pair energy and virial plain FP32 sums.
@@ -44,30 +42,7 @@ struct EAMFast {
     int stage_k0, stage_n;
     int first;
     int src_phi, src_rho, src_emb;  // table ids for error reports (DevTable::src)
-    float qh[3], ql[3];             // fixed-point step (FixFrame)
 };
-
-// 128-bit coherent load: the density pass writes the w words beside it.
-__device__ __forceinline__ int4 ld_ipos(const int4* p) {
-    int4 v;
-    asm volatile("ld.global.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-
-// steps q of an axis as a length, rounded once: both halves of q are exact in
-// FP32, and the step is an FP32 pair (one number would scale all lengths alike).
-// The result is the FP32 rounding of the difference, as pair_delta's is but where
-// the quantisation, a hundredth of that rounding, moves it across.
-__device__ __forceinline__ float fix_length(int q, float qh, float ql) {
-    const float h = (float)(q & ~0xfff), l = (float)(q & 0xfff);
-    return fmaf(h, qh, fmaf(l, qh, h * ql));
-}
-
-// x_i - x_j of the nearest images from the fixed-point positions (fix_coord).
-__device__ __forceinline__ float3 fix_delta(const EAMFast& p, const int4& a, const int4& b) {
-    return make_float3(fix_length(a.x - b.x, p.qh[0], p.ql[0]), fix_length(a.y - b.y, p.qh[1], p.ql[1]),
-                       fix_length(a.z - b.z, p.qh[2], p.ql[2]));
-}
 
 __device__ __forceinline__ void build_shift_table(const EAMFast& p, float4* s_hi, float4* s_lo) {
     for (int k = threadIdx.x; k < 64; k += blockDim.x) {
@@ -79,14 +54,26 @@ __device__ __forceinline__ void build_shift_table(const EAMFast& p, float4* s_hi
 }
 
 // d = x_i - (x_j + s L) with the shift from the table (exact hi differences,
-// see pair_delta in device_common.cuh).
+// see pair_delta in device_common.cuh).  Most entries of a large box have no
+// shift, and subtracting its zeros would change nothing: they skip the table's
+// two 16-byte loads.
+constexpr unsigned NO_SHIFT = 1u | 1u << 2 | 1u << 4;  // the image bits of (0, 0, 0)
+
 __device__ __forceinline__ float3 delta_tab(const float4& hi, const float4& lo, const float4& hj, const float4& lj,
-                                            const float4& sh, const float4& sl) {
-    float3 d;
-    d.x = __fadd_rn(__fsub_rn(__fsub_rn(hi.x, hj.x), sh.x), __fsub_rn(__fsub_rn(lo.x, lj.x), sl.x));
-    d.y = __fadd_rn(__fsub_rn(__fsub_rn(hi.y, hj.y), sh.y), __fsub_rn(__fsub_rn(lo.y, lj.y), sl.y));
-    d.z = __fadd_rn(__fsub_rn(__fsub_rn(hi.z, hj.z), sh.z), __fsub_rn(__fsub_rn(lo.z, lj.z), sl.z));
-    return d;
+                                            unsigned ent, const float4* s_hi, const float4* s_lo) {
+    float ax = __fsub_rn(hi.x, hj.x), ay = __fsub_rn(hi.y, hj.y), az = __fsub_rn(hi.z, hj.z);
+    float bx = __fsub_rn(lo.x, lj.x), by = __fsub_rn(lo.y, lj.y), bz = __fsub_rn(lo.z, lj.z);
+    const unsigned code = ent >> 26;
+    if (code != NO_SHIFT) {
+        const float4 sh = s_hi[code], sl = s_lo[code];
+        ax = __fsub_rn(ax, sh.x);
+        ay = __fsub_rn(ay, sh.y);
+        az = __fsub_rn(az, sh.z);
+        bx = __fsub_rn(bx, sl.x);
+        by = __fsub_rn(by, sl.y);
+        bz = __fsub_rn(bz, sl.z);
+    }
+    return make_float3(__fadd_rn(ax, bx), __fadd_rn(ay, by), __fadd_rn(az, bz));
 }
 
 template <int LANES>
@@ -110,15 +97,20 @@ __device__ __forceinline__ float plain_reduce(float v) {
     return v;
 }
 
-// Entries a lane prefetches into registers per pass over its row (packs).
-template <int LANES>
-struct Prefetch {
-    static constexpr int N = LANES >= 4 ? 64 / LANES : 16;
-};
+// Entries a lane holds in registers ahead of the one it evaluates: eight, so
+// that five blocks of the density pass fit a SM and the force pass spills
+// nothing (sixteen where the knots are staged).  Both passes are bound by the
+// L1's data path, 32 bytes a neighbour beside its knots, and by issue.
+// Density and force, us: 256,000 atoms 68.4 and 77.1, 1,048,576 247 and 295;
+// with sixteen ahead, four blocks and every entry's image shift loaded 73.2 and
+// 86.0, 267 and 331; four ahead 72.6 and 81.4; six blocks of the density pass
+// 83.3, five of the force pass 89.0 (256,000 atoms).
+constexpr int eam_ahead(int lanes, bool staged) { return lanes >= 8 ? 64 / lanes : (staged ? 16 : 8); }
+constexpr int DENSITY_CTAS = 5, FORCE_CTAS = 4;
 
 // Staged variants hold the knot window in shared memory (up to ~110 KB) and
 // run two 512-thread CTAs per SM, so 32 warps hide the gathers' latency.
-#define EAMF_BOUNDS(STAGED, N) __launch_bounds__((STAGED) ? 512 : 256, (STAGED) ? 2 : (N))
+#define EAMF_BOUNDS(STAGED, CTAS) __launch_bounds__((STAGED) ? 512 : 256, (STAGED) ? 2 : (CTAS))
 
 // Index of the rho knot below r, or -1 when r is closer than the first knot
 // (outside every tabulated range here).
@@ -137,7 +129,7 @@ __device__ __forceinline__ void gather_density_sum(const EAMFast& p, const PosPa
                                                    const unsigned* __restrict__ nbr, int ii, int m, int lane,
                                                    const float4* s_hi, const float4* s_lo, const float4* s_rho,
                                                    Kahan& acc, unsigned* status) {
-    constexpr int PF = Prefetch<LANES>::N;
+    constexpr int PF = eam_ahead(LANES, STAGED);
     const int step = LANES << p.hshift;
     const float rc2 = p.rc_rho * p.rc_rho * 1.0001f;
     const float offdr = p.off * p.inv_dr;
@@ -155,8 +147,7 @@ __device__ __forceinline__ void gather_density_sum(const EAMFast& p, const PosPa
             if (s0 + k * LANES >= m) break;
             float4 hn, ln;
             if (k + 1 < PF && s0 + (k + 1) * LANES < m) ld256(pack + (ent[k + 1] & (unsigned)INDEX_MASK), hn, ln);
-            const int code = (int)(ent[k] >> 26);
-            const float3 d = delta_tab(hi, lo, hj, lj, s_hi[code], s_lo[code]);
+            const float3 d = delta_tab(hi, lo, hj, lj, ent[k], s_hi, s_lo);
             hj = hn;
             lj = ln;
             const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
@@ -180,69 +171,9 @@ __device__ __forceinline__ void gather_density_sum(const EAMFast& p, const PosPa
     }
 }
 
-// The same from the fixed-point positions: half the bytes a neighbour (from the
-// packs both passes were at 75 % of the L1's data path) and no image shift to
-// look up or add.  What bounds them now is the latency of the chain from entry
-// to position to knot, and issue: a lane holds few entries ahead, so that more
-// warps fit (density, 256,000 atoms: four entries ahead and six blocks a SM
-// 58.6 us, five blocks 64.3; force: eight and four 70.6, four and four 74.6, eight
-// and five 75.2).  Packs and fixed point, us, 256,000 atoms: density 72.5 and
-// 58.6, force 85.7 and 70.6; 1,048,576 (two lanes an atom): 264 and 207, 329
-// and 256.  (Lengths rounded twice and a Newton step for the root take 55.7 and
-// 66.8, with a smaller error, but leave a trajectory four times as far from the
-// packs'.)
-constexpr int FIX_AHEAD_DENSITY = 4, FIX_CTAS_DENSITY = 6;
-constexpr int FIX_AHEAD_FORCE = 8, FIX_CTAS_FORCE = 4;
-constexpr int FIX_TWO_LANES_PER_SM = 3000;
-// Below this many atoms a SM launches and latency are all, and the packs serve
-// as well (both passes, us: 16,384 atoms 28.1 and 27.4, 32,000 34.8 and 30.6,
-// 55,296 52.5 and 40.1, before the lengths' second half).
-constexpr int FIX_PER_SM = 128;
-
-template <int LANES>
-__device__ __forceinline__ void fixed_density_sum(const EAMFast& p, const int4* ipos, const unsigned* __restrict__ nbr,
-                                                  int ii, int m, int lane, Kahan& acc, unsigned* status) {
-    constexpr int PF = FIX_AHEAD_DENSITY;
-    const int step = LANES << p.hshift;
-    const float rc2 = p.rc_rho * p.rc_rho * 1.0001f;
-    const float offdr = p.off * p.inv_dr;
-    const int4 xi = ld_ipos(ipos + ii);
-    const unsigned* rp = nbr + nbr_at(ii, lane, p.hshift, p.maxnb);
-    bool bad = false;
-    for (int s0 = lane; s0 < m; s0 += PF * LANES, rp += PF * step) {
-        unsigned ent[PF];
-#pragma unroll
-        for (int k = 0; k < PF; k++) ent[k] = (s0 + k * LANES < m) ? __ldg(rp + k * step) & (unsigned)INDEX_MASK : 0u;
-        int4 xj = ld_ipos(ipos + ent[0]);
-#pragma unroll
-        for (int k = 0; k < PF; k++) {
-            if (s0 + k * LANES >= m) break;
-            int4 xn;
-            if (k + 1 < PF && s0 + (k + 1) * LANES < m) xn = ld_ipos(ipos + ent[k + 1]);
-            const float3 d = fix_delta(p, xi, xj);
-            xj = xn;
-            const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
-            if (r2 > rc2) continue;
-            const float r = r2 * rsqrtf(r2);
-            if (!(r <= p.rc_rho)) continue;
-            float dx;
-            const int x = knot_of(p, r, offdr, dx);
-            if (x < 0) {
-                if (!bad) report_range(status, r, p.src_rho);
-                bad = true;
-                continue;
-            }
-            const float4 cf = __ldg(&p.coef2[2 * (size_t)x + 1]);
-            float v = fmaf(dx, fmaf(dx, fmaf(dx, cf.x, cf.y), cf.z), cf.w);
-            if (p.rmult_rho) v = v / r;
-            acc.add(v);
-        }
-    }
-}
-
 // F(rho), F'(rho) for atom i (TableReader::read on the EMBED section); F'
 // also travels with the position for the force pass.
-__device__ __forceinline__ void density_finish(const EAMFast& p, int i, float rho, float* spare, float* fp,
+__device__ __forceinline__ void density_finish(const EAMFast& p, int i, float rho, PosPack* pack, float* fp,
                                                float* femb, unsigned* status) {
     const float rval = rho - p.e_off;
     int x = __float2int_rz(rval * p.e_inv_dr);
@@ -266,19 +197,19 @@ __device__ __forceinline__ void density_finish(const EAMFast& p, int i, float rh
     }
     fp[i] = dF;
     femb[i] = F;
-    *spare = dF;
+    pack[i].lo.w = dF;
 }
 
-template <int LANES, bool STAGED, bool FIXED>
-__global__ void EAMF_BOUNDS(STAGED, FIXED ? FIX_CTAS_DENSITY : 4) k_eamf_density(EAMFast p, PosPack* pack, int4* ipos, const unsigned* __restrict__ nbr,
+template <int LANES, bool STAGED>
+__global__ void EAMF_BOUNDS(STAGED, DENSITY_CTAS) k_eamf_density(EAMFast p, PosPack* pack, const unsigned* __restrict__ nbr,
                                                    const int* __restrict__ nnb, float* __restrict__ fp,
                                                    float* __restrict__ femb, unsigned* status) {
-    __shared__ float4 s_hi[FIXED ? 1 : 64], s_lo[FIXED ? 1 : 64];
+    __shared__ float4 s_hi[64], s_lo[64];
     extern __shared__ float4 s_rho[];
-    if (!FIXED) build_shift_table(p, s_hi, s_lo);
+    build_shift_table(p, s_hi, s_lo);
     if (STAGED)
         for (int k = threadIdx.x; k < p.stage_n; k += blockDim.x) s_rho[k] = p.coef2[2 * (size_t)(p.stage_k0 + k) + 1];
-    if (!FIXED) __syncthreads();
+    __syncthreads();
     const int lane = threadIdx.x & (LANES - 1);
     const int per_block = blockDim.x / LANES;
     for (int base = blockIdx.x * per_block; base < p.n; base += gridDim.x * per_block) {
@@ -287,11 +218,10 @@ __global__ void EAMF_BOUNDS(STAGED, FIXED ? FIX_CTAS_DENSITY : 4) k_eamf_density
         const int ii = valid ? i : p.n - 1;
         const int m = valid ? nnb[ii] : 0;
         Kahan acc;
-        if (FIXED) fixed_density_sum<LANES>(p, ipos, nbr, ii, m, lane, acc, status);
-        else gather_density_sum<LANES, STAGED>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_rho, acc, status);
+        gather_density_sum<LANES, STAGED>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_rho, acc, status);
         float sum = acc.s, comp = acc.c;
         twosum_reduce<LANES>(sum, comp);
-        if (lane == 0 && valid) density_finish(p, i, __fsub_rn(sum, comp), FIXED ? reinterpret_cast<float*>(&ipos[i].w) : &pack[i].lo.w, fp, femb, status);
+        if (lane == 0 && valid) density_finish(p, i, __fsub_rn(sum, comp), pack, fp, femb, status);
     }
 }
 
@@ -324,7 +254,7 @@ __device__ __forceinline__ void gather_force_sum(const EAMFast& p, const PosPack
                                                  const float4* s_hi, const float4* s_lo, const float4* s_tab,
                                                  Kahan& ax, Kahan& ay, Kahan& az, float& ae, float& av,
                                                  unsigned* status) {
-    constexpr int PF = Prefetch<LANES>::N;
+    constexpr int PF = eam_ahead(LANES, STAGED);
     const int step = LANES << p.hshift;
     const float offdr = p.off * p.inv_dr;
     const float4 hi = pack[ii].hi, lo = pack[ii].lo;
@@ -342,8 +272,7 @@ __device__ __forceinline__ void gather_force_sum(const EAMFast& p, const PosPack
             if (s0 + k * LANES >= m) break;
             float4 hn, ln;
             if (k + 1 < PF && s0 + (k + 1) * LANES < m) ldg256(pack + (ent[k + 1] & (unsigned)INDEX_MASK), hn, ln);
-            const int code = (int)(ent[k] >> 26);
-            const float3 d = delta_tab(hi, lo, hj, lj, s_hi[code], s_lo[code]);
+            const float3 d = delta_tab(hi, lo, hj, lj, ent[k], s_hi, s_lo);
             const float fpj = lj.w;  // F'(rho_j) from the density pass
             hj = hn;
             lj = ln;
@@ -366,56 +295,6 @@ __device__ __forceinline__ void gather_force_sum(const EAMFast& p, const PosPack
             } else {
                 ldg256(&p.coef2[2 * (size_t)x], cp, cr);
             }
-            float fr, eh;
-            eam_pair_terms(p, r2, fpi + fpj, cp, cr, dx, r, rinv, fr, eh);
-            ax.add(d.x * fr);
-            ay.add(d.y * fr);
-            az.add(d.z * fr);
-            ae += eh;
-            av = fmaf(fr, r2, av);
-        }
-    }
-}
-
-// The same from the fixed-point positions (fixed_density_sum).
-template <int LANES>
-__device__ __forceinline__ void fixed_force_sum(const EAMFast& p, const int4* __restrict__ ipos,
-                                                const unsigned* __restrict__ nbr, int ii, int m, int lane, Kahan& ax,
-                                                Kahan& ay, Kahan& az, float& ae, float& av, unsigned* status) {
-    constexpr int PF = FIX_AHEAD_FORCE;
-    const int step = LANES << p.hshift;
-    const float offdr = p.off * p.inv_dr;
-    const int4 xi = __ldg(ipos + ii);
-    const float fpi = __int_as_float(xi.w);
-    const unsigned* rp = nbr + nbr_at(ii, lane, p.hshift, p.maxnb);
-    bool bad = false;
-    for (int s0 = lane; s0 < m; s0 += PF * LANES, rp += PF * step) {
-        unsigned ent[PF];
-#pragma unroll
-        for (int k = 0; k < PF; k++) ent[k] = (s0 + k * LANES < m) ? __ldg(rp + k * step) & (unsigned)INDEX_MASK : 0u;
-        int4 xj = __ldg(ipos + ent[0]);
-#pragma unroll
-        for (int k = 0; k < PF; k++) {
-            if (s0 + k * LANES >= m) break;
-            int4 xn;
-            if (k + 1 < PF && s0 + (k + 1) * LANES < m) xn = __ldg(ipos + ent[k + 1]);
-            const float3 d = fix_delta(p, xi, xj);
-            const float fpj = __int_as_float(xj.w);  // F'(rho_j) from the density pass
-            xj = xn;
-            const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
-            if (r2 > p.rc2) continue;
-            const float rinv = rsqrtf(r2);
-            const float r = r2 * rinv;
-            if (!(r <= p.rc_phi)) continue;
-            float dx;
-            const int x = knot_of(p, r, offdr, dx);
-            if (x < 0) {
-                if (!bad) report_range(status, r, p.src_phi);
-                bad = true;
-                continue;
-            }
-            float4 cp, cr;
-            ldg256(&p.coef2[2 * (size_t)x], cp, cr);
             float fr, eh;
             eam_pair_terms(p, r2, fpi + fpj, cp, cr, dx, r, rinv, fr, eh);
             ax.add(d.x * fr);
@@ -457,9 +336,8 @@ __device__ __forceinline__ void force_store(const EAMFast& p, int i, float vfx, 
 // KICK: the step's second half-kick and its ledger terms in the epilogue (the
 // force is final here: one potential, no force modifies), as k_kick does
 // them, one ledger partial per warp.
-template <int LANES, bool STAGED, bool KICK, bool FIXED>
-__global__ void EAMF_BOUNDS(STAGED, FIXED ? FIX_CTAS_FORCE : 4) k_eamf_force(EAMFast p, const PosPack* __restrict__ pack,
-                                                       const int4* __restrict__ ipos,
+template <int LANES, bool STAGED, bool KICK>
+__global__ void EAMF_BOUNDS(STAGED, FORCE_CTAS) k_eamf_force(EAMFast p, const PosPack* __restrict__ pack,
                                                        const unsigned* __restrict__ nbr, const int* __restrict__ nnb,
                                                        const float* __restrict__ femb, float* __restrict__ fx,
                                                        float* __restrict__ fy, float* __restrict__ fz,
@@ -478,16 +356,16 @@ __global__ void EAMF_BOUNDS(STAGED, FIXED ? FIX_CTAS_FORCE : 4) k_eamf_force(EAM
         s_kk[kslot] = s_ke[kslot] = s_kw[kslot] = F2{0.f, 0.f};
         s_kv[kslot] = 0ull;
     }
-    __shared__ float4 s_hi[FIXED ? 1 : 64], s_lo[FIXED ? 1 : 64];
+    __shared__ float4 s_hi[64], s_lo[64];
     extern __shared__ float4 s_tab[];  // phi knots [k0, k0+ns), then rho knots (separate arrays: a warp's
                                        // random knots spread over all eight 16-byte bank groups)
-    if (!FIXED) build_shift_table(p, s_hi, s_lo);
+    build_shift_table(p, s_hi, s_lo);
     if (STAGED)
         for (int k = threadIdx.x; k < 2 * p.stage_n; k += blockDim.x) {
             const int kk = k < p.stage_n ? k : k - p.stage_n;
             s_tab[k] = p.coef2[2 * (size_t)(p.stage_k0 + kk) + (k < p.stage_n ? 0 : 1)];
         }
-    if (!FIXED) __syncthreads();
+    __syncthreads();
     const int lane = threadIdx.x & (LANES - 1);
     const int per_block = blockDim.x / LANES;
     for (int base = blockIdx.x * per_block; base < p.n; base += gridDim.x * per_block) {
@@ -497,8 +375,7 @@ __global__ void EAMF_BOUNDS(STAGED, FIXED ? FIX_CTAS_FORCE : 4) k_eamf_force(EAM
         const int m = valid ? nnb[ii] : 0;
         Kahan ax, ay, az;
         float ae = 0.f, av = 0.f;
-        if (FIXED) fixed_force_sum<LANES>(p, ipos, nbr, ii, m, lane, ax, ay, az, ae, av, status);
-        else gather_force_sum<LANES, STAGED>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_tab, ax, ay, az, ae, av, status);
+        gather_force_sum<LANES, STAGED>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_tab, ax, ay, az, ae, av, status);
         force_reduce<LANES>(ax, ay, az, ae, av);
         if (lane == 0 && valid) {
             const float vfx = __fsub_rn(ax.s, ax.c), vfy = __fsub_rn(ay.s, ay.c), vfz = __fsub_rn(az.s, az.c);
@@ -732,7 +609,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) k_eamt_density(EAMFast p, EAM
         }
         float sum = acc.s, comp = acc.c;
         twosum_reduce<LANES>(sum, comp);
-        if (lane == 0 && valid) density_finish(p, i, __fsub_rn(sum, comp), &pack[i].lo.w, fp, femb, status);
+        if (lane == 0 && valid) density_finish(p, i, __fsub_rn(sum, comp), pack, fp, femb, status);
     }
 }
 
@@ -839,33 +716,33 @@ static void launch_tiles(Context* c, const EAMFast& p, const EAMTileArgs& a) {
     prof_end(c);
 }
 
-template <int LANES, bool STAGED, bool FIXED>
+template <int LANES, bool STAGED>
 static void launch_fast(Context* c, const EAMFast& p, int grid, int block, size_t smem1, size_t smem2,
                         const KickArgs* ka) {
     static bool attr = false;
     if (!attr) {
-        cudaFuncSetAttribute(k_eamf_density<LANES, STAGED, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, false, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_eamf_density<LANES, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              200 * 1024);
-        cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, true, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              200 * 1024);
         attr = true;
     }
     prof_begin(c, "eam_density");
-    k_eamf_density<LANES, STAGED, FIXED><<<grid, block, smem1, c->stream>>>(
-        p, c->pack, c->ipos, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->fp, c->femb, c->d_status);
+    k_eamf_density<LANES, STAGED><<<grid, block, smem1, c->stream>>>(
+        p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->fp, c->femb, c->d_status);
     prof_end(c);
     const unsigned* aflag = c->flags_used ? c->aflag : nullptr;
     if (ka) {
         prof_begin(c, "eam_force_kick");
-        k_eamf_force<LANES, STAGED, true, FIXED><<<grid, block, smem2, c->stream>>>(
-            p, c->pack, c->ipos, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->femb, c->fx, c->fy, c->fz, c->pe,
+        k_eamf_force<LANES, STAGED, true><<<grid, block, smem2, c->stream>>>(
+            p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->femb, c->fx, c->fy, c->fz, c->pe,
             c->vir, c->d_status, *ka, c->vx, c->vy, c->vz, aflag, c->d_ledger);
         launch_ledger_finalize(c, *ka, grid * (block >> 5));
     } else {
         prof_begin(c, "eam_force");
-        k_eamf_force<LANES, STAGED, false, FIXED><<<grid, block, smem2, c->stream>>>(
-            p, c->pack, c->ipos, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->femb, c->fx, c->fy, c->fz, c->pe,
+        k_eamf_force<LANES, STAGED, false><<<grid, block, smem2, c->stream>>>(
+            p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->femb, c->fx, c->fy, c->fz, c->pe,
             c->vir, c->d_status, KickArgs{}, nullptr, nullptr, nullptr, nullptr, nullptr);
     }
     prof_end(c);
@@ -886,13 +763,6 @@ bool tiles_apply(const Context* c) {
     return p.kind == POT_EAM && eam_fast_shape(c, p);
 }
 
-bool eam_uses_fixed(const Context* c) {
-    if (c->use_f64 || c->eam_stage || c->n < FIX_PER_SM * c->num_sms) return false;
-    for (const Potential& p : c->pots)
-        if (p.kind == POT_EAM && eam_fast_shape(c, p)) return true;
-    return false;
-}
-
 bool eam_fast_ok(const Context* c, const Potential& pot) { return pot.d_coef2 && eam_fast_shape(c, pot); }
 
 int eam_fast_launch(Context* c, Potential& pot, bool first) {
@@ -903,8 +773,6 @@ int eam_fast_launch(Context* c, Potential& pot, bool first) {
     for (int d = 0; d < 3; d++) {
         p.Lh[d] = c->box.Lh[d];
         p.Ll[d] = c->box.Ll[d];
-        p.qh[d] = c->fix.qh[d];
-        p.ql[d] = c->fix.ql[d];
     }
     p.coef2 = pot.d_coef2;
     p.emb = pot.dt[2].coef;
@@ -941,12 +809,7 @@ int eam_fast_launch(Context* c, Potential& pot, bool first) {
     }
     p.stage_k0 = k0;
     p.stage_n = ns;
-    const bool fixed = c->fix.on && c->ipos && ns == 0;
     int block = c->eam_block > 256 ? 256 : c->eam_block, lanes = c->eam_lanes;
-    // a large box fills the chip with two lanes an atom, and reduces less:
-    // density and force of 1,048,576 atoms 197 and 252 us with four, 188 and 236
-    // with two; of 256,000 54 and 65, 58 and 64 (before the lengths' second half)
-    if (fixed && !c->eam_lanes_set && c->n >= FIX_TWO_LANES_PER_SM * c->num_sms) lanes = 2;
     int per_block = block / lanes;
     int grid = grid_for(c->n, per_block);
     if (ns > 0) {
@@ -1000,9 +863,8 @@ int eam_fast_launch(Context* c, Potential& pot, bool first) {
         return check_cuda(c, cudaGetLastError(), "eam tiles");
     }
 #define OMDG_EAMF(L)                                                 \
-    (st      ? launch_fast<L, true, false>(c, p, grid, block, smem1, smem2, kap) \
-     : fixed ? launch_fast<L, false, true>(c, p, grid, block, smem1, smem2, kap) \
-             : launch_fast<L, false, false>(c, p, grid, block, smem1, smem2, kap))
+    (st ? launch_fast<L, true>(c, p, grid, block, smem1, smem2, kap) \
+        : launch_fast<L, false>(c, p, grid, block, smem1, smem2, kap))
     switch (lanes) {
         case 1: OMDG_EAMF(1); break;
         case 2: OMDG_EAMF(2); break;

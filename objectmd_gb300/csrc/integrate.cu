@@ -50,7 +50,6 @@ __device__ __forceinline__ bool drift_store(const IntParams& p, const DriftArgs&
     pk.hi.w = __int_as_float(t);
     pk.lo.w = 0.f;
     d.pack[i] = pk;
-    if (p.ipos) p.ipos[i] = fix_pos(X, Y, Z, p.fix);
     const float4 r0 = d.xref[i];
     const float dx = (pk.hi.x - r0.x) + pk.lo.x, dy = (pk.hi.y - r0.y) + pk.lo.y, dz = (pk.hi.z - r0.z) + pk.lo.z;
     return !(dx * dx + dy * dy + dz * dz <= p.half_skin2);
@@ -461,8 +460,6 @@ static IntParams int_params(Context* c) {
     }
     float hs = (float)(0.5 * c->skin);
     p.half_skin2 = hs * hs;
-    p.fix = c->fix;
-    p.ipos = c->fix.on ? c->ipos : nullptr;
     p.use_f64 = c->use_f64 ? 1 : 0;
     for (int d = 0; d < 3; d++) {
         p.Q[d] = c->box.P[d] - c->box.org[d];
@@ -831,7 +828,6 @@ __global__ void __launch_bounds__(IO_BLOCK) k_upload_state(IntParams p, const in
             pk.hi.w = __int_as_float(type[i]);
             pk.lo.w = 0.f;
             pack[i] = pk;
-            if (p.ipos) p.ipos[i] = fix_pos(X, Y, Z, p.fix);
             const float4 r0 = xref[i];
             const float dx = (pk.hi.x - r0.x) + pk.lo.x, dy = (pk.hi.y - r0.y) + pk.lo.y,
                         dz = (pk.hi.z - r0.z) + pk.lo.z;

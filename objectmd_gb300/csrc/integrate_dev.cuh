@@ -38,8 +38,6 @@ struct IntParams {
     unsigned range_group;                // group bits it acts on
     double range_lo[3], range_hi[3];     // box -/+ border
     int need_vmax;                       // measure SqrMaxVelocity (DynamicTimeStep)
-    FixFrame fix;
-    int4* ipos;                          // fixed-point positions to refresh (or null)
 };
 
 struct FinParams {

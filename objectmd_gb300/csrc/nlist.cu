@@ -300,8 +300,6 @@ struct AtomArrays {
 // by pack_coord (the integrator refreshes the pack with the same function).
 struct PackFrame {
     float Qh[3], Ql[3];
-    FixFrame fix;
-    int4* ipos;  // null: not kept
 };
 
 // loc: the position rounded to FP32, which the list build screens (w: the type)
@@ -316,7 +314,6 @@ __device__ __forceinline__ float pack_atom(int i, double X, double Y, double Z, 
     p.hi.w = __int_as_float(type);
     p.lo.w = 0.f;
     pack[i] = p;
-    if (f.ipos) f.ipos[i] = fix_pos(X, Y, Z, f.fix);
     if (xref) xref[i] = make_float4(p.hi.x, p.hi.y, p.hi.z, 0.f);
     if (!loc) return 0.f;
     if (!active) {
@@ -1000,41 +997,6 @@ void nlist_prepare_geometry(Context* c) {
     }
 }
 
-// The fixed-point frame, for the EAM passes that use it: every periodic axis
-// three list ranges long, so that a period of that length or up to twice it
-// divides it.
-void fix_prepare(Context* c) {
-    const FixFrame old = c->fix;
-    FixFrame f;
-    const double rv = c->rc_max + c->skin, least = std::max(3.0 * rv, 2.2 * (rv + c->skin));
-    f.on = c->nrep == 0 && !c->tile_want && eam_uses_fixed(c);
-    for (int d = 0; d < 3; d++) {
-        double range = 4.0 * rv;
-        if (c->box.periodic[d]) {
-            const double t = std::floor(c->box.L[d] / least);
-            if (!(t >= 1.0)) {
-                f.on = 0;
-                break;
-            }
-            range = c->box.L[d] / t;
-        }
-        f.range[d] = range;
-        f.S[d] = 4294967296.0 / range;
-        f.C[d] = 6755399441055744.0 - c->box.lo[d] * f.S[d];
-        f.qh[d] = (float)(range / 4294967296.0);
-        f.ql[d] = (float)(range / 4294967296.0 - (double)f.qh[d]);
-        if (!(std::fabs(c->box.lo[d]) < 65536.0 && range < 131072.0 && f.S[d] < 4.0e9)) f.on = 0;  // |x S + C| in range
-    }
-    if (f.on && !c->ipos && cudaMalloc(&c->ipos, sizeof(int4) * (size_t)std::max(1, c->cap)) != cudaSuccess) {
-        cudaGetLastError();
-        f.on = 0;  // no room: the packs serve
-    }
-    bool same = f.on == old.on;
-    for (int d = 0; d < 3 && same && f.on; d++) same = f.S[d] == old.S[d] && f.C[d] == old.C[d];
-    c->fix = f;
-    if (!same) invalidate_graph(c);  // a captured step holds the old frame
-}
-
 // Cell grids of the replicas (same rules as nlist_prepare_geometry, per
 // replica) and the replica of every atom; uploads both.
 int replica_prepare(Context* c) {
@@ -1208,8 +1170,6 @@ void tile_release(Context* c) {
 
 PackFrame pack_frame(const Context* c) {
     PackFrame f;
-    f.fix = c->fix;
-    f.ipos = c->fix.on ? c->ipos : nullptr;
     for (int d = 0; d < 3; d++) {
         const double Q = c->box.P[d] - c->box.org[d];
         f.Qh[d] = (float)Q;

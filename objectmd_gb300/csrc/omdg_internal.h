@@ -92,14 +92,6 @@ struct BoxGeom {
     double cell_org[3], cell_h[3];
 };
 
-// Positions as 32-bit fixed point (device_common.cuh, fix_coord): a period of
-// each axis is 2^32 steps.
-struct FixFrame {
-    int on = 0;
-    double S[3], C[3], range[3];  // steps per length, offset (with the rounding constant), period
-    float qh[3], ql[3];           // length of a step, as an FP32 pair
-};
-
 struct __align__(32) PosPack {
     float4 hi;  // hx, hy, hz, type (bit pattern)
     float4 lo;  // lx, ly, lz, per-atom auxiliary (EAM: F'(rho), written by the density pass)
@@ -249,8 +241,6 @@ struct Context {
     int nbr_capacity = 0;       // launch key: the first build's row capacity (0: from the density)
     long overflow_recoveries = 0;  // queued steps replayed after a row overflow
     int* rev = nullptr;       // slot of i in row j (three-body kernels)
-    FixFrame fix;                // fixed-point frame (nlist_prepare_geometry decides whether it is kept)
-    int4* ipos = nullptr;        // fixed-point positions; w: F'(rho) after the EAM density pass
     float4* slot_buf = nullptr;  // per-slot force contributions (three-body kernels), of the rows' hits only
     unsigned* row_hits = nullptr;  // hit bits of every row (rows.cuh), cap words per 32 entries
     int* ters_wide = nullptr;    // Tersoff centres past the register path: [0] count, then their indices
@@ -270,7 +260,6 @@ struct Context {
     int nbr_hshift = 3;        // sliced-ELL slice height H = 2^hshift
     int eam_block = 256;
     int eam_lanes = 4;         // threads per atom
-    bool eam_lanes_set = false;  // by the caller or the tuner: no rule by size
     int eam_stage = 0;         // 1: stage spline knots in shared memory
     double eam_stage_frac = 0.35;
     int eam_ctas_per_sm = 1;
@@ -383,9 +372,6 @@ void prof_collect(Context* c);
 // neighbour list (nlist.cu)
 int nlist_build(Context* c, bool on_request = false);
 void nlist_prepare_geometry(Context* c);
-void fix_prepare(Context* c);             // after tile_prepare
-bool eam_uses_fixed(const Context* c);    // an EAM pass reads the fixed-point positions (eam_fast.cu)
-void invalidate_graph(Context* c);
 int nlist_reserve(Context* c, int maxnb);
 size_t nlist_slots(const Context* c, int maxnb);
 // EAM cell tiles: decide whether the builds write tile slots and size the

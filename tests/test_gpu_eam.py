@@ -421,3 +421,39 @@ def test_fixed_point_positions(omdg_lib, oracle_lib, case):
         ctx.compute_forces()
         st = ctx.get_state()
     check_forces(st["f"], fref, st["pot"], eref)
+
+
+@pytest.mark.parametrize("cells,periodic", [(22, (1, 1, 1)), (22, (1, 1, 0)), (12, (1, 1, 1))])
+def test_small_components_keep_their_bits(omdg_lib, cells, periodic):
+    """Dimers along z, 10^-4 to 10^-3 A off the axis, on a grid wider than the
+    cutoff, some of them across the faces, in a box of 21,296 atoms and one of
+    3,456.  A pair's force is parallel to its separation: f_x / f_z is d_x / d_z
+    but for the FP32 rounding of the two components and the two products
+    (4 x 2^-24) and the packs' resolution of a position (2^-48 of the box,
+    in the difference twice)."""
+    rng = np.random.default_rng(11)
+    grid = np.stack(np.meshgrid(*[np.arange(cells)] * 3, indexing="ij"), -1).reshape(-1, 3) * 10.0
+    side = 10.0 * cells
+    n = len(grid)
+    d = rng.uniform(1e-4, 1e-3, (n, 3)) * rng.choice([-1.0, 1.0], (n, 3))
+    d[:, 2] = rng.uniform(2.6, 3.4, n)
+    at = grid + rng.uniform(-0.4, 0.4, (n, 3))
+    at[:, 2] = grid[:, 2] + (4.0 if not periodic[2] else 8.5)
+    x = np.vstack([at, at + d])
+    L = np.full(3, side)
+    x = np.where(np.asarray(periodic) != 0, x % L, x)
+    d = x[n:] - x[:n]
+    d -= L * np.round(d / L)
+    with omdg_lib.Context(0) as ctx:
+        ctx.set_box(np.zeros(3), L, tuple(bool(p) for p in periodic))
+        ctx.set_atoms(x, np.zeros_like(x), masses=[26.98], znum=[13.0])
+        ctx.add_eam(EAM_TABLE)
+        ctx.set_neighbor(0.3, 0)
+        ctx.compute_forces()
+        f = ctx.get_state()["f"].astype(np.float64)
+    assert np.abs(f[:, 2]).min() > 0.0
+    tol = 2.0 ** -22 + 4.0 * side * 2.0 ** -48 / np.abs(d[:, :2])
+    for part in (f[:n], f[n:]):
+        ratio = part[:, :2] / part[:, 2:]
+        want = d[:, :2] / d[:, 2:]
+        assert (np.abs(ratio / want - 1.0) <= tol).all(), np.abs(ratio / want - 1.0).max()
