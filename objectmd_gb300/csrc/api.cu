@@ -939,11 +939,7 @@ static int build_list(Context* c) {
     return set_error(c, OMDG_ESTATE, "neighbour list did not fit");
 }
 
-int forces_compute(Context* c) {
-    if (c->pots.empty()) return set_error(c, OMDG_ESTATE, "no force kernel");
-    c->kick_fused = false;
-    c->gather_deferred = false;
-    if (!c->fuse_kick) c->wide_cleared = false;  // not a step's evaluation
+static int issue_forces(Context* c) {
     bool first = true;
     // in a step the last potential's slot gather joins the kick, unless a modify
     // or the detector works on the forces in between (a potential after it would
@@ -967,12 +963,23 @@ int forces_compute(Context* c) {
             case POT_ZBL: rc = zbl_launch(c, p, first); break;
             case POT_NN: rc = nn_launch(c, p, first); break;
         }
-        c->defer_gather = false;
         if (rc) return rc;
         first = false;
     }
-    c->wide_cleared = false;
     return post_force_modifies(c);  // MODIFY_POST_FORCE (integrator.cpp:215)
+}
+
+int forces_compute(Context* c, bool after_drift) {
+    if (c->pots.empty()) return set_error(c, OMDG_ESTATE, "no force kernel");
+    c->kick_fused = false;
+    c->gather_deferred = false;
+    c->wide_cleared = after_drift;
+    const int rc = issue_forces(c);
+    // what holds for this evaluation only, whichever way it ended
+    c->wide_cleared = false;
+    c->defer_gather = false;
+    if (rc) c->kick_fused = c->gather_deferred = false;
+    return rc;
 }
 
 // Eager rebuild of the list when the device asks for it (reads the flag).
@@ -1024,7 +1031,7 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
     };
     cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return check_cuda(c, e, "capture begin");
-    const long launches0 = c->launches;
+    const long launches0 = c->launches, rebuilds0 = c->rebuilds;
     long l0 = 0, l1 = 0, l2 = 0, l3 = 0;
     int rc = OMDG_OK;
     bool drifted = false;  // the step's kick_drift was in the last one's kick
@@ -1094,7 +1101,7 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
         l2 = c->launches;
         if (!rc && io) rc = branch(0, io[0], nullptr, nullptr);
         c->fuse_kick = true;
-        if (!rc) rc = forces_compute(c);
+        if (!rc) rc = forces_compute(c, true);
         c->fuse_kick = false;
         const bool f_after = c->gather_deferred;  // the kick completes the forces
         if (!rc && io && !f_after) rc = branch(1, nullptr, nullptr, io[2]);
@@ -1114,7 +1121,6 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
             if (e != cudaSuccess) rc = check_cuda(c, e, "download join");
         }
         l3 = c->launches;
-        c->captured_builds += 1;
     }
     // captured launches are counted when the graph replays, not here
     if (steps == 1) {
@@ -1122,9 +1128,11 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
         c->graph_body_kernels = l2 - l1;
     }
     c->launches = launches0;
+    c->captured_builds += c->rebuilds - rebuilds0;
     cudaGraph_t graph = nullptr;
     e = cudaStreamEndCapture(s, &graph);
     if (rc) {
+        c->kick_fused = c->gather_deferred = false;  // nothing of the capture runs
         if (graph) cudaGraphDestroy(graph);
         return rc;
     }
@@ -1448,7 +1456,7 @@ int omdg_step_async(omdg_ctx* c, int nsteps) {
             c->build_in_step = false;
             if (rc) return rc;
             c->fuse_kick = true;
-            rc = forces_compute(c);
+            rc = forces_compute(c, true);
             c->fuse_kick = false;
             if (rc) return rc;
             if ((rc = integrate_kick(c, k))) return rc;

@@ -470,7 +470,6 @@ static IntParams int_params(Context* c) {
 }
 
 static DriftArgs drift_args(Context* c, const cudaGraphConditionalHandle* cond) {
-    c->wide_cleared = c->ters_wide != nullptr;  // in a step the first three-body pass finds its queue cleared
     const bool reps = c->nrep > 0;
     return DriftArgs{c->x, c->y, c->z, c->pack, c->xref, reps ? c->d_rep_of : nullptr, reps ? c->d_rep_flag : nullptr,
                      c->ters_wide, cond ? *cond : 0, cond ? 1 : 0};

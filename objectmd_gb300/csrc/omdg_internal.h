@@ -202,7 +202,7 @@ struct Context {
     bool defer_gather = false;           // the slot gather being issued may join the step's kick
     bool gather_deferred = false;        // ... and does: the kick collects the slots
     bool gather_zero_virial = false;
-    bool wide_cleared = false;           // this step's kick_drift cleared the queue of wide centres
+    bool wide_cleared = false;           // the queue of wide centres is empty (within forces_compute only)
     int ncell_cap = 0;
     int* scan_partials = nullptr;
     int* cell_sorted = nullptr;
@@ -382,7 +382,8 @@ int tile_reserve_slots(Context* c);
 void tile_release(Context* c);
 
 // forces (eam.cu, pair.cu, threebody.cu)
-int forces_compute(Context* c);
+// after_drift: this step's kick_drift was issued before (it clears the queue of wide centres)
+int forces_compute(Context* c, bool after_drift = false);
 int eam_launch(Context* c, Potential& p, bool first);
 int pair_launch(Context* c, Potential& p, bool first);
 int sw_launch(Context* c, Potential& p, bool first);
