@@ -1468,12 +1468,16 @@ int omdg_step_async(omdg_ctx* c, int nsteps) {
         if (!gs.valid) {
             if ((rc = capture_step(c, gs))) return rc;
         }
-        const std::string said = c->last_error;
-        if (!gs.many_valid && !gs.many_failed && nsteps >= GRAPH_STEPS && gs.replayed >= GRAPH_AFTER &&
-            capture_step(c, gs, nullptr, GRAPH_STEPS)) {
-            gs.many_failed = true;  // no room for it, say: the single steps go on
-            cudaGetLastError();
-            c->last_error = said;
+        if (!gs.many_valid && !gs.many_failed && nsteps >= GRAPH_STEPS && gs.replayed >= GRAPH_AFTER) {
+            const std::string said = c->last_error;
+            rc = capture_step(c, gs, nullptr, GRAPH_STEPS);
+            if (rc && rc != OMDG_ENOMEM) return rc;
+            if (rc) {  // no room for it: the single steps go on
+                gs.many_failed = true;
+                cudaGetLastError();
+                c->last_error = said;
+                rc = OMDG_OK;
+            }
         }
         for (int k = 0; k < nsteps;) {
             const bool many = gs.many_valid && nsteps - k >= GRAPH_STEPS;

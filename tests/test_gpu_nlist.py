@@ -229,3 +229,31 @@ def test_kick_and_drift_in_one_kernel(omdg_lib, kind, ncell, every):
     assert out[0][-1] > 3
     for o in out[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(o, out[0]))
+
+
+@pytest.mark.parametrize("ncell", [4, 17])
+def test_the_graph_of_steps_runs(omdg_lib, ncell):
+    """Calls of eight steps take the graph of eight once 64 steps were replayed,
+    with seven kicks and drifts of each eight in one kernel: seven launches
+    fewer.  What a call itself launches comes from calls of two and of four
+    steps; the rebuilds are the same in every run."""
+    from objectmd_gb300 import inputs
+
+    x, v, (lo, hi) = inputs.diamond_silicon(ncell=ncell, a=5.431, sigma=0.05, temp=1500.0, seed_pos=3, seed_vel=4)
+    launches, rebuilds = [], []
+    for size in (2, 4, 8):
+        with omdg_lib.Context(0) as ctx:
+            ctx.set_box(lo, hi)
+            ctx.set_atoms(x, v, masses=[inputs.md_mass("silicon")], znum=[14.0])
+            ctx.add_tersoff(os.path.join(TABLES, "tersoff.silicon27"))
+            ctx.set_neighbor(SKIN, 0)
+            ctx.set_timestep(0.001)
+            for _ in range(64):
+                ctx.step(1)
+            for _ in range(64 // size):
+                ctx.step(size)
+            launches.append(ctx.stats()["launches"])
+            rebuilds.append(ctx.stats()["rebuilds"])
+    assert rebuilds[0] == rebuilds[1] == rebuilds[2]
+    per_call = (launches[0] - launches[1]) / 16
+    assert launches[1] - launches[2] == 8 * per_call + 7 * 8
