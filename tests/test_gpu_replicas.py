@@ -189,3 +189,39 @@ def test_sort_of_replicas_at_its_edges(omdg_lib, sizes):
         d = whole[at:at + n] - run([k])[0]
         assert np.abs(d - L * np.round(d / L)).max() <= 1e-5, k
         at += n
+
+
+def test_a_smaller_skin_needs_more_cells(omdg_lib):
+    """A context of replicas whose list range shrinks from call to call: the
+    grid has more cells each time, and the cells' replicas grow with it.  The
+    list is each single box's."""
+    from objectmd_gb300 import inputs
+
+    parts = [inputs.diamond_silicon(ncell=n, a=5.431, sigma=0.05, temp=300.0, seed_pos=81 + k, seed_vel=82 + k)
+             for k, n in enumerate((4, 7, 5))]
+    natoms = [len(p[0]) for p in parts]
+    start = np.concatenate([[0], np.cumsum(natoms)])
+    with omdg_lib.Context(0) as ctx:
+        ctx.set_replicas(natoms, [p[2][0] for p in parts], [p[2][1] for p in parts], (1, 1, 0))
+        ctx.set_atoms(np.vstack([p[0] for p in parts]), np.vstack([p[1] for p in parts]),
+                      masses=[inputs.md_mass("silicon")], znum=[14.0])
+        ctx.add_tersoff(TERSOFF)
+        ctx.set_timestep(0.0005)
+        for skin in (6.0, 2.0, 0.3, 0.05):
+            ctx.set_neighbor(skin, 0)
+            ctx.compute_forces()
+            ctx.step(3)
+            ctx.build_neighbors()
+            x = ctx.get_state()["x"]
+            mine = nbr_set(*ctx.neighbors())
+            for k, p in enumerate(parts):
+                sl = slice(start[k], start[k + 1])
+                with omdg_lib.Context(0) as one:
+                    one.set_box(p[2][0], p[2][1], (True, True, False))
+                    one.set_atoms(x[sl], masses=[inputs.md_mass("silicon")], znum=[14.0])
+                    one.add_tersoff(TERSOFF)
+                    one.set_neighbor(skin, 0)
+                    one.build_neighbors()
+                    alone = nbr_set(*one.neighbors())
+                part = {(i - start[k], j - start[k], *rest) for i, j, *rest in mine if start[k] <= i < start[k + 1]}
+                assert part == alone, (skin, k)
