@@ -169,12 +169,13 @@ __global__ void __launch_bounds__(256) k_pair32_typed(PairParams p, const PosPac
 //   - the centre minus the image's length is formed once per centre and picked
 //     by the entry's image bits (integer selects cost nothing here);
 //   - 1/r comes from the hardware's reciprocal-square-root estimate and one
-//     third-order step (y + y e (1/2 + 3/8 e), e = 1 - r^2 y^2: the estimate's
-//     error cubed, below an ulp), r = r^2 / r takes one Newton step to half
-//     an ulp, and the force factor a product where the reference divides;
-//   - the knot index comes from FP32; a value it puts in the segment next
-//     door is off by the spline's third-derivative jump times 1e-4 knots
-//     cubed, far below an ulp;
+//     third-order step (Householder's for y^-2 = r^2: y + y e (1/2 + 3/8 e),
+//     e = 1 - r^2 y^2, leaves the estimate's error cubed, below an ulp), r =
+//     r^2 / r takes one Newton step to half an ulp, and the force factor a
+//     product where the reference divides;
+//   - the knot index comes from FP32, which near a knot may name the segment
+//     next door: the offset from the knot then is negative or a whole segment,
+//     one integer comparison, and the index is put right out of line;
 //   - value and slope share their Horner steps.
 // Reads below the first knot, with the reference's edge rules, go through
 // tab_read64 out of line.  The IEEE sequences (root, two divisions, separate
@@ -183,6 +184,13 @@ __global__ void __launch_bounds__(256) k_pair32_typed(PairParams p, const PosPac
 // theirs (1.3-1.4e-15 of the norm).
 __device__ __noinline__ void tab_read64_slow(const DevTable& t, double r, double* v, double* dv, unsigned* status) {
     tab_read64(t, r, *v, *dv, status);
+}
+
+// The knot next to k, and the offset from it; d: the offset from knot k.
+__device__ __noinline__ int knot64_next(const DevTable& t, double rval, int k, double* d) {
+    k = min(k + (__double_as_longlong(*d) < 0 ? -1 : 1), t.n - 2);
+    *d = fma(-(double)k, t.dr64, rval);
+    return k;
 }
 
 // double to float by the bits (truncated; normal, positive, in float's range)
@@ -213,6 +221,7 @@ __global__ void __launch_bounds__(P64_BLOCK) k_pair64(PairParams p, const double
     const bool any = valid && (p.all_types || ti == p.ta || ti == p.tb);
     const int m = any ? nnb[i] : 0;
     const long long rc_bits = __double_as_longlong(p.rc64);
+    const unsigned long long dr_bits = (unsigned long long)__double_as_longlong(p.phi.dr64);
     for (int s = lane; s < m; s += LANES) {
         const unsigned e = __ldg(&nbr[nbr_at(i, s, p.hshift, p.maxnb)]);
         const int j = nbr_index(e);
@@ -240,8 +249,9 @@ __global__ void __launch_bounds__(P64_BLOCK) k_pair64(PairParams p, const double
         if (tiny || __double_as_longlong(rval) < (1ll << 52) || p.phi.n > (1 << 16)) {
             tab_read64_slow(p.phi, r, &ph, &dph, status);
         } else {
-            const int k = min((int)(d2f_bits(rval) * p.phi.inv_dr), p.phi.n - 2);
-            const double d = fma(-f2d_exact((float)k), p.phi.dr64, rval);
+            int k = min((int)(d2f_bits(rval) * p.phi.inv_dr), p.phi.n - 2);
+            double d = fma(-f2d_exact((float)k), p.phi.dr64, rval);
+            if ((unsigned long long)__double_as_longlong(d) >= dr_bits) k = knot64_next(p.phi, rval, k, &d);
             const double4_32a cf = p.phi.coef64[k];
             const double u = fma(d, cf.x, cf.y), h = fma(d, u, cf.z);
             ph = fma(d, h, cf.w);

@@ -211,3 +211,102 @@ def test_typed_pair_in_a_large_box_matches_oracle(omdg_lib, oracle_lib, share, p
     clear[i[np.abs(r - phi.max_range()) < 4e-6]] = False
     assert clear.mean() > 0.99
     assert np.abs(st["pot"] - e)[clear].max() <= 2e-6
+
+
+def dimers(r, direction, spacing):
+    """Pairs at distances r along a direction, on a grid; returns the positions
+    (first atoms, then second ones) and the box."""
+    n = len(r)
+    side = int(np.ceil(n ** (1.0 / 3.0)))
+    grid = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n] * spacing + 1.0
+    d = np.asarray(direction, dtype=np.float64)
+    return np.vstack([grid, grid + np.asarray(r)[:, None] * d / np.linalg.norm(d)]), np.zeros(3), np.full(3, side * spacing)
+
+
+def dimer_forces(omdg, table, x, lo, hi):
+    with omdg.Context(0) as ctx:
+        ctx.set_box(lo, hi, (False, False, False))
+        ctx.set_atoms(x, masses=[39.948], znum=[18.0])
+        ctx.add_pair_table(str(table), fp64=True)
+        ctx.set_neighbor(0.3, 1)
+        ctx.compute_forces()
+        return ctx.get_state()["f"]
+
+
+def plain_table(path, off, dr, values):
+    lines = ["#$ NumberOfData %d" % len(values), "#$ Spacing %.17g" % dr, "#$ Offset %.17g" % off, "#$ Format PLAIN",
+             "#$ --"] + ["%.17g" % v for v in values]
+    path.write_text("\n".join(lines) + "\n")
+
+
+# Distances within 2e-4 of a segment of a knot, where FP32 may name the wrong
+# segment, in a table of measured values (LJ with noise of 1e-4 eV): the slope's
+# cubic term jumps from segment to segment, so the neighbouring segment's slope
+# is off by 1e-8 eV/A.  Allowed: the FP64 rounding of the four operations of the
+# slope (each at most its largest term's, eight ulps in all), and that of r and
+# of its offset from the knot (four ulps of r) times the curvature.
+def test_fp64_pair_next_to_the_knots(omdg_lib, oracle_lib, tmp_path):
+    oc = oracle_lib
+    rng = np.random.default_rng(21)
+    n, off, rc = 5000, 2.0, 8.5125
+    dr = (rc - off) / (n - 1)
+    at = off + dr * np.arange(n)
+    s6 = (3.405 / at) ** 6
+    plain_table(tmp_path / "noisy", off, dr, 4 * 0.0104 * (s6 * s6 - s6) + 1e-4 * rng.standard_normal(n))
+    t = oc.Table.from_file(str(tmp_path / "noisy"), "")
+    knot = rng.integers(1, n - 2, 1000)
+    x, lo, hi = dimers(off + dr * (knot + rng.uniform(1e-6, 2e-4, 1000) * rng.choice([-1.0, 1.0], 1000)), (1, 0, 0), 20.0)
+    f = dimer_forces(omdg_lib, tmp_path / "noisy", x, lo, hi)
+    r = x[1000:, 0] - x[:1000, 0]
+    k = ((r - off) / dr).astype(int)
+    d = np.longdouble(r) - np.longdouble(off) - k * np.longdouble(dr)
+    c3, c2, c1 = 3 * t.a[k] * d * d, 2 * t.b[k] * d, np.longdouble(t.c[k])
+    tol = 8 * 2.0 ** -53 * (abs(c3) + abs(c2) + abs(c1)) + 4 * 2.0 ** -53 * r * abs(2 * t.b[k] + 6 * t.a[k] * d)
+    assert (np.abs(f[:1000, 0] - (c3 + c2 + c1)) <= tol).all()
+    assert np.array_equal(f[:1000], -f[1000:])
+
+
+# The root and its reciprocal over the range of distances, against numpy's: in a
+# table of phi = r a pair's force is its unit vector, r^2's rounding (an ulp, half
+# of it in the root), the reciprocal's, and three products'.
+@pytest.mark.parametrize("direction", [(1, 0, 0), (0.3, -1.1, 0.7)])
+def test_fp64_pair_unit_vectors(omdg_lib, oracle_lib, tmp_path, direction):
+    n, off, rc = 2000, 1e-3, 40.0
+    dr = (rc - off) / (n - 1)
+    plain_table(tmp_path / "line", off, dr, off + dr * np.arange(n))
+    r = np.exp(np.random.default_rng(22).uniform(np.log(0.01), np.log(39.9), 500))
+    x, lo, hi = dimers(r, direction, 90.0)
+    f = dimer_forces(omdg_lib, tmp_path / "line", x, lo, hi)
+    t = oracle_lib.Table.from_file(str(tmp_path / "line"), "")
+    slope = np.abs(np.array([t.read(q)[1] for q in r]) - 1.0).max()  # the table's own rounding
+    d = np.longdouble(x[500:]) - np.longdouble(x[:500])
+    u = d / np.sqrt((d * d).sum(1))[:, None]
+    assert np.abs(f[:500] - u).max() <= 6 * 2.0 ** -53 + 2 * slope
+
+
+# The thermostat's factor from one root estimate, against the formula in extended
+# precision: atoms without neighbours, whose velocities only it changes.  Allowed:
+# the three roundings of its quotients (half an ulp each, in an argument whose
+# root halves them) and the root's, 4 x 2^-53; the velocities' product one more.
+@pytest.mark.parametrize("target,tau", [(300.0, 0.1), (0.0, 0.5), (5000.0, 0.02), (90.0, 10.0)])
+def test_thermostat_factor(omdg_lib, target, tau):
+    rng = np.random.default_rng(23)
+    x, lo, hi = dimers(np.full(32, 15.0), (0, 0, 1), 40.0)
+    v = rng.standard_normal(x.shape)
+    dt, n = 0.001, len(x)
+    with omdg_lib.Context(0) as ctx:
+        ctx.set_box(lo, hi, (False, False, False))
+        ctx.set_atoms(x, v, masses=[39.948], znum=[18.0])
+        ctx.add_pair_table(LJ)
+        ctx.set_neighbor(0.3, 0)
+        ctx.set_timestep(dt)
+        ctx.set_thermostat(target, tau)
+        last = None
+        for step in range(6):
+            ctx.step(1)
+            now, kin = ctx.get_state()["v"], ctx.ledger()["kinetic"]
+            if step:
+                T = np.longdouble(2.0 / 3.0 / 8.61734279e-05) * np.longdouble(kin) / n
+                want = np.sqrt(1 + np.longdouble(dt) / np.longdouble(tau) * (np.longdouble(target) / T - 1))
+                assert np.abs(now / (last * want) - 1).max() <= 6 * 2.0 ** -53, step
+            last = now
