@@ -408,6 +408,42 @@ __device__ __forceinline__ void for_nbrs(int nc, F&& f) {
         if (b < nc) f(b);
 }
 
+// a b + c d with one product rounded by itself
+__device__ __forceinline__ float fma2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
+
+// The arithmetic of a bond that both forms share.  Every product and sum is
+// written as the instruction it is, so that the forms round alike whatever the
+// compiler contracts (test_tersoff_forms_have_the_same_bits).
+struct TersTriplet {
+    float c, g, dg, ex, dex;  // cos, g and dg/dcos, exp(l3^3 (r_ij - r_ik)^3) and its derivative by r_ij
+    __device__ __forceinline__ TersTriplet(const TersDev& p, float g0, float ax, float ay, float az, float ra, float bx,
+                                           float by, float bz, float rb) {
+        c = fmaf(az, bz, fma2(ax, bx, ay, by));
+        const float hc = __fsub_rn(p.h, c);
+        const float rden = __fdividef(1.f, fmaf(hc, hc, p.d2));
+        g = fmaf(-p.c2, rden, g0);
+        dg = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(-2.f, p.c2), hc), rden), rden);
+        const float dr = __fsub_rn(ra, rb);
+        const float l = __fmul_rn(p.l3c, dr);
+        ex = __expf(__fmul_rn(__fmul_rn(l, dr), dr));
+        dex = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(3.f, p.l3c), dr), dr), ex);
+    }
+};
+
+// V_ij = f_c (f_R - b f_A) of a bond and its derivatives by r_ij and zeta
+struct TersBond {
+    float v, dr, dz;
+    __device__ __forceinline__ TersBond(const TersDev& p, float r, float fc, float dfc, float zeta) {
+        const float fR = __fmul_rn(p.A, __expf(__fmul_rn(-p.l1, r))), fA = __fmul_rn(p.B, __expf(__fmul_rn(-p.l2, r)));
+        float b, db;
+        ters_bond_order(p, zeta, b, db);
+        const float att = fmaf(-b, fA, fR);
+        v = __fmul_rn(fc, att);
+        dr = fma2(dfc, att, fc, fma2(__fmul_rn(b, p.l2), fA, -p.l1, fR));
+        dz = __fmul_rn(__fmul_rn(-fc, fA), db);
+    }
+};
+
 // The bonds centred on one atom, for its nc <= K in-cutoff neighbours in
 // registers (unit vectors u from the centre, distances r).  Per neighbour the
 // cutoff f_c(r), f_c'(r) and 1/r are evaluated once; per triplet (a, b) the
@@ -433,56 +469,45 @@ __device__ __forceinline__ void ters_bonds(const TersDev& p, const int nc, const
         float ck[K], cc[K], cs[K];
         for_nbrs<K>(nc, [&](int b) {
             if (b == a) return;
-            const float c = ex_ * ux[b] + ey_ * uy[b] + ez_ * uz[b];
-            const float hc = p.h - c;
-            const float rden = __fdividef(1.f, p.d2 + hc * hc);
-            const float g = g0 - p.c2 * rden;
-            const float dg = -2.f * p.c2 * hc * rden * rden;
-            const float dr = rij - rr[b];
-            const float ex = __expf(p.l3c * dr * dr * dr);
-            const float dex = 3.f * p.l3c * dr * dr * ex;
-            zeta += fc[b] * g * ex;
-            const float cj = fc[b] * dg * ex * ir[a], cu = fc[b] * g * dex;
-            gjx += cj * (ux[b] - c * ex_) + cu * ex_;
-            gjy += cj * (uy[b] - c * ey_) + cu * ey_;
-            gjz += cj * (uz[b] - c * ez_) + cu * ez_;
-            ck[b] = dfc[b] * g * ex - fc[b] * g * dex;
-            cc[b] = fc[b] * dg * ex * ir[b];
-            cs[b] = c;
+            const TersTriplet t(p, g0, ex_, ey_, ez_, rij, ux[b], uy[b], uz[b], rr[b]);
+            const float fg = __fmul_rn(fc[b], t.g), fd = __fmul_rn(__fmul_rn(fc[b], t.dg), t.ex);
+            zeta = fmaf(fg, t.ex, zeta);
+            const float cj = __fmul_rn(fd, ir[a]), cu = __fmul_rn(fg, t.dex);
+            gjx = __fadd_rn(gjx, fma2(cu, ex_, cj, fmaf(-t.c, ex_, ux[b])));
+            gjy = __fadd_rn(gjy, fma2(cu, ey_, cj, fmaf(-t.c, ey_, uy[b])));
+            gjz = __fadd_rn(gjz, fma2(cu, ez_, cj, fmaf(-t.c, ez_, uz[b])));
+            ck[b] = fma2(__fmul_rn(dfc[b], t.g), t.ex, -fg, t.dex);
+            cc[b] = __fmul_rn(fd, ir[b]);
+            cs[b] = t.c;
         });
-        const float fR = p.A * __expf(-p.l1 * rij), fA = p.B * __expf(-p.l2 * rij);
-        float bij, dbdz;
-        ters_bond_order(p, zeta, bij, dbdz);
-        const float vij = fc[a] * (fR - bij * fA);
-        const float dv_dr = dfc[a] * (fR - bij * fA) + fc[a] * (-p.l1 * fR + bij * p.l2 * fA);
-        const float dv_dz = -fc[a] * fA * dbdz;
+        const TersBond v(p, rij, fc[a], dfc[a], zeta);
         // gradient of 1/2 V_ij: x_j part
-        const float sjx = 0.5f * (dv_dr * ex_ + dv_dz * gjx);
-        const float sjy = 0.5f * (dv_dr * ey_ + dv_dz * gjy);
-        const float sjz = 0.5f * (dv_dr * ez_ + dv_dz * gjz);
-        fix += sjx;  // the x_i gradient is minus the sum of the others
-        fiy += sjy;
-        fiz += sjz;
-        const float s = 0.5f * dv_dz;
+        const float sjx = 0.5f * fma2(v.dr, ex_, v.dz, gjx);
+        const float sjy = 0.5f * fma2(v.dr, ey_, v.dz, gjy);
+        const float sjz = 0.5f * fma2(v.dr, ez_, v.dz, gjz);
+        fix = __fadd_rn(fix, sjx);  // the x_i gradient is minus the sum of the others
+        fiy = __fadd_rn(fiy, sjy);
+        fiz = __fadd_rn(fiz, sjz);
+        const float s = 0.5f * v.dz;
         // x_k parts
         for_nbrs<K>(nc, [&](int b) {
             if (b == a) return;
-            const float kx = s * (ck[b] * ux[b] + cc[b] * (ex_ - cs[b] * ux[b]));
-            const float ky = s * (ck[b] * uy[b] + cc[b] * (ey_ - cs[b] * uy[b]));
-            const float kz = s * (ck[b] * uz[b] + cc[b] * (ez_ - cs[b] * uz[b]));
-            fix += kx;
-            fiy += ky;
-            fiz += kz;
+            const float kx = fma2(ck[b], ux[b], cc[b], fmaf(-cs[b], ux[b], ex_));
+            const float ky = fma2(ck[b], uy[b], cc[b], fmaf(-cs[b], uy[b], ey_));
+            const float kz = fma2(ck[b], uz[b], cc[b], fmaf(-cs[b], uz[b], ez_));
+            fix = fmaf(s, kx, fix);
+            fiy = fmaf(s, ky, fiy);
+            fiz = fmaf(s, kz, fiz);
             // force on k = -gradient
-            skx[b] -= kx;
-            sky[b] -= ky;
-            skz[b] -= kz;
+            skx[b] = fmaf(-s, kx, skx[b]);
+            sky[b] = fmaf(-s, ky, sky[b]);
+            skz[b] = fmaf(-s, kz, skz[b]);
         });
-        skx[a] -= sjx;
-        sky[a] -= sjy;
-        skz[a] -= sjz;
-        ei += 0.5f * vij;
-        wi += 0.5f * dv_dr * rij;
+        skx[a] = __fsub_rn(skx[a], sjx);
+        sky[a] = __fsub_rn(sky[a], sjy);
+        skz[a] = __fsub_rn(skz[a], sjz);
+        ei = __fadd_rn(ei, 0.5f * v.v);
+        wi = fmaf(0.5f * v.dr, rij, wi);
     });
 }
 
@@ -581,14 +606,12 @@ __global__ void __launch_bounds__(TB_BLOCK, TERS_CTAS_PER_SM) k_tersoff_a(
     }
 }
 
-// a b + c d rounded as the compiler contracts it in ters_bonds
-__device__ __forceinline__ float fma2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
-
 // The bonds of one centre in the lane form, NJ neighbours a lane: the slots are
 // written, and lane 0 to 4 return the centre's sums.  wide: more neighbours than
-// the register path holds; gjx and the neighbour's part are then rounded as a loop
-// over arrays contracts them, so that a trajectory through a collision stays the one that
-// such a loop gave.  With one neighbour a lane (a small box, where the chain of
+// the register path holds, a centre that only this form takes; of two products
+// that are added the other one is then the one rounded by itself, in gjx and in
+// the neighbour's part.  Neither order is nearer to the exact sum; a collision
+// amplifies the difference, so they stay as trajectories have them.  With one neighbour a lane (a small box, where the chain of
 // one centre is all the time there is) the gradients of all bonds are kept, and
 // added up once at the end: centre pass of 512 atoms 11.9 -> 11.3 us with some 5
 // of launch.
@@ -616,32 +639,21 @@ __device__ __forceinline__ float ters_lanes_bonds(const TersDev& p, const LaneGr
             if (b == a) continue;
             const float4 ub = u[b];
             const float fb = f[b].x;
-            const float c = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
-            const float hc = p.h - c;
-            const float rden = __fdividef(1.f, p.d2 + hc * hc);
-            const float g = g0 - p.c2 * rden;
-            const float dg = -2.f * p.c2 * hc * rden * rden;
-            const float dr = ua.w - ub.w;
-            const float ex = __expf(p.l3c * dr * dr * dr);
-            const float dex = 3.f * p.l3c * dr * dr * ex;
-            zeta += fb * g * ex;
-            const float cj = fb * dg * ex * fa.z, cu = fb * g * dex;
-            gjx = __fadd_rn(gjx, wide ? fma2(cj, fmaf(-c, ua.x, ub.x), cu, ua.x)
-                                      : fma2(cu, ua.x, cj, fmaf(-c, ua.x, ub.x)));
-            gjy = __fadd_rn(gjy, fma2(cu, ua.y, cj, fmaf(-c, ua.y, ub.y)));
-            gjz = __fadd_rn(gjz, fma2(cu, ua.z, cj, fmaf(-c, ua.z, ub.z)));
+            const TersTriplet t(p, g0, ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w);
+            const float fg = __fmul_rn(fb, t.g);
+            zeta = fmaf(fg, t.ex, zeta);
+            const float cj = __fmul_rn(__fmul_rn(__fmul_rn(fb, t.dg), t.ex), fa.z), cu = __fmul_rn(fg, t.dex);
+            const float px = fmaf(-t.c, ua.x, ub.x);
+            gjx = __fadd_rn(gjx, wide ? fma2(cj, px, cu, ua.x) : fma2(cu, ua.x, cj, px));
+            gjy = __fadd_rn(gjy, fma2(cu, ua.y, cj, fmaf(-t.c, ua.y, ub.y)));
+            gjz = __fadd_rn(gjz, fma2(cu, ua.z, cj, fmaf(-t.c, ua.z, ub.z)));
         }
-        const float fR = p.A * __expf(-p.l1 * ua.w), fA = p.B * __expf(-p.l2 * ua.w);
-        float bij, dbdz;
-        ters_bond_order(p, zeta, bij, dbdz);
-        const float vij = fa.x * (fR - bij * fA);
-        const float dv_dr = fma2(fa.y, fmaf(-bij, fA, fR), fa.x, fma2(bij * p.l2, fA, -p.l1, fR));
-        const float dv_dz = -fa.x * fA * dbdz;
-        sjx[j] = 0.5f * (wide ? fma2(dv_dz, gjx, dv_dr, ua.x) : fma2(dv_dr, ua.x, dv_dz, gjx));
-        sjy[j] = 0.5f * (wide ? fma2(dv_dz, gjy, dv_dr, ua.y) : fma2(dv_dr, ua.y, dv_dz, gjy));
-        sjz[j] = 0.5f * (wide ? fma2(dv_dz, gjz, dv_dr, ua.z) : fma2(dv_dr, ua.z, dv_dz, gjz));
-        dz[j] = 0.5f * dv_dz;
-        ve[a] = make_float2(vij, dv_dr);
+        const TersBond v(p, ua.w, fa.x, fa.y, zeta);
+        sjx[j] = 0.5f * (wide ? fma2(v.dz, gjx, v.dr, ua.x) : fma2(v.dr, ua.x, v.dz, gjx));
+        sjy[j] = 0.5f * (wide ? fma2(v.dz, gjy, v.dr, ua.y) : fma2(v.dr, ua.y, v.dz, gjy));
+        sjz[j] = 0.5f * (wide ? fma2(v.dz, gjz, v.dr, ua.z) : fma2(v.dr, ua.z, v.dz, gjz));
+        dz[j] = 0.5f * v.dz;
+        ve[a] = make_float2(v.v, v.dr);
     }
     __syncwarp(g.mask);
 #pragma unroll
@@ -657,13 +669,13 @@ __device__ __forceinline__ float ters_lanes_bonds(const TersDev& p, const LaneGr
     const auto add = [&](int a, float s, const float4* row) {
         if (g.lane < 3) {
             const float* xc = &row[0].x + g.lane;
-            own += xc[4 * a];  // the x_i gradient is minus the sum of the others
+            own = __fadd_rn(own, xc[4 * a]);  // the x_i gradient is minus the sum of the others
             for (int b = 0; b < nc; b++)
                 if (b != a) own = fmaf(s, xc[4 * b], own);
         } else if (g.lane == 3) {
-            own += 0.5f * ve[a].x;
+            own = __fadd_rn(own, 0.5f * ve[a].x);
         } else if (g.lane == 4) {
-            own += 0.5f * ve[a].y * u[a].w;
+            own = fmaf(0.5f * ve[a].y, u[a].w, own);
         }
     };
 #pragma unroll (NJ == 1 ? 2 : 1)
@@ -683,19 +695,13 @@ __device__ __forceinline__ float ters_lanes_bonds(const TersDev& p, const LaneGr
                 continue;
             }
             const float4 uk = u[k], fk = f[k];
-            const float c = ua.x * uk.x + ua.y * uk.y + ua.z * uk.z;
-            const float hc = p.h - c;
-            const float rden = __fdividef(1.f, p.d2 + hc * hc);
-            const float g = g0 - p.c2 * rden;
-            const float dg = -2.f * p.c2 * hc * rden * rden;
-            const float dr = ua.w - uk.w;
-            const float ex = __expf(p.l3c * dr * dr * dr);
-            const float dex = 3.f * p.l3c * dr * dr * ex;
-            const float ck = fma2(fk.y * g, ex, -fk.x * g, dex);
-            const float cc = fk.x * dg * ex * fk.z;
-            const float kx = fma2(ck, uk.x, cc, fmaf(-c, uk.x, ua.x));
-            const float ky = fma2(ck, uk.y, cc, fmaf(-c, uk.y, ua.y));
-            const float kz = fma2(ck, uk.z, cc, fmaf(-c, uk.z, ua.z));
+            const TersTriplet t(p, g0, ua.x, ua.y, ua.z, ua.w, uk.x, uk.y, uk.z, uk.w);
+            const float fg = __fmul_rn(fk.x, t.g);
+            const float ck = fma2(__fmul_rn(fk.y, t.g), t.ex, -fg, t.dex);
+            const float cc = __fmul_rn(__fmul_rn(__fmul_rn(fk.x, t.dg), t.ex), fk.z);
+            const float kx = fma2(ck, uk.x, cc, fmaf(-t.c, uk.x, ua.x));
+            const float ky = fma2(ck, uk.y, cc, fmaf(-t.c, uk.y, ua.y));
+            const float kz = fma2(ck, uk.z, cc, fmaf(-t.c, uk.z, ua.z));
             row[k] = make_float4(kx, ky, kz, 0.f);
             // force on k = -gradient
             skx[j] = fmaf(-s, kx, skx[j]);
@@ -725,8 +731,8 @@ __device__ __forceinline__ float ters_lanes_bonds(const TersDev& p, const LaneGr
 // counted).  A lane owns a neighbour: its bond's zeta and gradient first, then
 // what each bond in turn gives to it as its third atom, for which the factors
 // of the triplet are evaluated again (some 30 instructions).  The centre's sums
-// are taken bond by bond in the register path's order, and the products that
-// join a sum are the ones that do there: both forms give the same bits, and a
+// are taken bond by bond in the register path's order, from the same
+// instructions (TersTriplet, TersBond): both forms give the same bits, and a
 // trajectory does not depend on which took a centre.  The queue was one thread a centre over local
 // arrays, a chain of some 190,000 cycles: 0.7 % of the 1.47 M
 // atoms of the impact ensemble, both passes 199 -> 141 us.

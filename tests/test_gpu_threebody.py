@@ -225,3 +225,38 @@ def test_nve_drift_over_10k_steps(omdg_lib, kind, bound):
         e1 = ctx.ledger()["energy"]
     assert np.isfinite(e1)
     assert abs(e1 - e0) / len(x) < bound
+
+
+@pytest.mark.parametrize("ncell", [6, 11])
+def test_tersoff_forms_have_the_same_bits(omdg_lib, tmp_path, ncell):
+    """The same box through both forms: with a surrogate whose training range
+    holds no atom, every centre takes the masked Tersoff pass (a thread a
+    centre, the crowded ones queued), where plain Tersoff takes eight lanes for
+    every centre of a box this small (1,731 atoms; 10,651 take the threads, and
+    the pass is its own check).  The list ranges are made equal: rows and order
+    of the sums are the same, and the surrogate's further hits add zeros."""
+    x, v, lo, hi = interstitial_silicon(ncell, 71)
+    model = str(tmp_path / "none.nn")
+    with omdg_lib.Network(0) as net:
+        net.set_normalization(np.zeros(32), np.ones(32), np.full(32, 1e9), np.full(32, 2e9))
+        net.set_weights(np.zeros(6337))
+        net.save(model)
+    out = []
+    for surrogate in (True, False):
+        with si_context(omdg_lib, x, v, lo, hi, "tersoff") if not surrogate else omdg_lib.Context(0) as ctx:
+            if surrogate:
+                from objectmd_gb300 import inputs
+
+                ctx.set_box(lo, hi)
+                ctx.set_atoms(x, v, masses=[inputs.md_mass("silicon")], znum=[14.0])
+                ctx.add_nn(model, TERSOFF_FILE)
+                reach = ctx.max_cut_radius() + 0.3
+            ctx.set_neighbor(reach - ctx.max_cut_radius(), 1)
+            ctx.compute_forces()
+            if surrogate:
+                assert ctx.nn_fallback_atoms() == len(x)
+            assert ctx.wide_centres() >= 3
+            st = ctx.get_state()
+            out.append((st["f"], st["pot"], st["vir"], np.concatenate(ctx.neighbors())))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
