@@ -296,17 +296,34 @@ struct AtomArrays {
     int extra_n;
 };
 
+// Replica mode: every replica has its own periodic lengths and cell grid,
+// and its cells occupy the global cell range [cell_base, cell_base + cells).
+struct RepGeom {
+    double lo[3], L[3], cell_org[3], cell_h[3], inv_h[3];
+    int nc[3], periodic[3];
+    int cell_base;
+    ShiftF S;
+};
+
 // The pack coordinate is X = x + Q with Q = P - org, formed as FP32 hi + lo
 // by pack_coord (the integrator refreshes the pack with the same function).
 struct PackFrame {
     float Qh[3], Ql[3];
 };
 
-// loc: the position rounded to FP32, which the list build screens (w: the type)
+struct Corner {
+    double lo[3];
+};
+
+// loc: the position from the box's (or the replica's) lower corner lo, rounded
+// to FP32, which the list build screens (w: the type).  From the origin the
+// band of pairs that take the FP64 test would grow with the box's distance from
+// it: 256,000 EAM atoms, build and sort 254 us at the origin, 586 at an offset
+// of 3e4 A, 3,550 at 1e6 A; now 254 at all three.
 // One atom's packs; returns its share of umax.
 __device__ __forceinline__ float pack_atom(int i, double X, double Y, double Z, int type, bool active,
-                                           const PackFrame& f, PosPack* __restrict__ pack, float4* __restrict__ xref,
-                                           float4* __restrict__ loc) {
+                                           const PackFrame& f, const double* lo, PosPack* __restrict__ pack,
+                                           float4* __restrict__ xref, float4* __restrict__ loc) {
     PosPack p;
     pack_coord(X, f.Qh[0], f.Ql[0], p.hi.x, p.lo.x);
     pack_coord(Y, f.Qh[1], f.Ql[1], p.hi.y, p.lo.y);
@@ -322,13 +339,13 @@ __device__ __forceinline__ float pack_atom(int i, double X, double Y, double Z, 
         loc[i] = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f);
         return 0.f;
     }
-    const float ux = f2_from(X).hi, uy = f2_from(Y).hi, uz = f2_from(Z).hi;
+    const float ux = f2_from(X - lo[0]).hi, uy = f2_from(Y - lo[1]).hi, uz = f2_from(Z - lo[2]).hi;
     loc[i] = make_float4(ux, uy, uz, p.hi.w);
     const float m = fmaxf(fabsf(ux), fmaxf(fabsf(uy), fabsf(uz)));
     return m <= 3.0e38f ? m : 3.0e38f;  // non-finite: flagged by the cell assignment
 }
 
-// The largest |x| sets the width of the screening band.  Whole warps.
+// The largest |x - lo| sets the width of the screening band.  Whole warps.
 __device__ __forceinline__ void pack_umax(float m, unsigned* umax) {
     m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
     if ((threadIdx.x & 31) == 0 && m > 0.f && __float_as_uint(m) > *(volatile unsigned*)umax)
@@ -343,7 +360,8 @@ __device__ __forceinline__ void pack_umax(float m, unsigned* umax) {
 __global__ void k_permute_gather(int n, const int* __restrict__ perm, AtomArrays a, AtomArrays st,
                                  const int* __restrict__ cell_old, int* __restrict__ cell_new,
                                  int* __restrict__ inv, const int* __restrict__ rep_of,
-                                 const int* __restrict__ rflag, PackFrame f, const unsigned* __restrict__ aflag,
+                                 const int* __restrict__ rflag, PackFrame f, Corner corner,
+                                 const RepGeom* __restrict__ rg, const unsigned* __restrict__ aflag,
                                  PosPack* __restrict__ pack, float4* __restrict__ xref, float4* __restrict__ loc,
                                  unsigned* umax) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -365,7 +383,7 @@ __global__ void k_permute_gather(int n, const int* __restrict__ perm, AtomArrays
         st.id[k] = a.id[o];
         st.flag[k] = flag;
         for (int q = 0; q < a.extra_n; q++) st.extra[(size_t)q * n + k] = a.extra[(size_t)q * n + o];
-        u = pack_atom(k, X, Y, Z, type, !aflag || (flag & 1u), f, pack, xref, loc);
+        u = pack_atom(k, X, Y, Z, type, !aflag || (flag & 1u), f, rg ? rg[rep_of[k]].lo : corner.lo, pack, xref, loc);
     }
     pack_umax(u, umax);
 }
@@ -444,20 +462,11 @@ __global__ void k_rep_build_done(int nrep, int full, int* __restrict__ rflag, in
 }
 
 
-// Replica mode: every replica has its own periodic lengths and cell grid,
-// and its cells occupy the global cell range [cell_base, cell_base + cells).
-struct RepGeom {
-    double lo[3], L[3], cell_org[3], cell_h[3], inv_h[3];
-    int nc[3], periodic[3];
-    int cell_base;
-    ShiftF S;
-};
-
 __global__ void k_pack(int n, const double* __restrict__ x, const double* __restrict__ y,
                        const double* __restrict__ z, const int* __restrict__ type, PackFrame f,
                        PosPack* __restrict__ pack) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) pack_atom(i, x[i], y[i], z[i], type[i], true, f, pack, nullptr, nullptr);
+    if (i < n) pack_atom(i, x[i], y[i], z[i], type[i], true, f, nullptr, pack, nullptr, nullptr);
 }
 
 // EAM cell tiles: besides the list entry, the build writes each entry's
@@ -486,6 +495,7 @@ struct BuildParams {
     double L64[3];
     double rsq;           // Rv*Rv in FP64 (VerletList.cpp:161)
     float rv;             // Rv rounded to FP32
+    float corner_err;     // FP64 rounding of two atoms' x - lo
     float lmax;           // largest periodic length (screening band)
 };
 
@@ -565,7 +575,7 @@ __device__ __noinline__ bool exact_within(double Lx, double Ly, double Lz, doubl
 // The list build.  The candidates of the 27 cells are 9 runs of back-to-back
 // atoms (axis_run); a candidate costs one 16-byte load of its FP32 position,
 // four of them in flight, and the squared length of the difference.  Every
-// FP32 step errs by at most an ulp of max|x| + L, so pairs within a band of
+// FP32 step errs by at most an ulp of the box's extent, so pairs within a band of
 // Rv (a few 1e-4 A for boxes of a few hundred A: one atom in thirty has such
 // a pair), and pairs close enough to be an overlap, take the reference's FP64
 // test, out of line: the list is the reference's exactly, in the traversal
@@ -667,7 +677,7 @@ __device__ __forceinline__ void build_centre(
     // differences each round by half an ulp of at most U; 2x margin, sqrt(3)
     // for the length and 1e-6 relative for the squares
     const float U = __uint_as_float(*umax) + p.lmax;
-    const float dlt = 1.7320509f * (6.f * U * 1.1920929e-7f) + 1e-6f * p.rv;
+    const float dlt = 1.7320509f * (6.f * U * 1.1920929e-7f + p.corner_err) + 1e-6f * p.rv;
     const float rl = fmaxf(p.rv - dlt, 0.f), rh = p.rv + dlt, ro = 1.0e-3f + dlt;
     const float rsq_lo = rl * rl * (1.f - 1e-6f), rsq_hi = rh * rh * (1.f + 1e-6f), rsq_ov = ro * ro;
     const int nx = REP ? g->nc[0] : p.nc[0], ny = REP ? g->nc[1] : p.nc[1], nz = REP ? g->nc[2] : p.nc[2];
@@ -1384,8 +1394,8 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
         a.a.flag[k] = flag[w];
         a.cell[k] = c[w];
         a.inv[id[w]] = k;
-        u = fmaxf(u, pack_atom(k, p[w][0], p[w][1], p[w][2], type[w], !a.aflag || (flag[w] & 1u), a.f, a.pack, a.xref,
-                               a.loc));
+        u = fmaxf(u, pack_atom(k, p[w][0], p[w][1], p[w][2], type[w], !a.aflag || (flag[w] & 1u), a.f, geom.lo, a.pack,
+                               a.xref, a.loc));
     }
     pack_umax(u, a.umax);
     for (int q = 0; q < a.a.extra_n; q++) {
@@ -1614,7 +1624,7 @@ int nlist_build(Context* c, bool on_request) {
                        c->stage_extra, c->extra_n};
         k_permute_gather<<<grid_for(n, 256), 256, 0, s>>>(n, c->perm, cur, stg, c->cell, cell_sorted, c->inv,
                                                           c->d_rep_of, rflag, pack_frame(c),
-                                                          c->flags_used ? c->aflag : nullptr, c->pack, c->xref, c->loc,
+                                                          Corner{g.lo[0], g.lo[1], g.lo[2]}, rg, c->flags_used ? c->aflag : nullptr, c->pack, c->xref, c->loc,
                                                           umax);
         k_permute_copyback<<<grid_for(n, 256), 256, 0, s>>>(n, stg, cur, c->d_rep_of, rflag);
         c->launches += 2;
@@ -1677,6 +1687,11 @@ int nlist_build(Context* c, bool on_request) {
     for (int d = 0; d < 3; d++)
         if (g.periodic[d]) bp.lmax = fmaxf(bp.lmax, (float)g.L[d]);
     if (reps) bp.lmax = (float)c->rep_lmax;
+    double far = 0.0;  // the corner farthest from the origin
+    for (int d = 0; d < 3; d++) far = std::max(far, std::fabs(g.lo[d]));
+    if (reps)
+        for (double q : c->rep_lo) far = std::max(far, std::fabs(q));
+    bp.corner_err = (float)(far * 0x1p-51);
     // shared-memory columns: maxnb is twice the mean row and 32 at first, so
     // half of it and 8 holds nearly every row; 64 entries (32 KB a block)
     // keep seven blocks on a SM.  Longer rows go out in pieces.

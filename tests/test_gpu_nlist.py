@@ -257,3 +257,64 @@ def test_the_graph_of_steps_runs(omdg_lib, ncell):
     assert rebuilds[0] == rebuilds[1] == rebuilds[2]
     per_call = (launches[0] - launches[1]) / 16
     assert launches[1] - launches[2] == 8 * per_call + 7 * 8
+
+
+@pytest.mark.parametrize("offset", [(0.0, 0.0, 0.0), (3.0e4, -7.0e5, 12.5), (1.0e6, 1.0e6, 1.0e6), (-5.0e8, 0.0, 3.0e3)])
+def test_boxes_far_from_the_origin(omdg_lib, oracle_lib, offset):
+    """The list is the oracle's wherever the box lies, from one thread and from
+    eight lanes a centre, as a box and as two replicas."""
+    from objectmd_gb300 import inputs
+
+    oc = oracle_lib
+    rv = cutoff(oc)
+    x, _, (lo, hi) = inputs.eam_aluminium(ncell=6, a=4.05, sigma=0.1, temp=0.0, seed_pos=31, seed_vel=32)
+    offset = np.asarray(offset)
+    x, lo, hi = x + offset, np.asarray(lo) + offset, np.asarray(hi) + offset
+    ref = nbr_set(*oc.neighbors(oc.make_box(lo, hi, (1, 1, 0)), x, rv))
+    for mode in (1, 8):
+        with context(omdg_lib, x, lo, hi, (1, 1, 0), mode) as ctx:
+            ctx.build_neighbors()
+            assert nbr_set(*ctx.neighbors()) == ref
+    n = len(x)
+    with omdg_lib.Context(0) as ctx:
+        far = np.array([2.0e5, 0.0, -4.0e4])
+        ctx.set_replicas([n, n], [lo, lo + far], [hi, hi + far], (1, 1, 0))
+        ctx.set_atoms(np.vstack([x, x + far]), masses=[inputs.md_mass("silicon")], znum=[14.0])
+        ctx.add_tersoff(os.path.join(TABLES, "tersoff.silicon27"))
+        ctx.set_neighbor(rv - ctx.max_cut_radius(), 1)
+        ctx.build_neighbors()
+        rows = nbr_set(*ctx.neighbors())
+    assert {q for q in rows if q[0] < n} == ref
+    moved = nbr_set(*oc.neighbors(oc.make_box(lo + far, hi + far, (1, 1, 0)), x + far, rv))
+    assert {(i - n, j - n, *s) for i, j, *s in rows if i >= n} == moved
+
+
+def test_a_build_takes_as_long_far_from_the_origin(omdg_lib):
+    """256,000 atoms at the origin and 10^6 A away: from the box's corner the
+    FP32 screen leaves as few pairs to the FP64 test (from the origin a build
+    there took 14 times as long)."""
+    import torch
+
+    from objectmd_gb300 import inputs
+
+    x, lo, hi = inputs.fcc((40, 40, 40), 4.05)
+    x = inputs.perturb(x, 0.05, 5, lo, hi)
+    best = []
+    for offset in (0.0, 1.0e6):
+        with omdg_lib.Context(0) as ctx:
+            ctx.set_box(np.asarray(lo) + offset, np.asarray(hi) + offset)
+            ctx.set_atoms(x + offset, masses=[inputs.md_mass("aluminum")], znum=[13.0])
+            ctx.add_eam(EAM_TABLE)
+            ctx.set_neighbor(SKIN, 0)
+            ctx.build_neighbors()
+            stream = torch.cuda.ExternalStream(ctx.stream())
+            times = []
+            for _ in range(10):
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record(stream)
+                ctx.build_neighbors()
+                b.record(stream)
+                b.synchronize()
+                times.append(a.elapsed_time(b))
+            best.append(min(times))
+    assert best[1] < 3.0 * best[0], best
