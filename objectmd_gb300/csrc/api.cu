@@ -1504,7 +1504,10 @@ namespace omdg {
 // or before the one that overflowed.  Restore it, grow the rows, redo that
 // rebuild and the rest of its step, then replay the steps still owed.  The counting sort and the list are deterministic functions of
 // that state, so the trajectory is the one an ample capacity gives, bit for
-// bit.  (The two-temperature model keeps electron state outside the
+// bit.  What the steps after the overflow did with truncated rows (a slot whose
+// writer was dropped holds anything) is discarded with the errors it raised;
+// an error from before the snapshot stands, and one from after it comes up
+// again in the replay.  (The two-temperature model keeps electron state outside the
 // snapshot; a run with it reports the overflow instead.)
 static int recover_overflow(omdg_ctx* c) {
     const long owed_total = c->async_steps;
@@ -1570,9 +1573,13 @@ int omdg_sync(omdg_ctx* c) {
     const int expect = (c->async_steps > 0 && c->async_steps <= c->ledger_cap) ? (int)c->async_steps : 0;
     int rc = step_state_fetch(c, &status, &step, &rows, &elapsed, expect);  // waits for the queued steps
     if (rc) return rc;
-    if ((status & ERR_NBR_OVERFLOW) && !(status & ~ERR_NBR_OVERFLOW) && c->async_steps > 0 && c->snap_d &&
-        !(c->ttm && ttm_active(c)))
-        return recover_overflow(c);
+    if ((status & ERR_NBR_OVERFLOW) && c->async_steps > 0 && c->snap_d && !(c->ttm && ttm_active(c))) {
+        int snap[2] = {0, 0};  // taken by these steps; the error bits before it
+        cudaError_t e = cudaMemcpy(snap, c->d_flags + 6, sizeof(snap), cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return check_cuda(c, e, "overflow recovery");
+        if (snap[0] && !snap[1]) return recover_overflow(c);
+        if (snap[0] && snap[1]) status = (unsigned)snap[1];
+    }
     if ((rc = status_error(c, status))) {
         if (rc == OMDG_ESTATE) {
             // a neighbour row overflowed during the run: grow for the next call

@@ -396,9 +396,10 @@ __global__ void k_permute_gather(int n, const int* __restrict__ perm, AtomArrays
 // that earlier state and replays from there, which reaches the same state.
 __global__ void k_snapshot(int n, const int* __restrict__ halted, const int* __restrict__ taken, AtomArrays a,
                            AtomArrays snap, const unsigned char* __restrict__ st, unsigned char* __restrict__ st_snap,
-                           int st_bytes) {
+                           int st_bytes, const unsigned* __restrict__ status, int* __restrict__ errors) {
     if (*halted || *taken) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0) *errors = (int)*status;
     if (k < st_bytes) st_snap[k] = st[k];
     if (k >= n) return;
     snap.x[k] = a.x[k];
@@ -1214,7 +1215,7 @@ struct SortArgs {
     PackFrame f;
     StepState* st;
     unsigned* status;
-    int* taken;
+    int* taken;  // [1]: the error bits at the time
     AtomArrays a, snap;  // snap.x null: no snapshot
     unsigned char* st_snap;
     int *count, *start, *perm, *cell, *inv;
@@ -1273,6 +1274,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
         }
     }
     const bool snap = !REP && a.snap.x && !a.st->halted && !*a.taken;
+    const unsigned errors = *a.status;  // before this sort
     double p[PER][3], v[PER][3];
     int type[PER], id[PER], c[PER], slot[PER];
     unsigned flag[PER];
@@ -1314,7 +1316,10 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(SortArgs a) {
         if (snap) {  // the state as it is after the request was taken
             __syncthreads();
             if (t < a.st_bytes) a.st_snap[t] = reinterpret_cast<const unsigned char*>(a.st)[t];
-            if (t == 0) *a.taken = 1;
+            if (t == 0) {
+                a.taken[0] = 1;
+                a.taken[1] = (int)errors;
+            }
         }
     }
 #pragma unroll
@@ -1574,7 +1579,7 @@ int nlist_build(Context* c, bool on_request) {
         int* taken = c->d_flags + 6;
         k_snapshot<<<grid_for(std::max(n, sb), 256), 256, 0, s>>>(
             n, step_state_halted(c), taken, cur0, snap, static_cast<const unsigned char*>(c->d_state),
-            static_cast<unsigned char*>(c->snap_state), sb);
+            static_cast<unsigned char*>(c->snap_state), sb, c->d_status, taken + 1);
         k_set_one<<<1, 1, 0, s>>>(taken);
         c->launches += 2;
     }

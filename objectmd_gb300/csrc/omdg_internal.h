@@ -329,7 +329,8 @@ struct Context {
     int* d_flags = nullptr;         // [0] rebuild request, [1] row length needed, [2] ghost count,
                                     // [3] largest coordinate of the last build (float bits),
                                     // [4] blocks done in the current kick (reset by the last block),
-                                    // [5] atoms of the replicas a partial build takes, [6] snapshot taken
+                                    // [5] atoms of the replicas a partial build takes, [6] snapshot taken,
+                                    // [7] error bits there were when it was
     double* d_red = nullptr;        // block partials
     int red_cap = 0;
     double* d_ledger = nullptr;     // per step LEDGER_W doubles: kinetic, potential, virial, lambda,

@@ -118,3 +118,63 @@ def test_a_replica_rebuilt_alone_overflows(omdg_lib, sizes):
         d = tight[at:at + n] - ample[at:at + n]
         assert np.abs(d - L * np.round(d / L)).max() <= 1e-5
         at += n
+
+
+def test_errors_of_discarded_steps_do_not_stop_the_recovery(omdg_lib):
+    """Many steps after the overflow in the same call: truncated rows may drive
+    atoms anywhere, to non-finite positions too, but those steps are replayed.
+    The same call ten times, since what a dropped slot holds is left open."""
+    case = converging_silicon(6, 12.0, 1.2)
+    with context(omdg_lib, "sw", *case, 0) as ctx:
+        ctx.step(2)
+        capacity = longest(ctx)
+        ctx.step(198)
+        ample = ctx.get_state()
+    for _ in range(10):
+        with context(omdg_lib, "sw", *case, capacity) as ctx:
+            ctx.step(2)
+            ctx.step(198)
+            st = ctx.get_state()
+            assert longest(ctx) > capacity
+        for k in ("x", "v", "f", "pot"):
+            assert np.array_equal(st[k], ample[k]), k
+
+
+@pytest.mark.parametrize("collide", [True, False])
+def test_an_error_before_the_overflow_stands(omdg_lib, collide):
+    """Two argon atoms shot at each other pass the table's first knot before the
+    call's first rebuild (a skin of 4 A, a rebuild every 200 steps); there the
+    rows, all alike in the crystal, overflow, as they do without the shot.  The table's error is reported, not lost in a replay."""
+    from objectmd_gb300 import inputs
+
+    table = os.path.join(TABLES, "pair.lj.argon")
+    x, v, (lo, hi) = inputs.lj_argon(ncell=8, temp=120.0)
+    if collide:
+        x = np.vstack([x, [[1.3, 1.3, 1.3], [4.3, 1.3, 1.3]]])
+        v = np.vstack([v, [[120.0, 0.0, 0.0], [-120.0, 0.0, 0.0]]])
+        keep = np.linalg.norm(x[:-2] - np.array([2.8, 1.3, 1.3]), axis=1) > 4.5
+        keep = np.append(keep, [True, True])
+        x, v = x[keep], v[keep]
+
+    def context(capacity):
+        ctx = omdg_lib.Context(0)
+        ctx.set_box(lo, hi)
+        ctx.set_atoms(x, v, masses=[inputs.md_mass("argon")], znum=[18.0])
+        ctx.add_pair_table(table)
+        if capacity:
+            ctx.set_launch("nbr_capacity", capacity)
+        ctx.set_neighbor(4.0, 200)
+        ctx.set_timestep(0.0005)
+        return ctx
+
+    with context(0) as ctx:
+        ctx.build_neighbors()
+        capacity = longest(ctx)
+    with context(capacity) as ctx:
+        if collide:
+            with pytest.raises(omdg_lib.OMDGError) as err:
+                ctx.step(600)
+            assert err.value.code == omdg_lib.OMDG_ERANGE
+        else:
+            ctx.step(600)
+            assert longest(ctx) > capacity
