@@ -1575,9 +1575,13 @@ int omdg_sync(omdg_ctx* c) {
     if (rc) return rc;
     if ((status & ERR_NBR_OVERFLOW) && c->async_steps > 0 && c->snap_d && !(c->ttm && ttm_active(c))) {
         int snap[2] = {0, 0};  // taken by these steps; the error bits before it
+        int need = 0;
         cudaError_t e = cudaMemcpy(snap, c->d_flags + 6, sizeof(snap), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaMemcpy(&need, c->d_flags + 1, sizeof(int), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return check_cuda(c, e, "overflow recovery");
-        if (snap[0] && !snap[1]) return recover_overflow(c);
+        // (a centre with more in-cutoff neighbours than its pass holds sets the
+        // same bit, and would set it again in the replay, whatever the rows)
+        if (snap[0] && !snap[1] && need > c->maxnb) return recover_overflow(c);
         if (snap[0] && snap[1]) status = (unsigned)snap[1];
     }
     if ((rc = status_error(c, status))) {

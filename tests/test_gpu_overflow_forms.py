@@ -178,3 +178,20 @@ def test_an_error_before_the_overflow_stands(omdg_lib, collide):
         else:
             ctx.step(600)
             assert longest(ctx) > capacity
+
+
+def test_more_neighbours_than_a_centre_holds_is_an_error(omdg_lib):
+    """Silicon driven together until a centre has more than the 24 neighbours
+    inside the cutoff that a three-body pass holds (with room in the rows): an
+    error, which no growth of the rows would mend."""
+    from objectmd_gb300 import inputs
+
+    x, lo, hi = inputs.diamond((6, 6, 6), 4.62)
+    d = x - 0.5 * (np.asarray(lo) + np.asarray(hi))
+    inner = np.linalg.norm(d, axis=1) < 12.0
+    v = np.zeros_like(x)
+    v[inner] = -3.0 * d[inner]
+    with context(omdg_lib, "sw", x, v, lo, hi, 400) as ctx:
+        with pytest.raises(omdg_lib.OMDGError) as err:
+            ctx.step(200)
+        assert err.value.code == omdg_lib.OMDG_ESTATE
