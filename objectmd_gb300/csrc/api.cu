@@ -266,7 +266,6 @@ struct GraphState {
     cudaGraphExec_t many_exec = nullptr;
     cudaGraph_t many_graph = nullptr;
     bool many_valid = false, many_failed = false;
-    int many_joined = 0;  // kernels fewer than as many single steps have
     long replayed = 0;
     // the same step with download branches into pinned host arrays
     // (omdg_step_io), keyed by the x, v, f output pointers
@@ -275,7 +274,7 @@ struct GraphState {
     cudaStream_t io_side = nullptr;
     cudaEvent_t io_ev[4] = {};
     double* io_key[3] = {};
-    long io_kernels = 0;
+    long kernels = 0, many_kernels = 0, io_kernels = 0;  // of a replay, outside the rebuild body
     bool io_valid = false;
 };
 static std::map<Context*, GraphState> g_graphs;
@@ -945,7 +944,7 @@ static int issue_forces(Context* c) {
     // or the detector works on the forces in between (a potential after it would
     // be added before the slots instead of after them: another rounding)
     const Potential* last_slots = nullptr;
-    if (c->fuse_kick && !c->use_f64 && c->post_ops.empty() && !c->ttm)
+    if (c->fuse_kick && !c->forces_out && !c->use_f64 && c->post_ops.empty() && !c->ttm)
         for (auto& p : c->pots)
             if (!p.fallback_only)
                 last_slots = p.kind == POT_SW || p.kind == POT_TERSOFF || p.kind == POT_NN ? &p : nullptr;
@@ -1010,6 +1009,14 @@ static int eager_maybe_rebuild(Context* c) {
 // eight; without the node 6.2, 2.6, 2.6), a capture and instantiation some 0.1
 // to 1 ms, so the graph is made once a run has replayed GRAPH_AFTER steps of
 // the same context one by one.
+//
+// io with forces: where the slot gather would join the kick it stays apart, so
+// that the forces go out beside the kick; with velocities to write as well,
+// which go out after it anyway, only where the copies are long.  us a step,
+// joined and apart, f alone: 8,000 Tersoff atoms 48.0 and 47.0, 512,000 186.6 and
+// 174.2, 195,112 SW atoms 147 and 137; x, v and f: 8,000 52.0 and 53.6, 125,000
+// 105.4 and 107.6, 195,112 SW 188.5 and 188.6, 512,000 294 and 289.6.
+constexpr int IO_APART_PER_SM = 2048;
 constexpr int GRAPH_STEPS = 8;
 constexpr long GRAPH_AFTER = 64;
 static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr, int steps = 1) {
@@ -1032,10 +1039,9 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
     cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return check_cuda(c, e, "capture begin");
     const long launches0 = c->launches, rebuilds0 = c->rebuilds;
-    long l0 = 0, l1 = 0, l2 = 0, l3 = 0;
+    long l0 = 0, l1 = 0, l2 = 0, kernels = 0;
     int rc = OMDG_OK;
     bool drifted = false;  // the step's kick_drift was in the last one's kick
-    int joined = 0;
     cudaGraphConditionalHandle h = 0;
     const bool on_request = small_sort(c);  // the rebuild's kernels are the step's own, and look for the request
     const auto new_handle = [&]() -> int {
@@ -1101,15 +1107,15 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
         l2 = c->launches;
         if (!rc && io) rc = branch(0, io[0], nullptr, nullptr);
         c->fuse_kick = true;
+        c->forces_out = io && io[2] && (!io[1] || c->n >= IO_APART_PER_SM * c->num_sms);
         if (!rc) rc = forces_compute(c, true);
-        c->fuse_kick = false;
+        c->fuse_kick = c->forces_out = false;
         const bool f_after = c->gather_deferred;  // the kick completes the forces
         if (!rc && io && !f_after) rc = branch(1, nullptr, nullptr, io[2]);
         if (!rc && k + 1 < steps && drift_joins(c)) {
             rc = new_handle();
             if (!rc) rc = integrate_kick_and_drift(c, on_request ? nullptr : &h);
             drifted = true;
-            joined++;
         } else if (!rc) {
             rc = integrate_kick(c, 0);
         }
@@ -1120,13 +1126,11 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
             if (e == cudaSuccess) e = cudaStreamWaitEvent(s, gs.io_ev[3], 0);
             if (e != cudaSuccess) rc = check_cuda(c, e, "download join");
         }
-        l3 = c->launches;
+        kernels += (l1 - l0) + (c->launches - l2);
     }
     // captured launches are counted when the graph replays, not here
-    if (steps == 1) {
-        c->graph_step_kernels = (l1 - l0) + (l3 - l2);
-        c->graph_body_kernels = l2 - l1;
-    }
+    (steps > 1 ? gs.many_kernels : io ? gs.io_kernels : gs.kernels) = kernels + io_launches;
+    c->graph_body_kernels = l2 - l1;
     c->launches = launches0;
     c->captured_builds += c->rebuilds - rebuilds0;
     cudaGraph_t graph = nullptr;
@@ -1148,12 +1152,10 @@ static int capture_step(Context* c, GraphState& gs, double* const* io = nullptr,
         gs.io_exec = exec;
         gs.io_valid = true;
         for (int k = 0; k < 3; k++) gs.io_key[k] = io[k];
-        gs.io_kernels = io_launches;
     } else if (steps > 1) {
         gs.many_graph = graph;
         gs.many_exec = exec;
         gs.many_valid = true;
-        gs.many_joined = joined;
     } else {
         gs.graph = graph;
         gs.exec = exec;
@@ -1484,10 +1486,9 @@ int omdg_step_async(omdg_ctx* c, int nsteps) {
             cudaError_t e = cudaGraphLaunch(many ? gs.many_exec : gs.exec, c->stream);
             if (e != cudaSuccess) return check_cuda(c, e, "graph launch");
             k += many ? GRAPH_STEPS : 1;
-            if (many) c->launches -= gs.many_joined;
+            c->launches += many ? gs.many_kernels : gs.kernels;
         }
         gs.replayed += nsteps;
-        c->graph_steps += nsteps;
     }
     c->async_steps += nsteps;
     if (nsteps > 0 && c->thermo_tau > 0.0) c->lambda_pending = true;
@@ -1680,7 +1681,6 @@ int omdg_step_io(omdg_ctx* c, const double* x_in, const double* v_in, int nsteps
     }
     cudaError_t e = cudaGraphLaunch(gs.io_exec, c->stream);
     if (e != cudaSuccess) return check_cuda(c, e, "graph launch");
-    c->graph_steps += 1;
     c->launches += gs.io_kernels;
     c->async_steps += 1;
     const long rec0 = c->overflow_recoveries;
@@ -1880,7 +1880,7 @@ int omdg_stats(omdg_ctx* c, long* rebuilds, long* launches) {
     long eager = c->rebuilds - c->captured_builds;
     if (rebuilds) *rebuilds = eager + graph_builds;
     // kernels issued so far: eager launches plus graph replays
-    if (launches) *launches = c->launches + c->graph_steps * c->graph_step_kernels + graph_builds * c->graph_body_kernels;
+    if (launches) *launches = c->launches + graph_builds * c->graph_body_kernels;
     (void)gs;
     return OMDG_OK;
 }

@@ -198,6 +198,7 @@ struct Context {
     int* d_cell_rep = nullptr;           // replica of each cell (rep_cells)
     bool build_partial = false;          // the build being issued rebuilds only the flagged replicas
     bool fuse_kick = false;              // the forces being issued are a step's: the kick may join them
+    bool forces_out = false;             // ... and go to the host beside the kick: no gather joins it
     bool kick_fused = false;             // the last force launch did the step's second half-kick
     bool defer_gather = false;           // the slot gather being issued may join the step's kick
     bool gather_deferred = false;        // ... and does: the kick collects the slots
@@ -221,8 +222,6 @@ struct Context {
     size_t io_cap = 0;
     long async_steps = 0;        // steps enqueued since the last omdg_sync
     long launches_at_sync = 0, last_launches = 0;
-    long graph_steps = 0;        // graph replays issued
-    long graph_step_kernels = 0; // kernels per replay (outside the rebuild body)
     long graph_body_kernels = 0; // kernels in the rebuild body
     long captured_builds = 0;    // list builds issued while capturing (never ran)
     void* d_state = nullptr;     // StepState (integrate.cu)

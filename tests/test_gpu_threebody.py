@@ -260,3 +260,36 @@ def test_tersoff_forms_have_the_same_bits(omdg_lib, tmp_path, ncell):
             out.append((st["f"], st["pot"], st["vir"], np.concatenate(ctx.neighbors())))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("kind,ncell", [("sw", 6), ("tersoff", 6), ("tersoff", 34)])
+def test_forces_go_out_beside_the_kick(omdg_lib, kind, ncell):
+    """omdg_step_io with forces: the slot gather stays a kernel of its own, so
+    that they need not wait for the kick (with velocities too, in a box above
+    2,048 atoms a SM): one launch more than a step that only velocities leave.
+    Values as get_state gives them."""
+    import torch
+
+    from objectmd_gb300 import inputs
+
+    x, v, (lo, hi) = inputs.diamond_silicon(ncell=ncell, a=5.431, sigma=0.03, temp=300.0, seed_pos=4, seed_vel=5)
+    n = len(x)
+    out = {k: torch.empty((n, 3), dtype=torch.float64).pin_memory().numpy() for k in ("x_out", "v_out", "f_out")}
+    launches = {}
+    with si_context(omdg_lib, x, v, lo, hi, kind) as ctx:
+        ctx.set_neighbor(1.0, 0)
+        ctx.set_timestep(0.0001)
+        for want in (("v_out",), ("f_out",), ("x_out", "v_out"), ("x_out", "v_out", "f_out")):
+            ctx.step_io(1, **{k: out[k] for k in want})
+            before = ctx.stats()
+            ctx.step_io(1, **{k: out[k] for k in want})
+            after = ctx.stats()
+            assert after["rebuilds"] == before["rebuilds"]
+            launches[want] = after["launches"] - before["launches"]
+            st = ctx.get_state()
+            for k in want:
+                assert np.array_equal(out[k], st[k[0]]), (want, k)
+    assert launches[("f_out",)] == launches[("v_out",)] + 1
+    # f beside the kick is a launch and a gather more, f with v after it nothing
+    apart = n >= 2048 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert launches[("x_out", "v_out", "f_out")] == launches[("x_out", "v_out")] + (2 if apart else 0)
