@@ -729,7 +729,7 @@ int step_state_read(Context* c, long long* step, int* row, int* rebuild) {
 }
 
 int step_state_init(Context* c) {
-    StepState h;
+    StepState h{};  // every word and the padding: the whole of it is copied
     h.step = 0;
     h.row = 0;
     h.rebuild = 0;
