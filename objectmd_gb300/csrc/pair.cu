@@ -304,9 +304,9 @@ static void launch64(Context* c, const PairParams& p) {
 // Few lanes an atom waste the least on ragged rows and on the sums' exchange,
 // many shorten the dependent chain where the chip is not full (a warp alone
 // takes about 2 us per row entry).  LJ argon, 79 entries, us with 8 / 16 / 32
-// lanes before the root's Newton step: 500 atoms 25.7 / 17.1 / 14.0, 2,048
-// atoms 26.1 / 19.9 / 23.7, 4,000 atoms 30.9 / 31.8 / 40.0, 16,384 atoms 95 /
-// 104 / 132.
+// lanes: 500 atoms 27.4 / 18.6 / 13.8, 1,372 27.4 / 19.1 / 18.8, 2,048 28.4 /
+// 21.5 / 24.4, 2,916 29.0 / 26.6 / 31.4, 4,000 33.1 / 33.6 / 41.0, 16,384 103 / 111 /
+// 140.  (8 and 16 meet between 3,000 and 4,000 atoms, where they are within 8 %.)
 static void launch64(Context* c, const PairParams& p) {
     if (c->n >= 20 * c->num_sms) launch64<8>(c, p);
     else if (c->n >= 8 * c->num_sms) launch64<16>(c, p);
