@@ -54,17 +54,18 @@ __device__ __forceinline__ void build_shift_table(const EAMFast& p, float4* s_hi
 }
 
 // d = x_i - (x_j + s L) with the shift from the table (exact hi differences,
-// see pair_delta in device_common.cuh).  Most entries of a large box have no
-// shift, and subtracting its zeros would change nothing: they skip the table's
-// two 16-byte loads.
+// see pair_delta in device_common.cuh).  SKIP: most entries of a large box have
+// no shift, and subtracting its zeros would change nothing: they skip the
+// table's two 16-byte loads.
 constexpr unsigned NO_SHIFT = 1u | 1u << 2 | 1u << 4;  // the image bits of (0, 0, 0)
 
+template <bool SKIP>
 __device__ __forceinline__ float3 delta_tab(const float4& hi, const float4& lo, const float4& hj, const float4& lj,
                                             unsigned ent, const float4* s_hi, const float4* s_lo) {
     float ax = __fsub_rn(hi.x, hj.x), ay = __fsub_rn(hi.y, hj.y), az = __fsub_rn(hi.z, hj.z);
     float bx = __fsub_rn(lo.x, lj.x), by = __fsub_rn(lo.y, lj.y), bz = __fsub_rn(lo.z, lj.z);
     const unsigned code = ent >> 26;
-    if (code != NO_SHIFT) {
+    if (!SKIP || code != NO_SHIFT) {
         const float4 sh = s_hi[code], sl = s_lo[code];
         ax = __fsub_rn(ax, sh.x);
         ay = __fsub_rn(ay, sh.y);
@@ -97,16 +98,21 @@ __device__ __forceinline__ float plain_reduce(float v) {
     return v;
 }
 
-// Entries a lane holds in registers ahead of the one it evaluates: eight, so
-// that five blocks of the density pass fit a SM and the force pass spills
-// nothing (sixteen where the knots are staged).  Both passes are bound by the
-// L1's data path, 32 bytes a neighbour beside its knots, and by issue.
-// Density and force, us: 256,000 atoms 68.4 and 77.1, 1,048,576 247 and 295;
-// with sixteen ahead, four blocks and every entry's image shift loaded 73.2 and
-// 86.0, 267 and 331; four ahead 72.6 and 81.4; six blocks of the density pass
-// 83.3, five of the force pass 89.0 (256,000 atoms).
-constexpr int eam_ahead(int lanes, bool staged) { return lanes >= 8 ? 64 / lanes : (staged ? 16 : 8); }
-constexpr int DENSITY_CTAS = 5, FORCE_CTAS = 4;
+// Entries a lane holds in registers ahead of the one it evaluates (sixteen where
+// the knots are staged).  Both passes are bound by the L1's data path, 32 bytes a
+// neighbour beside its knots, and by issue: with eight ahead the force pass
+// spills nothing, and in a large box (LARGE) five blocks of the density pass are
+// worth the registers, and the image shifts that are not loaded the branch.  A
+// smaller box waits for one lane's chain instead, and takes neither.
+// Density and force, us: 256,000 atoms 68.8 and 77.3, 1,048,576 243 and 295; with
+// sixteen ahead, four blocks and every shift loaded 73.2 and 86.0, 267 and 331;
+// four ahead 72.6 and 81.4, six blocks of the density pass 83.3, five of the
+// force pass 89.0 (256,000 atoms).  The density pass, LARGE and not: 13,500 atoms
+// 14.3 and 13.0, 23,328 14.8 and 14.8, 55,296 24.8 and 24.4, 87,808 29.6 and 32.1.
+constexpr int eam_ahead(int lanes, bool staged, int gather) { return lanes >= 8 ? 64 / lanes : (staged ? 16 : gather); }
+constexpr int DENSITY_AHEAD = 14, FORCE_AHEAD = 8;
+constexpr int DENSITY_CTAS = 4, DENSITY_CTAS_LARGE = 5, FORCE_CTAS = 4;
+constexpr int DENSITY_LARGE_PER_SM = 400;
 
 // Staged variants hold the knot window in shared memory (up to ~110 KB) and
 // run two 512-thread CTAs per SM, so 32 warps hide the gathers' latency.
@@ -124,12 +130,12 @@ __device__ __forceinline__ int knot_of(const EAMFast& p, float r, float offdr, f
 
 // One lane's share of rho_i over the gathered row of atom ii (entries lane,
 // lane + LANES, ...).
-template <int LANES, bool STAGED>
+template <int LANES, bool STAGED, bool LARGE>
 __device__ __forceinline__ void gather_density_sum(const EAMFast& p, const PosPack* pack,
                                                    const unsigned* __restrict__ nbr, int ii, int m, int lane,
                                                    const float4* s_hi, const float4* s_lo, const float4* s_rho,
                                                    Kahan& acc, unsigned* status) {
-    constexpr int PF = eam_ahead(LANES, STAGED);
+    constexpr int PF = eam_ahead(LANES, STAGED, DENSITY_AHEAD);
     const int step = LANES << p.hshift;
     const float rc2 = p.rc_rho * p.rc_rho * 1.0001f;
     const float offdr = p.off * p.inv_dr;
@@ -147,7 +153,7 @@ __device__ __forceinline__ void gather_density_sum(const EAMFast& p, const PosPa
             if (s0 + k * LANES >= m) break;
             float4 hn, ln;
             if (k + 1 < PF && s0 + (k + 1) * LANES < m) ld256(pack + (ent[k + 1] & (unsigned)INDEX_MASK), hn, ln);
-            const float3 d = delta_tab(hi, lo, hj, lj, ent[k], s_hi, s_lo);
+            const float3 d = delta_tab<LARGE>(hi, lo, hj, lj, ent[k], s_hi, s_lo);
             hj = hn;
             lj = ln;
             const float r2 = fmaf(d.z, d.z, fmaf(d.y, d.y, d.x * d.x));
@@ -200,8 +206,8 @@ __device__ __forceinline__ void density_finish(const EAMFast& p, int i, float rh
     pack[i].lo.w = dF;
 }
 
-template <int LANES, bool STAGED>
-__global__ void EAMF_BOUNDS(STAGED, DENSITY_CTAS) k_eamf_density(EAMFast p, PosPack* pack, const unsigned* __restrict__ nbr,
+template <int LANES, bool STAGED, bool LARGE>
+__global__ void EAMF_BOUNDS(STAGED, LARGE ? DENSITY_CTAS_LARGE : DENSITY_CTAS) k_eamf_density(EAMFast p, PosPack* pack, const unsigned* __restrict__ nbr,
                                                    const int* __restrict__ nnb, float* __restrict__ fp,
                                                    float* __restrict__ femb, unsigned* status) {
     __shared__ float4 s_hi[64], s_lo[64];
@@ -218,7 +224,7 @@ __global__ void EAMF_BOUNDS(STAGED, DENSITY_CTAS) k_eamf_density(EAMFast p, PosP
         const int ii = valid ? i : p.n - 1;
         const int m = valid ? nnb[ii] : 0;
         Kahan acc;
-        gather_density_sum<LANES, STAGED>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_rho, acc, status);
+        gather_density_sum<LANES, STAGED, LARGE>(p, pack, nbr, ii, m, lane, s_hi, s_lo, s_rho, acc, status);
         float sum = acc.s, comp = acc.c;
         twosum_reduce<LANES>(sum, comp);
         if (lane == 0 && valid) density_finish(p, i, __fsub_rn(sum, comp), pack, fp, femb, status);
@@ -254,7 +260,7 @@ __device__ __forceinline__ void gather_force_sum(const EAMFast& p, const PosPack
                                                  const float4* s_hi, const float4* s_lo, const float4* s_tab,
                                                  Kahan& ax, Kahan& ay, Kahan& az, float& ae, float& av,
                                                  unsigned* status) {
-    constexpr int PF = eam_ahead(LANES, STAGED);
+    constexpr int PF = eam_ahead(LANES, STAGED, FORCE_AHEAD);
     const int step = LANES << p.hshift;
     const float offdr = p.off * p.inv_dr;
     const float4 hi = pack[ii].hi, lo = pack[ii].lo;
@@ -272,7 +278,7 @@ __device__ __forceinline__ void gather_force_sum(const EAMFast& p, const PosPack
             if (s0 + k * LANES >= m) break;
             float4 hn, ln;
             if (k + 1 < PF && s0 + (k + 1) * LANES < m) ldg256(pack + (ent[k + 1] & (unsigned)INDEX_MASK), hn, ln);
-            const float3 d = delta_tab(hi, lo, hj, lj, ent[k], s_hi, s_lo);
+            const float3 d = delta_tab<true>(hi, lo, hj, lj, ent[k], s_hi, s_lo);
             const float fpj = lj.w;  // F'(rho_j) from the density pass
             hj = hn;
             lj = ln;
@@ -605,7 +611,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) k_eamt_density(EAMFast p, EAM
                 }
             }
         } else {
-            gather_density_sum<LANES, false>(p, pack, nbr, i, m, lane, s_shi, s_slo, nullptr, acc, status);
+            gather_density_sum<LANES, false, true>(p, pack, nbr, i, m, lane, s_shi, s_slo, nullptr, acc, status);
         }
         float sum = acc.s, comp = acc.c;
         twosum_reduce<LANES>(sum, comp);
@@ -721,7 +727,8 @@ static void launch_fast(Context* c, const EAMFast& p, int grid, int block, size_
                         const KickArgs* ka) {
     static bool attr = false;
     if (!attr) {
-        cudaFuncSetAttribute(k_eamf_density<LANES, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(k_eamf_density<LANES, STAGED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             200 * 1024);
         cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              200 * 1024);
         cudaFuncSetAttribute(k_eamf_force<LANES, STAGED, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -729,7 +736,9 @@ static void launch_fast(Context* c, const EAMFast& p, int grid, int block, size_
         attr = true;
     }
     prof_begin(c, "eam_density");
-    k_eamf_density<LANES, STAGED><<<grid, block, smem1, c->stream>>>(
+    const bool large = !STAGED && c->n >= DENSITY_LARGE_PER_SM * c->num_sms;
+    auto density = large ? k_eamf_density<LANES, STAGED, !STAGED> : k_eamf_density<LANES, STAGED, false>;
+    density<<<grid, block, smem1, c->stream>>>(
         p, c->pack, reinterpret_cast<const unsigned*>(c->nbr), c->nnb, c->fp, c->femb, c->d_status);
     prof_end(c);
     const unsigned* aflag = c->flags_used ? c->aflag : nullptr;
