@@ -333,16 +333,17 @@ def timed_steps(ctx, n, steps, stream, flush_l2, torch):
     return total_ms, kernels, st1["rebuilds"] - st0["rebuilds"], st1["launches"] - st0["launches"]
 
 
-# the solve's algorithmic bytes: T, con, cap, S, E (8 B each), map 4, mask 1 read; A 8 written (the kernel
-# reads each cell's three face conductances instead of con: 69 B)
-FDTD_CELL_BYTES = 53
+# the solve's bytes a cell: T 8, its three face conductances 24, capacity and its reciprocal 16, S and E 8
+# each, map 4, mask 1 read; A 8 written
+FDTD_CELL_BYTES = 77
 
 
 def fdtd_report(device, torch, n=256, steps=100):
     """The finite-difference heat solver (omdg_fdtd) on an n^3 periodic grid
     with a hot block: cells/s over `steps` host-driven steps (wall clock,
-    synchronised), and the stencil's HBM roof (53 algorithmic bytes per
-    cell; the grid, 1.3 GB of arrays at n = 256, is ten times the L2)."""
+    synchronised), and the stencil's HBM roof (FDTD_CELL_BYTES per cell; the
+    grid, 1.3 GB of arrays at n = 256, is ten times the L2).  The FP64 pipe
+    binds it (79 % busy in ncu)."""
     from objectmd_gb300 import omdg
 
     dim = n ** 3
