@@ -2,9 +2,9 @@
 // EDENS tables on the same knot grid, no OutOfRange values (a read outside
 // the table is an error, as in the reference).  Same arithmetic as eam.cu
 // (team.cpp:81-92, :116-145, :224-237), arranged for the GB300 memory system:
-//   - each lane loads all of its neighbour-list entries up front (one DRAM
-//     round trip per atom instead of one per neighbour) and gathers the next
-//     neighbour's pack while it evaluates the current one,
+//   - each lane loads its neighbour-list entries in batches up front (one or
+//     two DRAM round trips per atom instead of one per neighbour) and gathers the
+//     next neighbour's pack while it evaluates the current one,
 //   - a neighbour's position pack (with F'(rho) in its spare word) and an
 //     interleaved (phi, rho) knot are one 256-bit load each,
 //   - the periodic image comes from a 64-entry shared table of split shift

@@ -575,7 +575,7 @@ __device__ __noinline__ bool exact_within(double Lx, double Ly, double Lz, doubl
 
 // The list build.  The candidates of the 27 cells are 9 runs of back-to-back
 // atoms (axis_run); a candidate costs one 16-byte load of its FP32 position,
-// four of them in flight, and the squared length of the difference.  Every
+// six of them in flight, and the squared length of the difference.  Every
 // FP32 step errs by at most an ulp of the box's extent, so pairs within a band of
 // Rv (a few 1e-4 A for boxes of a few hundred A: one atom in thirty has such
 // a pair), and pairs close enough to be an overlap, take the reference's FP64
@@ -667,7 +667,7 @@ __device__ __forceinline__ void build_centre(
     extern __shared__ unsigned s_row[];
     const RepGeom* g = REP ? rg + rep_of[i] : nullptr;
     const float4 ui = loc[i];
-    if (ui.x == 3.0e38f) {  // inactive centre (k_pack): an empty row
+    if (ui.x == 3.0e38f) {  // inactive centre (pack_atom): an empty row
         if (lane == 0) {
             nnb[i] = 0;
             nbmask[i] = 0u;
@@ -1638,7 +1638,7 @@ int nlist_build(Context* c, bool on_request) {
 
     BuildParams bp;
     bp.to = TileOut{};
-    // tile slots: prepared per tile after the scan, written by the cell-local build
+    // tile slots: prepared per tile after the scan, written by the list build
     const bool tiles = c->tile_want && !reps && c->tslot && c->tile_stride >= c->maxnb;
     if (tiles) {
         TilePrep tp;

@@ -220,7 +220,7 @@ __global__ void k_nn_normalize(NNDescParams p, long n, const float* __restrict__
 // sums its terms in the order of the feature index, in FP32.  Bound by the
 // shared loads' latency and wavefronts at two blocks a SM (LSU 50 %).  For a
 // batch of 16 x 512 atoms a step's kernels take 17 (forward), 7 (forces), 6
-// (dL/du), 25 (gradient) and 12 us (sums and Adam) under ncu, a step 82 us in
+// (dL/du), 25 (gradient) and 12 us (sums and Adam) under ncu (warm caches), a step 82 us in
 // the loop; one thread per atom, as it was, ran 64 blocks of 128 threads with
 // 64-wide vectors in local memory and took 348 us a step.
 constexpr int NT_THREADS = 256;
