@@ -3,7 +3,7 @@
  *
  * TEST INFRASTRUCTURE ONLY.  Only tests/, __graft_entry__.smoke() and the
  * cpu_baseline / reference legs of bench.py may load this library, and only
- * as the checker.  The product (libomdg) never links or calls it.
+ * as the oracle.  The product (libomdg) never links or calls it.
  *
  * Each function names the reference lines it restates.  Its agreement with
  * the reference itself is pinned by tests/golden/ fixtures produced by the

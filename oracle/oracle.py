@@ -2,7 +2,7 @@
 
 Only ``tests/``, ``__graft_entry__.smoke()`` and the ``cpu_baseline`` /
 ``--impl reference`` legs of ``bench.py`` may import this module, and only as
-the checker.  The product library never loads it.
+the oracle.  The product library never loads it.
 
 This wraps ``liboracle.so`` (``oracle/omd_oracle.c``, a restatement of the
 reference's hot path in C) and runs ``oracle/_ref/ref_driver`` (the reference's
